@@ -1,0 +1,46 @@
+"""Kernels at the sizes where their decompositions change: edges of tiles, remainders, odd strides, the smallest and largest of a
+range, each against an fp32 / fp64 PyTorch statement of the same operation.
+
+Tolerances: a bf16 result is half a unit in the last place (2^-9 relative) off its exact value by rounding alone; 2^-8 of the value
+leaves room for the fp32 accumulation in front of it, plus an absolute term of a few fp32 roundings of the largest term."""
+import math
+
+import pytest
+import torch
+
+from tensor_parallel_b200.ops import functional as OF
+
+pytestmark = pytest.mark.gpu
+
+
+def _native():
+    from tensor_parallel_b200.ops import native
+
+    return native
+
+
+def _close(got, want, terms=1.0):
+    err = (got.double() - want).abs()
+    bound = want.abs() * 2.0 ** -8 + terms * 2.0 ** -18
+    assert bool((err <= bound).all()), f"largest excess {(err - bound).max().item():.3g} at value {want.flatten()[(err - bound).argmax()].item():.3g}"
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (8, 0), (4099, 0), (4096, 1)])
+@pytest.mark.parametrize("dtype,gdtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_adamw_remainders_and_alignment(n, offset, dtype, gdtype):
+    nat = _native()
+    torch.manual_seed(n)
+
+    def make(dt, scale=1.0):
+        return (torch.rand(n + offset, device="cuda") * scale).to(dt)[offset:]
+
+    p, g, m, v = make(dtype), make(gdtype, 0.1), make(torch.float32, 0.1), make(torch.float32, 0.01)
+    master = p.float().clone() if dtype == torch.bfloat16 else None
+    p0, m0, v0 = p.double(), m.double(), v.double()
+    nat.adamw_step(p, g, m, v, 3, 1e-2, 0.9, 0.99, 1e-8, 0.1, master=master)
+    m1, v1 = 0.9 * m0 + 0.1 * g.double(), 0.99 * v0 + 0.01 * g.double() ** 2
+    want = p0 * (1 - 1e-3) - 1e-2 * (m1 / (1 - 0.9 ** 3)) / ((v1 / (1 - 0.99 ** 3)).sqrt() + 1e-8)
+    for got, ref in ((m, m1), (v, v1), (p if master is None else master, want)):
+        assert (got.double() - ref).abs().max().item() <= 2e-6  # a few fp32 roundings of values below 1 (1 - 0.99f is 1e-6 off)
+    if master is not None:
+        assert torch.equal(p, master.to(torch.bfloat16))
