@@ -25,6 +25,19 @@ def _close(got, want, terms=1.0):
     assert bool((err <= bound).all()), f"largest excess {(err - bound).max().item():.3g} at value {want.flatten()[(err - bound).argmax()].item():.3g}"
 
 
+@pytest.mark.parametrize("heads,tokens", [(1, 3), (3, 700), (12, 65), (33, 2100)])
+@pytest.mark.parametrize("interleaved,rotary", [(False, 128), (False, 64), (True, 32)])
+def test_rope_head_groups(heads, tokens, interleaved, rotary):
+    torch.manual_seed(heads)
+    x = torch.randn(1, tokens, heads, 128, device="cuda", dtype=torch.bfloat16)
+    pos = torch.randint(0, 4000, (1, tokens), device="cuda")
+    got = OF.apply_rope(x, pos, 10000.0, rotary, interleaved)
+    want = OF.apply_rope_ref(x.float(), pos, 10000.0, rotary, interleaved)
+    # fp32 angles up to 4000 rad are 2.4e-4 rad off between two fp32 evaluations of the frequency
+    assert (got.float() - want).abs().max().item() <= 2.0 ** -8 * want.abs().max().item() + 5e-3
+    assert torch.equal(got[..., rotary:], x[..., rotary:])
+
+
 @pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (8, 0), (4099, 0), (4096, 1)])
 @pytest.mark.parametrize("dtype,gdtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
 def test_adamw_remainders_and_alignment(n, offset, dtype, gdtype):
