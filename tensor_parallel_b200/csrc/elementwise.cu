@@ -145,44 +145,91 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T
   }
 }
 
-// Backward: dx per row; dweight / dbias accumulated with fp32 atomics into zero-initialised buffers.
-// Each CTA handles ROWS_PER_CTA consecutive rows and keeps its column partial sums in registers.
+// Backward: dx per row; the column sums for dweight / dbias go through one fp32 partial row per CTA, which
+// norm_bwd_reduce_kernel adds up in a fixed order (deterministic, no atomics).  Memory-bound: x and dy are read and dx is
+// written once.  A CTA walks rows blockIdx.x, + gridDim.x, ... and holds its column sums in registers; the raw 16-byte vectors
+// of the next row are fetched before the block-wide sums of the current one (PREFETCH), which is what keeps enough bytes in
+// flight with two CTAs per SM.  V = vectors of 8 elements per thread.
 constexpr int NORM_BWD_MAXV = 4;  // cols <= 8192 in the backward kernel (register limit)
+constexpr int NORM_BWD_CTAS = 148 * 2;
 
-template <typename T, int MODE>
-__global__ void __launch_bounds__(NORM_THREADS)
+template <typename T> struct Raw8 { uint4 u[sizeof(T) / 2]; };  // 8 elements as they lie in memory
+template <typename T> __device__ __forceinline__ Raw8<T> load_raw(const T* p) {
+  Raw8<T> r;
+#pragma unroll
+  for (int i = 0; i < int(sizeof(T) / 2); ++i) r.u[i] = reinterpret_cast<const uint4*>(p)[i];
+  return r;
+}
+__device__ __forceinline__ void unpack(const Raw8<bf16>& r, float (&v)[8]) {
+  const uint32_t w[4] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+__device__ __forceinline__ void unpack(const Raw8<float>& r, float (&v)[8]) {
+  const uint32_t w[8] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w, r.u[1].x, r.u[1].y, r.u[1].z, r.u[1].w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
+}
+
+template <typename T, int MODE, int V>
+__global__ void __launch_bounds__(NORM_THREADS, (sizeof(T) == 4 && MODE == 1 && V == 4) ? 1 : 2)  // (that one would spill)
 norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ weight,
                 const float* __restrict__ rstd_in, const float* __restrict__ mean_in, T* __restrict__ dx,
-                float* __restrict__ dweight, float* __restrict__ dbias, int rows, int cols, int rows_per_cta) {
+                float* __restrict__ part_w, float* __restrict__ part_b, int rows, int cols) {
+  constexpr bool PREFETCH = sizeof(T) == 2 ? V <= 2 : V == 1;  // (wider rows keep enough bytes in flight by themselves)
   const int nvec = cols >> 3;
-  float dw_acc[NORM_BWD_MAXV][8], db_acc[NORM_BWD_MAXV][8];
+  float dw_acc[V][8], db_acc[V][8];
 #pragma unroll
-  for (int i = 0; i < NORM_BWD_MAXV; ++i)
+  for (int i = 0; i < V; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) { dw_acc[i][j] = 0.f; db_acc[i][j] = 0.f; }
-  const int row0 = blockIdx.x * rows_per_cta;
-  const int row1 = min(rows, row0 + rows_per_cta);
-  for (int row = row0; row < row1; ++row) {
-    const float rstd = rstd_in[row];
-    const float mean = MODE == 1 ? mean_in[row] : 0.f;
-    float xh[NORM_BWD_MAXV][8], g[NORM_BWD_MAXV][8];
+  Raw8<T> xr[V], dr[V];
+  auto fetch = [&](int row, Raw8<T> (&xo)[V], Raw8<T> (&dd)[V]) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int vi = threadIdx.x + i * NORM_THREADS;
+      if (vi < nvec) {
+        dd[i] = load_raw(dy + size_t(row) * cols + vi * 8);
+        xo[i] = load_raw(x + size_t(row) * cols + vi * 8);
+      }
+    }
+  };
+  int row = blockIdx.x;
+  float rstd = 0.f, mean = 0.f;
+  if (row < rows) {
+    fetch(row, xr, dr);
+    rstd = rstd_in[row];
+    if (MODE == 1) mean = mean_in[row];
+  }
+  while (row < rows) {
+    const int next = row + gridDim.x;
+    Raw8<T> xn[V], dn[V];
+    float rstd_n = 0.f, mean_n = 0.f;
+    if (next < rows) {
+      if (PREFETCH) fetch(next, xn, dn);
+      rstd_n = rstd_in[next];
+      if (MODE == 1) mean_n = mean_in[next];
+    }
     float s1 = 0.f, s2 = 0.f;  // sum(g), sum(g * xhat)
 #pragma unroll
-    for (int i = 0; i < NORM_BWD_MAXV; ++i) {
+    for (int i = 0; i < V; ++i) {
       const int vi = threadIdx.x + i * NORM_THREADS;
       if (vi < nvec) {
         float d[8], xv[8], w[8];
-        Vec8<T>::load(dy + size_t(row) * cols + vi * 8, d);
-        Vec8<T>::load(x + size_t(row) * cols + vi * 8, xv);
+        unpack(dr[i], d);
+        unpack(xr[i], xv);
         if (weight) Vec8<T>::load(weight + vi * 8, w);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] = (xv[j] - mean) * rstd;
-          dw_acc[i][j] += d[j] * xh[i][j];
+          const float xh = (xv[j] - mean) * rstd;
+          dw_acc[i][j] += d[j] * xh;
           db_acc[i][j] += d[j];
-          g[i][j] = weight ? d[j] * w[j] : d[j];
-          s1 += g[i][j];
-          s2 += g[i][j] * xh[i][j];
+          const float g = weight ? d[j] * w[j] : d[j];
+          s1 += g;
+          s2 += g * xh;
         }
       }
     }
@@ -191,27 +238,64 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
     const float c1 = MODE == 1 ? s1 * inv_n : 0.f;
     const float c2 = s2 * inv_n;
 #pragma unroll
-    for (int i = 0; i < NORM_BWD_MAXV; ++i) {
+    for (int i = 0; i < V; ++i) {
       const int vi = threadIdx.x + i * NORM_THREADS;
       if (vi < nvec) {
-        float o[8];
+        float d[8], xv[8], w[8], o[8];
+        unpack(dr[i], d);
+        unpack(xr[i], xv);
+        if (weight) Vec8<T>::load(weight + vi * 8, w);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = (g[i][j] - c1 - xh[i][j] * c2) * rstd;
+        for (int j = 0; j < 8; ++j) {
+          const float xh = (xv[j] - mean) * rstd;
+          const float g = weight ? d[j] * w[j] : d[j];
+          o[j] = (g - c1 - xh * c2) * rstd;
+        }
         Vec8<T>::store(dx + size_t(row) * cols + vi * 8, o);
       }
     }
+    if (PREFETCH) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) { xr[i] = xn[i]; dr[i] = dn[i]; }
+    } else if (next < rows) {
+      fetch(next, xr, dr);
+    }
+    rstd = rstd_n;
+    mean = mean_n;
+    row = next;
   }
 #pragma unroll
-  for (int i = 0; i < NORM_BWD_MAXV; ++i) {
+  for (int i = 0; i < V; ++i) {
     const int vi = threadIdx.x + i * NORM_THREADS;
     if (vi < nvec) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (dweight) atomicAdd(dweight + vi * 8 + j, dw_acc[i][j]);
-        if (MODE == 1 && dbias) atomicAdd(dbias + vi * 8 + j, db_acc[i][j]);
-      }
+      if (part_w) Vec8<float>::store(part_w + size_t(blockIdx.x) * cols + vi * 8, dw_acc[i]);
+      if (MODE == 1 && part_b) Vec8<float>::store(part_b + size_t(blockIdx.x) * cols + vi * 8, db_acc[i]);
     }
   }
+}
+
+// out[c] = sum over parts of part[p][c] (blockIdx.y: 0 = weight, 1 = bias).  32 columns x 32 rows of partials per step, so that
+// every partial row's loads are independent; the summation order depends on the number of partials only.
+template <typename O>
+__global__ void __launch_bounds__(1024)
+norm_bwd_reduce_kernel(const float* __restrict__ part_w, const float* __restrict__ part_b, O* __restrict__ dweight, O* __restrict__ dbias,
+                       int parts, int cols) {
+  __shared__ float tile[32][33];
+  const float* part = blockIdx.y ? part_b : part_w;
+  O* out = blockIdx.y ? dbias : dweight;
+  if (!out) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + tx;
+  float s = 0.f;
+  if (c < cols) {
+#pragma unroll 4
+    for (int r = ty; r < parts; r += 32) s += part[size_t(r) * cols + c];
+  }
+  tile[ty][tx] = s;
+  __syncthreads();
+  const float t = warp_sum(tile[tx][ty]);  // warp ty sums column ty of the tile
+  const int co = blockIdx.x * 32 + ty;
+  if (tx == 0 && co < cols) out[co] = from_f<O>(t);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -427,7 +511,8 @@ __device__ __forceinline__ void adamw_update(float g, float& p, float& m, float&
 }
 
 // VEC: 8 elements per thread and step with 16-byte accesses (all pointers 16-byte aligned; the last n % 8 elements are done one
-// by one): up to ten independent 16-byte loads per thread are in flight, where the element-wise form has five of 2 to 4 bytes.
+// by one): up to ten independent 16-byte loads per thread are in flight, where the element-wise form has five of 2 to 4 bytes
+// (202 M parameters with master weights: 1260 us element-wise, 944 us = 6.4 TB/s in vectors).
 template <typename P, typename G, bool VEC>
 __global__ void __launch_bounds__(256)
 adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, float* __restrict__ m, float* __restrict__ v, float* __restrict__ master,
@@ -501,21 +586,39 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   TPB_CHECK_LAUNCH();
 }
 
+// Rows of fp32 partials that tpb_norm_bwd needs for this row count: part_w / part_b hold that many rows of `cols` floats.
+extern "C" int tpb_norm_bwd_parts(int rows) { return rows < NORM_BWD_CTAS ? rows : NORM_BWD_CTAS; }
+
+// dweight / dbias (either may be null, with its partials) are written, not accumulated; grad_dtype: 0 = bf16, 1 = fp32.
 extern "C" int tpb_norm_bwd(const void* dy, const void* x, const void* weight, const float* rstd, const float* mean,
-                            void* dx, float* dweight, float* dbias, int rows, int cols, int mode, int dtype,
-                            void* stream_) {
-  if (!dy || !x || !dx || !rstd || rows <= 0) return TPB_ERR_ARG;
+                            void* dx, float* part_w, float* part_b, void* dweight, void* dbias, int rows, int cols, int mode, int dtype,
+                            int grad_dtype, void* stream_) {
+  if (!dy || !x || !dx || !rstd || rows <= 0 || cols <= 0 || (mode && !mean) || (dweight && !part_w) || (dbias && (!part_b || !mode))) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_BWD_MAXV) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  int rows_per_cta = (rows + 148 * 4 - 1) / (148 * 4);
-  if (rows_per_cta < 1) rows_per_cta = 1;
-  const int grid = (rows + rows_per_cta - 1) / rows_per_cta;
-#define LAUNCH(T, M)                                                                                                  \
-  norm_bwd_kernel<T, M><<<grid, NORM_THREADS, 0, s>>>((const T*)dy, (const T*)x, (const T*)weight, rstd, mean, (T*)dx, \
-                                                      dweight, dbias, rows, cols, rows_per_cta)
+  const int grid = tpb_norm_bwd_parts(rows);
+  if (!dweight) part_w = nullptr;
+  if (!dbias) part_b = nullptr;
+#define LAUNCH3(T, M, V)                                                                                              \
+  norm_bwd_kernel<T, M, V><<<grid, NORM_THREADS, 0, s>>>((const T*)dy, (const T*)x, (const T*)weight, rstd, mean, (T*)dx, part_w, part_b, rows, cols)
+#define LAUNCH(T, M)                                                                     \
+  do {                                                                                   \
+    if (cols <= NORM_THREADS * 8) LAUNCH3(T, M, 1);                                      \
+    else if (cols <= NORM_THREADS * 16) LAUNCH3(T, M, 2);                                \
+    else if (cols <= NORM_THREADS * 24) LAUNCH3(T, M, 3);                                \
+    else LAUNCH3(T, M, 4);                                                               \
+  } while (0)
   if (dtype == 0) { if (mode) LAUNCH(bf16, 1); else LAUNCH(bf16, 0); }
   else            { if (mode) LAUNCH(float, 1); else LAUNCH(float, 0); }
 #undef LAUNCH
+#undef LAUNCH3
+  if (dweight || dbias) {
+    const dim3 rgrid((cols + 31) / 32, dbias ? 2 : 1);
+    if (grad_dtype == 0)
+      norm_bwd_reduce_kernel<bf16><<<rgrid, 1024, 0, s>>>(part_w, part_b, (bf16*)dweight, (bf16*)dbias, grid, cols);
+    else
+      norm_bwd_reduce_kernel<float><<<rgrid, 1024, 0, s>>>(part_w, part_b, (float*)dweight, (float*)dbias, grid, cols);
+  }
   TPB_CHECK_LAUNCH();
 }
 
@@ -538,9 +641,11 @@ extern "C" int tpb_rope(const void* x, void* out, const int64_t* positions, cons
   const bool vec_ok = dtype == 0 && head_dim % 8 == 0 && (interleaved ? rotary_dim % 8 == 0 : half_ % 8 == 0) && rotary_dim > 0 &&
                       !(x_stride_tok & 7) && !(out_stride_tok & 7) && !((uintptr_t)x & 15) && !((uintptr_t)out & 15);
   if (vec_ok) {
-    const long long vwork = (long long)tokens * heads * (interleaved ? rotary_dim / 8 : half_ / 8);
-    rope_vec_kernel<<<grid_for(vwork, 256), 256, 0, s>>>((const bf16*)x, (bf16*)out, positions, base_pos, seq, tokens, heads, head_dim,
-                                                         rotary_dim, l2t, interleaved, inverse, x_stride_tok, out_stride_tok);
+    const int chunks = interleaved ? rotary_dim / 8 : half_ / 8;
+    const int groups = tpb_rope_head_groups((long long)tokens * chunks, heads);
+    rope_vec_kernel<<<grid_for((long long)tokens * chunks * groups, 256), 256, 0, s>>>((const bf16*)x, (bf16*)out, positions, base_pos, seq, tokens,
+                                                                                       heads, groups, head_dim, rotary_dim, l2t, interleaved,
+                                                                                       inverse, x_stride_tok, out_stride_tok);
   } else if (dtype == 0)
     rope_kernel<bf16><<<grid_for(work, 256), 256, 0, s>>>((const bf16*)x, (bf16*)out, positions, base_pos, seq, tokens, heads,
                                                           head_dim, rotary_dim, l2t, interleaved, inverse, x_stride_tok, out_stride_tok);
@@ -612,14 +717,6 @@ extern "C" int tpb_adamw(void* param, const void* grad, float* m, float* v, floa
   if (param_dtype == 0) { if (grad_is_fp32) LAUNCH(bf16, float); else LAUNCH(bf16, bf16); }
   else                  { if (grad_is_fp32) LAUNCH(float, float); else LAUNCH(float, bf16); }
 #undef LAUNCH
-#undef LAUNCH3
-  if (dweight || dbias) {
-    const dim3 rgrid((cols + 31) / 32, dbias ? 2 : 1);
-    if (grad_dtype == 0)
-      norm_bwd_reduce_kernel<bf16><<<rgrid, 1024, 0, s>>>(part_w, part_b, (bf16*)dweight, (bf16*)dbias, grid, cols);
-    else
-      norm_bwd_reduce_kernel<float><<<rgrid, 1024, 0, s>>>(part_w, part_b, (float*)dweight, (float*)dbias, grid, cols);
-  }
   TPB_CHECK_LAUNCH();
 }
 

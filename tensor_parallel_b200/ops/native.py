@@ -333,7 +333,7 @@ def linear(x, weight, bias=None):
 # ------------------------------------------------------------------------------------------------
 
 LIB.tpb_norm_fwd.argtypes = [c_void_p] * 8 + [c_int, c_int, c_float, c_int, c_int, c_void_p]
-LIB.tpb_norm_bwd.argtypes = [c_void_p] * 8 + [c_int, c_int, c_int, c_int, c_void_p]
+LIB.tpb_norm_bwd.argtypes = [c_void_p] * 10 + [c_int] * 5 + [c_void_p]
 
 
 def norm_supported(x: torch.Tensor) -> bool:
@@ -372,11 +372,17 @@ class _NormFn(torch.autograd.Function):
         g2d = grad.reshape(x2d.shape).to(x2d.dtype).contiguous()
         rows, cols = x2d.shape
         dx = torch.empty_like(x2d)
-        dw = torch.zeros(cols, dtype=torch.float32, device=x2d.device) if w is not None else None
-        db = torch.zeros(cols, dtype=torch.float32, device=x2d.device) if ctx.bdtype is not None else None
-        check(LIB.tpb_norm_bwd(_ptr(g2d), _ptr(x2d), _ptr(w), _ptr(rstd), _ptr(mean), _ptr(dx), _ptr(dw), _ptr(db), rows, cols,
-                               ctx.mode, _dtype_code(x2d), _stream()), "tpb_norm_bwd")
-        launch_count += 1
+        # column sums: one fp32 partial row per CTA, added up by a second kernel that writes the gradients in their own dtype
+        has_w, has_b = w is not None, ctx.bdtype is not None
+        gdtype = ctx.wdtype if has_w and (not has_b or ctx.bdtype == ctx.wdtype) and ctx.wdtype == torch.bfloat16 else torch.float32
+        parts = LIB.tpb_norm_bwd_parts(rows)
+        part_w = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_w else None
+        part_b = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_b else None
+        dw = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_w else None
+        db = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_b else None
+        check(LIB.tpb_norm_bwd(_ptr(g2d), _ptr(x2d), _ptr(w), _ptr(rstd), _ptr(mean), _ptr(dx), _ptr(part_w), _ptr(part_b), _ptr(dw), _ptr(db),
+                               rows, cols, ctx.mode, _dtype_code(x2d), int(gdtype == torch.float32), _stream()), "tpb_norm_bwd")
+        launch_count += 2 if has_w or has_b else 1
         return (dx.view(ctx.shape), None if dw is None else dw.to(ctx.wdtype), None if db is None else db.to(ctx.bdtype), None, None)
 
 

@@ -25,6 +25,29 @@ def _close(got, want, terms=1.0):
     assert bool((err <= bound).all()), f"largest excess {(err - bound).max().item():.3g} at value {want.flatten()[(err - bound).argmax()].item():.3g}"
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (2, 2048), (295, 2056), (297, 4096), (700, 5120), (61, 8192)])
+@pytest.mark.parametrize("mode", ["rms", "layer"])
+def test_norm_backward_row_and_column_edges(dtype, rows, cols, mode):
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, cols, device="cuda") * 2 + 0.1).to(dtype).requires_grad_()
+    w = (1 + 0.1 * torch.randn(cols, device="cuda")).to(dtype).requires_grad_()
+    b = torch.randn(cols, device="cuda").to(dtype).requires_grad_()
+    g = torch.randn(rows, cols, device="cuda").to(dtype)
+    xr, wr, br = (t.detach().double().requires_grad_() for t in (x, w, b))
+    if mode == "rms":
+        OF.rms_norm(x, w, 1e-6).backward(g)
+        (xr * (xr.square().mean(-1, keepdim=True) + 1e-6).rsqrt() * wr).backward(g.double())
+    else:
+        OF.layer_norm(x, w, b, 1e-5).backward(g)
+        torch.nn.functional.layer_norm(xr, (cols,), wr, br, 1e-5).backward(g.double())
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -17  # rounding of the result / of fp32 sums over up to 8192 terms
+    for got, want in ((x.grad, xr.grad), (w.grad, wr.grad)) + (((b.grad, br.grad),) if mode == "layer" else ()):
+        scale = want.square().mean().sqrt().item()
+        err = (got.double() - want).abs()
+        assert bool((err <= rel * (want.abs() + 2 * scale) + 1e-6).all()), (err.max().item(), scale)
+
+
 @pytest.mark.parametrize("heads,tokens", [(1, 3), (3, 700), (12, 65), (33, 2100)])
 @pytest.mark.parametrize("interleaved,rotary", [(False, 128), (False, 64), (True, 32)])
 def test_rope_head_groups(heads, tokens, interleaved, rotary):
