@@ -26,38 +26,86 @@ __device__ __forceinline__ float ce_warp_sum(float v) {
   return v;
 }
 
+// Both kernels are memory-bound: one CTA per row, 16-byte accesses.  A row starts at any element when the pitch is odd (a
+// vocabulary that is no multiple of 8): [0, head) and [tail, cols) are handled one by one, [head, tail) is 16-byte aligned.
+struct CeSpan { int head, tail; };
+__device__ __forceinline__ CeSpan ce_span(const bf16* x, int cols) {
+  const int head = min(cols, int((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / 2);
+  return {head, head + (cols - head) / 8 * 8};
+}
+__device__ __forceinline__ void ce_unpack(const uint4& u, float (&v)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+
+// One pass over the row: every thread keeps a running maximum and the sum of exp(x - maximum), rescaled when the maximum of a
+// group of loaded values exceeds it; the threads' pairs are merged at the end.
 __global__ void __launch_bounds__(CE_THREADS)
 ce_stats_kernel(const bf16* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ stats, int cols,
                 long long ld, int vocab_start, int ignore_index) {
   const long long row = blockIdx.x;
   const bf16* x = logits + row * ld;
-  __shared__ float red[CE_THREADS / 32];
-  __shared__ float bcast;
-  float m = -INFINITY;
-  for (int c = threadIdx.x; c < cols; c += CE_THREADS) m = fmaxf(m, __bfloat162float(x[c]));
-  m = ce_warp_max(m);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float t = threadIdx.x < CE_THREADS / 32 ? red[threadIdx.x] : -INFINITY;
-    t = ce_warp_max(t);
-    if (threadIdx.x == 0) bcast = t;
+  __shared__ float red_m[CE_THREADS / 32], red_s[CE_THREADS / 32];
+  const CeSpan span = ce_span(x, cols);
+  float m = -INFINITY, s = 0.f;
+  auto raise = [&](float group_max) {  // exp(-inf - -inf) must not arise while nothing finite has been seen
+    if (group_max > m) {
+      s *= expf(m - group_max);
+      m = group_max;
+    }
+    return m == -INFINITY ? 0.f : m;
+  };
+  constexpr int U = 4;  // vectors in flight per thread
+  for (int c = span.head + threadIdx.x * 8; c < span.tail; c += U * CE_THREADS * 8) {
+    uint4 raw[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int ck = c + k * CE_THREADS * 8;
+      raw[k] = ck < span.tail ? *reinterpret_cast<const uint4*>(x + ck) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);  // -inf
+    }
+    float v[U][8], gm = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      ce_unpack(raw[k], v[k]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) gm = fmaxf(gm, v[k][j]);
+    }
+    const float base = raise(gm);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      float part = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) part += expf(v[k][j] - base);
+      s += part;
+    }
+  }
+  const int edge = span.head + cols - span.tail;  // at most 14 elements outside the vectors
+  if (int(threadIdx.x) < edge) {
+    const float v = __bfloat162float(x[int(threadIdx.x) < span.head ? threadIdx.x : span.tail + threadIdx.x - span.head]);
+    const float base = raise(v);
+    s += expf(v - base);
+  }
+  // merge (maximum, sum) over the CTA; a pair without a finite maximum carries no mass (or a NaN that has to survive)
+  const float wm = ce_warp_max(m);
+  s = ce_warp_sum(m == wm ? s : s * expf(m - wm));
+  if ((threadIdx.x & 31) == 0) {
+    red_m[threadIdx.x >> 5] = wm;
+    red_s[threadIdx.x >> 5] = s;
   }
   __syncthreads();
-  m = bcast;
-  float s = 0.f;
-  for (int c = threadIdx.x; c < cols; c += CE_THREADS) s += expf(__bfloat162float(x[c]) - m);
-  s = ce_warp_sum(s);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
   if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < CE_THREADS / 32; ++w) t += red[w];
+    float mm = red_m[0], t = 0.f;
+    for (int w = 1; w < CE_THREADS / 32; ++w) mm = fmaxf(mm, red_m[w]);
+    for (int w = 0; w < CE_THREADS / 32; ++w) t += red_m[w] == mm ? red_s[w] : red_s[w] * expf(red_m[w] - mm);
+    if (mm == -INFINITY) t = NAN;  // no finite logit in this slice: exp(-inf - -inf)
     const long long label = labels[row];
     const long long local = label - vocab_start;
     const bool mine = label != ignore_index && local >= 0 && local < cols;
-    stats[row * 4 + 0] = m;
+    stats[row * 4 + 0] = mm;
     stats[row * 4 + 1] = t;
     stats[row * 4 + 2] = mine ? __bfloat162float(x[local]) : 0.f;
     stats[row * 4 + 3] = mine ? 1.f : 0.f;
@@ -69,18 +117,47 @@ ce_grad_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ labels, co
                long long ld, int vocab_start, int ignore_index, const float* __restrict__ scale_ptr) {
   const long long row = blockIdx.x;
   bf16* x = logits + row * ld;
+  const CeSpan span = ce_span(x, cols);
   const long long label = labels[row];
   const float scale = scale_ptr[0];
-  if (label == ignore_index) {
-    for (int c = threadIdx.x; c < cols; c += CE_THREADS) x[c] = __float2bfloat16(0.f);
-    return;
-  }
-  const float l = lse[row];
+  const bool ignored = label == ignore_index;
+  const float l = ignored ? 0.f : lse[row];
   const long long local = label - vocab_start;
-  for (int c = threadIdx.x; c < cols; c += CE_THREADS) {
-    float p = expf(__bfloat162float(x[c]) - l);
+  auto grad = [&](float v, int c) {
+    if (ignored) return 0.f;
+    float p = expf(v - l);
     if (c == local) p -= 1.f;
-    x[c] = __float2bfloat16(p * scale);
+    return p * scale;
+  };
+  constexpr int U = 4;
+  for (int c = span.head + threadIdx.x * 8; c < span.tail; c += U * CE_THREADS * 8) {
+    uint4 raw[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int ck = c + k * CE_THREADS * 8;
+      if (ck < span.tail && !ignored) raw[k] = *reinterpret_cast<const uint4*>(x + ck);
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int ck = c + k * CE_THREADS * 8;
+      if (ck < span.tail) {
+        float v[8];
+        ce_unpack(raw[k], v);
+        uint4 o;
+        uint32_t* ow = &o.x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(grad(v[2 * j], ck + 2 * j), grad(v[2 * j + 1], ck + 2 * j + 1));
+          ow[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(x + ck) = o;
+      }
+    }
+  }
+  const int edge = span.head + cols - span.tail;
+  if (int(threadIdx.x) < edge) {
+    const int c = int(threadIdx.x) < span.head ? threadIdx.x : span.tail + threadIdx.x - span.head;
+    x[c] = __float2bfloat16(grad(__bfloat162float(x[c]), c));
   }
 }
 

@@ -48,6 +48,45 @@ def test_norm_backward_row_and_column_edges(dtype, rows, cols, mode):
         assert bool((err <= rel * (want.abs() + 2 * scale) + 1e-6).all()), (err.max().item(), scale)
 
 
+@pytest.mark.parametrize("vocab", [8, 131, 4096, 5003])
+def test_head_loss_rows_at_any_alignment(vocab):
+    from tensor_parallel_b200.ops.loss import lm_head_cross_entropy
+
+    torch.manual_seed(vocab)
+    rows, hidden = 150, 128
+    x = torch.randn(rows, hidden, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    w = (torch.randn(vocab, hidden, device="cuda", dtype=torch.bfloat16) * 0.2).requires_grad_()
+    labels = torch.randint(0, vocab, (rows,), device="cuda")
+    labels[::7] = -100
+    loss = lm_head_cross_entropy(x, w, labels)
+    loss.backward()
+    xr, wr = x.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(xr @ wr.t(), labels)
+    want.backward()
+    assert abs(loss.item() - want.item()) <= 2e-3 * want.item() + 1e-3  # logits are rounded to bf16
+    for got, ref in ((x.grad, xr.grad), (w.grad, wr.grad)):
+        assert (got.double() - ref).norm() <= 0.02 * ref.norm()
+
+
+def test_loss_statistics_with_infinite_logits():
+    """Masked (-inf) logits carry no mass whatever vector, thread or edge they fall into."""
+    from tensor_parallel_b200.ops import loss as L
+
+    nat = _native()
+    torch.manual_seed(0)
+    rows, cols = 40, 4099
+    logits = torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16) * 4
+    logits[torch.rand(rows, cols, device="cuda") < 0.5] = -math.inf
+    logits[3, :4000] = -math.inf
+    logits[4, 1:] = -math.inf
+    logits[4, 0] = 1.0
+    labels = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    stats = torch.empty(rows, 4, device="cuda")
+    nat.check(L.LIB.tpb_ce_stats(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), rows, cols, cols, 0, -100, nat._stream()), "ce_stats")
+    lse = stats[:, 0].double() + stats[:, 1].double().log()
+    assert (lse - logits.double().logsumexp(-1)).abs().max().item() < 1e-5
+
+
 @pytest.mark.parametrize("heads,tokens", [(1, 3), (3, 700), (12, 65), (33, 2100)])
 @pytest.mark.parametrize("interleaved,rotary", [(False, 128), (False, 64), (True, 32)])
 def test_rope_head_groups(heads, tokens, interleaved, rotary):
