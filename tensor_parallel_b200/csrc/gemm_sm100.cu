@@ -43,6 +43,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include "gemm_pair.cuh"
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
 #include "tpb_api.h"
@@ -1179,6 +1180,7 @@ extern "C" int tpb_gemm_preload(void) {
   LOAD(16, 1, 8); LOAD(16, 2, 8); LOAD(16, 4, 8); LOAD(32, 1, 8); LOAD(32, 2, 8); LOAD(32, 4, 8);
   LOAD(64, 1, 2); LOAD(128, 1, 1); LOAD(256, 1, 1);
 #undef LOAD
+  if (e == cudaSuccess) e = gemm_pair_preload();
   return e == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
@@ -1289,6 +1291,9 @@ extern "C" int tpb_gemm_plan_ex(int tokens, int features, int k, int world, int 
     const int work = tiles * splits;
     plan->grid = work < sms ? work : sms;
   }
+  // Whole tiles of a many-token GEMM on one rank run on CTA pairs where that is faster (rule and figures: gemm_pair_tile);
+  // split-K, the cross-rank sum and the fused all-gather (force_splits = 1) stay with the single-CTA kernel.
+  plan->pair = (!plan->swapped && world == 1 && force_splits <= 0 && plan->k_splits == 1) ? gemm_pair_tile(tokens, features, sms) : 0;
   plan->tokens_pad = plan->swapped ? plan->n_tiles * bn : plan->m_tiles * BM;
   plan->slot_elems = size_t(tokens) * size_t(features);
   plan->tiles = tiles;
@@ -1404,6 +1409,20 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     }
     p.ag_push_counter = static_cast<uint32_t*>(ag->push_counter);
     p.ag_mc_dst = static_cast<__nv_bfloat16*>(ag->mc_gathered);
+  }
+
+  if (plan->pair && !ag) {
+    PairGemm g;
+    g.x = x; g.w = w;
+    g.tokens = tokens; g.features = features; g.k = k; g.ldx = ldx; g.ldw = ldw;
+    g.x_mn = p.a_mn; g.w_mn = p.b_mn;
+    g.out = p.out; g.ld_out = ld_out;
+    g.bias = p.bias; g.bias_scale = bias_scale;
+    g.residual = p.residual;
+    g.act = act;
+    g.status = p.status;
+    g.out_elems = p.out_elems;
+    return gemm_pair_launch(g, plan->pair, sm_count(), stream);
   }
 
   const void* a_ptr = plan->swapped ? w : x;

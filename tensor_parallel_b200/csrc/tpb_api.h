@@ -35,6 +35,7 @@ typedef struct {
   size_t slot_elems;  // fp32 elements one slot must hold
   int stream_k;       // 1: the (tile, k-block) units are dealt out as one contiguous range per CTA; k_splits then is an
                       // upper bound of the CTAs that contribute to one tile
+  int pair;           // columns of the CTA-pair tile (256 or 128) when the many-token pair kernel runs this shape, else 0
 } tpb_gemm_plan_t;
 
 // Workspace of the fused split-K / all-reduce epilogue.  All pointers are device pointers valid on the

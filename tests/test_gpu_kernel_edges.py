@@ -25,6 +25,51 @@ def _close(got, want, terms=1.0):
     assert bool((err <= bound).all()), f"largest excess {(err - bound).max().item():.3g} at value {want.flatten()[(err - bound).argmax()].item():.3g}"
 
 
+def _gemm_ref(x, w, bias=None, act=None, residual=None):
+    y = x.double() @ w.double().t()
+    if bias is not None:
+        y = y + bias.double()
+    if act == "swiglu16":
+        g = y.reshape(y.shape[0], -1, 2, 16)
+        y = (torch.nn.functional.silu(g[:, :, 0]) * g[:, :, 1]).reshape(y.shape[0], -1)
+    elif act == "gelu":
+        y = torch.nn.functional.gelu(y)
+    elif act == "relu":
+        y = torch.relu(y)
+    return y if residual is None else y + residual.double()
+
+
+@pytest.mark.parametrize("tokens,features,k", PAIR)
+@pytest.mark.parametrize("x_t,w_t", [(False, False), (False, True), (True, True)])
+def test_pair_gemm(tokens, features, k, x_t, w_t):
+    nat = _native()
+    torch.manual_seed(tokens + features)
+    assert nat.gemm_plan(tokens, features, k, no_swap=x_t or w_t).pair in (128, 256)
+    x = torch.randn(tokens, k, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(features, k, device="cuda", dtype=torch.bfloat16) / math.sqrt(k)
+    bias = torch.randn(features, device="cuda", dtype=torch.bfloat16)
+    res = torch.randn(tokens, features, device="cuda", dtype=torch.bfloat16)
+    args = (x.t().contiguous() if x_t else x, w.t().contiguous() if w_t else w)
+    out = nat.gemm_nt(*args, bias=bias, residual=res, act="gelu", x_t=x_t, w_t=w_t)
+    _close(out, _gemm_ref(x, w, bias, "gelu", res), terms=8)
+    _close(nat.gemm_nt(*args, x_t=x_t, w_t=w_t), _gemm_ref(x, w), terms=8)
+    nat.device_state(x.device).check_status()
+
+
+@pytest.mark.parametrize("tokens", [2305, 8192])
+def test_pair_gemm_gated_into_a_wider_buffer(tokens):
+    nat = _native()
+    torch.manual_seed(tokens)
+    f, k = 1376, 264
+    x = torch.randn(tokens, k, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(2 * f, k, device="cuda", dtype=torch.bfloat16) / math.sqrt(k)
+    assert nat.gemm_plan(tokens, 2 * f, k).pair
+    wide = torch.full((tokens, f + 24), 7.0, device="cuda", dtype=torch.bfloat16)
+    nat.gemm_nt(x, w, act="swiglu16", out=wide[:, 16 : 16 + f])
+    _close(wide[:, 16 : 16 + f], _gemm_ref(x, w, act="swiglu16"), terms=8)
+    assert bool((wide[:, :16] == 7).all()) and bool((wide[:, 16 + f :] == 7).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (2, 2048), (295, 2056), (297, 4096), (700, 5120), (61, 8192)])
 @pytest.mark.parametrize("mode", ["rms", "layer"])
