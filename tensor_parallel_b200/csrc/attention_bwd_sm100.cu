@@ -64,6 +64,7 @@ struct BwParams {
   int bias_kind;       // 0 none, 1 fp32, 2 bf16
   long long b_sb, b_sh, b_sq, b_sk;
   float* dbias;        // fp32, the bias' own strides, zero-initialised by the caller; written by the dQ launch only (or null)
+  int bias_vec;        // bias rows readable as aligned vectors of eight keys (bias_vector_rows); so is dbias then
   float inv_scale;
   uint32_t* status;
 };
@@ -306,14 +307,14 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         hi = min(HC, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
       }
       const bool masked = lo > 0 || hi < HC;
-      // score bias: element (query, key) = (col0 + c, ri) for dK / dV and (ri, col0 + c) for dQ
-      const float* bias_f = static_cast<const float*>(p.bias);
-      const bf16* bias_h = static_cast<const bf16*>(p.bias);
+      // score bias: element (query, key) = (col0 + c, ri) for dK / dV - there the lanes of a warp own consecutive keys - and
+      // (ri, col0 + c) for dQ, where a thread's columns are consecutive keys of one row and are read eight at a time
       const int b_head = DKV ? head + g : head;
       const long long bias_base = BIAS ? (long long)b * p.b_sb + (long long)b_head * p.b_sh + (long long)ri * (DKV ? p.b_sk : p.b_sq) : 0;
       const long long bias_step = DKV ? p.b_sq : p.b_sk;  // per column
       const int col_limit = DKV ? p.sq : p.sk, row_limit = DKV ? p.sk : p.sq;
       uint32_t pp[HC / 2], ds[HC / 2];
+      float bv[8], db[4];
 #pragma unroll
       for (int c = 0; c < HC; c += 2) {
         float l0, l1, d0, d1;
@@ -325,17 +326,14 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
           l0 = l1 = my_lse2;
           d0 = d1 = my_del;
         }
+        if (BIAS && (c & 7) == 0)
+          load_bias8(p.bias, p.bias_kind, bias_base + (long long)(col0 + c) * bias_step, bias_step, ri < row_limit ? col_limit - col0 - c : 0,
+                     !DKV && p.bias_vec, bv);
         float x0, x1, p0, p1, g0, g1;
         ffma2(x0, x1, __uint_as_float(sv[c]), __uint_as_float(sv[c + 1]), p.scale_log2e, p.scale_log2e, -l0, -l1);
-        long long bi0 = 0, bi1 = 0;
         if (BIAS) {
-          bi0 = bias_base + (long long)(col0 + c) * bias_step;
-          bi1 = bi0 + bias_step;
-          const bool in0 = ri < row_limit && col0 + c < col_limit, in1 = ri < row_limit && col0 + c + 1 < col_limit;
-          const float b0 = !in0 ? 0.f : (p.bias_kind == 1 ? __ldg(bias_f + bi0) : __bfloat162float(bias_h[bi0]));
-          const float b1 = !in1 ? 0.f : (p.bias_kind == 1 ? __ldg(bias_f + bi1) : __bfloat162float(bias_h[bi1]));
-          x0 += b0 * 1.4426950408889634f;
-          x1 += b1 * 1.4426950408889634f;
+          x0 += bv[c & 7] * 1.4426950408889634f;
+          x1 += bv[(c & 7) + 1] * 1.4426950408889634f;
         }
         p0 = ex2_approx(x0);
         p1 = ex2_approx(x1);
@@ -346,8 +344,20 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         ffma2(g0, g1, __uint_as_float(dv[c]), __uint_as_float(dv[c + 1]), p.scale, p.scale, -d0, -d1);  // (dP - delta) * scale
         ffma2(g0, g1, g0, g1, p0, p1, 0.f, 0.f);
         if (BIAS && !DKV && p.dbias) {  // d(bias) = P (dP - delta) = dS / scale; pairs that are masked or out of range contribute nothing
-          if (p0 != 0.f && ri < row_limit && col0 + c < col_limit) atomicAdd(p.dbias + bi0, g0 * p.inv_scale);
-          if (p1 != 0.f && ri < row_limit && col0 + c + 1 < col_limit) atomicAdd(p.dbias + bi1, g1 * p.inv_scale);
+          db[c & 3] = p0 != 0.f ? g0 * p.inv_scale : 0.f;
+          db[(c & 3) + 1] = p1 != 0.f ? g1 * p.inv_scale : 0.f;
+          if ((c & 3) == 2 && ri < row_limit) {
+            const int c4 = c - 2;
+            float* dst = p.dbias + bias_base + (long long)(col0 + c4) * bias_step;
+            if (p.bias_vec && col0 + c4 + 4 <= col_limit) {
+              // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (db[i] != 0.f && col0 + c4 + i < col_limit) atomicAdd(dst + i * bias_step, db[i]);
+            }
+          }
         }
         if (DKV) pp[c >> 1] = pack_bf16x2(p0, p1);
         ds[c >> 1] = pack_bf16x2(g0, g1);
@@ -484,6 +494,7 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   p.bias = bias;
   p.bias_kind = !bias ? 0 : (bias_dtype == 1 ? 1 : 2);
   p.b_sb = bias_sb; p.b_sh = bias_sh; p.b_sq = bias_sq; p.b_sk = bias_sk;
+  p.bias_vec = bias && bias_vector_rows(bias, bias_sb, bias_sh, bias_sq, bias_sk) && !(reinterpret_cast<uintptr_t>(dbias) & 15);
   p.dbias = nullptr;  // (the dK / dV launch leaves it alone)
   p.inv_scale = scale > 0.f ? 1.f / scale : 0.f;
   // dK / dV: the dk strides serve dv too (the existing contract)

@@ -56,6 +56,7 @@ struct FaParams {
   const void* bias;  // additive score bias in natural-log units, -inf masks a key; element strides, 0 broadcasts
   int bias_kind;     // 0 none, 1 fp32, 2 bf16
   long long bias_sb, bias_sh, bias_sq, bias_sk;
+  int bias_vec;      // rows readable as aligned vectors of eight keys (bias_vector_rows)
   uint32_t* status;
 };
 
@@ -203,8 +204,6 @@ attn_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 #pragma unroll
     for (int i = 0; i < HD; ++i) o_reg[i] = 0.f;
     float m_run = -INFINITY, l_run = 0.f, alpha_prev = 1.f;
-    const float* bias_f = static_cast<const float*>(p.bias);
-    const bf16* bias_h = static_cast<const bf16*>(p.bias);
     const long long bias_row = p.bias_kind ? (b * p.bias_sb + h * p.bias_sh + (long long)min(qi, p.sq - 1) * p.bias_sq) : 0;
     bool alive = true;
 
@@ -247,18 +246,18 @@ attn_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           for (int i = 0; i < HN; i += 2) m_half = fmax3(m_half, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
           m_half *= p.scale_log2e;  // (the scale is positive: the maximum commutes with it)
         } else {
+          const int visible = min(p.sk, p.causal ? qi + shift + 1 : p.sk) - key0;  // the others become -inf
 #pragma unroll
-          for (int i = 0; i < HN; ++i) {
-            const int key = key0 + i;
-            const bool dead = key >= p.sk || (p.causal && key > qi + shift);
-            float sv = dead ? -INFINITY : __uint_as_float(r[i]) * p.scale_log2e;
-            if (p.bias_kind && !dead) {
-              const long long bi = bias_row + (long long)key * p.bias_sk;
-              const float bv = p.bias_kind == 1 ? __ldg(bias_f + bi) : __bfloat162float(bias_h[bi]);
-              sv += bv * 1.4426950408889634f;
+          for (int c = 0; c < HN; c += 8) {
+            float bv[8];
+            if (p.bias_kind) load_bias8(p.bias, p.bias_kind, bias_row + (long long)(key0 + c) * p.bias_sk, p.bias_sk, visible - c, p.bias_vec, bv);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              float sv = c + i < visible ? __uint_as_float(r[c + i]) * p.scale_log2e : -INFINITY;
+              if (p.bias_kind && c + i < visible) sv += bv[i] * 1.4426950408889634f;
+              r[c + i] = __float_as_uint(sv);
+              m_half = fmaxf(m_half, sv);
             }
-            r[i] = __float_as_uint(sv);
-            m_half = fmaxf(m_half, sv);
           }
         }
       }
@@ -541,8 +540,6 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     const uint32_t s_addr = tmem_base + (uint32_t(quarter * 32) << 16) + t * FA_N;  // scores, and in their first 64 columns P
     const uint32_t o_addr = tmem_base + (uint32_t(quarter * 32) << 16) + O_COL0 + t * FA_N;
     float m_run = -INFINITY, l_run = 0.f;
-    const float* bias_f = static_cast<const float*>(p.bias);
-    const bf16* bias_h = static_cast<const bf16*>(p.bias);
     const long long bias_row = p.bias_kind ? (b * p.bias_sb + h * p.bias_sh + (long long)min(qi, p.sq - 1) * p.bias_sq) : 0;
     bool alive = true;
 
@@ -577,18 +574,18 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         m_tile = fmaxf(m0, m1) * p.scale_log2e;  // (the scale is positive: the maximum commutes with it)
       } else {
         m_tile = -INFINITY;
+        const int visible = min(p.sk, p.causal ? qi + shift + 1 : p.sk) - key0;  // the others become -inf
 #pragma unroll
-        for (int i = 0; i < FA_N; ++i) {
-          const int key = key0 + i;
-          const bool dead = key >= p.sk || (p.causal && key > qi + shift);
-          float sv = dead ? -INFINITY : __uint_as_float(r[i]) * p.scale_log2e;
-          if (!dead) {
-            const long long bi = bias_row + (long long)key * p.bias_sk;
-            const float bv = p.bias_kind == 1 ? __ldg(bias_f + bi) : __bfloat162float(bias_h[bi]);
-            sv += bv * 1.4426950408889634f;
+        for (int c = 0; c < FA_N; c += 8) {
+          float bv[8];
+          load_bias8(p.bias, p.bias_kind, bias_row + (long long)(key0 + c) * p.bias_sk, p.bias_sk, visible - c, p.bias_vec, bv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float sv = c + i < visible ? __uint_as_float(r[c + i]) * p.scale_log2e : -INFINITY;
+            if (c + i < visible) sv += bv[i] * 1.4426950408889634f;
+            r[c + i] = __float_as_uint(sv);
+            m_tile = fmaxf(m_tile, sv);
           }
-          r[i] = __float_as_uint(sv);
-          m_tile = fmaxf(m_tile, sv);
         }
       }
       // ---- lazy running maximum; rescale the accumulated output only after a large rise ----
@@ -761,6 +758,7 @@ extern "C" int tpb_attn_prefill_sm100(const void* q, const void* k, const void* 
   p.bias = bias;
   p.bias_kind = !bias ? 0 : (bias_dtype == 1 ? 1 : 2);
   p.bias_sb = bias_sb; p.bias_sh = bias_sh; p.bias_sq = bias_sq; p.bias_sk = bias_sk;
+  p.bias_vec = bias && bias_vector_rows(bias, bias_sb, bias_sh, bias_sq, bias_sk);
   p.status = static_cast<uint32_t*>(status);
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   static const bool one_tile = getenv("TPB_ATTN_ONE_TILE") != nullptr;  // (A/B switch: the kernel with one query tile per CTA)

@@ -2,6 +2,7 @@
 // tensor maps over strided [batch, seq, head, head_dim] views.
 #pragma once
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -58,6 +59,39 @@ __device__ __forceinline__ void ex2_poly2(float& x0, float& x1) {
   ffma2(p0, p1, p0, p1, f0, f1, 0.9999280572f, 0.9999280572f);
   x0 = __int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23));
   x1 = __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23));
+}
+
+// Eight consecutive keys of one score-bias row, starting at element `idx`; `valid` of them exist (the others become 0).
+// kind: 1 fp32, 2 bf16.  `vec` (see bias_vector_rows): the eight elements are contiguous and 16-byte aligned - one or two wide
+// loads instead of eight scattered ones, each of which costs its own 32-byte sector when the lanes of a warp own different rows
+// (16 x 512 tokens, 32 heads of 64, one bias for all batches: forward 1084 -> 210 us, dQ with the bias gradient 1138 -> 353 us).
+__device__ __forceinline__ void load_bias8(const void* bias, int kind, long long idx, long long step, int valid, bool vec, float (&v)[8]) {
+  if (vec && valid >= 8) {
+    if (kind == 1) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(bias) + idx));
+      const float4 b = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(bias) + idx) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(bias) + idx));
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[2 * i] = __uint_as_float(w[i] << 16);
+        v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const long long at = idx + i * step;
+    v[i] = i >= valid ? 0.f : (kind == 1 ? __ldg(static_cast<const float*>(bias) + at) : __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[at]));
+  }
+}
+// True if eight keys from a multiple of 8 on are one aligned vector in every row of this bias (fp32 needs multiples of 4 only,
+// but the keys come in eights anyway).
+__host__ __device__ __forceinline__ bool bias_vector_rows(const void* bias, long long sb, long long sh, long long sq, long long sk) {
+  return sk == 1 && !((sb | sh | sq) & 7) && !(reinterpret_cast<uintptr_t>(bias) & 15);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

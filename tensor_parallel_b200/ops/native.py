@@ -651,7 +651,19 @@ class _AttentionFn(torch.autograd.Function):
         return grads[0], grads[1], grads[2], None, None, dbias
 
 
+def _keys_contiguous(bias):
+    """``bias`` with consecutive keys adjacent in memory (a differentiable copy if they are not): the kernels then read a row of
+    it in 16-byte vectors.  Relative-position tables arrive as permuted ``[query, key, head]`` lookups, whose keys lie a whole
+    row of heads apart.  Views that broadcast a dimension are left alone (a copy would materialise it)."""
+    if bias is None or bias.ndim == 0 or bias.shape[-1] == 1 or bias.stride(-1) == 1:
+        return bias
+    if any(st == 0 and n > 1 for st, n in zip(bias.stride(), bias.shape)):
+        return bias
+    return bias.contiguous()
+
+
 def attention(q, k, v, causal, bias=None, scale=None):
+    bias = _keys_contiguous(bias)
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad or (bias is not None and bias.requires_grad))
     if needs_grad:
         return _AttentionFn.apply(q, k, v, bool(causal), scale, bias)

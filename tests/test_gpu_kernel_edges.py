@@ -164,3 +164,31 @@ def test_adamw_remainders_and_alignment(n, offset, dtype, gdtype):
         assert (got.double() - ref).abs().max().item() <= 2e-6  # a few fp32 roundings of values below 1 (1 - 0.99f is 1e-6 off)
     if master is not None:
         assert torch.equal(p, master.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("sq,sk", [(64, 128), (150, 152), (150, 150), (300, 520)])
+@pytest.mark.parametrize("layout", ["dense", "heads_last", "padding", "fp32"])
+def test_bias_rows_in_vectors_and_one_by_one(sq, sk, layout):
+    torch.manual_seed(sq + sk)
+    b, h, d = 3, 4, 64
+    q = torch.randn(b, sq, h, d, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    k, v = (torch.randn(b, sk, h, d, device="cuda", dtype=torch.bfloat16).requires_grad_() for _ in range(2))
+    if layout == "heads_last":
+        leaf = torch.randn(sq, sk, h, device="cuda", dtype=torch.bfloat16).requires_grad_()
+        bias = leaf.permute(2, 0, 1)[None]
+    elif layout == "padding":
+        leaf = torch.zeros(b, 1, 1, sk, device="cuda", dtype=torch.bfloat16)
+        leaf[1, :, :, sk // 2 :] = -math.inf
+        bias = leaf
+    else:
+        leaf = torch.randn(1, h, sq, sk, device="cuda", dtype=torch.float32 if layout == "fp32" else torch.bfloat16).requires_grad_()
+        bias = leaf
+    g = torch.randn(b, sq, h, d, device="cuda", dtype=torch.bfloat16)
+    OF.attention(q, k, v, False, bias=bias).backward(g)
+    ref = [t.detach().double().requires_grad_() for t in (q, k, v, bias)]
+    scores = torch.einsum("bqhd,bkhd->bhqk", ref[0], ref[1]) / math.sqrt(d) + ref[3]
+    torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1), ref[2]).backward(g.double())
+    got = [q.grad, k.grad, v.grad] + ([] if layout == "padding" else [leaf.grad.permute(2, 0, 1)[None] if layout == "heads_last" else leaf.grad])
+    for a, r in zip(got, ref):
+        # probabilities and dS pass through bf16 (2^-9 each) on their way into sums that cancel
+        assert (a.double() - r.grad).norm() <= 0.02 * r.grad.norm()
