@@ -72,11 +72,10 @@ class T5Attention(nn.Module):
             self.relative_attention_bias = nn.Embedding(self.relative_attention_num_buckets, self.n_heads)
 
     def compute_bias(self, query_length: int, key_length: int, device):
-        ctx = torch.arange(key_length - query_length, key_length, device=device)[:, None]
-        mem = torch.arange(key_length, device=device)[None, :]
-        buckets = relative_position_bucket(mem - ctx, not self.is_decoder, self.relative_attention_num_buckets,
-                                           self.relative_attention_max_distance)
-        return self.relative_attention_bias(buckets).permute(2, 0, 1)[None]  # [1, heads, q, k]
+        # query i sits at position i + key_length - query_length: the distances run from -(key_length - 1) to query_length - 1
+        distance = torch.arange(1 - key_length, query_length, device=device)
+        buckets = relative_position_bucket(distance, not self.is_decoder, self.relative_attention_num_buckets, self.relative_attention_max_distance)
+        return OF.relative_bias(self.relative_attention_bias, buckets, query_length, key_length)  # [1, heads, q, k]
 
     def forward(self, hidden_states, mask=None, key_value_states=None, position_bias=None, past_key_value=None, use_cache=False):
         b, s, _ = hidden_states.shape

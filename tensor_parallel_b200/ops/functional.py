@@ -100,6 +100,12 @@ def geglu_ref(gate, up, approximate: str = "tanh"):
     return F.gelu(gate, approximate=approximate) * up
 
 
+def relative_bias_ref(embedding, buckets, queries: int, keys: int):
+    i = torch.arange(queries, device=buckets.device)[:, None]
+    j = torch.arange(keys, device=buckets.device)[None, :]
+    return embedding(buckets[j - i + queries - 1]).permute(2, 0, 1)[None]
+
+
 # -- dispatching front-end ---------------------------------------------------------------------
 
 
@@ -136,6 +142,19 @@ def attention(q, k, v, causal: bool, bias=None, scale: Optional[float] = None):
     if nat is not None and nat.attention_supported(q, k, v, bias):
         return nat.attention(q, k, v, causal, bias, scale)
     return attention_ref(q, k, v, causal, bias, scale)
+
+
+def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
+    """Score bias ``[1, heads, queries, keys]`` of a learned table over position buckets; ``buckets`` holds the bucket of each distance
+    ``key - query``, from ``-(queries - 1)`` up, in ``queries + keys - 1`` entries.  An embedding that does more than look rows up (a
+    wrapper, hooks, renormalisation, sparse gradients) is called as the module it is."""
+    plain = (type(embedding) is torch.nn.Embedding and embedding.max_norm is None and embedding.padding_idx is None and not embedding.sparse
+             and not embedding.scale_grad_by_freq and not (embedding._forward_hooks or embedding._forward_pre_hooks or embedding._backward_hooks
+                                                           or embedding._backward_pre_hooks))
+    nat = _native(embedding.weight) if plain and buckets.is_cuda else None
+    if nat is not None and nat.relative_bias_supported(embedding.weight):
+        return nat.relative_bias(embedding.weight, buckets, queries, keys)
+    return relative_bias_ref(embedding, buckets, queries, keys)
 
 
 def gelu(x, approximate: str = "none"):

@@ -743,6 +743,46 @@ def qkv_rope_append(q, k, v, q_out, kcache, vcache, base_pos, batch, seq, rotary
     return q_out
 
 
+LIB.tpb_relative_bias.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
+LIB.tpb_relative_bias_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
+
+
+def relative_bias_supported(table: torch.Tensor) -> bool:
+    return table.dtype in (torch.bfloat16, torch.float32) and table.ndim == 2 and table.numel() > 0
+
+
+class _RelativeBiasFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, table, buckets, queries, keys):
+        global launch_count
+        n, heads = table.shape
+        table = table.contiguous()
+        buckets = buckets.to(torch.int32).contiguous()
+        out = torch.empty(1, heads, queries, keys, dtype=table.dtype, device=table.device)
+        check(LIB.tpb_relative_bias(_ptr(table), _ptr(buckets), _ptr(out), heads, queries, keys, _dtype_code(table), _stream()), "tpb_relative_bias")
+        launch_count += 1
+        ctx.save_for_backward(buckets)
+        ctx.meta = (n, heads, queries, keys, table.dtype)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        global launch_count
+        (buckets,) = ctx.saved_tensors
+        n, heads, queries, keys, dtype = ctx.meta
+        g = grad.to(dtype).contiguous()
+        partial = torch.empty(LIB.tpb_relative_bias_parts(queries), n, heads, dtype=torch.float32, device=g.device)
+        check(LIB.tpb_relative_bias_bwd(_ptr(g), _ptr(buckets), _ptr(partial), heads, queries, keys, n, _dtype_code(g), _stream()), "tpb_relative_bias_bwd")
+        launch_count += 1
+        return partial.sum(0).to(dtype), None, None, None
+
+
+def relative_bias(table, buckets, queries, keys):
+    """``out[0, h, i, j] = table[buckets[j - i + queries - 1], h]`` for a ``[n_buckets, heads]`` table and the bucket of each of the
+    ``queries + keys - 1`` distances (values must be valid rows of the table)."""
+    return _RelativeBiasFn.apply(table, buckets, int(queries), int(keys))
+
+
 # ------------------------------------------------------------------------------------------------
 # embedding / optimizer / casts
 # ------------------------------------------------------------------------------------------------

@@ -192,3 +192,23 @@ def test_bias_rows_in_vectors_and_one_by_one(sq, sk, layout):
     for a, r in zip(got, ref):
         # probabilities and dS pass through bf16 (2^-9 each) on their way into sums that cancel
         assert (a.double() - r.grad).norm() <= 0.02 * r.grad.norm()
+
+
+@pytest.mark.parametrize("queries,keys", [(1, 1), (1, 9), (17, 40), (64, 1032), (65, 2100), (512, 512)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_relative_bias_and_its_gradient(queries, keys, dtype):
+    torch.manual_seed(queries + keys)
+    heads, n = 5, 40
+    emb = torch.nn.Embedding(n, heads, device="cuda", dtype=dtype)
+    ref = torch.nn.Embedding(n, heads, device="cuda", dtype=torch.float64)
+    ref.weight.data.copy_(emb.weight.data)
+    buckets = torch.randint(0, n, (queries + keys - 1,), device="cuda")
+    out = OF.relative_bias(emb, buckets, queries, keys)
+    want = OF.relative_bias_ref(ref, buckets, queries, keys)
+    assert out.is_contiguous() and torch.equal(out.double(), want)
+    g = torch.randn(1, heads, queries, keys, device="cuda").to(dtype)
+    out.backward(g)
+    want.backward(g.double())
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+    err = (emb.weight.grad.double() - ref.weight.grad).abs()
+    assert bool((err <= rel * ref.weight.grad.abs() + 2.0 ** -22 * queries * keys ** 0.5).all())
