@@ -195,10 +195,11 @@ template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm vol
 // cp.async into its private slots of a DEC_STAGES-deep ring, so several groups are in flight per lane without holding
 // them in registers, and nobody reads another thread's slot (no barrier).  kbase / vbase already point at this
 // lane's first chunk (element 8 * part of key 0); see dec_elem for the slice layout.  The trip count is uniform across the warp
-// (consume() shuffles); lanes whose key is out of range copy nothing and pass valid = false.
-template <int D, typename Consume>
+// (consume() shuffles); lanes whose key is out of range copy nothing and pass valid = false.  `prepare` (run once by every
+// thread of the CTA) is what consume() needs; it runs while the first groups are on their way.
+template <int D, typename Prepare, typename Consume>
 __device__ __forceinline__ void stream_keys(const bf16* kbase, const bf16* vbase, int k_begin, int k_end, int warp, int sub,
-                                            uint4* ring, Consume&& consume) {
+                                            uint4* ring, Prepare&& prepare, Consume&& consume) {
   constexpr int EPL = D / 8, C = EPL / 8, STEP = DEC_WARPS * 4;
   auto slot = [&](int stage, int kv, int c) { return ring + ((stage * 2 + kv) * C + c) * DEC_THREADS + threadIdx.x; };
   auto issue = [&](int stage, int group_base) {
@@ -217,6 +218,7 @@ __device__ __forceinline__ void stream_keys(const bf16* kbase, const bf16* vbase
   int key_base = k_begin + warp * 4;
 #pragma unroll
   for (int st = 0; st < DEC_STAGES - 1; ++st) issue(st, key_base + st * STEP);
+  prepare();
   for (int it = 0; key_base < k_end; key_base += STEP, ++it) {
     issue((it + DEC_STAGES - 1) % DEC_STAGES, key_base + (DEC_STAGES - 1) * STEP);
     cp_async_wait_group<DEC_STAGES - 1>();
@@ -260,12 +262,14 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kcache, 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane >> 3;   // which of the 4 keys of this warp iteration
   const int part = lane & 7;   // which D/8 slice
-  for (int i = threadIdx.x; i < G * D; i += DEC_THREADS) {
-    const int g = i / D, d = i % D;
-    const int qh = kvh * g_total + g_offset + g;
-    q_s[g][d] = __bfloat162float(q[((long long)b * q_heads + qh) * D + d]) * scale_log2e;
-  }
-  __syncthreads();
+  auto prepare = [&]() {
+    for (int i = threadIdx.x; i < G * D; i += DEC_THREADS) {
+      const int g = i / D, d = i % D;
+      const int qh = kvh * g_total + g_offset + g;
+      q_s[g][d] = __bfloat162float(q[((long long)b * q_heads + qh) * D + d]) * scale_log2e;
+    }
+    __syncthreads();
+  };
 
   float m[G], l[G], acc[G][EPL];
 #pragma unroll
@@ -279,7 +283,7 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kcache, 
   const bf16* vbase = vcache + (long long)bh * max_seq * D + part * 8;
 
   extern __shared__ uint4 dec_ring[];
-  stream_keys<D>(kbase, vbase, k0, k1, warp, sub, dec_ring, [&](const float (&kf)[EPL], const float (&vf)[EPL], bool valid) {
+  stream_keys<D>(kbase, vbase, k0, k1, warp, sub, dec_ring, prepare, [&](const float (&kf)[EPL], const float (&vf)[EPL], bool valid) {
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       float s = 0.f;
@@ -396,9 +400,11 @@ attn_decode_fused_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
                          float* __restrict__ part_o, float* __restrict__ part_ml, uint32_t* __restrict__ counters,
                          const int* __restrict__ pos_ptr, int q_heads, int kv_heads, int g_total, int g_offset, int max_seq,
                          int splits, float scale_log2e, int rotary_dim, float log2_theta, int interleaved, long long q_ld,
-                         long long k_ld, long long v_ld, const float2* __restrict__ rope_table, long long out_ld) {
+                         long long k_ld, long long v_ld, const float2* __restrict__ rope_table, long long out_ld, int early) {
   constexpr int EPL = D / 8;
-  pdl_wait();
+  // early: the cache rows before `pos` and `pos` itself were written before the previous kernel of the stream began, so the
+  // first keys are on their way before that kernel (the q / k / v projection) has finished
+  if (!early) pdl_wait();
   const int bh = blockIdx.x;
   const int b = bh / kv_heads, kvh = bh % kv_heads;
   const int split = blockIdx.y;
@@ -422,43 +428,49 @@ attn_decode_fused_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
   const int sub = lane >> 3, part = lane & 7;
   const int half = rotary_dim >> 1;
 
-  // rotate q (G heads) and the new k into shared memory; one thread per element pair
-  for (int i = threadIdx.x; i < (G + 1) * (D / 2); i += DEC_THREADS) {
-    const int hsel = i / (D / 2), p = i % (D / 2);
-    const bool is_k = hsel == G;
-    const bf16* src = is_k ? k + b * k_ld + (long long)kvh * D : q + b * q_ld + (long long)(kvh * g_total + g_offset + hsel) * D;
-    float* dst = is_k ? knew_s : q_s[hsel];
-    const float mul = is_k ? 1.f : scale_log2e;
-    if (p < half) {
-      const int ia = interleaved ? 2 * p : p;
-      const int ib = interleaved ? 2 * p + 1 : p + half;
-      float sn, cs;
-      if (rope_table) {  // (cos, sin) of every position, filled by rope_table_kernel with the formula below
-        const float2 t = __ldg(rope_table + (long long)pos * half + p);
-        cs = t.x;
-        sn = t.y;
+  auto prepare = [&]() {
+    if (early) {
+      pdl_wait();
+      pdl_trigger();
+    }
+    // rotate q (G heads) and the new k into shared memory; one thread per element pair
+    for (int i = threadIdx.x; i < (G + 1) * (D / 2); i += DEC_THREADS) {
+      const int hsel = i / (D / 2), p = i % (D / 2);
+      const bool is_k = hsel == G;
+      const bf16* src = is_k ? k + b * k_ld + (long long)kvh * D : q + b * q_ld + (long long)(kvh * g_total + g_offset + hsel) * D;
+      float* dst = is_k ? knew_s : q_s[hsel];
+      const float mul = is_k ? 1.f : scale_log2e;
+      if (p < half) {
+        const int ia = interleaved ? 2 * p : p;
+        const int ib = interleaved ? 2 * p + 1 : p + half;
+        float sn, cs;
+        if (rope_table) {  // (cos, sin) of every position, filled by rope_table_kernel with the formula below
+          const float2 t = __ldg(rope_table + (long long)pos * half + p);
+          cs = t.x;
+          sn = t.y;
+        } else {
+          const float inv_freq = exp2f(-log2_theta * (2.f * float(p) / float(rotary_dim)));
+          sincosf(float(pos) * inv_freq, &sn, &cs);
+        }
+        const float a = __bfloat162float(src[ia]), c = __bfloat162float(src[ib]);
+        // round through bf16 like the stand-alone append kernel, so cached and in-flight keys agree bit for bit
+        dst[ia] = __bfloat162float(__float2bfloat16(a * cs - c * sn)) * mul;
+        dst[ib] = __bfloat162float(__float2bfloat16(c * cs + a * sn)) * mul;
       } else {
-        const float inv_freq = exp2f(-log2_theta * (2.f * float(p) / float(rotary_dim)));
-        sincosf(float(pos) * inv_freq, &sn, &cs);
+        const int e = rotary_dim + 2 * (p - half);
+        dst[e] = __bfloat162float(src[e]) * mul;
+        dst[e + 1] = __bfloat162float(src[e + 1]) * mul;
       }
-      const float a = __bfloat162float(src[ia]), c = __bfloat162float(src[ib]);
-      // round through bf16 like the stand-alone append kernel, so cached and in-flight keys agree bit for bit
-      dst[ia] = __bfloat162float(__float2bfloat16(a * cs - c * sn)) * mul;
-      dst[ib] = __bfloat162float(__float2bfloat16(c * cs + a * sn)) * mul;
-    } else {
-      const int e = rotary_dim + 2 * (p - half);
-      dst[e] = __bfloat162float(src[e]) * mul;
-      dst[e + 1] = __bfloat162float(src[e + 1]) * mul;
     }
-  }
-  for (int i = threadIdx.x; i < D; i += DEC_THREADS) vnew_s[i] = __bfloat162float(v[b * v_ld + (long long)kvh * D + i]);
-  __syncthreads();
-  if (owns_new) {  // persist the new key / value for later steps
-    for (int i = threadIdx.x; i < D; i += DEC_THREADS) {
-      kcache[((long long)bh * max_seq + pos) * D + i] = __float2bfloat16(knew_s[i]);
-      vcache[((long long)bh * max_seq + pos) * D + i] = __float2bfloat16(vnew_s[i]);
+    for (int i = threadIdx.x; i < D; i += DEC_THREADS) vnew_s[i] = __bfloat162float(v[b * v_ld + (long long)kvh * D + i]);
+    __syncthreads();
+    if (owns_new) {  // persist the new key / value for later steps
+      for (int i = threadIdx.x; i < D; i += DEC_THREADS) {
+        kcache[((long long)bh * max_seq + pos) * D + i] = __float2bfloat16(knew_s[i]);
+        vcache[((long long)bh * max_seq + pos) * D + i] = __float2bfloat16(vnew_s[i]);
+      }
     }
-  }
+  };
 
   float m[G], l[G], acc[G][EPL];
 #pragma unroll
@@ -493,7 +505,7 @@ attn_decode_fused_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
   };
 
   extern __shared__ uint4 dec_ring[];
-  stream_keys<D>(kbase, vbase, k0, k1_cache, warp, sub, dec_ring, consume);
+  stream_keys<D>(kbase, vbase, k0, k1_cache, warp, sub, dec_ring, prepare, consume);
   if (owns_new && warp == 0) {  // the new token's key / value come straight from shared memory (warp-uniform branch)
     float kf[EPL], vf[EPL];
 #pragma unroll
@@ -939,11 +951,13 @@ extern "C" int tpb_rope_table(void* table, int positions, int rotary_dim, float 
 // with batch * q_heads of them every group of query heads of a KV head fits into ONE launch (GQA / MQA with large groups).
 // rope_table: optional output of tpb_rope_table covering every position < max_seq (null: angles are computed in place).
 // out: [batch][q_heads * head_dim] with a row pitch of out_ld elements (<= 0: dense).
+// early: launch as a programmatic dependent of the previous kernel of the stream and read pos_ptr and the cache rows before it
+// while that kernel still runs: it may produce q / k / v, but not those.
 extern "C" int tpb_attn_decode_fused(const void* q, const void* k, const void* v, void* kcache, void* vcache, void* out,
                                      float* part_o, float* part_ml, void* counters, const int* pos_ptr, int batch, int q_heads,
                                      int kv_heads, int head_dim, int max_seq, int splits, float scale, int rotary_dim, float theta,
                                      int interleaved, long long q_ld, long long k_ld, long long v_ld, const void* rope_table,
-                                     long long out_ld, int counter_elems, void* stream_) {
+                                     long long out_ld, int counter_elems, int early, void* stream_) {
   if (!q || !k || !v || !kcache || !vcache || !out || !pos_ptr || batch <= 0 || splits < 1 || q_heads % kv_heads) return TPB_ERR_ARG;
   if (splits > 1 && (!part_o || !part_ml || !counters)) return TPB_ERR_ARG;
   if (head_dim != 64 && head_dim != 128) return TPB_ERR_SIZE;
@@ -965,9 +979,10 @@ extern "C" int tpb_attn_decode_fused(const void* q, const void* k, const void* v
     dim3 grid(batch * kv_heads, splits, reps);
 #define DECF(D, G)                                                                                                           \
   if (!dec_smem_ready<attn_decode_fused_kernel<D, G>>(dec_ring_bytes<D>())) return TPB_ERR_CUDA;                               \
-  launch_kernel(attn_decode_fused_kernel<D, G>, grid, dim3(DEC_THREADS), dec_ring_bytes<D>(), s, (const bf16*)q, (const bf16*)k, (const bf16*)v, \
+  launch_dependent(attn_decode_fused_kernel<D, G>, grid, dim3(DEC_THREADS), dec_ring_bytes<D>(), s, first && (early || pdl_enabled()), (const bf16*)q, (const bf16*)k, (const bf16*)v, \
                 (bf16*)kcache, (bf16*)vcache, (bf16*)out, part_o, part_ml, (uint32_t*)counters, pos_ptr, q_heads, kv_heads, g_total, \
-                done, max_seq, splits, sl2, rotary_dim, l2t, interleaved, q_ld, k_ld, v_ld, (const float2*)rope_table, out_ld)
+                done, max_seq, splits, sl2, rotary_dim, l2t, interleaved, q_ld, k_ld, v_ld, (const float2*)rope_table, out_ld, (early && first) ? 1 : 0)
+    const bool first = launches == 0;  // (a second group of heads follows the first group's launch, which writes the new cache row)
     if (head_dim == 128) {
       if (gnow == 1) { DECF(128, 1); } else if (gnow == 2) { DECF(128, 2); } else { DECF(128, 4); }
     } else {

@@ -44,6 +44,7 @@
 #include <string.h>
 
 #include "gemm_pair.cuh"
+#include "gemm_stream.cuh"
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
 #include "tpb_api.h"
@@ -1181,6 +1182,7 @@ extern "C" int tpb_gemm_preload(void) {
   LOAD(64, 1, 2); LOAD(128, 1, 1); LOAD(256, 1, 1);
 #undef LOAD
   if (e == cudaSuccess) e = gemm_pair_preload();
+  if (e == cudaSuccess) e = gemm_stream_preload();
   return e == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
@@ -1294,6 +1296,8 @@ extern "C" int tpb_gemm_plan_ex(int tokens, int features, int k, int world, int 
   // Whole tiles of a many-token GEMM on one rank run on CTA pairs where that is faster (rule and figures: gemm_pair_tile);
   // split-K, the cross-rank sum and the fused all-gather (force_splits = 1) stay with the single-CTA kernel.
   plan->pair = (!plan->swapped && world == 1 && force_splits <= 0 && plan->k_splits == 1) ? gemm_pair_tile(tokens, features, sms) : 0;
+  // Few tokens on one rank: rows dealt out evenly to all SMs, no partial sums (gemm_stream_sm100.cu).
+  plan->stream = plan->swapped && world == 1 && force_splits <= 0 && force_kbox <= 0 && !plan->stream_k && gemm_stream_fits(features, k, sms);
   plan->tokens_pad = plan->swapped ? plan->n_tiles * bn : plan->m_tiles * BM;
   plan->slot_elems = size_t(tokens) * size_t(features);
   plan->tiles = tiles;
@@ -1358,10 +1362,11 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.act = act;
   p.bias_scale = bias_scale;
-  p.reduce = plan->reduce;
+  const bool streamed = plan->stream && !ag && !(rc && rc->world > 1);  // (whole rows per CTA: no partial sums, no workspace)
+  p.reduce = plan->reduce && !streamed;
   p.world = 1;
   p.rank = 0;
-  if (plan->reduce) {
+  if (p.reduce) {
     if (!rc || rc->world < 1 || rc->world > MAX_WORLD) return TPB_ERR_ARG;
     if (size_t(tokens) * size_t(act == 5 ? features : ld_out) > rc->slot_stride) return TPB_ERR_WORKSPACE;
     if (rc->world + plan->k_splits > rc->max_slots || plan->tiles > rc->max_tiles || !rc->split_counters) return TPB_ERR_WORKSPACE;
@@ -1423,6 +1428,22 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     g.status = p.status;
     g.out_elems = p.out_elems;
     return gemm_pair_launch(g, plan->pair, sm_count(), stream);
+  }
+
+  if (streamed) {
+    StreamGemm g;
+    g.x = x; g.w = w;
+    g.tokens = tokens; g.features = features; g.k = k; g.ldx = ldx; g.ldw = ldw;
+    g.out = p.out; g.ld_out = ld_out;
+    g.bias = p.bias; g.bias_scale = bias_scale;
+    g.residual = p.residual;
+    g.act = act;
+    g.norm_mode = p.norm_mode; g.norm_eps = p.norm_eps; g.norm_x = p.norm_x; g.norm_ld = p.norm_ld; g.norm_k = p.norm_k;
+    g.norm_rowsum = p.norm_rowsum;
+    g.early = opts ? opts->early : 0;
+    g.status = p.status;
+    g.out_elems = p.out_elems;
+    return gemm_stream_launch(g, sm_count(), stream);
   }
 
   const void* a_ptr = plan->swapped ? w : x;

@@ -1,7 +1,8 @@
 // Kernel launch helper.  With TPB_PDL=1 the decode-path kernels are launched with the programmatic-dependent-launch
 // attribute: between two dependent kernels of a CUDA graph lie about 3.7 us on B200 (measured with %globaltimer stamps
 // inside the kernels), part of it launch latency that a successor scheduled ahead of time hides.
-// Off by default.  Measured on one B200 with the per-rank shapes of a Llama-2-7B decode step: 2.35 vs 2.40 ms at
+// TPB_PDL is off by default (a decode step on one GPU asks for early launches by itself, kernel by kernel, see `early` in
+// gemm_stream_sm100.cu: those kernels fetch weights before the wait, which the figures below do not include).  Measured on one B200 with the per-rank shapes of a Llama-2-7B decode step: 2.35 vs 2.40 ms at
 // 8-way, 2.96 vs 3.09 ms at 4-way shard shapes, but 4.79 vs 3.91 ms at 2-way and 5.76 vs 5.65 ms unsharded.
 // Discipline of every such kernel: do the work that does not depend on earlier kernels (barrier init, TMEM
 // allocation), then griddepcontrol.wait, and only THEN griddepcontrol.launch_dependents.  A successor is scheduled
@@ -26,8 +27,10 @@ inline bool pdl_enabled() {
   return enabled == 1;
 }
 
+// `early`: set the attribute for this launch whatever TPB_PDL says (the caller vouches that the kernel reads nothing an earlier
+// kernel of the stream writes before its griddepcontrol.wait).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool early, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -37,8 +40,13 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_dependent(kernel, grid, block, smem, stream, pdl_enabled(), args...);
 }
 
 }  // namespace tpb

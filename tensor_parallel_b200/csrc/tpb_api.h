@@ -36,6 +36,7 @@ typedef struct {
   int stream_k;       // 1: the (tile, k-block) units are dealt out as one contiguous range per CTA; k_splits then is an
                       // upper bound of the CTAs that contribute to one tile
   int pair;           // columns of the CTA-pair tile (256 or 128) when the many-token pair kernel runs this shape, else 0
+  int stream;         // 1: the few-token weight-streaming kernel runs this shape (the tile fields then describe its fallback)
 } tpb_gemm_plan_t;
 
 // Workspace of the fused split-K / all-reduce epilogue.  All pointers are device pointers valid on the
@@ -83,6 +84,8 @@ typedef struct {
   const float* norm_rowsum;  // LayerNorm: fp32 [features], sum over k of w'[f, k]; the caller folds W beta into the bias
   double wait_seconds;       // bound of the waits for peer GPUs; <= 0: the library default (tpb_set_wait_limit)
   size_t out_elems;          // extent of `out` in elements, for the index checks of a -DTPB_BOUNDS build; 0: derived from the shape
+  int early;                 // launch as a programmatic dependent of the previous kernel of the stream and read w before that
+                             // kernel has finished (few-token streaming kernel only): w must not be an output of that kernel
 } tpb_gemm_opts_t;
 
 // 1 if this library was built with -DTPB_BOUNDS (kernels check their store indices and report STATUS_BAD_ARG = 3 in the

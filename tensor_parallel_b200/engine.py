@@ -311,11 +311,11 @@ class DecoderEngine:
 
     # -- building blocks --------------------------------------------------------------------------
 
-    def _row_parallel(self, x2d, weight, bias, residual_out):
+    def _row_parallel(self, x2d, weight, bias, residual_out, early=False):
         """``residual_out += all-reduce(x2d @ weight.T) + bias`` in place (``bias`` is the shard's copy, bias / world)."""
         tokens = x2d.shape[0]
         if self.world == 1:
-            native.gemm_nt(x2d, weight, bias=bias, residual=residual_out, out=residual_out)
+            native.gemm_nt(x2d, weight, bias=bias, residual=residual_out, out=residual_out, early=early)
         elif tokens <= 64 and self.comm.fits_fused(tokens, weight.shape[0], weight.shape[1]):
             self.comm.gemm_allreduce(x2d, weight, bias=bias, residual=residual_out, out=residual_out, bias_scale=float(self.world))
         else:
@@ -325,20 +325,24 @@ class DecoderEngine:
             if bias is not None:
                 residual_out.add_(bias * self.world)
 
-    def _projection(self, x, n, weight, bias, rowsum, out, act=None):
+    def _projection(self, x, n, weight, bias, rowsum, out, act=None, early=False):
         """``act(norm(x) @ weight.T + bias)`` where ``weight`` already carries the norm weight: for up to 64 tokens the
         GEMM normalises on the fly, otherwise ``n`` holds the rows normalised (without weight) by a kernel in front."""
         if n is None:
-            return native.gemm_nt(x, weight, bias=bias, act=act, out=out, norm=(self.mode, self.eps, rowsum))
+            return native.gemm_nt(x, weight, bias=bias, act=act, out=out, norm=(self.mode, self.eps, rowsum), early=early)
         return native.gemm_nt(n, weight, bias=bias, act=act, out=out)
 
     def _layer(self, i, x, n, qkv, q_rot, cat, act_buf, batch, seq, decode: bool):
         L = self.layers[i]
         D, spec = self.head_dim, self.spec
         fold = n is None
+        # A decode step on one GPU is a chain of kernels that each stream megabytes nothing in the chain writes (weights, older
+        # cache rows): every kernel may start while its predecessor drains and fetch those first.  With several ranks a
+        # predecessor may be waiting for a peer, and kernels parked behind it take the SMs it needs: not there.
+        early = decode and fold and self.world == 1
         if not fold:
             native.norm_forward(x, None, None, self.eps, self.mode - 1, out=n)
-        self._projection(x, n, L["wqkv"], L["bqkv"], L["sqkv"], qkv)
+        self._projection(x, n, L["wqkv"], L["bqkv"], L["sqkv"], qkv, early=early)
         nq_w, nk_w = self.nq * D, self.nkv * D
         q2, k2, v2 = qkv[:, :nq_w], qkv[:, nq_w : nq_w + nk_w], qkv[:, nq_w + nk_w :]
         attn = cat[:, :nq_w]
@@ -346,7 +350,7 @@ class DecoderEngine:
             # RoPE, cache append, split-KV attention and the split merge: one launch
             native.attn_decode_fused(q2, k2, v2, self.kcache[i][:batch], self.vcache[i][:batch], self.pos, spec.rotary_dim, self.theta,
                                      interleaved=spec.rope_interleaved, splits=self.splits, workspace=self.attn_ws,
-                                     out=attn, rope_angles=self.rope_angles)
+                                     out=attn, rope_angles=self.rope_angles, early=early)
         else:
             native.qkv_rope_append(q2, k2, v2, q_rot, self.kcache[i], self.vcache[i], self.pos, batch, seq, spec.rotary_dim, self.theta,
                                    interleaved=spec.rope_interleaved)
@@ -358,16 +362,16 @@ class DecoderEngine:
         if self.parallel:
             # the MLP reads the block input as well (through its own norm weights, folded into w1; the statistics are
             # the same rows'), and both partial results leave through one row-parallel GEMM
-            self._projection(x, n, L["w1"], L["b1"], L["s1"], cat[:, nq_w:], act=self.act)
-            self._row_parallel(cat, L["wcat"], L["bcat"], x)
+            self._projection(x, n, L["w1"], L["b1"], L["s1"], cat[:, nq_w:], act=self.act, early=early)
+            self._row_parallel(cat, L["wcat"], L["bcat"], x, early)
             return
-        self._row_parallel(attn, L["wo"], L["bo"], x)
+        self._row_parallel(attn, L["wo"], L["bo"], x, early)
         if not fold:
             native.norm_forward(x, None, None, self.eps, self.mode - 1, out=n)
-        self._projection(x, n, L["w1"], L["b1"], L["s1"], act_buf, act=self.act)
-        self._row_parallel(act_buf, L["wd"], L["bd"], x)
+        self._projection(x, n, L["w1"], L["b1"], L["s1"], act_buf, act=self.act, early=early)
+        self._row_parallel(act_buf, L["wd"], L["bd"], x, early)
 
-    def _head(self, x, logits_local, batch):
+    def _head(self, x, logits_local, batch, decode: bool = False):
         """Final norm + head on ``x [batch, hidden]``; returns full logits ``[batch, vocab]``."""
         n = None
         if batch > 64:  # too many rows for the in-kernel statistics
@@ -383,7 +387,7 @@ class DecoderEngine:
             if self.comm is None:  # (preload: this rank alone)
                 return logits_local[:batch]
             return self.comm.all_reduce(logits_local[:batch].contiguous())
-        self._projection(x, n, self.lm_head, self.head_bias, self.head_rowsum, logits_local)
+        self._projection(x, n, self.lm_head, self.head_bias, self.head_rowsum, logits_local, early=decode and self.world == 1)
         if self.world == 1:
             return logits_local[:batch]
         gathered = self.comm.all_gather(logits_local[:batch].contiguous())  # [world, batch, vocab_local]
@@ -529,7 +533,7 @@ class DecoderEngine:
         for i in range(len(self.layers)):
             self._layer(i, x, self.n[:batch] if batch > 64 else None, self.qkv[:batch], None, self.cat[:batch],
                         None if self.parallel else self.act_buf[:batch], batch, 1, decode=True)
-        logits = self._head(x, self.logits_local[:batch], batch)
+        logits = self._head(x, self.logits_local[:batch], batch, decode=True)
         torch.argmax(logits.float(), dim=-1, out=self.next_ids[:batch])
         self.ids[:batch].copy_(self.next_ids[:batch])
         self.pos.add_(1)

@@ -39,7 +39,7 @@ c_void_p, c_int, c_float, c_ll, c_size_t = ctypes.c_void_p, ctypes.c_int, ctypes
 class GemmPlan(ctypes.Structure):
     _fields_ = [("swapped", c_int), ("bn", c_int), ("kbox", c_int), ("m_tiles", c_int), ("n_tiles", c_int), ("k_blocks", c_int),
                 ("k_splits", c_int), ("kb_per_split", c_int), ("reduce", c_int), ("grid", c_int), ("tokens_pad", c_int),
-                ("tiles", c_int), ("slot_elems", c_size_t), ("stream_k", c_int), ("pair", c_int)]
+                ("tiles", c_int), ("slot_elems", c_size_t), ("stream_k", c_int), ("pair", c_int), ("stream", c_int)]
 
 
 class ReduceCtx(ctypes.Structure):
@@ -51,7 +51,7 @@ class ReduceCtx(ctypes.Structure):
 class GemmOpts(ctypes.Structure):
     _fields_ = [("x_mn", c_int), ("w_mn", c_int), ("norm_mode", c_int), ("norm_eps", c_float), ("norm_x", c_void_p),
                 ("norm_ld", c_ll), ("norm_k", c_int), ("norm_rowsum", c_void_p), ("wait_seconds", ctypes.c_double),
-                ("out_elems", c_size_t)]
+                ("out_elems", c_size_t), ("early", c_int)]
 
 
 def device_wait_seconds() -> float:
@@ -200,7 +200,7 @@ def gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
 def gemm_nt(x2d: torch.Tensor, w: torch.Tensor, bias=None, residual=None, act=None, out=None, force_splits: int = 0,
             reduce_ctx: Optional[ReduceCtx] = None, world: int = 1, bias_scale: float = 1.0, force_kbox: int = 0,
             x_t: bool = False, w_t: bool = False, norm: Optional[Tuple] = None, norm_rows: Optional[torch.Tensor] = None,
-            out_elems: int = 0) -> torch.Tensor:
+            out_elems: int = 0, early: bool = False) -> torch.Tensor:
     """``out[tokens, features] = act(x2d @ w.T + bias) + residual`` on the tcgen05 kernel.
 
     ``x_t`` / ``w_t``: the operand is passed transposed, ``x2d`` as ``[k, tokens]`` / ``w`` as ``[k, features]`` (row
@@ -209,7 +209,8 @@ def gemm_nt(x2d: torch.Tensor, w: torch.Tensor, bias=None, residual=None, act=No
     into the kernel (at most 64 tokens): ``w`` must already be multiplied by the norm weight along k.  ``norm_rows``
     ``[tokens, n]`` are the rows the statistics are taken over when ``x2d`` is only a column slice of them.
     ``out_elems`` (a library built with ``-DTPB_BOUNDS`` only): extent of ``out`` that the kernel checks its store
-    indices against; 0 derives it from the shape."""
+    indices against; 0 derives it from the shape.  ``early``: the kernel may start, and read ``w``, while the previous kernel
+    of the stream is still running (that kernel must not write ``w``); everything else is read after it."""
     global launch_count
     if x_t:
         k, tokens = x2d.shape
@@ -223,12 +224,13 @@ def gemm_nt(x2d: torch.Tensor, w: torch.Tensor, bias=None, residual=None, act=No
     state = device_state(x2d.device)
     ctx = reduce_ctx
     if ctx is None:
-        if plan.reduce:
+        if plan.reduce and not plan.stream:
             state.ensure_slots(tokens * (features if act == "swiglu16" else out.stride(0)))
         ctx = state.ctx
     opts = None
-    if x_t or w_t or norm is not None or out_elems:
+    if x_t or w_t or norm is not None or out_elems or early:
         opts = GemmOpts()
+        opts.early = int(early)
         opts.x_mn, opts.w_mn, opts.out_elems = int(x_t), int(w_t), int(out_elems)
         if norm is not None:
             mode, eps, rowsum = norm
@@ -689,7 +691,7 @@ def attn_decode(q, kcache, vcache, len_ptr, len_add, scale=None, splits=1, works
     return out
 
 
-LIB.tpb_attn_decode_fused.argtypes = [c_void_p] * 10 + [c_int] * 6 + [c_float, c_int, c_float, c_int, c_ll, c_ll, c_ll, c_void_p, c_ll, c_int, c_void_p]
+LIB.tpb_attn_decode_fused.argtypes = [c_void_p] * 10 + [c_int] * 6 + [c_float, c_int, c_float, c_int, c_ll, c_ll, c_ll, c_void_p, c_ll, c_int, c_int, c_void_p]
 LIB.tpb_rope_table.argtypes = [c_void_p, c_int, c_int, c_float, c_void_p]
 
 
@@ -704,11 +706,12 @@ def rope_table(positions: int, rotary_dim: int, theta: float, device) -> torch.T
 
 
 def attn_decode_fused(q, k, v, kcache, vcache, pos_ptr, rotary_dim, theta, interleaved=False, scale=None, splits=1,
-                      workspace=None, out=None, rope_angles=None):
+                      workspace=None, out=None, rope_angles=None, early=False):
     """One decode step of attention in a single launch: rotate q / k of the new token (``q/k/v``: 2-D row views of the
     projection output), append k, v to the cache at ``pos_ptr[0]``, attend over ``[0, pos]`` and merge the key splits.
     ``workspace = (part_o, part_ml, counters)`` with ``counters`` an int32 tensor of at least ``batch * kv_heads`` elements
-    zeroed once (``batch * q_heads``: all query-head groups of a KV head share one launch)."""
+    zeroed once (``batch * q_heads``: all query-head groups of a KV head share one launch).  ``early``: the kernel may start while
+    the previous kernel of the stream is still running and read ``pos_ptr`` and the cached rows, which that kernel must not write."""
     global launch_count
     d = kcache.shape[3]
     b, hq, hkv, smax = q.shape[0], q.shape[1] // d, kcache.shape[1], kcache.shape[2]
@@ -724,7 +727,7 @@ def attn_decode_fused(q, k, v, kcache, vcache, pos_ptr, rotary_dim, theta, inter
     check(LIB.tpb_attn_decode_fused(_ptr(q), _ptr(k), _ptr(v), _ptr(kcache), _ptr(vcache), _ptr(out), _ptr(part_o), _ptr(part_ml),
                                     _ptr(counters), _ptr(pos_ptr), b, hq, hkv, d, smax, splits, scale, rotary_dim, theta,
                                     int(interleaved), q.stride(0), k.stride(0), v.stride(0), _ptr(rope_angles),
-                                    out.stride(0) if out.stride(0) != hq * d else 0, 0 if counters is None else counters.numel(), _stream()),
+                                    out.stride(0) if out.stride(0) != hq * d else 0, 0 if counters is None else counters.numel(), int(early), _stream()),
           "tpb_attn_decode_fused")
     launch_count += LIB.tpb_last_launches()
     return out

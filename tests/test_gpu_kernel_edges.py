@@ -70,6 +70,67 @@ def test_pair_gemm_gated_into_a_wider_buffer(tokens):
     assert bool((wide[:, :16] == 7).all()) and bool((wide[:, 16 + f :] == 7).all())
 
 
+# one unit of 32 rows, a ragged last unit, one unit per SM, one CTA with two, more than one pass of 128 rows per CTA
+@pytest.mark.parametrize("features,k", [(32, 64), (40, 136), (1000, 520), (4736, 256), (4768, 1032), (4096, 4096), (22016, 264), (32003, 512)])
+@pytest.mark.parametrize("tokens", [1, 8, 17, 64])
+def test_streamed_few_token_gemm(tokens, features, k):
+    nat = _native()
+    torch.manual_seed(tokens + features)
+    assert nat.gemm_plan(tokens, features, k).stream
+    x = torch.randn(tokens, k, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(features, k, device="cuda", dtype=torch.bfloat16) / math.sqrt(k)
+    bias = torch.randn(features, device="cuda", dtype=torch.bfloat16)
+    res = torch.randn(tokens, features, device="cuda", dtype=torch.bfloat16)
+    _close(nat.gemm_nt(x, w, bias=bias, residual=res, act="relu"), _gemm_ref(x, w, bias, "relu", res), terms=8)
+    _close(nat.gemm_nt(x, w, act="gelu"), _gemm_ref(x, w, act="gelu"), terms=8)
+    if features % 32 == 0:
+        _close(nat.gemm_nt(x, w, bias=bias, act="swiglu16"), _gemm_ref(x, w, bias, "swiglu16"), terms=8)
+    nat.device_state(x.device).check_status()
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 40])
+def test_early_launch_reads_what_its_predecessor_wrote(tokens):
+    """A chain of dependent GEMMs launched ahead of one another gives the bits of the same chain in stream order."""
+    nat = _native()
+    torch.manual_seed(tokens)
+    widths = [512, 4096, 1376, 4768, 512]
+    ws = [torch.randn(b, a, device="cuda", dtype=torch.bfloat16) / math.sqrt(a) for a, b in zip(widths, widths[1:])]
+    x0 = torch.randn(tokens, widths[0], device="cuda", dtype=torch.bfloat16)
+
+    def chain(early):
+        x = x0
+        for _ in range(3):
+            for w in ws:
+                x = nat.gemm_nt(x, w, act="gelu", norm=(1, 1e-6, None), early=early)
+        return x
+
+    want = chain(False)
+    for _ in range(5):
+        assert torch.equal(chain(True), want)
+
+
+@pytest.mark.parametrize("hq,hkv,d,splits", [(8, 8, 128, 1), (8, 2, 64, 4), (12, 2, 128, 2)])
+def test_early_decode_attention_follows_the_projection(hq, hkv, d, splits):
+    nat = _native()
+    torch.manual_seed(hq)
+    b, smax, hidden = 3, 320, 256
+    x = torch.randn(b, hidden, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn((hq + 2 * hkv) * d, hidden, device="cuda", dtype=torch.bfloat16) / 16
+    kc, vc = (torch.randn(b, hkv, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    for pos in (0, 1, 31, 250, smax - 1):
+        at = torch.tensor([pos], device="cuda", dtype=torch.int32)
+        torch.cuda.synchronize()
+        outs = []
+        for early in (False, True, True):
+            k2, v2 = kc.clone(), vc.clone()
+            qkv = torch.zeros(b, w.shape[0], device="cuda", dtype=torch.bfloat16)
+            nat.gemm_nt(x, w, out=qkv, early=early)
+            q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+            outs.append((nat.attn_decode_fused(q, k, v, k2, v2, at, d, 10000.0, splits=splits, early=early), k2, v2))
+        for other in outs[1:]:
+            assert all(torch.equal(a, o) for a, o in zip(outs[0], other))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (2, 2048), (295, 2056), (297, 4096), (700, 5120), (61, 8192)])
 @pytest.mark.parametrize("mode", ["rms", "layer"])
