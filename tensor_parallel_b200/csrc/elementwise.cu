@@ -765,3 +765,70 @@ extern "C" int tpb_transpose_bf16(const void* in, void* out, int rows, int cols,
       static_cast<const tpb::bf16*>(in), static_cast<tpb::bf16*>(out), rows, cols, in_ld, out_ld);
   TPB_CHECK_LAUNCH();
 }
+
+// ------------------------------------------------------------------------------------------------
+// End of a greedy decode step in one launch: ids[b] = next_ids[b] = argmax of logits row b (the first one of equal values, a NaN
+// above everything, like torch.argmax), pos[0] += 1.  One CTA per row; a row of 32000 logits is 64 KB, so the time is launch
+// latency plus about one microsecond - as separate cast, argmax, copy and add kernels it was four launches.
+// ------------------------------------------------------------------------------------------------
+namespace tpb {
+constexpr int PICK_THREADS = 512;
+struct Best { float v; int i; };
+__device__ __forceinline__ bool beats(const Best& a, const Best& b) {  // a comes before b in the order of torch.argmax
+  const bool an = a.v != a.v, bn = b.v != b.v;
+  if (an != bn) return an;
+  if (an || a.v == b.v) return a.i < b.i;
+  return a.v > b.v;
+}
+__global__ void __launch_bounds__(PICK_THREADS)
+greedy_pick_kernel(const bf16* __restrict__ logits, long long ld, int cols, int64_t* __restrict__ next_ids, int64_t* __restrict__ ids,
+                   int* __restrict__ pos) {
+  __shared__ Best red[PICK_THREADS / 32];
+  pdl_wait();
+  const bf16* x = logits + blockIdx.x * ld;
+  const int head = min(cols, int((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / 2), tail = head + (cols - head) / 8 * 8;
+  Best best = {-INFINITY, cols};  // (loses against every element)
+#pragma unroll 4
+  for (int c = head + int(threadIdx.x) * 8; c < tail; c += PICK_THREADS * 8) {
+    float v[8];
+    Vec8<bf16>::load(x + c, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const Best cand = {v[j], c + j};
+      if (beats(cand, best)) best = cand;
+    }
+  }
+  const int edge = head + cols - tail;  // at most 14 elements outside the 16-byte vectors
+  if (int(threadIdx.x) < edge) {
+    const int c = int(threadIdx.x) < head ? int(threadIdx.x) : tail + int(threadIdx.x) - head;
+    const Best cand = {to_f<bf16>(x[c]), c};
+    if (beats(cand, best)) best = cand;
+  }
+  auto merge = [&]() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const Best other = {__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+      if (beats(other, best)) best = other;
+    }
+  };
+  merge();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = threadIdx.x < PICK_THREADS / 32 ? red[threadIdx.x] : Best{-INFINITY, cols};
+    merge();
+    if (threadIdx.x == 0) {
+      next_ids[blockIdx.x] = best.i;
+      ids[blockIdx.x] = best.i;
+      if (blockIdx.x == 0) pos[0] += 1;
+    }
+  }
+}
+}  // namespace tpb
+
+// early: launch as a programmatic dependent (the kernel reads nothing before the previous kernel of the stream is complete).
+extern "C" int tpb_greedy_pick(const void* logits, long long ld, int rows, int cols, int64_t* next_ids, int64_t* ids, int* pos, int early, void* stream_) {
+  if (!logits || !next_ids || !ids || !pos || rows <= 0 || cols <= 0 || ld < cols) return TPB_ERR_ARG;
+  return launch_dependent(tpb::greedy_pick_kernel, dim3(rows), dim3(tpb::PICK_THREADS), 0, static_cast<cudaStream_t>(stream_), early != 0 || pdl_enabled(),
+                          static_cast<const tpb::bf16*>(logits), ld, cols, next_ids, ids, pos) == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
+}

@@ -534,9 +534,7 @@ class DecoderEngine:
             self._layer(i, x, self.n[:batch] if batch > 64 else None, self.qkv[:batch], None, self.cat[:batch],
                         None if self.parallel else self.act_buf[:batch], batch, 1, decode=True)
         logits = self._head(x, self.logits_local[:batch], batch, decode=True)
-        torch.argmax(logits.float(), dim=-1, out=self.next_ids[:batch])
-        self.ids[:batch].copy_(self.next_ids[:batch])
-        self.pos.add_(1)
+        native.greedy_pick(logits, self.next_ids[:batch], self.ids[:batch], self.pos, early=self.world == 1)
         self.kernels_per_step = native.launch_count - before
 
     @traced("tpb.engine.decode_step")

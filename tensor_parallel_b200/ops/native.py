@@ -807,6 +807,19 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, out=None):
     return out.view(*ids.shape, cols) if out.shape[0] == flat.numel() and out.is_contiguous() else out
 
 
+LIB.tpb_greedy_pick.argtypes = [c_void_p, c_ll, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
+
+
+def greedy_pick(logits: torch.Tensor, next_ids: torch.Tensor, ids: torch.Tensor, pos: torch.Tensor, early: bool = False):
+    """End of a greedy decode step in one launch: ``next_ids[:] = ids[:] = logits.argmax(-1)`` (bf16 ``[rows, cols]``, ties and
+    NaN like ``torch.argmax``; int64 ids), ``pos[0] += 1`` (int32).  ``early``: see :func:`gemm_nt`."""
+    global launch_count
+    rows, cols = logits.shape
+    check(LIB.tpb_greedy_pick(_ptr(logits), logits.stride(0), rows, cols, _ptr(next_ids), _ptr(ids), _ptr(pos), int(early), _stream()),
+          "tpb_greedy_pick")
+    launch_count += 1
+
+
 def adamw_step(param, grad, exp_avg, exp_avg_sq, step, lr, beta1, beta2, eps, weight_decay, master=None, grad_scale=1.0):
     global launch_count
     check(LIB.tpb_adamw(_ptr(param), _ptr(grad), _ptr(exp_avg), _ptr(exp_avg_sq), _ptr(master), param.numel(), lr, beta1, beta2, eps,

@@ -39,6 +39,10 @@ def _gemm_ref(x, w, bias=None, act=None, residual=None):
     return y if residual is None else y + residual.double()
 
 
+# tokens, features, k: whole pair tiles, one row / column / k-block more and less, a ragged last band of token tiles, an odd pitch
+PAIR = [(2560, 2048, 256), (2561, 2047, 200), (4000, 1288, 72), (2303, 4100, 136), (8192, 384, 64), (5000, 1000, 1032)]
+
+
 @pytest.mark.parametrize("tokens,features,k", PAIR)
 @pytest.mark.parametrize("x_t,w_t", [(False, False), (False, True), (True, True)])
 def test_pair_gemm(tokens, features, k, x_t, w_t):
@@ -225,6 +229,24 @@ def test_adamw_remainders_and_alignment(n, offset, dtype, gdtype):
         assert (got.double() - ref).abs().max().item() <= 2e-6  # a few fp32 roundings of values below 1 (1 - 0.99f is 1e-6 off)
     if master is not None:
         assert torch.equal(p, master.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("cols", [1, 5, 8, 515, 32000, 50257])
+def test_greedy_pick_matches_torch_argmax(cols):
+    nat = _native()
+    torch.manual_seed(cols)
+    rows = 9
+    logits = torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16)  # bf16: ties are common
+    logits[1] = 0.25
+    logits[2] = -math.inf
+    logits[3, cols // 2] = math.nan
+    logits[4, cols // 3 :] = math.nan
+    logits[5, -1] = 1000.0
+    nxt, ids = torch.zeros(rows, dtype=torch.int64, device="cuda"), torch.zeros(rows, dtype=torch.int64, device="cuda")
+    pos = torch.tensor([41], dtype=torch.int32, device="cuda")
+    nat.greedy_pick(logits, nxt, ids, pos)
+    want = logits.cpu().float().argmax(-1)
+    assert torch.equal(nxt.cpu(), want) and torch.equal(ids, nxt) and pos.item() == 42
 
 
 @pytest.mark.parametrize("sq,sk", [(64, 128), (150, 152), (150, 150), (300, 520)])
