@@ -36,6 +36,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "attention_sm100.cuh"
 #include "ptx_sm100.cuh"
@@ -49,6 +50,7 @@ constexpr int BW_R = 128;      // resident rows = TMEM lanes
 constexpr int BW_T = 64;       // streamed rows per step = TMEM columns of one score buffer
 constexpr int BW_STAGES = 3;
 constexpr int BW_THREADS = 320;
+constexpr int BW_BIAS_BYTES = BW_R * BW_T * 2;  // bias elements of one step
 constexpr int BW_T_BLOCK_BYTES = BW_T * 128;  // one [64 rows][64 elements] swizzled block
 
 struct BwParams {
@@ -69,10 +71,15 @@ struct BwParams {
   uint32_t* status;
 };
 
-template <int D, bool DKV, bool BIAS>  // BIAS: the score-bias code exists only in the instantiations that need it
+// BIAS: the score-bias code exists only in the instantiations that need it.  1: elements are loaded by the threads that use them;
+// 2: a dense bf16 bias whose rows TMA can address travels with the streamed tiles, [64 queries][128 keys] (dK / dV) or
+// [128 queries][64 keys] (dQ) per step, so that no elementwise warp ever waits for a global load (16 x 512 tokens, 32 heads of 64,
+// one bias for all batches: dK / dV 1093 -> 205 us, dQ 316 -> 231 us).
+template <int D, bool DKV, int BIAS>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_constant__ CUtensorMap tmap_r2,
-                        const __grid_constant__ CUtensorMap tmap_t1, const __grid_constant__ CUtensorMap tmap_t2, const BwParams p) {
+                        const __grid_constant__ CUtensorMap tmap_t1, const __grid_constant__ CUtensorMap tmap_t2,
+                        const __grid_constant__ CUtensorMap tmap_b, const BwParams p) {
   constexpr int DB = D / 64;
   constexpr uint32_t R_BYTES = DB * FA_BLOCK_BYTES;    // one resident tile (128 rows)
   constexpr uint32_t T_BYTES = DB * BW_T_BLOCK_BYTES;  // one streamed tile (64 rows)
@@ -87,9 +94,11 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   uint8_t* r2_s = r1_s + R_BYTES;
   uint8_t* t1_s = r2_s + R_BYTES;              // [stages]
   uint8_t* t2_s = t1_s + BW_STAGES * T_BYTES;  // [stages]
-  float* lse_s = reinterpret_cast<float*>(t2_s + BW_STAGES * T_BYTES);  // [stages][64]: lse * log2(e), +inf = no such query
-  float* del_s = lse_s + BW_STAGES * BW_T;                              // [stages][64]: delta * scale
-  uint64_t* bars = reinterpret_cast<uint64_t*>(del_s + BW_STAGES * BW_T);
+  // [stages][32 pairs of streamed queries]: {-lse * log2(e) of both (-inf = no such query), -delta * scale of both}
+  float4* stat_s = reinterpret_cast<float4*>(t2_s + BW_STAGES * T_BYTES);
+  uint8_t* bias_s = reinterpret_cast<uint8_t*>(t2_s + BW_STAGES * T_BYTES);  // [stages], BIAS == 2 only (1024-byte aligned for the swizzle)
+  if (BIAS == 2) stat_s = reinterpret_cast<float4*>(bias_s + BW_STAGES * BW_BIAS_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + BW_STAGES * BW_T / 2);
   uint64_t* r_full = bars;
   uint64_t* t_full = bars + 1;                   // [stages]
   uint64_t* t_empty = bars + 1 + BW_STAGES;      // [stages]
@@ -99,7 +108,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be uniform)
   const int b = blockIdx.z;
   const int shift = p.sk - p.sq;  // query i may see keys j <= i + shift when causal
   const int group = p.q_heads / p.kv_heads;
@@ -179,7 +188,9 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         const int row0 = (step0 + (DKV ? n - g * per_head : n)) * BW_T;  // first streamed row of the step
         const int t_head = DKV ? head + g : kvh;
         if (lane == 0) {
-          mbar_expect_tx(&t_full[s], 2 * T_BYTES);
+          mbar_expect_tx(&t_full[s], 2 * T_BYTES + (BIAS == 2 ? BW_BIAS_BYTES : 0));
+          if (BIAS == 2)
+            tma_load_4d(bias_s + s * BW_BIAS_BYTES, &tmap_b, &t_full[s], DKV ? r0 : row0, DKV ? row0 : r0, p.b_sh ? (DKV ? t_head : head) : 0, p.b_sb ? b : 0);
 #pragma unroll
           for (int d = 0; d < DB; ++d) {
             tma_load_4d(t1_s + s * T_BYTES + d * BW_T_BLOCK_BYTES, &tmap_t1, &t_full[s], d * 64, row0, t_head, b);
@@ -190,15 +201,16 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 #pragma unroll
           for (int c = lane; c < BW_T; c += 32) {
             const int qi = row0 + c;
-            float l2 = INFINITY, dl = 0.f;
+            float l2 = -INFINITY, dl = 0.f;
             if (qi < p.sq) {
               const long long idx = ((long long)b * p.q_heads + t_head) * p.sq + qi;
               const float l = __ldg(p.lse + idx);
-              if (l != -INFINITY) l2 = l * 1.4426950408889634f;  // (a query without a visible key has P = 0 everywhere)
-              dl = __ldg(p.delta + idx) * p.scale;
+              if (l != -INFINITY) l2 = -l * 1.4426950408889634f;  // (a query without a visible key has P = 0 everywhere)
+              dl = -__ldg(p.delta + idx) * p.scale;
             }
-            lse_s[s * BW_T + c] = l2;
-            del_s[s * BW_T + c] = dl;
+            float* pair = reinterpret_cast<float*>(stat_s + s * (BW_T / 2) + (c >> 1)) + (c & 1);
+            pair[0] = l2;
+            pair[2] = dl;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&t_full[s]);
@@ -206,65 +218,67 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (elect_one() && n_steps > 0) {
-      const uint32_t r1_addr = smem_u32(r1_s), r2_addr = smem_u32(r2_s);
+    // ---------------- MMA issuer (the warp stays together, one lane issues: see umma_bf16_lead) ----------------
+    if (n_steps > 0) {
+      const uint32_t leader = elect_one();
+      const uint32_t r1_lo = desc_kmajor_lo(smem_u32(r1_s)), r2_lo = desc_kmajor_lo(smem_u32(r2_s));
       auto issue_scores = [&](int n) {  // S[n & 1] = R1 T1(n)^T, dP[n & 1] = R2 T2(n)^T
         const int s = n % BW_STAGES, buf = n & 1;
-        const uint32_t t1_addr = smem_u32(t1_s + s * T_BYTES), t2_addr = smem_u32(t2_s + s * T_BYTES);
+        const uint32_t t1_lo = desc_kmajor_lo(smem_u32(t1_s + s * T_BYTES)), t2_lo = desc_kmajor_lo(smem_u32(t2_s + s * T_BYTES));
 #pragma unroll
         for (int d = 0; d < DB; ++d) {
 #pragma unroll
-          for (int kk = 0; kk < 64 / 16; ++kk) {
-            umma_bf16(tmem_base + S_COL0 + buf * BW_T, make_desc_kmajor_sw128(r1_addr + d * FA_BLOCK_BYTES + kk * 32),
-                      make_desc_kmajor_sw128(t1_addr + d * BW_T_BLOCK_BYTES + kk * 32), IDESC_S, (d | kk) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < 64 / 16; ++kk)
+            umma_bf16_lead(leader, tmem_base + S_COL0 + buf * BW_T, r1_lo + d * (FA_BLOCK_BYTES >> 4) + kk * 2,
+                           t1_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
         }
 #pragma unroll
         for (int d = 0; d < DB; ++d) {
 #pragma unroll
-          for (int kk = 0; kk < 64 / 16; ++kk) {
-            umma_bf16(tmem_base + DP_COL0 + buf * BW_T, make_desc_kmajor_sw128(r2_addr + d * FA_BLOCK_BYTES + kk * 32),
-                      make_desc_kmajor_sw128(t2_addr + d * BW_T_BLOCK_BYTES + kk * 32), IDESC_S, (d | kk) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < 64 / 16; ++kk)
+            umma_bf16_lead(leader, tmem_base + DP_COL0 + buf * BW_T, r2_lo + d * (FA_BLOCK_BYTES >> 4) + kk * 2,
+                           t2_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
         }
-        umma_commit(&s_full[buf]);
+        umma_commit_lead(leader, &s_full[buf]);
       };
       auto issue_accumulate = [&](int n) {
         const int s = n % BW_STAGES, buf = n & 1;
-        const uint32_t t1_addr = smem_u32(t1_s + s * T_BYTES), t2_addr = smem_u32(t2_s + s * T_BYTES);
+        const uint32_t t1_lo = desc_mnmajor_lo(smem_u32(t1_s + s * T_BYTES), BW_T_BLOCK_BYTES);
+        const uint32_t t2_lo = desc_mnmajor_lo(smem_u32(t2_s + s * T_BYTES), BW_T_BLOCK_BYTES);
 #pragma unroll
         for (int kk = 0; kk < BW_T / 16; ++kk) {
           // the bf16 operand of the 16 streamed rows kk: written by the thread that owns their column half, inside that half
           const uint32_t a_col = (kk >> 1) * 32 + (kk & 1) * 8;
           if (DKV)  // dV += P^T dO
-            umma_bf16_tmem_a(tmem_base + ACC1_COL, tmem_base + S_COL0 + buf * BW_T + a_col,
-                             make_desc_mnmajor_sw128(t2_addr + kk * 16 * 128, BW_T_BLOCK_BYTES), IDESC_ACC, (n | kk) ? 1u : 0u);
+            umma_bf16_tmem_a_lead(leader, tmem_base + ACC1_COL, tmem_base + S_COL0 + buf * BW_T + a_col, t2_lo + kk * (16 * 128 >> 4), IDESC_ACC,
+                                  (n | kk) ? 1u : 0u);
           // dK += dS^T Q   or   dQ += dS K
-          umma_bf16_tmem_a(tmem_base + ACC0_COL, tmem_base + DP_COL0 + buf * BW_T + a_col,
-                           make_desc_mnmajor_sw128(t1_addr + kk * 16 * 128, BW_T_BLOCK_BYTES), IDESC_ACC, (n | kk) ? 1u : 0u);
+          umma_bf16_tmem_a_lead(leader, tmem_base + ACC0_COL, tmem_base + DP_COL0 + buf * BW_T + a_col, t1_lo + kk * (16 * 128 >> 4), IDESC_ACC,
+                                (n | kk) ? 1u : 0u);
         }
       };
-      bool ok = mbar_wait(r_full, 0) && mbar_wait(&t_full[0], 0);
-      if (!ok) give_up(STATUS_TIMEOUT_MBAR);
-      if (ok) {
+      auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+        const bool there = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+        if (!there && leader) give_up(STATUS_TIMEOUT_MBAR);
         tc_fence_after();
-        issue_scores(0);
-      }
-      for (int n = 0; ok && n < n_steps && !*abort_flag; ++n) {
+        return there;
+      };
+      bool ok = wait_all(r_full, 0) && wait_all(&t_full[0], 0);
+      if (ok) issue_scores(0);
+      for (int n = 0; ok && n < n_steps; ++n) {
         if (n + 1 < n_steps) {
           // scores of the next step: their TMEM buffer was last read by the accumulate MMAs of step n - 1 (issued
           // before these) and by the elementwise warps of step n - 1 (who delivered before those were issued)
-          if (!mbar_wait(&t_full[(n + 1) % BW_STAGES], ((n + 1) / BW_STAGES) & 1)) { give_up(STATUS_TIMEOUT_MBAR); break; }
-          tc_fence_after();
+          ok = wait_all(&t_full[(n + 1) % BW_STAGES], ((n + 1) / BW_STAGES) & 1);
+          if (!ok) break;
           issue_scores(n + 1);
         }
-        if (!mbar_wait(&p_full[n & 1], (n >> 1) & 1)) { give_up(STATUS_TIMEOUT_MBAR); break; }
-        tc_fence_after();
+        ok = wait_all(&p_full[n & 1], (n >> 1) & 1);
+        if (!ok) break;
         issue_accumulate(n);
-        umma_commit(&t_empty[n % BW_STAGES]);  // the streamed tiles of step n may be overwritten once these MMAs retire
+        umma_commit_lead(leader, &t_empty[n % BW_STAGES]);  // the streamed tiles of step n may be overwritten once these MMAs retire
       }
-      umma_commit(acc_full);
+      umma_commit_lead(leader, acc_full);
     }
   } else {
     // ---------------- elementwise warps ----------------
@@ -275,18 +289,18 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
     const int row = quarter * 32 + lane;
     const int ri = r0 + row;  // key (DKV) or query
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
-    float my_lse2 = INFINITY, my_del = 0.f;
+    float my_lse2 = -INFINITY, my_del = 0.f;  // negated
     if (!DKV && ri < p.sq) {
       const long long idx = ((long long)b * p.q_heads + head) * p.sq + ri;
       const float l = __ldg(p.lse + idx);
-      if (l != -INFINITY) my_lse2 = l * 1.4426950408889634f;
-      my_del = __ldg(p.delta + idx) * p.scale;
+      if (l != -INFINITY) my_lse2 = -l * 1.4426950408889634f;
+      my_del = -__ldg(p.delta + idx) * p.scale;
     }
     bool alive = true;
 
     for (int n = 0; n < n_steps; ++n) {
       const int s = n % BW_STAGES, buf = n & 1;
-      if (*abort_flag || (DKV && !mbar_wait(&t_full[s], (n / BW_STAGES) & 1)) || !mbar_wait(&s_full[buf], (n >> 1) & 1)) {
+      if (*abort_flag || ((DKV || BIAS == 2) && !mbar_wait(&t_full[s], (n / BW_STAGES) & 1)) || !mbar_wait(&s_full[buf], (n >> 1) & 1)) {
         if (!*abort_flag) give_up(STATUS_TIMEOUT_MBAR);
         alive = false;
         break;
@@ -306,7 +320,11 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       } else {
         hi = min(HC, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
       }
-      const bool masked = lo > 0 || hi < HC;
+      // ... as bits; only steps that touch the diagonal or an end have any cleared (decided per warp: the common loop has no masks)
+      uint32_t visible = 0xffffffffu;
+      if (lo > 0) visible = lo < HC ? visible << lo : 0u;
+      if (hi < HC) visible = hi > 0 ? visible & (0xffffffffu >> (HC - hi)) : 0u;
+      const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);
       // score bias: element (query, key) = (col0 + c, ri) for dK / dV - there the lanes of a warp own consecutive keys - and
       // (ri, col0 + c) for dQ, where a thread's columns are consecutive keys of one row and are read eight at a time
       const int b_head = DKV ? head + g : head;
@@ -315,53 +333,73 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       const int col_limit = DKV ? p.sq : p.sk, row_limit = DKV ? p.sk : p.sq;
       uint32_t pp[HC / 2], ds[HC / 2];
       float bv[8], db[4];
+      auto pairs = [&](auto with_masks) {
+        constexpr bool MASKED = decltype(with_masks)::value;
 #pragma unroll
-      for (int c = 0; c < HC; c += 2) {
-        float l0, l1, d0, d1;
-        if (DKV) {
-          const float2 l = *reinterpret_cast<const float2*>(lse_s + s * BW_T + half * HC + c);
-          const float2 d = *reinterpret_cast<const float2*>(del_s + s * BW_T + half * HC + c);
-          l0 = l.x; l1 = l.y; d0 = d.x; d1 = d.y;
-        } else {
-          l0 = l1 = my_lse2;
-          d0 = d1 = my_del;
-        }
-        if (BIAS && (c & 7) == 0)
-          load_bias8(p.bias, p.bias_kind, bias_base + (long long)(col0 + c) * bias_step, bias_step, ri < row_limit ? col_limit - col0 - c : 0,
-                     !DKV && p.bias_vec, bv);
-        float x0, x1, p0, p1, g0, g1;
-        ffma2(x0, x1, __uint_as_float(sv[c]), __uint_as_float(sv[c + 1]), p.scale_log2e, p.scale_log2e, -l0, -l1);
-        if (BIAS) {
-          x0 += bv[c & 7] * 1.4426950408889634f;
-          x1 += bv[(c & 7) + 1] * 1.4426950408889634f;
-        }
-        p0 = ex2_approx(x0);
-        p1 = ex2_approx(x1);
-        if (masked) {
-          if (c < lo || c >= hi) p0 = 0.f;
-          if (c + 1 < lo || c + 1 >= hi) p1 = 0.f;
-        }
-        ffma2(g0, g1, __uint_as_float(dv[c]), __uint_as_float(dv[c + 1]), p.scale, p.scale, -d0, -d1);  // (dP - delta) * scale
-        ffma2(g0, g1, g0, g1, p0, p1, 0.f, 0.f);
-        if (BIAS && !DKV && p.dbias) {  // d(bias) = P (dP - delta) = dS / scale; pairs that are masked or out of range contribute nothing
-          db[c & 3] = p0 != 0.f ? g0 * p.inv_scale : 0.f;
-          db[(c & 3) + 1] = p1 != 0.f ? g1 * p.inv_scale : 0.f;
-          if ((c & 3) == 2 && ri < row_limit) {
-            const int c4 = c - 2;
-            float* dst = p.dbias + bias_base + (long long)(col0 + c4) * bias_step;
-            if (p.bias_vec && col0 + c4 + 4 <= col_limit) {
-              // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
-            } else {
+        for (int c = 0; c < HC; c += 2) {
+          float l0, l1, d0, d1;
+          if (DKV) {
+            const float4 st = stat_s[s * (BW_T / 2) + ((half * HC + c) >> 1)];
+            l0 = st.x; l1 = st.y; d0 = st.z; d1 = st.w;
+          } else {
+            l0 = l1 = my_lse2;
+            d0 = d1 = my_del;
+          }
+          if (BIAS == 2 && (c & 7) == 0) {
+            const uint8_t* tile = bias_s + s * BW_BIAS_BYTES;
+            if (DKV) {  // column = query row of the tile, lanes read consecutive keys
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (db[i] != 0.f && col0 + c4 + i < col_limit) atomicAdd(dst + i * bias_step, db[i]);
+              for (int i = 0; i < 8; ++i)
+                bv[i] = __bfloat162float(*reinterpret_cast<const bf16*>(tile + (half * HC + c + i) * (BW_R * 2) + row * 2));
+            } else {  // eight keys of this thread's query: one swizzled 16-byte chunk
+              const uint4 u = *reinterpret_cast<const uint4*>(tile + row * 128 + ((((half * HC + c) >> 3) ^ (row & 7)) << 4));
+              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                bv[2 * i] = __uint_as_float(w[i] << 16);
+                bv[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+              }
             }
           }
+          if (BIAS == 1 && (c & 7) == 0)
+            load_bias8(p.bias, p.bias_kind, bias_base + (long long)(col0 + c) * bias_step, bias_step, ri < row_limit ? col_limit - col0 - c : 0,
+                       !DKV && p.bias_vec, bv);
+          float x0, x1, p0, p1, g0, g1;
+          ffma2(x0, x1, __uint_as_float(sv[c]), __uint_as_float(sv[c + 1]), p.scale_log2e, p.scale_log2e, l0, l1);
+          if (BIAS) {
+            x0 += bv[c & 7] * 1.4426950408889634f;
+            x1 += bv[(c & 7) + 1] * 1.4426950408889634f;
+          }
+          p0 = ex2_approx(x0);
+          p1 = ex2_approx(x1);
+          if (MASKED) {
+            if (!(visible >> c & 1)) p0 = 0.f;
+            if (!(visible >> (c + 1) & 1)) p1 = 0.f;
+          }
+          ffma2(g0, g1, __uint_as_float(dv[c]), __uint_as_float(dv[c + 1]), p.scale, p.scale, d0, d1);  // (dP - delta) * scale
+          ffma2(g0, g1, g0, g1, p0, p1, 0.f, 0.f);
+          if (BIAS && !DKV && p.dbias) {  // d(bias) = P (dP - delta) = dS / scale; pairs that are masked or out of range contribute nothing
+            db[c & 3] = p0 != 0.f ? g0 * p.inv_scale : 0.f;
+            db[(c & 3) + 1] = p1 != 0.f ? g1 * p.inv_scale : 0.f;
+            if ((c & 3) == 2 && ri < row_limit) {
+              const int c4 = c - 2;
+              float* dst = p.dbias + bias_base + (long long)(col0 + c4) * bias_step;
+              if (p.bias_vec && col0 + c4 + 4 <= col_limit) {
+                // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
+              } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (db[i] != 0.f && col0 + c4 + i < col_limit) atomicAdd(dst + i * bias_step, db[i]);
+              }
+            }
+          }
+          if (DKV) pp[c >> 1] = pack_bf16x2(p0, p1);
+          ds[c >> 1] = pack_bf16x2(g0, g1);
         }
-        if (DKV) pp[c >> 1] = pack_bf16x2(p0, p1);
-        ds[c >> 1] = pack_bf16x2(g0, g1);
-      }
+      };
+      if (masked) pairs(std::true_type{});
+      else pairs(std::false_type{});
       // bf16 pairs over the first 16 columns of this thread's own half (nobody else reads or writes those)
       if (DKV) tmem_st_x16(t_lane + S_COL0 + buf * BW_T + half * HC, pp);
       tmem_st_x16(t_lane + DP_COL0 + buf * BW_T + half * HC, ds);
@@ -426,10 +464,11 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-template <int D, bool DKV, bool BIAS>
-static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const BwParams& p, dim3 grid,
-                     cudaStream_t stream) {
-  constexpr size_t smem = size_t(D / 64) * (2 * FA_BLOCK_BYTES + 2 * BW_STAGES * BW_T_BLOCK_BYTES) + 2 * BW_STAGES * BW_T * sizeof(float) + 1024 + 256;
+template <int D, bool DKV, int BIAS>
+static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& tb, const BwParams& p,
+                     dim3 grid, cudaStream_t stream) {
+  constexpr size_t smem = size_t(D / 64) * (2 * FA_BLOCK_BYTES + 2 * BW_STAGES * BW_T_BLOCK_BYTES) + (BIAS == 2 ? BW_STAGES * BW_BIAS_BYTES : 0) +
+                          2 * BW_STAGES * BW_T * sizeof(float) + 1024 + 256;
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
@@ -438,8 +477,23 @@ static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtenso
       return TPB_ERR_CUDA;
     configured[dev].store(true, std::memory_order_release);
   }
-  attn_bwd_tcgen05_kernel<D, DKV, BIAS><<<grid, BW_THREADS, smem, stream>>>(r1, r2, t1, t2, p);
+  attn_bwd_tcgen05_kernel<D, DKV, BIAS><<<grid, BW_THREADS, smem, stream>>>(r1, r2, t1, t2, tb, p);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
+}
+
+// Tensor map over a bf16 score bias [batch or 1][heads or 1][sq][sk] (keys contiguous); box = [rows queries][keys].
+static int bw_bias_tmap(CUtensorMap* map, const void* bias, int batch, int heads, int sq, int sk, long long sb, long long sh, long long sqs, int rows,
+                        int keys, bool swizzled) {
+  EncodeTiledFn fn = fa_encode_fn();
+  if (!fn) return TPB_ERR_DRIVER;
+  cuuint64_t dims[4] = {cuuint64_t(sk), cuuint64_t(sq), cuuint64_t(sh ? heads : 1), cuuint64_t(sb ? batch : 1)};
+  cuuint64_t strides[3] = {cuuint64_t(sqs) * 2, cuuint64_t(sh ? sh : sqs) * 2, cuuint64_t(sb ? sb : sqs) * 2};
+  cuuint32_t box[4] = {cuuint32_t(keys), cuuint32_t(rows), 1, 1}, estr[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(bias), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? TPB_OK
+             : TPB_ERR_TMAP;
 }
 
 }  // namespace tpb
@@ -501,17 +555,28 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   p.out0 = static_cast<bf16*>(dk); p.o0_sb = dk_sb; p.o0_ss = dk_ss; p.o0_sh = dk_sh;
   p.out1 = static_cast<bf16*>(dv); p.o1_sb = dk_sb; p.o1_ss = dk_ss; p.o1_sh = dk_sh;
   dim3 grid_kv((sk + BW_R - 1) / BW_R, kv_heads, batch);
-  const bool with_bias = bias != nullptr;
-  if (head_dim == 128)
-    rc = with_bias ? bw_launch<128, true, true>(k128, v128, q64, do64, p, grid_kv, s) : bw_launch<128, true, false>(k128, v128, q64, do64, p, grid_kv, s);
-  else
-    rc = with_bias ? bw_launch<64, true, true>(k128, v128, q64, do64, p, grid_kv, s) : bw_launch<64, true, false>(k128, v128, q64, do64, p, grid_kv, s);
+  // a dense bf16 bias travels by TMA (strides and base are multiples of 16 bytes); fp32 ones, unaligned rows and masks that
+  // broadcast over the queries are loaded element by element
+  const int bias_mode = !bias ? 0 : (p.bias_kind == 2 && p.bias_vec && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0 ? 2 : 1);
+  CUtensorMap b_kv = q64, b_q = q64;
+  if (bias_mode == 2) {
+    rc = bw_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_T, BW_R, false);
+    if (rc == TPB_OK) rc = bw_bias_tmap(&b_q, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_R, BW_T, true);
+    if (rc != TPB_OK) return rc;
+  }
+#define BW_DISPATCH(DKV, R1, R2, T1, T2, TB, GRID)                                                                                        \
+  (head_dim == 128 ? (bias_mode == 0   ? bw_launch<128, DKV, 0>(R1, R2, T1, T2, TB, p, GRID, s)                                           \
+                      : bias_mode == 1 ? bw_launch<128, DKV, 1>(R1, R2, T1, T2, TB, p, GRID, s)                                           \
+                                       : bw_launch<128, DKV, 2>(R1, R2, T1, T2, TB, p, GRID, s))                                          \
+                   : (bias_mode == 0   ? bw_launch<64, DKV, 0>(R1, R2, T1, T2, TB, p, GRID, s)                                            \
+                      : bias_mode == 1 ? bw_launch<64, DKV, 1>(R1, R2, T1, T2, TB, p, GRID, s)                                            \
+                                       : bw_launch<64, DKV, 2>(R1, R2, T1, T2, TB, p, GRID, s)))
+  rc = BW_DISPATCH(true, k128, v128, q64, do64, b_kv, grid_kv);
   if (rc != TPB_OK) return rc;
   p.out0 = static_cast<bf16*>(dq); p.o0_sb = dq_sb; p.o0_ss = dq_ss; p.o0_sh = dq_sh;
   p.out1 = nullptr;
   p.dbias = dbias;
   dim3 grid_q((sq + BW_R - 1) / BW_R, q_heads, batch);
-  if (head_dim == 128)
-    return with_bias ? bw_launch<128, false, true>(q128, do128, k64, v64, p, grid_q, s) : bw_launch<128, false, false>(q128, do128, k64, v64, p, grid_q, s);
-  return with_bias ? bw_launch<64, false, true>(q128, do128, k64, v64, p, grid_q, s) : bw_launch<64, false, false>(q128, do128, k64, v64, p, grid_q, s);
+  return BW_DISPATCH(false, q128, do128, k64, v64, b_q, grid_q);
+#undef BW_DISPATCH
 }

@@ -399,7 +399,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be uniform)
   const int qblk = gridDim.x - 1 - blockIdx.x;  // heavy (late) causal tiles first
   const int h = blockIdx.y, b = blockIdx.z;
   const int kvh = h / (p.q_heads / p.kv_heads);
@@ -469,63 +469,62 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         }
       }
     } else if (warp == 1) {
-      // ---------------- MMA issuer ----------------
-      if (elect_one() && n_max > 0) {
-        const uint32_t q_addr = smem_u32(q_s);
+      // ---------------- MMA issuer (the warp stays together, one lane issues: see umma_bf16_lead) ----------------
+      if (n_max > 0) {
+        const uint32_t leader = elect_one();
+        const uint32_t q_lo = desc_kmajor_lo(smem_u32(q_s));
         auto issue_qk = [&](int t, int j) {  // S_t = Q_t K(j)^T
-          const uint32_t k_addr = smem_u32(k_s + (j & 1) * T_BYTES);
-          const uint32_t d_tmem = tmem_base + t * FA_N;
+          const uint32_t k_lo = desc_kmajor_lo(smem_u32(k_s + (j & 1) * T_BYTES));
 #pragma unroll
           for (int d = 0; d < DB; ++d) {
 #pragma unroll
-            for (int kk = 0; kk < 64 / 16; ++kk) {
-              const uint64_t adesc = make_desc_kmajor_sw128(q_addr + t * T_BYTES + d * FA_BLOCK_BYTES + kk * 32);
-              const uint64_t bdesc = make_desc_kmajor_sw128(k_addr + d * FA_BLOCK_BYTES + kk * 32);
-              umma_bf16(d_tmem, adesc, bdesc, IDESC_QK, (d | kk) ? 1u : 0u);
-            }
+            for (int kk = 0; kk < 64 / 16; ++kk)
+              umma_bf16_lead(leader, tmem_base + t * FA_N, q_lo + (t * T_BYTES + d * FA_BLOCK_BYTES) / 16 + kk * 2, k_lo + d * (FA_BLOCK_BYTES / 16) + kk * 2,
+                             IDESC_QK, (d | kk) ? 1u : 0u);
           }
-          umma_commit(&s_full[t]);
+          umma_commit_lead(leader, &s_full[t]);
         };
         auto issue_pv = [&](int t, int j) {  // O_t (+)= P_t(j) V(j): P from tensor memory, V tile [128 keys][D] MN-major
-          const uint32_t v_addr = smem_u32(v_s + (j & 1) * T_BYTES);
+          const uint32_t v_lo = desc_mnmajor_lo(smem_u32(v_s + (j & 1) * T_BYTES), FA_BLOCK_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < FA_N / 16; ++kk) {
-            const uint64_t bdesc = make_desc_mnmajor_sw128(v_addr + kk * 16 * 128, FA_BLOCK_BYTES);
-            umma_bf16_tmem_a(tmem_base + O_COL0 + t * FA_N, tmem_base + t * FA_N + kk * 8, bdesc, IDESC_PV, (j | kk) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < FA_N / 16; ++kk)
+            umma_bf16_tmem_a_lead(leader, tmem_base + O_COL0 + t * FA_N, tmem_base + t * FA_N + kk * 8, v_lo + kk * (16 * 128 / 16), IDESC_PV,
+                                  (j | kk) ? 1u : 0u);
         };
-        bool ok = mbar_wait(q_full, 0) && mbar_wait(&k_full[0], 0);
-        if (!ok) give_up(STATUS_TIMEOUT_MBAR);
-        if (ok) {
+        auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+          const bool there = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+          if (!there && leader) give_up(STATUS_TIMEOUT_MBAR);
           tc_fence_after();
+          return there;
+        };
+        bool ok = wait_all(q_full, 0) && wait_all(&k_full[0], 0);
+        if (ok) {
 #pragma unroll
           for (int t = 0; t < 2; ++t)
             if (n_tiles[t] > 0) issue_qk(t, 0);
-          umma_commit(&k_empty[0]);
+          umma_commit_lead(leader, &k_empty[0]);
         }
-        for (int j = 0; ok && j < n_max && !*abort_flag; ++j) {
+        for (int j = 0; ok && j < n_max; ++j) {
           const bool next = j + 1 < n_max;
-          if (next && !mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) { give_up(STATUS_TIMEOUT_MBAR); break; }
-          if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1)) { give_up(STATUS_TIMEOUT_MBAR); break; }
+          if (next) ok = wait_all(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1);
+          ok = ok && wait_all(&v_full[j & 1], (j >> 1) & 1);
+          if (!ok) break;
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             if (ok && j < n_tiles[t]) {
-              if (!mbar_wait(&p_full[t], j & 1)) {
-                give_up(STATUS_TIMEOUT_MBAR);
-                ok = false;
-              } else {
-                tc_fence_after();
+              ok = wait_all(&p_full[t], j & 1);
+              if (ok) {
                 issue_pv(t, j);
                 if (j == n_tiles[t] - 1)
-                  umma_commit(&o_full[t]);
+                  umma_commit_lead(leader, &o_full[t]);
                 else
                   issue_qk(t, j + 1);
               }
             }
           }
           if (!ok) break;
-          umma_commit(&v_empty[j & 1]);          // V(j) may be overwritten once these MMAs retire
-          if (next) umma_commit(&k_empty[(j + 1) & 1]);  // and K(j + 1)
+          umma_commit_lead(leader, &v_empty[j & 1]);          // V(j) may be overwritten once these MMAs retire
+          if (next) umma_commit_lead(leader, &k_empty[(j + 1) & 1]);  // and K(j + 1)
         }
       }
     }

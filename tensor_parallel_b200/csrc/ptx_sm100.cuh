@@ -209,6 +209,71 @@ __device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_
       : "memory");
 }
 
+// Forms for an issue loop that the WHOLE warp walks, with only its `leader` lane issuing.  An MMA takes its descriptors from
+// uniform registers; in code that only the elected lane runs, every operand of every instruction is moved there one by one,
+// and a stream of short MMAs (N <= 64) is then bound by its issue loop (attention backward 4 x 2048, 32 heads of 128, causal: 606 ->
+// 554 us with this form and mask-free common steps, forward 204 -> 194 us).  Descriptors come as 32-bit halves: the high half is
+// a constant of the layout, the low half (address field) advances by plain 32-bit additions.
+constexpr uint32_t DESC_KMAJOR_HI = (1024u >> 4) | (1u << 14) | (2u << 29);  // stride 1024 B, version 1, 128-byte swizzle
+__device__ __forceinline__ uint32_t desc_kmajor_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+__device__ __forceinline__ uint32_t desc_mnmajor_lo(uint32_t smem_addr, uint32_t mn_block_bytes) {
+  return ((smem_addr & 0x3FFFFu) >> 4) | (((mn_block_bytes >> 4) & 0x3FFFu) << 16);
+}
+__device__ __forceinline__ void umma_bf16_lead(uint32_t leader, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 da, db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "mov.b64 da, {%1, %6};\n"
+      "mov.b64 db, {%2, %6};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(leader), "n"(DESC_KMAJOR_HI)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_tmem_a_lead(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "mov.b64 db, {%2, %6};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(leader), "n"(DESC_KMAJOR_HI)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_lead(uint32_t leader, uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %2, 0;\n"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+      "}\n" ::"r"(smem_u32(bar)), "r"(bytes), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_lead(uint32_t leader, uint32_t smem_dst, const void* tmap, uint64_t* bar, int x, int y) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+      "}\n" ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_lead(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(smem_u32(bar)), "r"(leader)
+      : "memory");
+}
+
 // Register reallocation between warpgroups (every warp of a group of four executes the same one).
 template <int REGS>
 __device__ __forceinline__ void setmaxnreg_inc() {
