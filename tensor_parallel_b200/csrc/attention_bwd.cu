@@ -40,6 +40,48 @@ __device__ __forceinline__ float bias_at(const BiasArgs& ba, long long idx) {
   return ba.kind == 1 ? __ldg(static_cast<const float*>(ba.bias) + idx) : __bfloat162float(static_cast<const bf16*>(ba.bias)[idx]);
 }
 
+// 16-byte accesses: D / 8 lanes per row, four rows per lane group in flight, rows in memory order (head fastest), so that a warp
+// reads whole contiguous stretches of `out` and `dout`.  Memory-bound: 4 x 2048 x 32 heads of 128, 134 MB, 68 -> 33 us against a
+// warp per row with 2-byte loads.
+template <int D>
+__global__ void __launch_bounds__(256)
+attn_bwd_delta_vec_kernel(const bf16* __restrict__ out, const bf16* __restrict__ dout, float* __restrict__ delta, int sq, int heads,
+                          long long o_sb, long long o_ss, long long o_sh, long long do_sb, long long do_ss, long long do_sh, long long rows) {
+  constexpr int LANES = D / 8, GROUPS = 256 / LANES, U = 4;
+  const int part = threadIdx.x % LANES;
+  const long long r0 = blockIdx.x * (long long)(GROUPS * U) + threadIdx.x / LANES;
+  uint4 o[U], g[U];
+  long long dst[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long r = r0 + u * GROUPS;  // (b, i, h)
+    o[u] = g[u] = make_uint4(0, 0, 0, 0);
+    dst[u] = -1;
+    if (r < rows) {
+      const long long t = r / heads;
+      const int h = int(r - t * heads);
+      const long long b = t / sq;
+      const int i = int(t - b * sq);
+      o[u] = *reinterpret_cast<const uint4*>(out + b * o_sb + (long long)i * o_ss + (long long)h * o_sh + part * 8);
+      g[u] = *reinterpret_cast<const uint4*>(dout + b * do_sb + (long long)i * do_ss + (long long)h * do_sh + part * 8);
+      dst[u] = (b * heads + h) * sq + i;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t ow[4] = {o[u].x, o[u].y, o[u].z, o[u].w}, gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      acc += __uint_as_float(ow[k] << 16) * __uint_as_float(gw[k] << 16);
+      acc += __uint_as_float(ow[k] & 0xFFFF0000u) * __uint_as_float(gw[k] & 0xFFFF0000u);
+    }
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (part == 0 && dst[u] >= 0) delta[dst[u]] = acc;
+  }
+}
+
 __global__ void attn_bwd_delta_kernel(const bf16* __restrict__ out, const bf16* __restrict__ dout, float* __restrict__ delta,
                                       int sq, int heads, int d, long long o_sb, long long o_ss, long long o_sh,
                                       long long do_sb, long long do_ss, long long do_sh, long long rows) {
@@ -353,7 +395,15 @@ extern "C" int tpb_attn_bwd_delta(const void* out, const void* dout, float* delt
                                   void* stream_) {
   if (!out || !dout || !delta || batch <= 0 || sq <= 0 || heads <= 0 || head_dim <= 0) return TPB_ERR_ARG;
   const long long rows = (long long)batch * heads * sq;
-  attn_bwd_delta_kernel<<<int((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream_)>>>(
+  const bool vec = !((o_sb | o_ss | o_sh | do_sb | do_ss | do_sh) & 7) && !((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout)) & 15);
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  if (vec && head_dim == 128)
+    attn_bwd_delta_vec_kernel<128><<<int((rows + 63) / 64), 256, 0, s>>>((const bf16*)out, (const bf16*)dout, delta, sq, heads, o_sb, o_ss, o_sh, do_sb,
+                                                                         do_ss, do_sh, rows);
+  else if (vec && head_dim == 64)
+    attn_bwd_delta_vec_kernel<64><<<int((rows + 127) / 128), 256, 0, s>>>((const bf16*)out, (const bf16*)dout, delta, sq, heads, o_sb, o_ss, o_sh, do_sb,
+                                                                          do_ss, do_sh, rows);
+  else attn_bwd_delta_kernel<<<int((rows + 7) / 8), 256, 0, s>>>(
       (const bf16*)out, (const bf16*)dout, delta, sq, heads, head_dim, o_sb, o_ss, o_sh, do_sb, do_ss, do_sh, rows);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
