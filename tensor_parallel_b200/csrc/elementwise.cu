@@ -147,11 +147,11 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T
 
 // Backward: dx per row; the column sums for dweight / dbias go through one fp32 partial row per CTA, which
 // norm_bwd_reduce_kernel adds up in a fixed order (deterministic, no atomics).  Memory-bound: x and dy are read and dx is
-// written once.  A CTA walks rows blockIdx.x, + gridDim.x, ... and holds its column sums in registers; the raw 16-byte vectors
-// of the next row are fetched before the block-wide sums of the current one (PREFETCH), which is what keeps enough bytes in
-// flight with two CTAs per SM.  V = vectors of 8 elements per thread.
-constexpr int NORM_BWD_MAXV = 4;  // cols <= 8192 in the backward kernel (register limit)
-constexpr int NORM_BWD_CTAS = 148 * 2;
+// written once.  A thread owns 8 columns (a CTA has as many threads as the row has vectors, so that its registers admit 1024
+// threads per SM whatever the width) and walks rows blockIdx.x, + gridDim.x, ... with the column sums in registers; bf16 rows are
+// fetched one ahead, before the block-wide sums of the current row.  RMSNorm 8192 x 4096 bf16: 57 us (3.5 TB/s; 73 us with half as
+// many threads of two vectors each), LayerNorm 1999 x 5120 fp32: 40 us.
+constexpr int NORM_BWD_MAXC = 8192;  // 1024 threads
 
 template <typename T> struct Raw8 { uint4 u[sizeof(T) / 2]; };  // 8 elements as they lie in memory
 template <typename T> __device__ __forceinline__ Raw8<T> load_raw(const T* p) {
@@ -174,103 +174,76 @@ __device__ __forceinline__ void unpack(const Raw8<float>& r, float (&v)[8]) {
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
 }
 
-template <typename T, int MODE, int V>
-__global__ void __launch_bounds__(NORM_THREADS, (sizeof(T) == 4 && MODE == 1 && V == 4) ? 1 : 2)  // (that one would spill)
+template <typename T, int MODE>
+__global__ void __launch_bounds__(1024)
 norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ weight,
                 const float* __restrict__ rstd_in, const float* __restrict__ mean_in, T* __restrict__ dx,
                 float* __restrict__ part_w, float* __restrict__ part_b, int rows, int cols) {
-  constexpr bool PREFETCH = sizeof(T) == 2 ? V <= 2 : V == 1;  // (wider rows keep enough bytes in flight by themselves)
-  const int nvec = cols >> 3;
-  float dw_acc[V][8], db_acc[V][8];
+  constexpr bool PREFETCH = sizeof(T) == 2;  // (an fp32 row has twice the bytes in flight, and no registers left for another)
+  const int c0 = threadIdx.x * 8;
+  const bool mine = c0 < cols;
+  float dw_acc[8], db_acc[8];
 #pragma unroll
-  for (int i = 0; i < V; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { dw_acc[i][j] = 0.f; db_acc[i][j] = 0.f; }
-  Raw8<T> xr[V], dr[V];
-  auto fetch = [&](int row, Raw8<T> (&xo)[V], Raw8<T> (&dd)[V]) {
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int vi = threadIdx.x + i * NORM_THREADS;
-      if (vi < nvec) {
-        dd[i] = load_raw(dy + size_t(row) * cols + vi * 8);
-        xo[i] = load_raw(x + size_t(row) * cols + vi * 8);
-      }
+  for (int j = 0; j < 8; ++j) { dw_acc[j] = 0.f; db_acc[j] = 0.f; }
+  Raw8<T> wr, xr, dr;
+  if (mine && weight) wr = load_raw(weight + c0);
+  auto fetch = [&](int row, Raw8<T>& xo, Raw8<T>& dd) {
+    if (mine) {
+      dd = load_raw(dy + size_t(row) * cols + c0);
+      xo = load_raw(x + size_t(row) * cols + c0);
     }
   };
+  const float inv_n = 1.f / float(cols);
   int row = blockIdx.x;
-  float rstd = 0.f, mean = 0.f;
-  if (row < rows) {
-    fetch(row, xr, dr);
-    rstd = rstd_in[row];
-    if (MODE == 1) mean = mean_in[row];
-  }
+  if (row < rows) fetch(row, xr, dr);
   while (row < rows) {
     const int next = row + gridDim.x;
-    Raw8<T> xn[V], dn[V];
-    float rstd_n = 0.f, mean_n = 0.f;
-    if (next < rows) {
-      if (PREFETCH) fetch(next, xn, dn);
-      rstd_n = rstd_in[next];
-      if (MODE == 1) mean_n = mean_in[next];
-    }
+    const float rstd = rstd_in[row], mean = MODE == 1 ? mean_in[row] : 0.f;
+    Raw8<T> xn, dn;
+    if (PREFETCH && next < rows) fetch(next, xn, dn);
     float s1 = 0.f, s2 = 0.f;  // sum(g), sum(g * xhat)
+    if (mine) {
+      float d[8], xv[8], w[8];
+      unpack(dr, d);
+      unpack(xr, xv);
+      if (weight) unpack(wr, w);
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int vi = threadIdx.x + i * NORM_THREADS;
-      if (vi < nvec) {
-        float d[8], xv[8], w[8];
-        unpack(dr[i], d);
-        unpack(xr[i], xv);
-        if (weight) Vec8<T>::load(weight + vi * 8, w);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = (xv[j] - mean) * rstd;
-          dw_acc[i][j] += d[j] * xh;
-          db_acc[i][j] += d[j];
-          const float g = weight ? d[j] * w[j] : d[j];
-          s1 += g;
-          s2 += g * xh;
-        }
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (xv[j] - mean) * rstd;
+        dw_acc[j] += d[j] * xh;
+        db_acc[j] += d[j];
+        const float g = weight ? d[j] * w[j] : d[j];
+        s1 += g;
+        s2 += g * xh;
       }
     }
     block_sum2(s1, s2);
-    const float inv_n = 1.f / float(cols);
     const float c1 = MODE == 1 ? s1 * inv_n : 0.f;
     const float c2 = s2 * inv_n;
+    if (mine) {
+      float d[8], xv[8], w[8], o[8];
+      unpack(dr, d);
+      unpack(xr, xv);
+      if (weight) unpack(wr, w);
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int vi = threadIdx.x + i * NORM_THREADS;
-      if (vi < nvec) {
-        float d[8], xv[8], w[8], o[8];
-        unpack(dr[i], d);
-        unpack(xr[i], xv);
-        if (weight) Vec8<T>::load(weight + vi * 8, w);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = (xv[j] - mean) * rstd;
-          const float g = weight ? d[j] * w[j] : d[j];
-          o[j] = (g - c1 - xh * c2) * rstd;
-        }
-        Vec8<T>::store(dx + size_t(row) * cols + vi * 8, o);
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (xv[j] - mean) * rstd;
+        const float g = weight ? d[j] * w[j] : d[j];
+        o[j] = (g - c1 - xh * c2) * rstd;
       }
+      Vec8<T>::store(dx + size_t(row) * cols + c0, o);
     }
     if (PREFETCH) {
-#pragma unroll
-      for (int i = 0; i < V; ++i) { xr[i] = xn[i]; dr[i] = dn[i]; }
+      xr = xn;
+      dr = dn;
     } else if (next < rows) {
       fetch(next, xr, dr);
     }
-    rstd = rstd_n;
-    mean = mean_n;
     row = next;
   }
-#pragma unroll
-  for (int i = 0; i < V; ++i) {
-    const int vi = threadIdx.x + i * NORM_THREADS;
-    if (vi < nvec) {
-      if (part_w) Vec8<float>::store(part_w + size_t(blockIdx.x) * cols + vi * 8, dw_acc[i]);
-      if (MODE == 1 && part_b) Vec8<float>::store(part_b + size_t(blockIdx.x) * cols + vi * 8, db_acc[i]);
-    }
+  if (mine) {
+    if (part_w) Vec8<float>::store(part_w + size_t(blockIdx.x) * cols + c0, dw_acc);
+    if (MODE == 1 && part_b) Vec8<float>::store(part_b + size_t(blockIdx.x) * cols + c0, db_acc);
   }
 }
 
@@ -634,32 +607,30 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   TPB_CHECK_LAUNCH();
 }
 
-// Rows of fp32 partials that tpb_norm_bwd needs for this row count: part_w / part_b hold that many rows of `cols` floats.
-extern "C" int tpb_norm_bwd_parts(int rows) { return rows < NORM_BWD_CTAS ? rows : NORM_BWD_CTAS; }
+// Rows of fp32 partials that tpb_norm_bwd needs (= its CTAs): part_w / part_b hold that many rows of `cols` floats.  As many CTAs
+// as 1024 threads per SM make, up to 16 (narrow rows: more partials would cost more than their CTAs bring).
+static inline int norm_bwd_threads(int cols) { return (cols / 8 + 31) / 32 * 32; }
+extern "C" int tpb_norm_bwd_parts(int rows, int cols) {
+  const int per_sm = 1024 / norm_bwd_threads(cols);
+  const int ctas = 148 * (per_sm > 16 ? 16 : (per_sm < 1 ? 1 : per_sm));
+  return rows < ctas ? rows : ctas;
+}
 
 // dweight / dbias (either may be null, with its partials) are written, not accumulated; grad_dtype: 0 = bf16, 1 = fp32.
 extern "C" int tpb_norm_bwd(const void* dy, const void* x, const void* weight, const float* rstd, const float* mean,
                             void* dx, float* part_w, float* part_b, void* dweight, void* dbias, int rows, int cols, int mode, int dtype,
                             int grad_dtype, void* stream_) {
   if (!dy || !x || !dx || !rstd || rows <= 0 || cols <= 0 || (mode && !mean) || (dweight && !part_w) || (dbias && (!part_b || !mode))) return TPB_ERR_ARG;
-  if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_BWD_MAXV) return TPB_ERR_SIZE;
+  if ((cols & 7) || cols > NORM_BWD_MAXC) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  const int grid = tpb_norm_bwd_parts(rows);
+  const int grid = tpb_norm_bwd_parts(rows, cols), threads = norm_bwd_threads(cols);
   if (!dweight) part_w = nullptr;
   if (!dbias) part_b = nullptr;
-#define LAUNCH3(T, M, V)                                                                                              \
-  norm_bwd_kernel<T, M, V><<<grid, NORM_THREADS, 0, s>>>((const T*)dy, (const T*)x, (const T*)weight, rstd, mean, (T*)dx, part_w, part_b, rows, cols)
-#define LAUNCH(T, M)                                                                     \
-  do {                                                                                   \
-    if (cols <= NORM_THREADS * 8) LAUNCH3(T, M, 1);                                      \
-    else if (cols <= NORM_THREADS * 16) LAUNCH3(T, M, 2);                                \
-    else if (cols <= NORM_THREADS * 24) LAUNCH3(T, M, 3);                                \
-    else LAUNCH3(T, M, 4);                                                               \
-  } while (0)
+#define LAUNCH(T, M) \
+  norm_bwd_kernel<T, M><<<grid, threads, 0, s>>>((const T*)dy, (const T*)x, (const T*)weight, rstd, mean, (T*)dx, part_w, part_b, rows, cols)
   if (dtype == 0) { if (mode) LAUNCH(bf16, 1); else LAUNCH(bf16, 0); }
   else            { if (mode) LAUNCH(float, 1); else LAUNCH(float, 0); }
 #undef LAUNCH
-#undef LAUNCH3
   if (dweight || dbias) {
     const dim3 rgrid((cols + 31) / 32, dbias ? 2 : 1);
     if (grad_dtype == 0)

@@ -377,7 +377,7 @@ class _NormFn(torch.autograd.Function):
         # column sums: one fp32 partial row per CTA, added up by a second kernel that writes the gradients in their own dtype
         has_w, has_b = w is not None, ctx.bdtype is not None
         gdtype = ctx.wdtype if has_w and (not has_b or ctx.bdtype == ctx.wdtype) and ctx.wdtype == torch.bfloat16 else torch.float32
-        parts = LIB.tpb_norm_bwd_parts(rows)
+        parts = LIB.tpb_norm_bwd_parts(rows, cols)
         part_w = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_w else None
         part_b = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_b else None
         dw = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_w else None
