@@ -75,11 +75,12 @@ def check(code: int, what: str):
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
+    return t.data_ptr() if t is not None else None  # (ctypes converts plain integers for a c_void_p argument)
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of the calling thread's current stream on the current device (no Stream object is built for it)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dtype_code(t: torch.Tensor) -> int:
