@@ -75,8 +75,8 @@ def test_pair_gemm_gated_into_a_wider_buffer(tokens):
 
 
 # one unit of 32 rows, a ragged last unit, one unit per SM, one CTA with two, more than one pass of 128 rows per CTA
-@pytest.mark.parametrize("features,k", [(32, 64), (40, 136), (1000, 520), (4736, 256), (4768, 1032), (4096, 4096), (22016, 264), (32003, 512)])
-@pytest.mark.parametrize("tokens", [1, 8, 17, 64])
+@pytest.mark.parametrize("features,k", [(32, 64), (40, 136), (1000, 520), (4736, 256), (4768, 1032), (2080, 1400), (4096, 4096), (22016, 264), (32003, 512)])
+@pytest.mark.parametrize("tokens", [1, 8, 16, 17, 64])
 def test_streamed_few_token_gemm(tokens, features, k):
     nat = _native()
     torch.manual_seed(tokens + features)
