@@ -25,7 +25,7 @@
 //               of step n (two TMEM buffers), so the tensor core always has work
 //   warps 2-9 : elementwise - two threads per TMEM lane, one per half of the step's 64 columns
 //
-// TMEM (512 columns): S 2 x 64 | dP 2 x 64 | accumulator 0 (dK or dQ) | accumulator 1 (dV).  Shared memory at head_dim
+// TMEM (512 columns): S 2 x 64 | dP 2 x 64 | accumulator 0 (dK or dQ) | accumulator 1 (dV) | resident tiles (RES_TMEM).  Shared memory at head_dim
 // 128: 2 x 32 KB resident + 3 x 2 x 16 KB streamed = 160 KB.  Every mbarrier wait is bounded; on expiry the CTA records
 // a status code and drains.  No TMA load has a multicast qualifier.
 #include <cuda.h>
@@ -85,6 +85,12 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   constexpr uint32_t T_BYTES = DB * BW_T_BLOCK_BYTES;  // one streamed tile (64 rows)
   constexpr uint32_t TMEM_COLS = 512;
   constexpr uint32_t S_COL0 = 0, DP_COL0 = 2 * BW_T, ACC0_COL = 4 * BW_T, ACC1_COL = 4 * BW_T + D;
+  // The resident tiles as tensor-memory A operands where 512 columns leave room for them (all of dQ, dK / dV at head_dim 64): from
+  // shared memory, a score MMA of 128 x 64 x 16 reads 6 KB for 32 clocks of work and is bound by that (dQ of 4 x 2048, 32 heads of
+  // 128, causal: 248 -> 233 us; whole backward of 16 x 512, 32 heads of 64: 291 -> 273 us).
+  constexpr bool RES_TMEM = !DKV || D == 64;
+  constexpr uint32_t RES_COL0 = ACC0_COL + (DKV ? 2 : 1) * D;  // resident 1, then resident 2: D / 2 columns each (two bf16 per column)
+  static_assert(!RES_TMEM || RES_COL0 + D <= TMEM_COLS, "tensor memory columns");
   constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BW_T, false, false);
   constexpr uint32_t IDESC_ACC = make_idesc_bf16(BW_R, D, false, true);
 
@@ -105,7 +111,8 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   uint64_t* s_full = bars + 1 + 2 * BW_STAGES;   // [2]
   uint64_t* p_full = s_full + 2;                 // [2]
   uint64_t* acc_full = p_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* res_full = acc_full + 1;             // RES_TMEM: the resident tiles are in tensor memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be uniform)
@@ -148,6 +155,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       mbar_init(&p_full[s], 8);  // one arrival per elementwise warp
     }
     mbar_init(acc_full, 1);
+    mbar_init(res_full, 8);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -176,6 +184,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
           tma_load_4d(r2_s + d * FA_BLOCK_BYTES, &tmap_r2, r_full, d * 64, r0, DKV ? kvh : head, b);
         }
       }
+      int g = 0, local = 0;  // query head of the group (dK / dV), step within it
       for (int n = 0; n < n_steps; ++n) {
         const int s = n % BW_STAGES;
         const uint32_t par = ((n / BW_STAGES) & 1) ^ 1;
@@ -184,9 +193,9 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
           if (lane == 0 && !*abort_flag) give_up(STATUS_TIMEOUT_MBAR);
           break;
         }
-        const int g = DKV ? n / per_head : 0;
-        const int row0 = (step0 + (DKV ? n - g * per_head : n)) * BW_T;  // first streamed row of the step
+        const int row0 = (step0 + local) * BW_T;  // first streamed row of the step
         const int t_head = DKV ? head + g : kvh;
+        if (++local == per_head) { local = 0; ++g; }
         if (lane == 0) {
           mbar_expect_tx(&t_full[s], 2 * T_BYTES + (BIAS == 2 ? BW_BIAS_BYTES : 0));
           if (BIAS == 2)
@@ -229,15 +238,23 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         for (int d = 0; d < DB; ++d) {
 #pragma unroll
           for (int kk = 0; kk < 64 / 16; ++kk)
-            umma_bf16_lead(leader, tmem_base + S_COL0 + buf * BW_T, r1_lo + d * (FA_BLOCK_BYTES >> 4) + kk * 2,
-                           t1_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
+            if (RES_TMEM)
+              umma_bf16_tmem_a_lead(leader, tmem_base + S_COL0 + buf * BW_T, tmem_base + RES_COL0 + (d * 4 + kk) * 8,
+                                    t1_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
+            else
+              umma_bf16_lead(leader, tmem_base + S_COL0 + buf * BW_T, r1_lo + d * (FA_BLOCK_BYTES >> 4) + kk * 2,
+                             t1_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
         }
 #pragma unroll
         for (int d = 0; d < DB; ++d) {
 #pragma unroll
           for (int kk = 0; kk < 64 / 16; ++kk)
-            umma_bf16_lead(leader, tmem_base + DP_COL0 + buf * BW_T, r2_lo + d * (FA_BLOCK_BYTES >> 4) + kk * 2,
-                           t2_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
+            if (RES_TMEM)
+              umma_bf16_tmem_a_lead(leader, tmem_base + DP_COL0 + buf * BW_T, tmem_base + RES_COL0 + D / 2 + (d * 4 + kk) * 8,
+                                    t2_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
+            else
+              umma_bf16_lead(leader, tmem_base + DP_COL0 + buf * BW_T, r2_lo + d * (FA_BLOCK_BYTES >> 4) + kk * 2,
+                             t2_lo + d * (BW_T_BLOCK_BYTES >> 4) + kk * 2, IDESC_S, (d | kk) ? 1u : 0u);
         }
         umma_commit_lead(leader, &s_full[buf]);
       };
@@ -263,7 +280,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         tc_fence_after();
         return there;
       };
-      bool ok = wait_all(r_full, 0) && wait_all(&t_full[0], 0);
+      bool ok = wait_all(RES_TMEM ? res_full : r_full, 0) && wait_all(&t_full[0], 0);
       if (ok) issue_scores(0);
       for (int n = 0; ok && n < n_steps; ++n) {
         if (n + 1 < n_steps) {
@@ -297,8 +314,32 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       my_del = -__ldg(p.delta + idx) * p.scale;
     }
     bool alive = true;
+    int g = 0, local = 0;  // as in the producer
+    if (RES_TMEM && n_steps > 0) {
+      // resident tiles: swizzled shared memory -> tensor memory, a row per thread, one tile per half
+      if (!mbar_wait(r_full, 0)) {
+        give_up(STATUS_TIMEOUT_MBAR);
+        alive = false;
+      }
+      const uint8_t* tile = half ? r2_s : r1_s;
+#pragma unroll
+      for (int d = 0; d < DB; ++d) {
+        uint32_t w[32];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 u = *reinterpret_cast<const uint4*>(tile + d * FA_BLOCK_BYTES + row * 128 + ((c ^ (row & 7)) << 4));
+          w[4 * c] = u.x; w[4 * c + 1] = u.y; w[4 * c + 2] = u.z; w[4 * c + 3] = u.w;
+        }
+        __syncwarp();
+        tmem_st_x32(t_lane + RES_COL0 + half * (D / 2) + d * 32, w);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(res_full);
+    }
 
-    for (int n = 0; n < n_steps; ++n) {
+    for (int n = 0; alive && n < n_steps; ++n) {
       const int s = n % BW_STAGES, buf = n & 1;
       if (*abort_flag || ((DKV || BIAS == 2) && !mbar_wait(&t_full[s], (n / BW_STAGES) & 1)) || !mbar_wait(&s_full[buf], (n >> 1) & 1)) {
         if (!*abort_flag) give_up(STATUS_TIMEOUT_MBAR);
@@ -306,8 +347,9 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         break;
       }
       tc_fence_after();
-      const int g = DKV ? n / per_head : 0;
-      const int col0 = (step0 + (DKV ? n - g * per_head : n)) * BW_T + half * HC;  // first query (DKV) or key of my columns
+      const int col0 = (step0 + local) * BW_T + half * HC;  // first query (DKV) or key of my columns
+      const int b_head = DKV ? head + g : head;
+      if (++local == per_head) { local = 0; ++g; }
       uint32_t sv[HC], dv[HC];
       tmem_ld_x32(t_lane + S_COL0 + buf * BW_T + half * HC, sv);
       tmem_ld_x32(t_lane + DP_COL0 + buf * BW_T + half * HC, dv);
@@ -327,7 +369,6 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);
       // score bias: element (query, key) = (col0 + c, ri) for dK / dV - there the lanes of a warp own consecutive keys - and
       // (ri, col0 + c) for dQ, where a thread's columns are consecutive keys of one row and are read eight at a time
-      const int b_head = DKV ? head + g : head;
       const long long bias_base = BIAS ? (long long)b * p.b_sb + (long long)b_head * p.b_sh + (long long)ri * (DKV ? p.b_sk : p.b_sq) : 0;
       const long long bias_step = DKV ? p.b_sq : p.b_sk;  // per column
       const int col_limit = DKV ? p.sq : p.sk, row_limit = DKV ? p.sk : p.sq;
