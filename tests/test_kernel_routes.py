@@ -1,0 +1,74 @@
+"""Rules that choose a kernel, checked on the CPU: which GEMM shapes may take the single-rank kernels, how the few-token kernel deals
+out its rows, and the relative-position bias by distance against the lookup of every pair."""
+import ctypes
+
+import pytest
+import torch
+
+from tensor_parallel_b200 import build
+from tensor_parallel_b200.models.t5 import T5Attention, T5Config, relative_position_bucket
+
+
+def _plan(tokens, features, k, world=1, splits=0, kbox=0, no_swap=0):
+    from tensor_parallel_b200.ops import native
+
+    plan = native.GemmPlan()
+    native.check(native.LIB.tpb_gemm_plan_ex(tokens, features, k, world, splits, kbox, no_swap, ctypes.byref(plan)), "gemm_plan")
+    return plan
+
+
+needs_library = pytest.mark.skipif(not build.LIB_PATH.exists(), reason="native library not built")
+
+
+@needs_library
+@pytest.mark.parametrize("tokens", [1, 16, 64, 65, 300, 4096, 8192])
+@pytest.mark.parametrize("features,k", [(32, 64), (4096, 4096), (12288, 4096), (512, 16384), (1000, 520), (32003, 4096)])
+def test_single_rank_kernels_leave_the_other_forms_alone(tokens, features, k):
+    plan = _plan(tokens, features, k)
+    assert not (plan.pair and plan.stream)
+    assert not plan.pair or (not plan.swapped and plan.k_splits == 1 and plan.pair in (128, 256))
+    assert not plan.stream or (plan.swapped and tokens <= 64)
+    for other in (_plan(tokens, features, k, world=2), _plan(tokens, features, k, splits=1), _plan(tokens, features, k, splits=2)):
+        assert other.pair == 0 and other.stream == 0
+    assert _plan(tokens, features, k, no_swap=1).stream == 0
+    # the fields of the tiled kernels do not depend on the choice
+    forced = _plan(tokens, features, k, splits=plan.k_splits)
+    assert (plan.swapped, plan.m_tiles, plan.n_tiles) == (forced.swapped, forced.m_tiles, forced.n_tiles)
+
+
+@pytest.mark.parametrize("features", [1, 32, 33, 1000, 4736, 4737, 4768, 9472, 12288, 22016, 32003, 65024, 151936])
+def test_row_ranges_cover_every_row_once_in_even_passes(features, sms=148):
+    """The integer arithmetic of the few-token kernel: ranges of 32-row units, the same number of passes everywhere, a box no pass is
+    shorter than."""
+    units = -(-features // 32)
+    grid = min(units, sms)
+    most, least = -(-units // grid), units // grid
+    passes = -(-most // 4)
+    longest, box = -(-most // passes), least // passes
+    assert 1 <= box and longest <= 4
+    covered = []
+    for c in range(grid):
+        u0, u1 = c * units // grid, (c + 1) * units // grid
+        n = u1 - u0
+        assert least <= n <= most
+        starts = [u0 + n * i // passes for i in range(passes + 1)]
+        assert starts[0] == u0 and starts[-1] == u1
+        assert all(box <= b - a <= longest for a, b in zip(starts, starts[1:]))
+        covered += list(range(u0, u1))
+    assert covered == list(range(units))
+
+
+@pytest.mark.parametrize("decoder", [False, True])
+@pytest.mark.parametrize("queries,keys", [(1, 1), (1, 40), (7, 12), (130, 130), (5, 300)])
+def test_relative_bias_by_distance_equals_the_lookup_of_every_pair(decoder, queries, keys):
+    torch.manual_seed(0)
+    attention = T5Attention(T5Config(num_heads=3, d_kv=8), True, decoder)
+    position = torch.arange(keys - queries, keys)[:, None]
+    buckets = relative_position_bucket(torch.arange(keys)[None, :] - position, not decoder, 32, 128)
+    want = attention.relative_attention_bias(buckets).permute(2, 0, 1)[None]
+    got = attention.compute_bias(queries, keys, "cpu")
+    assert torch.equal(got, want)
+    g = torch.randn_like(got)
+    table = attention.relative_attention_bias.weight
+    (a,), (b,) = torch.autograd.grad(got, table, g), torch.autograd.grad(want, table, g)
+    torch.testing.assert_close(a, b)
