@@ -488,11 +488,13 @@ bool gemm_stream_fits(int features, int k, int sms) {
   return (features + GS_UNIT - 1) / GS_UNIT >= sms / 2 || unit_bytes <= 1024 * 1024;
 }
 
-// 512 contiguous bytes of every weight row per stage where rows are long, else 256 in twice as many stages: 8192 x 40960 101 us with
-// 512 bytes and 117 us with 256, a decode step of four 7B layers (rows of 8 KB) 587 and 575 us.
+// 512 contiguous bytes of every weight row per stage where rows are long and a stage stays small, else 256 in twice as many stages:
+// 8192 x 40960 (two units per CTA) 101 us with 512 bytes and 117 us with 256, 32768 x 8192 (seven) 85 and 83 us, a decode step of
+// four 7B layers (rows of 8 KB) 587 and 575 us.
 template <int BN, int NACC>
 static int gs_pick(const StreamGemm& g, int sms, cudaStream_t stream) {
-  return g.k >= 8192 ? gs_launch<BN, NACC, 4, 1>(g, sms, stream) : gs_launch<BN, NACC, 2, 1>(g, sms, stream);
+  const bool small = (g.features + GS_UNIT - 1) / GS_UNIT <= 2 * sms;
+  return g.k >= 8192 && small ? gs_launch<BN, NACC, 4, 1>(g, sms, stream) : gs_launch<BN, NACC, 2, 1>(g, sms, stream);
 }
 
 int gemm_stream_launch(const StreamGemm& g, int sms, cudaStream_t stream) {
