@@ -73,7 +73,9 @@ __global__ void qkv_rope_append_kernel(const bf16* __restrict__ q, const bf16* _
 // 16-byte accesses.  Work of a token: (1) rot_chunks x groups threads that own one rotary chunk - 8 consecutive elements of the
 // first rotary half with their partners in the second, or 4 adjacent pairs when interleaved - and walk the q and k heads hg,
 // hg + groups, ... with it, so that the angles (exp2f and sincosf per pair, what bounded the kernel when every head
-// evaluated its own: 64 -> 51 us for 4000 tokens of 32 + 32 heads of 128) are computed once per thread; (2) one thread per 16-byte chunk of the non-rotary tails and of v.
+// evaluated its own: 64 -> 51 us for 4000 tokens of 32 + 32 heads of 128, 43 us with v by head groups and 32-bit divisions) are
+// computed once per thread; (2) one thread per 16-byte chunk of the non-rotary tails, and v_chunks x v_groups threads that
+// copy a chunk of v for several heads each.
 // Requires head_dim, rotary_dim / 2 (non-interleaved) or rotary_dim (interleaved) to be multiples of 8.
 __device__ __forceinline__ void rope_unpack(const uint4& u, float (&v)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -90,7 +92,7 @@ __device__ __forceinline__ uint4 rope_pack(const float (&v)[8]) {
 __global__ void __launch_bounds__(256)
 qkv_rope_append_vec_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
                            bf16* __restrict__ q_out, bf16* __restrict__ kcache, bf16* __restrict__ vcache,
-                           const int* __restrict__ base_pos, int batch, int seq, int q_heads, int kv_heads, int groups,
+                           const int* __restrict__ base_pos, int batch, int seq, int q_heads, int kv_heads, int groups, int v_groups,
                            int head_dim, int rotary_dim, float log2_theta, int interleaved, int max_seq,
                            long long q_ld, long long k_ld, long long v_ld) {
   const int half = rotary_dim >> 1;
@@ -99,13 +101,14 @@ qkv_rope_append_vec_kernel(const bf16* __restrict__ q, const bf16* __restrict__ 
   const int tail_chunks = (head_dim - rotary_dim) / 8;
   const int v_chunks = head_dim / 8;
   const int rot_work = rot_chunks * groups, tail_work = heads * tail_chunks;
-  const int per_token = rot_work + tail_work + kv_heads * v_chunks;
+  const int per_token = rot_work + tail_work + v_groups * v_chunks;
   const long long total = (long long)batch * seq * per_token;
   const int pos0 = base_pos ? base_pos[0] : 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per_token;
+    // (a 64-bit division costs as much as the rest of a copy: only for launches that need it)
+    const long long t = total <= 0xffffffffll ? (long long)(uint32_t(i) / uint32_t(per_token)) : i / per_token;
     int w = int(i - t * per_token);
-    const int b = int(t / seq);
+    const int b = int(uint32_t(t) / uint32_t(seq));  // (batch * seq is an int)
     const int pos = pos0 + int(t - (long long)b * seq);
     if (pos >= max_seq) continue;
     const bf16* qt = q + t * q_ld;
@@ -117,9 +120,12 @@ qkv_rope_append_vec_kernel(const bf16* __restrict__ q, const bf16* __restrict__ 
     };
     if (w >= rot_work + tail_work) {  // v: straight copy into the cache
       w -= rot_work + tail_work;
-      const int hv = w / v_chunks, c = (w - hv * v_chunks) * 8;
-      const uint4 val = *reinterpret_cast<const uint4*>(v + t * v_ld + hv * head_dim + c);
-      *reinterpret_cast<uint4*>(vcache + (((long long)b * kv_heads + hv) * max_seq + pos) * head_dim + c) = val;
+      const int hg = w / v_chunks, c = (w - hg * v_chunks) * 8;
+#pragma unroll 4
+      for (int hv = hg; hv < kv_heads; hv += v_groups) {
+        const uint4 val = *reinterpret_cast<const uint4*>(v + t * v_ld + hv * head_dim + c);
+        *reinterpret_cast<uint4*>(vcache + (((long long)b * kv_heads + hv) * max_seq + pos) * head_dim + c) = val;
+      }
       continue;
     }
     if (w >= rot_work) {  // non-rotary tail of q / k
@@ -815,13 +821,14 @@ extern "C" int tpb_qkv_rope_append(const void* q, const void* k, const void* v, 
   if (vec_ok) {
     const int rot_chunks = interleaved ? rotary_dim / 8 : half_ / 8;
     const int groups = tpb_rope_head_groups((long long)batch * seq * rot_chunks, q_heads + kv_heads);
+    const int v_groups = tpb_rope_head_groups((long long)batch * seq * (head_dim / 8), kv_heads);
     const long long per_token = (long long)rot_chunks * groups + (long long)(q_heads + kv_heads) * ((head_dim - rotary_dim) / 8) +
-                                (long long)kv_heads * (head_dim / 8);
+                                (long long)v_groups * (head_dim / 8);
     const long long vwork = (long long)batch * seq * per_token;
     long long vgrid = (vwork + 255) / 256;
     if (vgrid > 148 * 32) vgrid = 148 * 32;
     qkv_rope_append_vec_kernel<<<int(vgrid), 256, 0, s>>>((const bf16*)q, (const bf16*)k, (const bf16*)v, (bf16*)q_out, (bf16*)kcache,
-                                                          (bf16*)vcache, base_pos, batch, seq, q_heads, kv_heads, groups, head_dim,
+                                                          (bf16*)vcache, base_pos, batch, seq, q_heads, kv_heads, groups, v_groups, head_dim,
                                                           rotary_dim, log2f(theta), interleaved, max_seq, q_ld, k_ld, v_ld);
     return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
   }
