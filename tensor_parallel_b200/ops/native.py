@@ -211,14 +211,17 @@ def gemm_nt(x2d: torch.Tensor, w: torch.Tensor, bias=None, residual=None, act=No
     ``[tokens, n]`` are the rows the statistics are taken over when ``x2d`` is only a column slice of them.
     ``out_elems`` (a library built with ``-DTPB_BOUNDS`` only): extent of ``out`` that the kernel checks its store
     indices against; 0 derives it from the shape.  ``early``: the kernel may start, and read ``w``, while the previous kernel
-    of the stream is still running (that kernel must not write ``w``); everything else is read after it."""
+    of the stream is still running (that kernel must not write ``w``); everything else is read after it.  It has no effect on a
+    ``w`` that TMA cannot read in place."""
     global launch_count
     if x_t:
         k, tokens = x2d.shape
     else:
         tokens, k = x2d.shape
     features = w.shape[1] if w_t else w.shape[0]
-    x2d, w = _tma_ready(x2d), _tma_ready(w)
+    x2d, given = _tma_ready(x2d), w
+    w = _tma_ready(w)
+    early = early and w is given  # (a copy is written by the previous kernel of the stream, which early reads do not wait for)
     if out is None:
         out = torch.empty(tokens, features // 2 if act == "swiglu16" else features, dtype=torch.bfloat16, device=x2d.device)
     plan = gemm_plan(tokens, features, k, world, force_splits, force_kbox, no_swap=x_t or w_t)

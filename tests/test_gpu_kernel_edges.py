@@ -113,6 +113,42 @@ def test_early_launch_reads_what_its_predecessor_wrote(tokens):
         assert torch.equal(chain(True), want)
 
 
+def test_decode_step_with_weights_that_tma_cannot_address():
+    """An OPT block of ffn_dim 100 copies its second MLP weight on every step (its pitch is no multiple of 16 bytes): a step with
+    early launches gives the bits of a step without them."""
+    import tensor_parallel_b200 as tp
+    from tensor_parallel_b200.models.opt import OPTConfig, OPTForCausalLM
+
+    nat = _native()
+    torch.manual_seed(0)
+    cfg = OPTConfig(vocab_size=512, hidden_size=256, num_hidden_layers=2, ffn_dim=100, num_attention_heads=4, max_position_embeddings=128)
+    model = OPTForCausalLM(cfg).to("cuda", torch.bfloat16).eval()
+    wrapped = tp.tensor_parallel(model, ["cuda:0"])
+    wrapped.prefill(torch.randint(0, 512, (2, 9)), max_new_tokens=16)
+    engine = wrapped._engine
+    engine.use_graph = False
+    start = engine.pos.clone()
+    plain = nat.gemm_nt
+
+    def steps():
+        engine.pos.copy_(start)
+        engine.ids[:2] = torch.tensor([3, 5], device="cuda")
+        out = []
+        for _ in range(5):
+            engine.decode_step(2)
+            out.append(engine.logits_local[:2].clone())
+        return torch.stack(out)
+
+    got = steps()
+    try:
+        nat.gemm_nt = lambda *a, early=False, **k: plain(*a, **k)
+        want = steps()
+    finally:
+        nat.gemm_nt = plain
+    assert torch.equal(got, want)
+    engine.check_status()
+
+
 @pytest.mark.parametrize("hq,hkv,d,splits", [(8, 8, 128, 1), (8, 2, 64, 4), (12, 2, 128, 2)])
 def test_early_decode_attention_follows_the_projection(hq, hkv, d, splits):
     nat = _native()

@@ -72,3 +72,36 @@ def test_relative_bias_by_distance_equals_the_lookup_of_every_pair(decoder, quer
     table = attention.relative_attention_bias.weight
     (a,), (b,) = torch.autograd.grad(got, table, g), torch.autograd.grad(want, table, g)
     torch.testing.assert_close(a, b)
+
+
+class _Launches:
+    """Stands in for the native library: keeps the options of every GEMM that would have been launched."""
+
+    def __init__(self):
+        self.early = []
+
+    def tpb_gemm_bf16_ex(self, *args):
+        opts = args[15]
+        self.early.append(bool(opts is not None and opts._obj.early))
+        return 0
+
+
+@needs_library
+@pytest.mark.parametrize("pitch,offset,early", [(104, 0, True), (100, 0, False), (104, 1, False), (104, 8, True)])
+def test_a_weight_that_has_to_be_copied_is_not_read_early(monkeypatch, pitch, offset, early):
+    """An early launch reads its weights while the previous kernel of the stream runs; the copy of a weight that TMA cannot address
+    (a pitch that is no multiple of 8 elements, a base off a 16-byte boundary) is exactly that kernel."""
+    from tensor_parallel_b200.ops import native
+
+    lib = _Launches()
+    monkeypatch.setattr(native, "LIB", lib)
+    monkeypatch.setattr(native, "gemm_plan", lambda *a, **k: native.GemmPlan(stream=1))
+    monkeypatch.setattr(native, "device_state", lambda device: type("State", (), {"ctx": native.ReduceCtx()}))
+    monkeypatch.setattr(native, "_stream", lambda: 0)
+    storage = torch.zeros(64 * 104 + 64, dtype=torch.bfloat16)
+    storage = storage[(-storage.data_ptr() % 16) // 2:]
+    w = storage[offset:].as_strided((48, 100), (pitch, 1))
+    x = torch.zeros(2, 104, dtype=torch.bfloat16)[:, :100]
+    native.gemm_nt(x, w, early=True)
+    native.gemm_nt(x, w)
+    assert lib.early == [early, False]
