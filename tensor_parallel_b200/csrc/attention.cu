@@ -405,7 +405,7 @@ __global__ void attn_decode_combine_kernel(const float* __restrict__ part_o, con
 // counters: uint32 [batch * kv_heads], zero-initialised once; they re-arm themselves.
 template <int D, int G>
 __global__ void __launch_bounds__(DEC_THREADS)
-attn_decode_fused_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
+attn_decode_fused_kernel(const bf16* q, const bf16* k, const bf16* v,
                          bf16* __restrict__ kcache, bf16* __restrict__ vcache, bf16* __restrict__ out,
                          float* __restrict__ part_o, float* __restrict__ part_ml, uint32_t* __restrict__ counters,
                          const int* __restrict__ pos_ptr, int q_heads, int kv_heads, int g_total, int g_offset, int max_seq,
@@ -443,6 +443,8 @@ attn_decode_fused_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
       pdl_wait();
       pdl_trigger();
     }
+    static_assert(D <= DEC_THREADS, "one element of v per thread");
+    const float v_new = threadIdx.x < D ? bf16_bits_to_float(ld_after_wait_u16(v + b * v_ld + (long long)kvh * D + threadIdx.x)) : 0.f;
     // rotate q (G heads) and the new k into shared memory; one thread per element pair
     for (int i = threadIdx.x; i < (G + 1) * (D / 2); i += DEC_THREADS) {
       const int hsel = i / (D / 2), p = i % (D / 2);
@@ -462,17 +464,17 @@ attn_decode_fused_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
           const float inv_freq = exp2f(-log2_theta * (2.f * float(p) / float(rotary_dim)));
           sincosf(float(pos) * inv_freq, &sn, &cs);
         }
-        const float a = __bfloat162float(src[ia]), c = __bfloat162float(src[ib]);
+        const float a = bf16_bits_to_float(ld_after_wait_u16(src + ia)), c = bf16_bits_to_float(ld_after_wait_u16(src + ib));
         // round through bf16 like the stand-alone append kernel, so cached and in-flight keys agree bit for bit
         dst[ia] = __bfloat162float(__float2bfloat16(a * cs - c * sn)) * mul;
         dst[ib] = __bfloat162float(__float2bfloat16(c * cs + a * sn)) * mul;
       } else {
         const int e = rotary_dim + 2 * (p - half);
-        dst[e] = __bfloat162float(src[e]) * mul;
-        dst[e + 1] = __bfloat162float(src[e + 1]) * mul;
+        dst[e] = bf16_bits_to_float(ld_after_wait_u16(src + e)) * mul;
+        dst[e + 1] = bf16_bits_to_float(ld_after_wait_u16(src + e + 1)) * mul;
       }
     }
-    for (int i = threadIdx.x; i < D; i += DEC_THREADS) vnew_s[i] = __bfloat162float(v[b * v_ld + (long long)kvh * D + i]);
+    if (threadIdx.x < D) vnew_s[threadIdx.x] = v_new;
     __syncthreads();
     if (owns_new) {  // persist the new key / value for later steps
       for (int i = threadIdx.x; i < D; i += DEC_THREADS) {

@@ -818,7 +818,7 @@ __device__ __forceinline__ bool beats(const Best& a, const Best& b) {  // a come
   return a.v > b.v;
 }
 __global__ void __launch_bounds__(PICK_THREADS)
-greedy_pick_kernel(const bf16* __restrict__ logits, long long ld, int cols, int64_t* __restrict__ next_ids, int64_t* __restrict__ ids,
+greedy_pick_kernel(const bf16* logits, long long ld, int cols, int64_t* __restrict__ next_ids, int64_t* __restrict__ ids,
                    int* __restrict__ pos) {
   __shared__ Best red[PICK_THREADS / 32];
   pdl_wait();
@@ -828,7 +828,7 @@ greedy_pick_kernel(const bf16* __restrict__ logits, long long ld, int cols, int6
 #pragma unroll 4
   for (int c = head + int(threadIdx.x) * 8; c < tail; c += PICK_THREADS * 8) {
     float v[8];
-    Vec8<bf16>::load(x + c, v);
+    unpack(Raw8<bf16>{{ld_after_wait_v4(x + c)}}, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const Best cand = {v[j], c + j};
@@ -838,7 +838,7 @@ greedy_pick_kernel(const bf16* __restrict__ logits, long long ld, int cols, int6
   const int edge = head + cols - tail;  // at most 14 elements outside the 16-byte vectors
   if (int(threadIdx.x) < edge) {
     const int c = int(threadIdx.x) < head ? int(threadIdx.x) : tail + int(threadIdx.x) - head;
-    const Best cand = {to_f<bf16>(x[c]), c};
+    const Best cand = {bf16_bits_to_float(ld_after_wait_u16(x + c)), c};
     if (beats(cand, best)) best = cand;
   }
   auto merge = [&]() {

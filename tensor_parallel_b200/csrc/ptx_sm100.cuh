@@ -407,6 +407,18 @@ __device__ __forceinline__ bool wait_flag_ge(const uint32_t* p, uint32_t target,
 // kernel launched the ordinary way.  Nothing that depends on earlier kernels may be touched before pdl_wait().
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of what the predecessor writes.  Through a `const T* __restrict__` parameter the compiler may take data for constant over
+// the kernel's whole life (non-coherent loads, moved anywhere); these are volatile like pdl_wait() and stay behind it.
+__device__ __forceinline__ uint16_t ld_after_wait_u16(const void* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_after_wait_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float(static_cast<uint32_t>(b) << 16); }
 

@@ -1,6 +1,7 @@
 """Rules that choose a kernel, checked on the CPU: which GEMM shapes may take the single-rank kernels, how the few-token kernel deals
 out its rows, and the relative-position bias by distance against the lookup of every pair."""
 import ctypes
+import re
 
 import pytest
 import torch
@@ -105,3 +106,15 @@ def test_a_weight_that_has_to_be_copied_is_not_read_early(monkeypatch, pitch, of
     native.gemm_nt(x, w, early=True)
     native.gemm_nt(x, w)
     assert lib.early == [early, False]
+
+
+@pytest.mark.parametrize("file,kernel,inputs", [("attention.cu", "attn_decode_fused_kernel", ["q", "k", "v"]), ("elementwise.cu", "greedy_pick_kernel", ["logits"])])
+def test_early_kernels_do_not_call_their_predecessors_output_read_only(file, kernel, inputs):
+    """A kernel that starts before its predecessor ends must not promise the compiler that what the predecessor writes is constant
+    for the kernel's whole life (``const T* __restrict__`` allows read-only loads that move in front of the wait)."""
+    source = (build.CSRC / file).read_text()
+    (parameters,) = re.findall(r"\n" + kernel + r"\((.*?)\) \{", source, re.S)
+    declared = [d.strip() for d in parameters.replace("\n", " ").split(",")]
+    for name in inputs:
+        (declaration,) = [d for d in declared if d.split()[-1] == name]
+        assert "*" in declaration and "__restrict__" not in declaration
