@@ -307,6 +307,8 @@ class DecoderEngine:
             if embed_split:
                 self.embed_split, self.embed, self.pos_embed = True, None, None
         if comm is not None:
+            # what the passes above did not launch: the kernels of the multi-rank projections, whose forms depend on rank count and batch
+            native.check(native.LIB.tpb_gemm_preload(), "tpb_gemm_preload")
             native.check(native.LIB.tpb_comm_preload(), "tpb_comm_preload")
 
     # -- building blocks --------------------------------------------------------------------------

@@ -2,6 +2,7 @@
 out its rows, and the relative-position bias by distance against the lookup of every pair."""
 import ctypes
 import re
+import types
 
 import pytest
 import torch
@@ -118,3 +119,22 @@ def test_early_kernels_do_not_call_their_predecessors_output_read_only(file, ker
     for name in inputs:
         (declaration,) = [d for d in declared if d.split()[-1] == name]
         assert "*" in declaration and "__restrict__" not in declaration
+
+
+@needs_library
+def test_preload_of_a_rank_loads_every_kernel_a_step_may_launch(monkeypatch):
+    """A pass of one rank alone runs other GEMM kernels than a step of several ranks does, and one batch size runs only some of them:
+    ``preload`` loads all of them by name."""
+    from tensor_parallel_b200.engine import DecoderEngine
+    from tensor_parallel_b200.ops import native
+
+    loaded = []
+    library = types.SimpleNamespace(tpb_gemm_preload=lambda: loaded.append("gemm") or 0, tpb_comm_preload=lambda: loaded.append("comm") or 0)
+    monkeypatch.setattr(native, "LIB", library)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    for comm, want in ((object(), {"gemm", "comm"}), (None, set())):
+        engine = types.SimpleNamespace(comm=comm, world=2, head_split="vocab", embed_split=False, max_seq=80, device="cpu", vocab_local=32, x=torch.zeros(1, 8),
+                                       logits_local=torch.zeros(1, 32), pos=torch.zeros(1), ids=torch.zeros(1), prefill=lambda ids: None, _decode_body=lambda batch: None)
+        loaded.clear()
+        DecoderEngine.preload(engine)
+        assert set(loaded) == want and engine.comm is comm and engine.world == 2
