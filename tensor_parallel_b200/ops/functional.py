@@ -144,14 +144,22 @@ def attention(q, k, v, causal: bool, bias=None, scale: Optional[float] = None):
     return attention_ref(q, k, v, causal, bias, scale)
 
 
+def _only_looks_rows_up(embedding: torch.nn.Module) -> bool:
+    """False for an embedding whose call does more than look rows of its weight up: another class, a ``forward`` put on the instance
+    (offloading libraries), hooks of its own or of all modules, renormalisation, sparse or scaled gradients, a weight that is
+    a tensor subclass."""
+    every = torch.nn.modules.module
+    hooks = (embedding._forward_hooks, embedding._forward_pre_hooks, embedding._backward_hooks, embedding._backward_pre_hooks, every._global_forward_hooks,
+             every._global_forward_pre_hooks, every._global_backward_hooks, every._global_backward_pre_hooks)
+    return (type(embedding) is torch.nn.Embedding and "forward" not in vars(embedding) and type(embedding.weight) in (torch.nn.Parameter, torch.Tensor)
+            and embedding.max_norm is None and embedding.padding_idx is None and not embedding.sparse and not embedding.scale_grad_by_freq and not any(hooks))
+
+
 def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
     """Score bias ``[1, heads, queries, keys]`` of a learned table over position buckets; ``buckets`` holds the bucket of each distance
-    ``key - query``, from ``-(queries - 1)`` up, in ``queries + keys - 1`` entries.  An embedding that does more than look rows up (a
-    wrapper, hooks, renormalisation, sparse gradients) is called as the module it is."""
-    plain = (type(embedding) is torch.nn.Embedding and embedding.max_norm is None and embedding.padding_idx is None and not embedding.sparse
-             and not embedding.scale_grad_by_freq and not (embedding._forward_hooks or embedding._forward_pre_hooks or embedding._backward_hooks
-                                                           or embedding._backward_pre_hooks))
-    nat = _native(embedding.weight) if plain and buckets.is_cuda else None
+    ``key - query``, from ``-(queries - 1)`` up, in ``queries + keys - 1`` entries.  An embedding that does more than look rows up is
+    called as the module it is."""
+    nat = _native(embedding.weight) if _only_looks_rows_up(embedding) and buckets.is_cuda else None
     if nat is not None and nat.relative_bias_supported(embedding.weight):
         return nat.relative_bias(embedding.weight, buckets, queries, keys)
     return relative_bias_ref(embedding, buckets, queries, keys)

@@ -9,6 +9,7 @@ import torch
 
 from tensor_parallel_b200 import build
 from tensor_parallel_b200.models.t5 import T5Attention, T5Config, relative_position_bucket
+from tensor_parallel_b200.ops import functional as OF
 
 
 def _plan(tokens, features, k, world=1, splits=0, kbox=0, no_swap=0):
@@ -138,3 +139,65 @@ def test_preload_of_a_rank_loads_every_kernel_a_step_may_launch(monkeypatch):
         loaded.clear()
         DecoderEngine.preload(engine)
         assert set(loaded) == want and engine.comm is comm and engine.world == 2
+
+
+class _OnTheGpu(torch.Tensor):
+    """A CPU tensor that says it is a CUDA tensor: the route of a call is chosen as it is on a GPU."""
+
+    is_cuda = True
+
+
+class _Kernel:
+    """Stands in for the native module: notes that the relative-bias kernel was chosen."""
+
+    taken = False
+
+    def relative_bias_supported(self, *a):
+        return True
+
+    def relative_bias(self, table, buckets, queries, keys):
+        self.taken = True
+        return torch.zeros(1, table.shape[1], queries, keys)
+
+
+def _relative_bias_route(monkeypatch, embedding, buckets, queries, keys):
+    kernel = _Kernel()
+    monkeypatch.setattr(OF, "_native", lambda t: kernel)
+    out = OF.relative_bias(embedding, buckets.as_subclass(_OnTheGpu), queries, keys)
+    monkeypatch.undo()
+    return kernel.taken, out
+
+
+class _OtherEmbedding(torch.nn.Embedding):
+    pass
+
+
+@pytest.mark.parametrize("kind", ["plain", "subclass", "forward on the instance", "hook", "pre-hook", "hook of all modules", "pre-hook of all modules",
+                                  "backward hook of all modules", "padding", "sparse", "weight subclass"])
+def test_an_embedding_that_does_more_than_look_up_is_called(monkeypatch, kind):
+    embedding = (_OtherEmbedding if kind == "subclass" else torch.nn.Embedding)(8, 3, padding_idx=1 if kind == "padding" else None, sparse=kind == "sparse")
+    handle, factor = None, 1.0
+    if kind == "forward on the instance":
+        embedding.forward = lambda index, plain=embedding.forward: plain(index) * 2
+        factor = 2.0
+    elif kind.startswith("hook"):
+        register = embedding.register_forward_hook if kind == "hook" else torch.nn.modules.module.register_module_forward_hook
+        handle = register(lambda module, args, out: out * 2)
+        factor = 2.0
+    elif kind.startswith("pre-hook"):
+        register = embedding.register_forward_pre_hook if kind == "pre-hook" else torch.nn.modules.module.register_module_forward_pre_hook
+        handle = register(lambda module, args: None)
+    elif kind.startswith("backward"):
+        handle = torch.nn.modules.module.register_module_full_backward_hook(lambda module, before, after: None)
+    elif kind == "weight subclass":
+        embedding.weight = torch.nn.Parameter(embedding.weight.data.as_subclass(_OnTheGpu), requires_grad=False)
+    buckets = torch.randint(0, 8, (9,))
+    try:
+        taken, out = _relative_bias_route(monkeypatch, embedding, buckets, 4, 6)
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert taken == (kind == "plain")
+    if not taken:
+        distance = torch.arange(6)[None, :] - torch.arange(4)[:, None] + 3
+        assert torch.equal(torch.as_tensor(out), embedding.weight[buckets[distance]].permute(2, 0, 1)[None] * factor)
