@@ -160,7 +160,7 @@ def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
     ``key - query``, from ``-(queries - 1)`` up, in ``queries + keys - 1`` entries.  An embedding that does more than look rows up is
     called as the module it is."""
     nat = _native(embedding.weight) if _only_looks_rows_up(embedding) and buckets.is_cuda else None
-    if nat is not None and nat.relative_bias_supported(embedding.weight):
+    if nat is not None and nat.relative_bias_supported(embedding.weight, queries, keys):
         return nat.relative_bias(embedding.weight, buckets, queries, keys)
     return relative_bias_ref(embedding, buckets, queries, keys)
 

@@ -754,8 +754,10 @@ LIB.tpb_relative_bias.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_
 LIB.tpb_relative_bias_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
 
 
-def relative_bias_supported(table: torch.Tensor) -> bool:
-    return table.dtype in (torch.bfloat16, torch.float32) and table.ndim == 2 and table.numel() > 0
+def relative_bias_supported(table: torch.Tensor, queries: int, keys: int) -> bool:
+    """Some pair of a query and a key, and a grid that CUDA can launch (16 queries and one head per block)."""
+    return (table.dtype in (torch.bfloat16, torch.float32) and table.ndim == 2 and table.numel() > 0 and table.shape[1] <= 65535 and 0 < queries <= 65535 * 16
+            and keys > 0)
 
 
 class _RelativeBiasFn(torch.autograd.Function):

@@ -62,7 +62,7 @@ def test_row_ranges_cover_every_row_once_in_even_passes(features, sms=148):
 
 
 @pytest.mark.parametrize("decoder", [False, True])
-@pytest.mark.parametrize("queries,keys", [(1, 1), (1, 40), (7, 12), (130, 130), (5, 300)])
+@pytest.mark.parametrize("queries,keys", [(1, 1), (1, 40), (7, 12), (130, 130), (5, 300), (0, 0), (0, 4), (4, 0)])
 def test_relative_bias_by_distance_equals_the_lookup_of_every_pair(decoder, queries, keys):
     torch.manual_seed(0)
     attention = T5Attention(T5Config(num_heads=3, d_kv=8), True, decoder)
@@ -201,3 +201,14 @@ def test_an_embedding_that_does_more_than_look_up_is_called(monkeypatch, kind):
     if not taken:
         distance = torch.arange(6)[None, :] - torch.arange(4)[:, None] + 3
         assert torch.equal(torch.as_tensor(out), embedding.weight[buckets[distance]].permute(2, 0, 1)[None] * factor)
+
+
+@needs_library
+@pytest.mark.parametrize("queries,keys,heads,taken", [(1, 1, 1, True), (0, 5, 2, False), (5, 0, 2, False), (0, 0, 2, False), (65535 * 16 + 1, 1, 1, False), (1, 1, 65536, False)])
+def test_relative_bias_sizes_that_no_grid_covers_are_looked_up(queries, keys, heads, taken):
+    from tensor_parallel_b200.ops import native
+
+    table = torch.zeros(4, heads)
+    assert native.relative_bias_supported(table, queries, keys) == taken
+    if queries * keys == 0:  # the lookup has always taken these
+        assert OF.relative_bias(torch.nn.Embedding(4, heads), torch.zeros(max(0, queries + keys - 1), dtype=torch.int64), queries, keys).shape == (1, heads, queries, keys)
