@@ -106,6 +106,15 @@ def relative_bias_ref(embedding, buckets, queries: int, keys: int):
     return embedding(buckets[j - i + queries - 1]).permute(2, 0, 1)[None]
 
 
+def relative_bias_table_grad_ref(grad, buckets, rows: int):
+    """Gradient of a ``[rows, heads]`` table from that of its bias, ``[1, heads, queries, keys]``; differentiable itself."""
+    heads, queries, keys = grad.shape[1:]
+    i = torch.arange(queries, device=buckets.device)[:, None]
+    j = torch.arange(keys, device=buckets.device)[None, :]
+    pairs = grad[0].permute(1, 2, 0).reshape(queries * keys, heads).float()
+    return torch.zeros(rows, heads, dtype=torch.float32, device=grad.device).index_add(0, buckets[j - i + queries - 1].reshape(-1), pairs)
+
+
 # -- dispatching front-end ---------------------------------------------------------------------
 
 
@@ -155,11 +164,22 @@ def _only_looks_rows_up(embedding: torch.nn.Module) -> bool:
             and embedding.max_norm is None and embedding.padding_idx is None and not embedding.sparse and not embedding.scale_grad_by_freq and not any(hooks))
 
 
+def transformed(t: torch.Tensor) -> bool:
+    """True where an autograd function over raw pointers would drop out of what is going on around it: a functorch transform (vmap,
+    grad, jvp), a batch of gradients (``is_grads_batched``), a forward-mode tangent, a dispatch mode (fake tensors, ``make_fx``), tracing
+    or compilation."""
+    functorch = torch._C._functorch
+    return (functorch.peek_interpreter_stack() is not None or functorch.is_functorch_wrapped_tensor(t) or functorch.is_legacy_batchedtensor(t)
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()
+            or torch.autograd.forward_ad.unpack_dual(t).tangent is not None)
+
+
 def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
     """Score bias ``[1, heads, queries, keys]`` of a learned table over position buckets; ``buckets`` holds the bucket of each distance
     ``key - query``, from ``-(queries - 1)`` up, in ``queries + keys - 1`` entries.  An embedding that does more than look rows up is
     called as the module it is."""
-    nat = _native(embedding.weight) if _only_looks_rows_up(embedding) and buckets.is_cuda else None
+    direct = _only_looks_rows_up(embedding) and not transformed(embedding.weight) and buckets.device == embedding.weight.device
+    nat = _native(embedding.weight) if direct else None
     if nat is not None and nat.relative_bias_supported(embedding.weight, queries, keys):
         return nat.relative_bias(embedding.weight, buckets, queries, keys)
     return relative_bias_ref(embedding, buckets, queries, keys)

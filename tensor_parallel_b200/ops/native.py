@@ -15,6 +15,7 @@ from typing import Dict, Optional, Tuple
 import torch
 
 from tensor_parallel_b200 import build as _build
+from tensor_parallel_b200.ops import functional as OF
 
 _ERRORS = {1: "bad argument", 2: "alignment rule violated", 3: "CUDA runtime error", 4: "driver entry point missing",
            5: "tensor map rejected", 6: "reduction workspace too small", 7: "size beyond compiled-in maximum"}
@@ -779,6 +780,8 @@ class _RelativeBiasFn(torch.autograd.Function):
         global launch_count
         (buckets,) = ctx.saved_tensors
         n, heads, queries, keys, dtype = ctx.meta
+        if torch.is_grad_enabled() or OF.transformed(grad):  # a second derivative, or a batch of gradients
+            return OF.relative_bias_table_grad_ref(grad, buckets, n).to(dtype), None, None, None
         g = grad.to(dtype).contiguous()
         partial = torch.empty(LIB.tpb_relative_bias_parts(queries), n, heads, dtype=torch.float32, device=g.device)
         check(LIB.tpb_relative_bias_bwd(_ptr(g), _ptr(buckets), _ptr(partial), heads, queries, keys, n, _dtype_code(g), _stream()), "tpb_relative_bias_bwd")

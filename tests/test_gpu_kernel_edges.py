@@ -331,3 +331,32 @@ def test_relative_bias_and_its_gradient(queries, keys, dtype):
     rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
     err = (emb.weight.grad.double() - ref.weight.grad).abs()
     assert bool((err <= rel * ref.weight.grad.abs() + 2.0 ** -22 * queries * keys ** 0.5).all())
+
+
+def test_relative_bias_under_transforms():
+    """Second derivative, a batch of output gradients and forward mode, as the lookup itself gives them."""
+    torch.manual_seed(0)
+    heads, n, queries, keys = 5, 12, 33, 40
+    emb = torch.nn.Embedding(n, heads, device="cuda")
+    buckets = torch.randint(0, n, (queries + keys - 1,), device="cuda")
+    out = OF.relative_bias(emb, buckets, queries, keys)
+    want = OF.relative_bias_ref(emb, buckets, queries, keys)
+    assert type(out.grad_fn).__name__.startswith("_RelativeBiasFn")
+    gs = torch.randn(3, *out.shape, device="cuda")
+    (batched,) = torch.autograd.grad(out, emb.weight, gs, is_grads_batched=True, retain_graph=True)
+    for got, g in zip(batched, gs):
+        torch.testing.assert_close(got, torch.autograd.grad(want, emb.weight, g, retain_graph=True)[0], atol=1e-4, rtol=1e-5)
+    g = gs[0].clone().requires_grad_()
+    (first,) = torch.autograd.grad(out, emb.weight, g, create_graph=True)
+    weights = torch.randn(n, heads, device="cuda")
+    (second,) = torch.autograd.grad((first * weights).sum(), g)
+    table = torch.nn.Embedding(n, heads, device="cuda", _weight=weights)
+    assert torch.equal(second, OF.relative_bias_ref(table, buckets, queries, keys))
+
+    with torch.autograd.forward_ad.dual_level():
+        emb.weight.requires_grad_(False)
+        stand_in = torch.nn.Embedding(n, heads, device="cuda")
+        del stand_in.weight
+        stand_in.weight = torch.autograd.forward_ad.make_dual(emb.weight.data, weights)
+        moved = torch.autograd.forward_ad.unpack_dual(OF.relative_bias(stand_in, buckets, queries, keys)).tangent
+        assert torch.equal(moved, OF.relative_bias_ref(table, buckets, queries, keys))

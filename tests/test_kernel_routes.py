@@ -141,10 +141,8 @@ def test_preload_of_a_rank_loads_every_kernel_a_step_may_launch(monkeypatch):
         assert set(loaded) == want and engine.comm is comm and engine.world == 2
 
 
-class _OnTheGpu(torch.Tensor):
-    """A CPU tensor that says it is a CUDA tensor: the route of a call is chosen as it is on a GPU."""
-
-    is_cuda = True
+class _Subclass(torch.Tensor):
+    pass
 
 
 class _Kernel:
@@ -163,7 +161,7 @@ class _Kernel:
 def _relative_bias_route(monkeypatch, embedding, buckets, queries, keys):
     kernel = _Kernel()
     monkeypatch.setattr(OF, "_native", lambda t: kernel)
-    out = OF.relative_bias(embedding, buckets.as_subclass(_OnTheGpu), queries, keys)
+    out = OF.relative_bias(embedding, buckets, queries, keys)
     monkeypatch.undo()
     return kernel.taken, out
 
@@ -190,7 +188,7 @@ def test_an_embedding_that_does_more_than_look_up_is_called(monkeypatch, kind):
     elif kind.startswith("backward"):
         handle = torch.nn.modules.module.register_module_full_backward_hook(lambda module, before, after: None)
     elif kind == "weight subclass":
-        embedding.weight = torch.nn.Parameter(embedding.weight.data.as_subclass(_OnTheGpu), requires_grad=False)
+        embedding.weight = torch.nn.Parameter(embedding.weight.data.as_subclass(_Subclass), requires_grad=False)
     buckets = torch.randint(0, 8, (9,))
     try:
         taken, out = _relative_bias_route(monkeypatch, embedding, buckets, 4, 6)
@@ -212,3 +210,73 @@ def test_relative_bias_sizes_that_no_grid_covers_are_looked_up(queries, keys, he
     assert native.relative_bias_supported(table, queries, keys) == taken
     if queries * keys == 0:  # the lookup has always taken these
         assert OF.relative_bias(torch.nn.Embedding(4, heads), torch.zeros(max(0, queries + keys - 1), dtype=torch.int64), queries, keys).shape == (1, heads, queries, keys)
+
+
+@pytest.mark.parametrize("kind", ["vmap", "grad", "jvp", "forward mode", "trace", "fake tensors"])
+def test_a_transformed_lookup_stays_with_pytorch(monkeypatch, kind):
+    embedding = torch.nn.Embedding(8, 3)
+    buckets = torch.randint(0, 8, (9,))
+    kernel = _Kernel()
+    monkeypatch.setattr(OF, "_native", lambda t: kernel)
+
+    def bias(table):
+        return torch.func.functional_call(_Bias(embedding, buckets), {"embedding.weight": table})
+
+    table, tangent = embedding.weight.detach(), torch.randn(8, 3)
+    want = OF.relative_bias_ref(embedding, buckets, 4, 6).detach()
+    if kind == "vmap":
+        assert torch.equal(torch.func.vmap(bias)(torch.stack([table, 2 * table])), torch.stack([want, 2 * want]))
+    elif kind == "grad":
+        assert torch.func.grad(lambda t: bias(t).sum())(table).sum() == want.numel()
+    elif kind == "jvp":
+        out, moved = torch.func.jvp(bias, (table,), (tangent,))
+        assert torch.equal(out, want) and moved.shape == want.shape and moved.abs().sum() > 0
+    elif kind == "forward mode":
+        with torch.autograd.forward_ad.dual_level():
+            out = bias(torch.autograd.forward_ad.make_dual(table, tangent))
+            assert torch.autograd.forward_ad.unpack_dual(out).tangent is not None
+    elif kind == "trace":
+        traced = torch.jit.trace(_Bias(embedding, buckets), (), check_trace=False)
+        with torch.no_grad():
+            embedding.weight.mul_(2)
+        assert torch.equal(traced(), 2 * want)
+    else:
+        from torch._subclasses.fake_tensor import FakeTensorMode
+
+        with FakeTensorMode(allow_non_fake_inputs=True):
+            assert OF.relative_bias(embedding, buckets, 4, 6).shape == want.shape
+    assert not kernel.taken
+    OF.relative_bias(embedding, buckets, 4, 6)
+    assert kernel.taken
+
+
+class _Bias(torch.nn.Module):
+    def __init__(self, embedding, buckets):
+        super().__init__()
+        self.embedding, self.buckets = embedding, buckets
+
+    def forward(self):
+        return OF.relative_bias(self.embedding, self.buckets, 4, 6)
+
+
+def test_table_gradient_of_a_relative_bias():
+    embedding = torch.nn.Embedding(8, 3, dtype=torch.float64)
+    buckets = torch.randint(0, 8, (9,))
+    out = OF.relative_bias_ref(embedding, buckets, 4, 6)
+    g = torch.randn_like(out)
+    out.backward(g)
+    torch.testing.assert_close(OF.relative_bias_table_grad_ref(g, buckets, 8).double(), embedding.weight.grad, atol=1e-5, rtol=1e-5)
+
+    class Lookup(torch.autograd.Function):  # a batch of gradients reaches a backward as one batched tensor
+        @staticmethod
+        def forward(ctx, table):
+            return OF.relative_bias_ref(lambda index: table[index], buckets, 4, 6)
+
+        @staticmethod
+        def backward(ctx, grad):
+            assert OF.transformed(grad)
+            return OF.relative_bias_table_grad_ref(grad, buckets, 8)
+
+    table = embedding.weight.detach().float().requires_grad_()
+    (batched,) = torch.autograd.grad(Lookup.apply(table), table, torch.stack([g, 2 * g]).float(), is_grads_batched=True)
+    torch.testing.assert_close(batched.double(), torch.stack([embedding.weight.grad, 2 * embedding.weight.grad]), atol=1e-5, rtol=1e-5)
