@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
 #include "tpb_api.h"
 
 namespace tpb {
@@ -26,15 +27,27 @@ constexpr int RB_DIAGS = 1024;           // diagonals folded at a time
 
 __device__ __forceinline__ float rb_float(bf16 x) { return __bfloat162float(x); }
 __device__ __forceinline__ float rb_float(float x) { return x; }
+__device__ __forceinline__ void rb_nan(bf16& x) { x = __ushort_as_bfloat16(0x7FFF); }
+__device__ __forceinline__ void rb_nan(float& x) { x = __int_as_float(0x7FFFFFFF); }
 
+// A bucket that is no row of the table is not looked up: its distance gets NaN, and the status word says so.
 template <typename T>
 __global__ void __launch_bounds__(RB_THREADS)
-relative_bias_kernel(const T* __restrict__ table, const int* __restrict__ buckets, T* __restrict__ out, int heads, int queries, int keys) {
+relative_bias_kernel(const T* __restrict__ table, const int64_t* __restrict__ buckets, T* __restrict__ out, int heads, int queries, int keys,
+                     int n_buckets, uint32_t* status) {
   __shared__ T vals[RB_COLS + RB_ROWS];
   const int h = blockIdx.z, i0 = blockIdx.y * RB_ROWS, j0 = blockIdx.x * RB_COLS;
   const int rows = min(RB_ROWS, queries - i0), cols = min(RB_COLS, keys - j0);
   const int d0 = j0 - (i0 + rows - 1) + queries - 1;  // smallest distance index of the tile
-  for (int e = threadIdx.x; e < cols + rows - 1; e += RB_THREADS) vals[e] = table[(long long)buckets[d0 + e] * heads + h];
+  for (int e = threadIdx.x; e < cols + rows - 1; e += RB_THREADS) {
+    const int64_t b = buckets[d0 + e];
+    if (uint64_t(b) < uint64_t(n_buckets)) {
+      vals[e] = table[b * heads + h];
+    } else {
+      rb_nan(vals[e]);
+      atomicMax(status, uint32_t(STATUS_BAD_ARG));
+    }
+  }
   __syncthreads();
   const int c = threadIdx.x * 8;
   if (c >= cols) return;
@@ -57,7 +70,7 @@ relative_bias_kernel(const T* __restrict__ table, const int* __restrict__ bucket
 // partial: fp32 [ceil(queries / RB_BWD_ROWS)][n_buckets][heads]
 template <typename T>
 __global__ void __launch_bounds__(RB_BWD_THREADS)
-relative_bias_bwd_kernel(const T* __restrict__ grad, const int* __restrict__ buckets, float* __restrict__ partial, int heads, int queries,
+relative_bias_bwd_kernel(const T* __restrict__ grad, const int64_t* __restrict__ buckets, float* __restrict__ partial, int heads, int queries,
                          int keys, int n_buckets) {
   __shared__ float diag[RB_DIAGS];
   __shared__ int which[RB_DIAGS];
@@ -76,7 +89,8 @@ relative_bias_bwd_kernel(const T* __restrict__ grad, const int* __restrict__ buc
 #pragma unroll 8
       for (int r = r_lo; r < r_hi; ++r) s += rb_float(g[(long long)r * keys + j0 + r]);
       diag[e] = s;
-      which[e] = buckets[d0 + e0 + e];
+      const int64_t b = buckets[d0 + e0 + e];
+      which[e] = uint64_t(b) < uint64_t(n_buckets) ? int(b) : -1;  // (reported by the forward)
     }
     __syncthreads();
     for (int b0 = 0; b0 < n_buckets; b0 += 32) {  // 32 buckets x 8 slices of the diagonals
@@ -100,25 +114,29 @@ relative_bias_bwd_kernel(const T* __restrict__ grad, const int* __restrict__ buc
 
 using namespace tpb;
 
-// table: [n_buckets, heads] contiguous; buckets: int32 [queries + keys - 1], every value in [0, n_buckets); out: [heads, queries, keys].
-// dtype: 0 = bf16, 1 = fp32.
-extern "C" int tpb_relative_bias(const void* table, const int* buckets, void* out, int heads, int queries, int keys, int dtype, void* stream_) {
-  if (!table || !buckets || !out || heads <= 0 || queries <= 0 || keys <= 0 || heads > 65535 || (queries + RB_ROWS - 1) / RB_ROWS > 65535) return TPB_ERR_ARG;
+// table: [n_buckets, heads] contiguous; buckets: int64 [queries + keys - 1]; out: [heads, queries, keys]; dtype: 0 = bf16, 1 = fp32.
+// status: device word that becomes STATUS_BAD_ARG if a bucket is not in [0, n_buckets).
+extern "C" int tpb_relative_bias(const void* table, const int64_t* buckets, void* out, int heads, int queries, int keys, int n_buckets, int dtype,
+                                 void* status, void* stream_) {
+  if (!table || !buckets || !out || !status || heads <= 0 || queries <= 0 || keys <= 0 || n_buckets <= 0 || heads > 65535 ||
+      (queries + RB_ROWS - 1) / RB_ROWS > 65535)
+    return TPB_ERR_ARG;
   if (reinterpret_cast<uintptr_t>(out) & 15) return TPB_ERR_ALIGN;
   const dim3 grid((keys + RB_COLS - 1) / RB_COLS, (queries + RB_ROWS - 1) / RB_ROWS, heads);
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  uint32_t* st = static_cast<uint32_t*>(status);
   if (dtype == 0)
-    relative_bias_kernel<bf16><<<grid, RB_THREADS, 0, s>>>((const bf16*)table, buckets, (bf16*)out, heads, queries, keys);
+    relative_bias_kernel<bf16><<<grid, RB_THREADS, 0, s>>>((const bf16*)table, buckets, (bf16*)out, heads, queries, keys, n_buckets, st);
   else
-    relative_bias_kernel<float><<<grid, RB_THREADS, 0, s>>>((const float*)table, buckets, (float*)out, heads, queries, keys);
+    relative_bias_kernel<float><<<grid, RB_THREADS, 0, s>>>((const float*)table, buckets, (float*)out, heads, queries, keys, n_buckets, st);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
 // Rows of partial tables that tpb_relative_bias_bwd writes.
 extern "C" int tpb_relative_bias_parts(int queries) { return (queries + RB_BWD_ROWS - 1) / RB_BWD_ROWS; }
 
-// grad: [heads, queries, keys] contiguous; partial: fp32 [tpb_relative_bias_parts(queries)][n_buckets][heads], to be summed by the caller.
-extern "C" int tpb_relative_bias_bwd(const void* grad, const int* buckets, float* partial, int heads, int queries, int keys, int n_buckets, int dtype,
+// grad: [heads, queries, keys] contiguous; buckets as above, those out of range contribute nothing; partial: fp32 [tpb_relative_bias_parts(queries)][n_buckets][heads], to be summed by the caller.
+extern "C" int tpb_relative_bias_bwd(const void* grad, const int64_t* buckets, float* partial, int heads, int queries, int keys, int n_buckets, int dtype,
                                      void* stream_) {
   if (!grad || !buckets || !partial || heads <= 0 || queries <= 0 || keys <= 0 || n_buckets <= 0 || heads > 65535) return TPB_ERR_ARG;
   const dim3 grid(tpb_relative_bias_parts(queries), heads);

@@ -178,7 +178,8 @@ def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
     """Score bias ``[1, heads, queries, keys]`` of a learned table over position buckets; ``buckets`` holds the bucket of each distance
     ``key - query``, from ``-(queries - 1)`` up, in ``queries + keys - 1`` entries.  An embedding that does more than look rows up is
     called as the module it is."""
-    direct = _only_looks_rows_up(embedding) and not transformed(embedding.weight) and buckets.device == embedding.weight.device
+    direct = (_only_looks_rows_up(embedding) and not transformed(embedding.weight) and buckets.device == embedding.weight.device
+              and buckets.dtype in (torch.int64, torch.int32) and buckets.ndim == 1 and buckets.shape[0] >= queries + keys - 1)
     nat = _native(embedding.weight) if direct else None
     if nat is not None and nat.relative_bias_supported(embedding.weight, queries, keys):
         return nat.relative_bias(embedding.weight, buckets, queries, keys)

@@ -136,7 +136,8 @@ class DeviceState:
         code = int(self.status[0].item())
         if code:
             self.status.zero_()
-            raise RuntimeError({1: "an mbarrier wait", 2: "a peer flag wait"}.get(code, f"status {code}") + " timed out inside a kernel")
+            raise RuntimeError({1: "an mbarrier wait timed out inside a kernel", 2: "a peer flag wait timed out inside a kernel",
+                                3: "a kernel met an index outside its range"}.get(code, f"status {code} from a kernel"))
 
 
 _states: Dict[int, DeviceState] = {}
@@ -751,7 +752,7 @@ def qkv_rope_append(q, k, v, q_out, kcache, vcache, base_pos, batch, seq, rotary
     return q_out
 
 
-LIB.tpb_relative_bias.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
+LIB.tpb_relative_bias.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
 LIB.tpb_relative_bias_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
 
 
@@ -767,9 +768,10 @@ class _RelativeBiasFn(torch.autograd.Function):
         global launch_count
         n, heads = table.shape
         table = table.contiguous()
-        buckets = buckets.to(torch.int32).contiguous()
+        buckets = buckets.to(torch.int64).contiguous()
         out = torch.empty(1, heads, queries, keys, dtype=table.dtype, device=table.device)
-        check(LIB.tpb_relative_bias(_ptr(table), _ptr(buckets), _ptr(out), heads, queries, keys, _dtype_code(table), _stream()), "tpb_relative_bias")
+        check(LIB.tpb_relative_bias(_ptr(table), _ptr(buckets), _ptr(out), heads, queries, keys, n, _dtype_code(table),
+                                    _ptr(device_state(table.device).status), _stream()), "tpb_relative_bias")
         launch_count += 1
         ctx.save_for_backward(buckets)
         ctx.meta = (n, heads, queries, keys, table.dtype)
@@ -791,7 +793,8 @@ class _RelativeBiasFn(torch.autograd.Function):
 
 def relative_bias(table, buckets, queries, keys):
     """``out[0, h, i, j] = table[buckets[j - i + queries - 1], h]`` for a ``[n_buckets, heads]`` table and the bucket of each of the
-    ``queries + keys - 1`` distances (values must be valid rows of the table)."""
+    ``queries + keys - 1`` distances.  A bucket that is no row of the table gives NaN and sets the device's status word
+    (:meth:`DeviceState.check_status` raises)."""
     return _RelativeBiasFn.apply(table, buckets, int(queries), int(keys))
 
 

@@ -360,3 +360,25 @@ def test_relative_bias_under_transforms():
         stand_in.weight = torch.autograd.forward_ad.make_dual(emb.weight.data, weights)
         moved = torch.autograd.forward_ad.unpack_dual(OF.relative_bias(stand_in, buckets, queries, keys)).tangent
         assert torch.equal(moved, OF.relative_bias_ref(table, buckets, queries, keys))
+
+
+@pytest.mark.parametrize("bad", [12, -1, 2 ** 32, -(2 ** 32) + 3])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_relative_bias_with_a_bucket_out_of_range(bad, dtype):
+    """No row is read for it: its distance is NaN in every head, the status word says so, and its gradient goes nowhere."""
+    nat = _native()
+    torch.manual_seed(0)
+    heads, n, queries, keys = 3, 12, 20, 33
+    emb = torch.nn.Embedding(n, heads, device="cuda", dtype=dtype)
+    buckets = torch.randint(0, n, (queries + keys - 1,), device="cuda")
+    want = OF.relative_bias_ref(emb, buckets, queries, keys).detach()
+    distance = torch.arange(keys, device="cuda")[None, :] - torch.arange(queries, device="cuda")[:, None] + queries - 1
+    hit = (distance == 30)[None, None].expand_as(want)
+    buckets[30] = bad
+    out = OF.relative_bias(emb, buckets, queries, keys)
+    assert bool(out[hit].isnan().all()) and torch.equal(out[~hit], want[~hit])
+    with pytest.raises(RuntimeError, match="index"):
+        nat.device_state(out.device).check_status()
+    out.backward(hit.to(dtype))
+    assert emb.weight.grad.abs().max().item() == 0
+    nat.device_state(out.device).check_status()

@@ -280,3 +280,17 @@ def test_table_gradient_of_a_relative_bias():
     table = embedding.weight.detach().float().requires_grad_()
     (batched,) = torch.autograd.grad(Lookup.apply(table), table, torch.stack([g, 2 * g]).float(), is_grads_batched=True)
     torch.testing.assert_close(batched.double(), torch.stack([embedding.weight.grad, 2 * embedding.weight.grad]), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("buckets", [torch.zeros(8, dtype=torch.int64), torch.zeros(9), torch.zeros(9, dtype=torch.bool), torch.zeros(9, device="meta", dtype=torch.int64)])
+def test_buckets_that_a_lookup_does_not_take_do_not_reach_the_kernel(monkeypatch, buckets):
+    """Too few of them, of a type that is no index, on another device: PyTorch's own answer, mostly an error."""
+    kernel = _Kernel()
+    monkeypatch.setattr(OF, "_native", lambda t: kernel)
+    embedding = torch.nn.Embedding(8, 3)
+    if buckets.device.type == "meta":
+        OF.relative_bias(embedding, buckets, 4, 6)
+    else:
+        with pytest.raises((IndexError, RuntimeError)):
+            OF.relative_bias(embedding, buckets, 4, 6)
+    assert not kernel.taken
