@@ -233,6 +233,34 @@ def test_loss_statistics_with_infinite_logits():
     assert (lse - logits.double().logsumexp(-1)).abs().max().item() < 1e-5
 
 
+def _rounded_between(got, low, high):
+    """Every bf16 of ``got`` is the rounding of some value from ``low`` to ``high`` (fp64)."""
+    low, high = torch.minimum(low, high), torch.maximum(low, high)
+    return bool(((got >= low.float().to(torch.bfloat16)) & (got <= high.float().to(torch.bfloat16))).all())
+
+
+def test_loss_gradient_has_the_accuracy_of_the_fp32_exponential():
+    """Probabilities from 1 down to exp(-70), confident labels (p - 1 near 0) among them.  Given the fp32 difference of logit and
+    log-sum-exp, the exponential is within 2 units in the last place: what is rounded to bf16 lies in that interval."""
+    from tensor_parallel_b200.ops import loss as L
+
+    nat = _native()
+    torch.manual_seed(0)
+    rows, cols = 1024, 4096
+    logits = (-70 * torch.rand(rows, cols, device="cuda")).to(torch.bfloat16)
+    labels = torch.randint(0, cols, (rows,), device="cuda")
+    at = (torch.arange(rows, device="cuda"), labels)
+    logits[at] = 0.0
+    lse = torch.logspace(-7, 0, rows, device="cuda")  # (the label has all but 1e-7 .. all but 1 - 1 / e of the mass)
+    p = (logits.float() - lse[:, None]).double().exp()
+    low, high = p * (1 - 2.0 ** -22), p * (1 + 2.0 ** -22)
+    low[at] -= 1
+    high[at] -= 1
+    scale = torch.ones(1, device="cuda")
+    nat.check(L.LIB.tpb_ce_grad(logits.data_ptr(), labels.data_ptr(), lse.data_ptr(), rows, cols, cols, 0, -100, scale.data_ptr(), nat._stream()), "ce_grad")
+    assert _rounded_between(logits, low, high)
+
+
 @pytest.mark.parametrize("heads,tokens", [(1, 3), (3, 700), (12, 65), (33, 2100)])
 @pytest.mark.parametrize("interleaved,rotary", [(False, 128), (False, 64), (True, 32)])
 def test_rope_head_groups(heads, tokens, interleaved, rotary):
