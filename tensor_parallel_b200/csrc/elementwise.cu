@@ -382,17 +382,8 @@ __global__ void rope_tail_kernel(const T* __restrict__ x, T* __restrict__ out, i
 // ------------------------------------------------------------------------------------------------
 // Activations.  kind: 1 relu, 2 gelu(erf), 3 gelu(tanh), 4 silu.  Gated variants compute act(gate) * up.
 // ------------------------------------------------------------------------------------------------
-// FAST (bf16 data): the logistic function from the hardware exponential and reciprocal, a few units in the 22nd bit off - far
-// below the bf16 rounding of the result - instead of the IEEE sequences, which made the gated kernels compute-bound.  The
-// exponential is taken of -|x|, so the divisor stays in [1, 2].
-template <bool FAST>
-__device__ __forceinline__ float logistic(float x) {
-  if (!FAST) return 1.f / (1.f + expf(-x));
-  const float e = __expf(-fabsf(x)), r = __fdividef(1.f, 1.f + e);
-  return x >= 0.f ? r : e * r;
-}
 // act(x), and with GRAD its derivative, sharing the transcendental
-template <int KIND, bool FAST, bool GRAD>
+template <int KIND, bool GRAD>
 __device__ __forceinline__ float act_eval(float x, float& grad) {
   if (KIND == 1) {
     if (GRAD) grad = x > 0.f ? 1.f : 0.f;
@@ -409,22 +400,26 @@ __device__ __forceinline__ float act_eval(float x, float& grad) {
     return 0.5f * x * (1.f + t);
   }
   if (KIND == 4) {
-    const float s = logistic<FAST>(x);
-    if (GRAD) grad = s * (1.f + x * (1.f - s));
-    return FAST ? x * s : x / (1.f + expf(-x));
+    const float e = 1.f + expf(-x);
+    if (GRAD) {
+      const float s = 1.f / e;
+      grad = s * (1.f + x * (1.f - s));
+    }
+    return x / e;
   }
   if (GRAD) grad = 1.f;
   return x;
 }
 
-// Memory-bound when the arithmetic above fits beside it (8192 x 11008 gated silu, 541 MB forward and 902 MB backward: 136 -> 83 us
-// and 247 -> 143 us against IEEE divisions and a row division per vector): two 8-element vectors per thread and step, one instantiation per
-// activation.  Logical shape [rows, cols]; gate / up may be column slices of a wider fused projection (leading dims); DENSE:
-// they are not, and a vector's position is its index.
+// Two 8-element vectors per thread and step, one instantiation per activation, no row division where rows lie one after another
+// (8192 x 11008 gated, 541 MB forward and 902 MB backward: silu 134 -> 108 us and 227 -> 165 us, gelu 145 -> 113 and 321 -> 172,
+// gelu(tanh) 128 -> 98 and 226 -> 148).  Memory-bound with relu (89 and 146 us); expf, erff and the IEEE divisions cost the others
+// up to 24 us on top.  The hardware exponential and reciprocal would take silu to 92 and 147 us, at the cost of digits (an error of
+// 1.16 |x| units in the last place).  Logical shape [rows, cols]; gate / up may be column slices of a wider fused projection
+// (leading dims); DENSE: they are not, and a vector's position is its index.
 template <typename T, int KIND, bool DENSE>
 __global__ void __launch_bounds__(256)
 act_fwd_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ out, long long nvec, int cols, long long gate_ld, long long up_ld) {
-  constexpr bool FAST = sizeof(T) == 2;
   constexpr int U = 2;
   const int vec_per_row = cols >> 3;
   const long long step = (long long)gridDim.x * blockDim.x;
@@ -448,7 +443,7 @@ act_fwd_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restri
         unpack(g[k], gv);
         if (up) unpack(u[k], uv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = act_eval<KIND, FAST, false>(gv[j], unused) * (up ? uv[j] : 1.f);
+        for (int j = 0; j < 8; ++j) o[j] = act_eval<KIND, false>(gv[j], unused) * (up ? uv[j] : 1.f);
         Vec8<T>::store(out + i * 8, o);
       }
     }
@@ -458,7 +453,6 @@ act_fwd_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restri
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256)
 act_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ dgate, T* __restrict__ dup, long long nvec) {
-  constexpr bool FAST = sizeof(T) == 2;
   constexpr int U = 2;
   const long long step = (long long)gridDim.x * blockDim.x;
   for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < nvec; i0 += U * step) {
@@ -483,7 +477,7 @@ act_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gate, const T* 
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float grad;
-          const float f = act_eval<KIND, FAST, true>(gv[j], grad);
+          const float f = act_eval<KIND, true>(gv[j], grad);
           dg[j] = dv[j] * grad * (up ? uv[j] : 1.f);
           du[j] = dv[j] * f;
         }
