@@ -34,20 +34,17 @@
 
 namespace tpb {
 
-constexpr int GS_UNIT = 32;      // rows of a unit = rows of a weight box; the gated activation pairs 16 gate rows with their 16 up rows
+constexpr int GS_UNIT = StreamRows::UNIT;
 constexpr int GS_BK = 64;        // columns of a box: 128-byte swizzled rows
 constexpr int GS_THREADS = 192;
 constexpr int GS_EPI = 128;
 constexpr int GS_MAX_STAGES = 16;
-constexpr int GS_PASS_UNITS = 4;
 __host__ __device__ constexpr size_t GS_SLICE_BYTES(int ks) { return ks > 1 ? 9 * 1024 : 0; }
 
 struct GsParams {
-  int features, tokens, k_stages, units;
-  int passes;           // of every CTA
+  int features, tokens, k_stages;
+  StreamRows rows;      // (a stage's layout follows its pass_units; tmap_w loads boxes of its box_units, tmap_w1 of one unit)
   int slice_cols;       // KS > 1: columns of a slice
-  int pass_units;       // units of the longest pass of any CTA: the shared-memory layout of a stage follows it
-  int box_units;        // units of a full weight box (tmap_w); what is left of a pass comes in boxes of one unit (tmap_w1)
   int stages, early;
   int ld_out, act;
   float bias_scale;
@@ -92,7 +89,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   constexpr int STEPS = KBOX * (GS_BK / 16);  // MMAs of a stage; step n of the pass goes to accumulator n % NACC
   static_assert(TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0 && TMEM_COLS >= 32, "TMEM allocation");
   constexpr int TOK = BN / KS;  // token columns of a slice
-  const uint32_t w_box = uint32_t(KS > 1 ? KS : p.pass_units) * GS_UNIT * 128;  // [rows of a pass, or of all slices][64 columns]
+  const uint32_t w_box = uint32_t(KS > 1 ? KS : p.rows.pass_units) * GS_UNIT * 128;  // [rows of a pass, or of all slices][64 columns]
   const uint32_t w_bytes = KBOX * w_box, stage_bytes = w_bytes + X_BYTES;
 
   extern __shared__ uint8_t gs_smem_raw[];
@@ -109,12 +106,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   uint8_t* ring = smem + 1024 + GS_SLICE_BYTES(KS);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be uniform)
-  const int unit0 = int((long long)blockIdx.x * p.units / gridDim.x), unit1 = int((long long)(blockIdx.x + 1) * p.units / gridDim.x);
-  // the same number of passes everywhere, of even length: a short pass behind a full one would stream with most of the ring empty
-  // (22016 rows, 4 or 5 units per CTA: 4 + 1 units 39 us, 2 + 3 units 33 us)
-  const int passes = p.passes, my_units = unit1 - unit0;
-  auto pass_start = [&](int i) { return unit0 + my_units * i / passes; };
-  auto pass_units = [&](int i) { return my_units * (i + 1) / passes - my_units * i / passes; };
+  const int unit0 = p.rows.first(blockIdx.x), my_units = p.rows.first(blockIdx.x + 1) - unit0, passes = p.rows.passes;
+  auto pass_start = [&](int i) { return p.rows.pass_start(unit0, my_units, i); };
+  auto pass_units = [&](int i) { return pass_start(i + 1) - pass_start(i); };
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_w);
@@ -168,7 +162,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         return;
       }
       int done = 0;
-      for (; done + p.box_units <= u; done += p.box_units) {
+      for (; done + p.rows.box_units <= u; done += p.rows.box_units) {
 #pragma unroll
         for (int j = 0; j < KBOX; ++j)  // (columns and rows past the end arrive as zeros)
           tma_load_2d_lead(leader, dst + j * w_box + done * GS_UNIT * 128, &tmap_w, bar, col0 + j * GS_BK, row0 + done * GS_UNIT);
@@ -433,14 +427,8 @@ static int gs_launch(const StreamGemm& g, int sms, cudaStream_t stream) {
   p.tokens = g.tokens;
   p.k_stages = ((g.k + KS - 1) / KS + KBOX * GS_BK - 1) / (KBOX * GS_BK);  // (of a slice)
   p.slice_cols = p.k_stages * KBOX * GS_BK;
-  p.units = (g.features + GS_UNIT - 1) / GS_UNIT;
-  const int grid = p.units < sms ? p.units : sms;
-  const int most = (p.units + grid - 1) / grid;  // units of the CTA with the longest range
-  const int least = p.units / grid;              // and of the one with the shortest
-  p.passes = (most + GS_PASS_UNITS - 1) / GS_PASS_UNITS;
-  p.pass_units = (most + p.passes - 1) / p.passes;
-  p.box_units = least / p.passes;                // the shortest pass is one box (what longer ones have beyond it: boxes of one unit)
-  const size_t w_box = size_t(KS > 1 ? KS : p.pass_units) * GS_UNIT * 128;
+  p.rows = gemm_stream_rows(g.features, sms);
+  const size_t w_box = size_t(KS > 1 ? KS : p.rows.pass_units) * GS_UNIT * 128;
   const size_t stage_bytes = size_t(KBOX) * (w_box + BN * GS_BK * 2);
   // an MMA of M = 64 / 128 rows reads that many rows from the last weight box of the ring: what lies behind the last token box
   const size_t need = size_t(128) * 128, have = w_box + size_t(KBOX) * BN * GS_BK * 2;
@@ -458,7 +446,7 @@ static int gs_launch(const StreamGemm& g, int sms, cudaStream_t stream) {
     configured[dev].store(true, std::memory_order_release);
   }
   CUtensorMap tw, tw1, tx;
-  int rc = gs_tmap(&tw, g.w, g.features, g.k, g.ldw, p.box_units * GS_UNIT);
+  int rc = gs_tmap(&tw, g.w, g.features, g.k, g.ldw, p.rows.box_units * GS_UNIT);
   if (rc == TPB_OK) rc = gs_tmap(&tw1, g.w, g.features, g.k, g.ldw, GS_UNIT);
   if (rc == TPB_OK) rc = gs_tmap(&tx, g.x, g.tokens, g.k, g.ldx, BN / KS);
   if (rc != TPB_OK) return rc;
@@ -477,7 +465,7 @@ static int gs_launch(const StreamGemm& g, int sms, cudaStream_t stream) {
   p.norm_rowsum = g.norm_rowsum;
   p.status = g.status;
   p.out_elems = g.out_elems;
-  return launch_dependent(gemm_stream_kernel<BN, NACC, KBOX, KS>, dim3(grid), dim3(GS_THREADS), smem, stream, g.early != 0 || pdl_enabled(), tw, tw1, tx, p) ==
+  return launch_dependent(gemm_stream_kernel<BN, NACC, KBOX, KS>, dim3(p.rows.grid), dim3(GS_THREADS), smem, stream, g.early != 0 || pdl_enabled(), tw, tw1, tx, p) ==
                  cudaSuccess
              ? TPB_OK
              : TPB_ERR_CUDA;
@@ -520,3 +508,16 @@ cudaError_t gemm_stream_preload() {
 }
 
 }  // namespace tpb
+
+// The decomposition of a few-token GEMM, for tests: shape = {units, grid, passes, pass_units, box_units}, and at starts[0 .. passes] the
+// units at which the passes of CTA `cta` begin and the last one ends (room for `capacity` of them).
+extern "C" int tpb_gemm_stream_rows(int features, int sms, int cta, int* shape, int* starts, int capacity) {
+  if (features <= 0 || sms <= 0 || cta < 0 || !shape || !starts) return TPB_ERR_ARG;
+  const tpb::StreamRows r = tpb::gemm_stream_rows(features, sms);
+  if (cta >= r.grid || r.passes >= capacity) return TPB_ERR_ARG;
+  const int values[5] = {r.units, r.grid, r.passes, r.pass_units, r.box_units};
+  memcpy(shape, values, sizeof(values));
+  const int unit0 = r.first(cta), mine = r.first(cta + 1) - unit0;
+  for (int i = 0; i <= r.passes; ++i) starts[i] = r.pass_start(unit0, mine, i);
+  return TPB_OK;
+}

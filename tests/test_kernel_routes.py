@@ -39,25 +39,27 @@ def test_single_rank_kernels_leave_the_other_forms_alone(tokens, features, k):
     assert (plan.swapped, plan.m_tiles, plan.n_tiles) == (forced.swapped, forced.m_tiles, forced.n_tiles)
 
 
+@needs_library
 @pytest.mark.parametrize("features", [1, 32, 33, 1000, 4736, 4737, 4768, 9472, 12288, 22016, 32003, 65024, 151936])
 def test_row_ranges_cover_every_row_once_in_even_passes(features, sms=148):
-    """The integer arithmetic of the few-token kernel: ranges of 32-row units, the same number of passes everywhere, a box no pass is
-    shorter than."""
-    units = -(-features // 32)
-    grid = min(units, sms)
-    most, least = -(-units // grid), units // grid
-    passes = -(-most // 4)
-    longest, box = -(-most // passes), least // passes
-    assert 1 <= box and longest <= 4
+    """The decomposition that the few-token kernel and its launch use: ranges of 32-row units, the same number of passes everywhere, none
+    longer than the shared-memory layout or the 128 rows of an accumulator, none shorter than a box."""
+    from tensor_parallel_b200.ops import native
+
+    shape, starts = (ctypes.c_int * 5)(), (ctypes.c_int * 64)()
+
+    def rows(cta):
+        native.check(native.LIB.tpb_gemm_stream_rows(features, sms, cta, shape, starts, 64), "gemm_stream_rows")
+        units, grid, passes, longest, box = shape
+        return units, grid, passes, longest, box, list(starts[: passes + 1])
+
+    units, grid, _, longest, box, _ = rows(0)
+    assert units == -(-features // 32) and grid == min(units, sms) and 1 <= box <= longest <= 4
     covered = []
-    for c in range(grid):
-        u0, u1 = c * units // grid, (c + 1) * units // grid
-        n = u1 - u0
-        assert least <= n <= most
-        starts = [u0 + n * i // passes for i in range(passes + 1)]
-        assert starts[0] == u0 and starts[-1] == u1
-        assert all(box <= b - a <= longest for a, b in zip(starts, starts[1:]))
-        covered += list(range(u0, u1))
+    for cta in range(grid):
+        *_, at = rows(cta)
+        assert all(box <= b - a <= longest for a, b in zip(at, at[1:]))
+        covered += list(range(at[0], at[-1]))
     assert covered == list(range(units))
 
 
