@@ -364,6 +364,33 @@ def test_bias_rows_in_vectors_and_one_by_one(sq, sk, layout):
         assert (a.double() - r.grad).norm() <= 0.02 * r.grad.norm()
 
 
+# head_dim 128 and 64, causal with several key tiles and with a shift, grouped heads, a bias for each batch or for all heads, ragged tiles
+@pytest.mark.parametrize("b,sq,sk,hq,hkv,d,causal,shape", [
+    (2, 304, 304, 4, 2, 128, True, (1, 4, 304, 304)), (2, 200, 328, 4, 2, 64, True, (2, 4, 200, 328)), (1, 136, 264, 8, 8, 128, False, (1, 1, 136, 264)),
+    (3, 128, 128, 2, 2, 128, False, (3, 2, 128, 128)), (2, 65, 72, 4, 1, 64, True, (1, 4, 65, 72)), (2, 257, 384, 6, 2, 128, True, (2, 1, 257, 384))])
+def test_dense_bf16_bias_that_travels_with_the_tiles(b, sq, sk, hq, hkv, d, causal, shape):
+    torch.manual_seed(sq + sk)
+    q = torch.randn(b, sq, hq, d, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    k, v = (torch.randn(b, sk, hkv, d, device="cuda", dtype=torch.bfloat16).requires_grad_() for _ in range(2))
+    bias = torch.randn(shape, device="cuda", dtype=torch.bfloat16)
+    bias[..., 1:].masked_fill_(torch.rand(shape, device="cuda")[..., 1:] < 0.1, -math.inf)
+    bias.requires_grad_()
+    g = torch.randn(b, sq, hq, d, device="cuda", dtype=torch.bfloat16)
+    out = OF.attention(q, k, v, causal, bias=bias)
+    out.backward(g)
+    ref = [t.detach().double().requires_grad_() for t in (q, k, v, bias)]
+    keys, values = (t.repeat_interleave(hq // hkv, 2) for t in ref[1:3])
+    scores = torch.einsum("bqhd,bkhd->bhqk", ref[0], keys) / math.sqrt(d) + ref[3]
+    if causal:
+        scores = scores.masked_fill(torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(sk - sq + 1), -math.inf)
+    want = torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1), values)
+    want.backward(g.double())
+    # probabilities and dS pass through bf16 (2^-9 each) on their way into sums that cancel
+    for a, r in zip((out.detach(), q.grad, k.grad, v.grad, bias.grad), (want.detach(), *(t.grad for t in ref))):
+        assert (a.double() - r).norm() <= 0.02 * r.norm()
+    _native().device_state(q.device).check_status()
+
+
 @pytest.mark.parametrize("queries,keys", [(1, 1), (1, 9), (17, 40), (64, 1032), (65, 2100), (512, 512)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_relative_bias_and_its_gradient(queries, keys, dtype):
