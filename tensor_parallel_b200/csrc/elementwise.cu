@@ -527,7 +527,12 @@ __device__ __forceinline__ void adamw_update(float g, float& p, float& m, float&
 
 // VEC: 8 elements per thread and step with 16-byte accesses (all pointers 16-byte aligned; the last n % 8 elements are done one
 // by one): up to ten independent 16-byte loads per thread are in flight, where the element-wise form has five of 2 to 4 bytes
-// (202 M parameters with master weights: 1260 us element-wise, 944 us = 6.4 TB/s in vectors).
+// (202 M parameters with master weights: 1260 us element-wise, 944 us = 6.4 TB/s in vectors).  A thread's eight updates are a chain
+// of square roots and divisions that few threads do not hide: below ADAMW_VEC_MIN elements one thread per element is faster (bf16
+// with master weights, element-wise and in vectors: 4096 elements 2.1 and 3.3 us, 100 000 2.6 and 3.6, 400 000 4.4 and 4.6,
+// 600 000 5.6 and 4.8).
+constexpr long long ADAMW_VEC_MIN = 1 << 19;
+
 template <typename P, typename G, bool VEC>
 __global__ void __launch_bounds__(256)
 adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, float* __restrict__ m, float* __restrict__ v, float* __restrict__ master,
@@ -738,7 +743,7 @@ extern "C" int tpb_adamw(void* param, const void* grad, float* m, float* v, floa
   if (!param || !grad || !m || !v || n <= 0 || step < 1) return TPB_ERR_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const AdamwArgs a = {lr, beta1, beta2, eps, weight_decay, 1.f - powf(beta1, float(step)), 1.f - powf(beta2, float(step)), grad_scale};
-  const bool vec = !((reinterpret_cast<uintptr_t>(param) | reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(m) |
+  const bool vec = n >= ADAMW_VEC_MIN && !((reinterpret_cast<uintptr_t>(param) | reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(m) |
                       reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(master)) & 15);
 #define LAUNCH(P, G)                                                                                                                  \
   do {                                                                                                                                \

@@ -297,7 +297,8 @@ def test_rope_head_groups(heads, tokens, interleaved, rotary):
     assert torch.equal(got[..., rotary:], x[..., rotary:])
 
 
-@pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (8, 0), (4099, 0), (4096, 1)])
+# (vectors of eight from 2^19 elements on)
+@pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (8, 0), (4099, 0), (4096, 1), ((1 << 19) - 1, 0), (1 << 19, 0), ((1 << 19) + 7, 0), (1 << 19, 1)])
 @pytest.mark.parametrize("dtype,gdtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
 def test_adamw_remainders_and_alignment(n, offset, dtype, gdtype):
     nat = _native()
