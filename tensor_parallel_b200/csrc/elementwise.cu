@@ -411,8 +411,8 @@ __device__ __forceinline__ float act_eval(float x, float& grad) {
   return x;
 }
 
-// Two 8-element vectors per thread and step, one instantiation per activation, no row division where rows lie one after another
-// (8192 x 11008 gated, 541 MB forward and 902 MB backward: silu 134 -> 108 us and 227 -> 165 us, gelu 145 -> 113 and 321 -> 172,
+// Two 8-element vectors per thread and step (see act_grid), one instantiation per activation, no row division where rows lie one
+// after another (8192 x 11008 gated, 541 MB forward and 902 MB backward: silu 134 -> 108 us and 227 -> 165 us, gelu 145 -> 113 and 321 -> 172,
 // gelu(tanh) 128 -> 98 and 226 -> 148).  Memory-bound with relu (89 and 146 us); expf, erff and the IEEE divisions cost the others
 // up to 24 us on top.  The hardware exponential and reciprocal would take silu to 92 and 147 us, at the cost of digits (an error of
 // 1.16 |x| units in the last place).  Logical shape [rows, cols]; gate / up may be column slices of a wider fused projection
@@ -576,6 +576,11 @@ static inline int grid_for(long long work, int threads) {
   return int(g);
 }
 
+// The activation kernels take two vectors per thread where the chip is full; below 2^18 vectors (all threads resident at once) a
+// thread takes one, so that the chain of one thread is half as long (gated silu, two per thread and one: 100 x 768 2.8 and 2.4 us
+// forward, 3.6 and 2.6 us backward; 700 x 2048 3.7 and 3.4, 5.0 and 4.8; relu of 1000 x 3072 3.0 and 3.4).
+static inline int act_grid(long long nvec) { return grid_for(nvec < (1 << 18) ? nvec : (nvec + 1) / 2, 256); }
+
 }  // namespace tpb
 
 using namespace tpb;
@@ -689,8 +694,8 @@ extern "C" int tpb_act_fwd(const void* gate, const void* up, void* out, long lon
   const bool dense = (gate_ld == cols || rows == 1) && (!up || up_ld == cols || rows == 1);
 #define LAUNCH2(T, K)                                                                                                                                   \
   do {                                                                                                                                                  \
-    if (dense) act_fwd_kernel<T, K, true><<<grid_for((nvec + 1) / 2, 256), 256, 0, s>>>((const T*)gate, (const T*)up, (T*)out, nvec, cols, gate_ld, up_ld);   \
-    else act_fwd_kernel<T, K, false><<<grid_for((nvec + 1) / 2, 256), 256, 0, s>>>((const T*)gate, (const T*)up, (T*)out, nvec, cols, gate_ld, up_ld);        \
+    if (dense) act_fwd_kernel<T, K, true><<<act_grid(nvec), 256, 0, s>>>((const T*)gate, (const T*)up, (T*)out, nvec, cols, gate_ld, up_ld);   \
+    else act_fwd_kernel<T, K, false><<<act_grid(nvec), 256, 0, s>>>((const T*)gate, (const T*)up, (T*)out, nvec, cols, gate_ld, up_ld);        \
   } while (0)
 #define LAUNCH(T)                                                                                                           \
   do {                                                                                                                      \
@@ -711,7 +716,7 @@ extern "C" int tpb_act_bwd(const void* dout, const void* gate, const void* up, v
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const long long nvec = n / 8;
 #define LAUNCH2(T, K) \
-  act_bwd_kernel<T, K><<<grid_for((nvec + 1) / 2, 256), 256, 0, s>>>((const T*)dout, (const T*)gate, (const T*)up, (T*)dgate, (T*)dup, nvec)
+  act_bwd_kernel<T, K><<<act_grid(nvec), 256, 0, s>>>((const T*)dout, (const T*)gate, (const T*)up, (T*)dgate, (T*)dup, nvec)
 #define LAUNCH(T)                                                                                                           \
   do {                                                                                                                      \
     if (kind == 1) LAUNCH2(T, 1); else if (kind == 2) LAUNCH2(T, 2); else if (kind == 3) LAUNCH2(T, 3);                       \

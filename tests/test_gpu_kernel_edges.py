@@ -261,15 +261,16 @@ def test_loss_gradient_has_the_accuracy_of_the_fp32_exponential():
     assert _rounded_between(logits, low, high)
 
 
+# (a thread takes one vector of eight below 2^18 of them, two from there on)
+@pytest.mark.parametrize("vectors", [5, 1 << 17, (1 << 18) - 1, (1 << 18) + 3])
 @pytest.mark.parametrize("gated", [False, True])
-def test_silu_has_the_accuracy_of_the_fp32_functions(gated):
+def test_silu_has_the_accuracy_of_the_fp32_functions(gated, vectors):
     """On bf16 data too: expf (1 unit in the last place), the sum, the division and the products (half a unit each) stay within 2^-21 of
     the 64-bit value, 2^-20 of the terms of the derivative; what is rounded to bf16 lies in that interval."""
     torch.manual_seed(0)
-    n = 1 << 20
-    x = (160 * torch.rand(n // 8, 8, device="cuda") - 80).to(torch.bfloat16).requires_grad_()
-    u = (torch.rand(n // 8, 8, device="cuda") + 0.5).to(torch.bfloat16).requires_grad_()
-    g = torch.randn(n // 8, 8, device="cuda").to(torch.bfloat16)
+    x = (160 * torch.rand(vectors, 8, device="cuda") - 80).to(torch.bfloat16).requires_grad_()
+    u = (torch.rand(vectors, 8, device="cuda") + 0.5).to(torch.bfloat16).requires_grad_()
+    g = torch.randn(vectors, 8, device="cuda").to(torch.bfloat16)
     out = OF.swiglu(x, u) if gated else _native()._ActFn.apply(x, None, 4)
     out.backward(g)
     xd, ud, gd = x.detach().double(), u.detach().double() if gated else 1.0, g.double()
