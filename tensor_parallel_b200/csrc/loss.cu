@@ -26,10 +26,19 @@ __device__ __forceinline__ float ce_warp_sum(float v) {
   return v;
 }
 
-// One CTA per row, 16-byte accesses (8192 x 32000: statistics 200 -> 134 us against element-wise accesses and two passes, gradient
-// 249 -> 222 us against element-wise accesses).  The statistics are bound by memory; the gradient by expf as well (204 us with
-// __expf, which costs digits).  A row starts at any element when the pitch is odd (a vocabulary that is no multiple of 8):
+// One CTA per row, 16-byte accesses.  A row starts at any element when the pitch is odd (a vocabulary that is no multiple of 8):
 // [0, head) and [tail, cols) are handled one by one, [head, tail) is 16-byte aligned.
+// U vectors in flight per thread, or U = 0: every element is its own access.  Long rows hide their latency with four (8192 x 32000, 1
+// and 4: statistics 130 and 117 us, gradient 174 and 162 us; 65 x 32000 8.0 and 5.8, 7.0 and 5.5 us).  Below 8192 columns a thread has
+// no four vectors and their registers only cost CTAs per SM (8192 x 4000, 1 and 4: 24.8 and 29.0, 21.8 and 22.6 us; 8192 x 1000: 14.5 and
+// 22.4, 9.7 and 12.3 us), below 256 most threads have none (1000 x 131, 0 and 1: 3.0 and 3.6, 2.4 and 3.2 us).  Element-wise accesses and
+// two passes took 178 and 239 us for 8192 x 32000, 30 and 27 us for 8192 x 4000.
+#define CE_DISPATCH(cols, LAUNCH) \
+  do {                            \
+    if (cols >= 8192) LAUNCH(4);  \
+    else if (cols >= 256) LAUNCH(1); \
+    else LAUNCH(0);               \
+  } while (0)
 struct CeSpan { int head, tail; };
 __device__ __forceinline__ CeSpan ce_span(const bf16* x, int cols) {
   const int head = min(cols, int((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / 2);
@@ -46,13 +55,14 @@ __device__ __forceinline__ void ce_unpack(const uint4& u, float (&v)[8]) {
 
 // One pass over the row: every thread keeps a running maximum and the sum of exp(x - maximum), rescaled when the maximum of a
 // group of loaded values exceeds it; the threads' pairs are merged at the end.
+template <int U>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_stats_kernel(const bf16* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ stats, int cols,
                 long long ld, int vocab_start, int ignore_index) {
   const long long row = blockIdx.x;
   const bf16* x = logits + row * ld;
   __shared__ float red_m[CE_THREADS / 32], red_s[CE_THREADS / 32];
-  const CeSpan span = ce_span(x, cols);
+  const CeSpan span = U ? ce_span(x, cols) : CeSpan{cols, cols};
   float m = -INFINITY, s = 0.f;
   auto raise = [&](float group_max) {  // exp(-inf - -inf) must not arise while nothing finite has been seen
     if (group_max > m) {
@@ -61,8 +71,8 @@ ce_stats_kernel(const bf16* __restrict__ logits, const int64_t* __restrict__ lab
     }
     return m == -INFINITY ? 0.f : m;
   };
-  constexpr int U = 4;  // vectors in flight per thread
-  for (int c = span.head + threadIdx.x * 8; c < span.tail; c += U * CE_THREADS * 8) {
+  if constexpr (U > 0)
+    for (int c = span.head + threadIdx.x * 8; c < span.tail; c += U * CE_THREADS * 8) {
     uint4 raw[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) {
@@ -85,9 +95,9 @@ ce_stats_kernel(const bf16* __restrict__ logits, const int64_t* __restrict__ lab
       s += part;
     }
   }
-  const int edge = span.head + cols - span.tail;  // at most 14 elements outside the vectors
-  if (int(threadIdx.x) < edge) {
-    const float v = __bfloat162float(x[int(threadIdx.x) < span.head ? threadIdx.x : span.tail + threadIdx.x - span.head]);
+  const int edge = span.head + cols - span.tail;  // outside the vectors: at most 14 elements, or the whole row (U = 0)
+  for (int i = threadIdx.x; i < edge; i += CE_THREADS) {
+    const float v = __bfloat162float(x[i < span.head ? i : span.tail + i - span.head]);
     const float base = raise(v);
     s += expf(v - base);
   }
@@ -114,30 +124,35 @@ ce_stats_kernel(const bf16* __restrict__ logits, const int64_t* __restrict__ lab
   }
 }
 
+template <int U>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ labels, const float* __restrict__ lse, int cols,
                long long ld, int vocab_start, int ignore_index, const float* __restrict__ scale_ptr) {
   const long long row = blockIdx.x;
   bf16* x = logits + row * ld;
-  const CeSpan span = ce_span(x, cols);
+  const CeSpan span = U ? ce_span(x, cols) : CeSpan{cols, cols};
   const long long label = labels[row];
-  const float scale = scale_ptr[0];
-  const bool ignored = label == ignore_index;
-  const float l = ignored ? 0.f : lse[row];
+  const int edge = span.head + cols - span.tail;
+  if (label == ignore_index) {
+    for (int c = span.head + threadIdx.x * 8; c < span.tail; c += CE_THREADS * 8) *reinterpret_cast<uint4*>(x + c) = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < edge; i += CE_THREADS) x[i < span.head ? i : span.tail + i - span.head] = __float2bfloat16(0.f);
+    return;
+  }
+  const float scale = scale_ptr[0], l = lse[row];
   const long long local = label - vocab_start;
+  const int mark = local >= 0 && local < cols ? int(local) : -1;
   auto grad = [&](float v, int c) {
-    if (ignored) return 0.f;
     float p = expf(v - l);  // (not __expf, whose error grows with |v - l| and, next to a label's -1, decides whole digits)
-    if (c == local) p -= 1.f;
+    if (c == mark) p -= 1.f;
     return p * scale;
   };
-  constexpr int U = 4;
-  for (int c = span.head + threadIdx.x * 8; c < span.tail; c += U * CE_THREADS * 8) {
+  if constexpr (U > 0)
+    for (int c = span.head + threadIdx.x * 8; c < span.tail; c += U * CE_THREADS * 8) {
     uint4 raw[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       const int ck = c + k * CE_THREADS * 8;
-      if (ck < span.tail && !ignored) raw[k] = *reinterpret_cast<const uint4*>(x + ck);
+      if (ck < span.tail) raw[k] = *reinterpret_cast<const uint4*>(x + ck);
     }
 #pragma unroll
     for (int k = 0; k < U; ++k) {
@@ -156,9 +171,8 @@ ce_grad_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ labels, co
       }
     }
   }
-  const int edge = span.head + cols - span.tail;
-  if (int(threadIdx.x) < edge) {
-    const int c = int(threadIdx.x) < span.head ? threadIdx.x : span.tail + threadIdx.x - span.head;
+  for (int i = threadIdx.x; i < edge; i += CE_THREADS) {
+    const int c = i < span.head ? i : span.tail + i - span.head;
     x[c] = __float2bfloat16(grad(__bfloat162float(x[c]), c));
   }
 }
@@ -168,15 +182,21 @@ ce_grad_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ labels, co
 extern "C" int tpb_ce_stats(const void* logits, const int64_t* labels, float* stats, int rows, int cols, long long ld,
                             int vocab_start, int ignore_index, void* stream_) {
   if (!logits || !labels || !stats || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
-  tpb::ce_stats_kernel<<<rows, tpb::CE_THREADS, 0, static_cast<cudaStream_t>(stream_)>>>(
-      static_cast<const tpb::bf16*>(logits), labels, stats, cols, ld, vocab_start, ignore_index);
+#define LAUNCH(U)                                                                                    \
+  tpb::ce_stats_kernel<U><<<rows, tpb::CE_THREADS, 0, static_cast<cudaStream_t>(stream_)>>>(          \
+      static_cast<const tpb::bf16*>(logits), labels, stats, cols, ld, vocab_start, ignore_index)
+  CE_DISPATCH(cols, LAUNCH);
+#undef LAUNCH
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
 extern "C" int tpb_ce_grad(void* logits, const int64_t* labels, const float* lse, int rows, int cols, long long ld,
                            int vocab_start, int ignore_index, const float* scale_ptr, void* stream_) {
   if (!logits || !labels || !lse || !scale_ptr || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
-  tpb::ce_grad_kernel<<<rows, tpb::CE_THREADS, 0, static_cast<cudaStream_t>(stream_)>>>(
-      static_cast<tpb::bf16*>(logits), labels, lse, cols, ld, vocab_start, ignore_index, scale_ptr);
+#define LAUNCH(U)                                                                                    \
+  tpb::ce_grad_kernel<U><<<rows, tpb::CE_THREADS, 0, static_cast<cudaStream_t>(stream_)>>>(           \
+      static_cast<tpb::bf16*>(logits), labels, lse, cols, ld, vocab_start, ignore_index, scale_ptr)
+  CE_DISPATCH(cols, LAUNCH);
+#undef LAUNCH
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }

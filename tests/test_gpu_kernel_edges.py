@@ -214,6 +214,44 @@ def test_head_loss_rows_at_any_alignment(vocab):
         assert (got.double() - ref).norm() <= 0.02 * ref.norm()
 
 
+# (every element by itself below 256 columns, one vector per thread below 8192, four from there on)
+@pytest.mark.parametrize("cols", [1, 7, 255, 256, 261, 2049, 8191, 8192, 8203, 17000])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_loss_kernels_at_the_edges_of_a_row(cols, pad):
+    """Labels in the first and last element of each part of a row, outside this slice of the vocabulary, ignored; what lies between
+    the rows stays."""
+    from tensor_parallel_b200.ops import loss as L
+
+    nat = _native()
+    torch.manual_seed(cols + pad)
+    rows, start = 24, 100
+    wide = (3 * torch.randn(rows, cols + pad, device="cuda")).to(torch.bfloat16)
+    logits, before = wide[:, :cols], wide.clone()
+    local = torch.randint(0, cols, (rows,), device="cuda")
+    local[:6] = torch.tensor([0, cols - 1, min(7, cols - 1), max(0, cols - 8), cols // 8 * 8 % cols, min(2048, cols - 1)])
+    labels = local + start
+    labels[6], labels[7], labels[8] = -100, start - 1, start + cols
+    mine = (labels >= start) & (labels < start + cols)
+    exact = logits.double()
+    stats = torch.empty(rows, 4, device="cuda")
+    nat.check(L.LIB.tpb_ce_stats(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), rows, cols, cols + pad, start, -100, nat._stream()), "ce_stats")
+    lse = exact.logsumexp(-1)
+    assert torch.equal(stats[:, 0].double(), exact.amax(-1)) and torch.equal(stats[:, 3] != 0, mine)
+    # (the sum of up to 17000 fp32 exponentials: 1 + 2 units each, and a tree of additions of less than 80 levels)
+    assert (stats[:, 0].double() + stats[:, 1].double().log() - lse).abs().max().item() <= 2.0 ** -17
+    assert torch.equal(stats[mine, 2], exact[mine, local[mine]].float())
+    lse, scale = lse.float(), torch.full((1,), 0.5, device="cuda")
+    p = (logits.float() - lse[:, None]).double().exp()
+    low, high = p * (1 - 2.0 ** -22), p * (1 + 2.0 ** -22)
+    at = (torch.arange(rows, device="cuda")[mine], local[mine])
+    low[at] -= 1
+    high[at] -= 1
+    low[6] = high[6] = 0
+    nat.check(L.LIB.tpb_ce_grad(logits.data_ptr(), labels.data_ptr(), lse.data_ptr(), rows, cols, cols + pad, start, -100, scale.data_ptr(), nat._stream()), "ce_grad")
+    assert _rounded_between(logits, 0.5 * low, 0.5 * high)
+    assert torch.equal(wide[:, cols:], before[:, cols:])
+
+
 def test_loss_statistics_with_infinite_logits():
     """Masked (-inf) logits carry no mass whatever vector, thread or edge they fall into."""
     from tensor_parallel_b200.ops import loss as L
