@@ -75,7 +75,9 @@ __global__ void qkv_rope_append_kernel(const bf16* __restrict__ q, const bf16* _
 // hg + groups, ... with it, so that the angles (exp2f and sincosf per pair, what bounded the kernel when every head
 // evaluated its own: 64 -> 51 us for 4000 tokens of 32 + 32 heads of 128, 43 us with v by head groups and 32-bit divisions) are
 // computed once per thread; (2) one thread per 16-byte chunk of the non-rotary tails, and v_chunks x v_groups threads that
-// copy a chunk of v for several heads each.
+// copy a chunk of v for several heads each.  SINGLE: every rotary thread has one head (groups == q_heads + kv_heads); its
+// instantiation needs 40 registers instead of 60, so that more of such a launch is resident (700 tokens of 32 + 32 heads of 128, 32 of
+// them rotary: 11.3 -> 9.8 us).
 // Requires head_dim, rotary_dim / 2 (non-interleaved) or rotary_dim (interleaved) to be multiples of 8.
 __device__ __forceinline__ void rope_unpack(const uint4& u, float (&v)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -89,6 +91,7 @@ __device__ __forceinline__ uint4 rope_pack(const float (&v)[8]) {
   return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
 }
 
+template <bool SINGLE>
 __global__ void __launch_bounds__(256)
 qkv_rope_append_vec_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
                            bf16* __restrict__ q_out, bf16* __restrict__ kcache, bf16* __restrict__ vcache,
@@ -135,6 +138,37 @@ qkv_rope_append_vec_kernel(const bf16* __restrict__ q, const bf16* __restrict__ 
       continue;
     }
     const int hg = w / rot_chunks, e = (w - hg * rot_chunks) * 8;
+    if constexpr (SINGLE) {
+      const bf16* src = src_of(hg);
+      bf16* dst = dst_of(hg);
+      float x[8], r[8];
+      rope_unpack(*reinterpret_cast<const uint4*>(src + e), x);
+      if (!interleaved) {
+        float y[8], ry[8];
+        rope_unpack(*reinterpret_cast<const uint4*>(src + e + half), y);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float inv_freq = exp2f(-log2_theta * (2.f * float(e + u) / float(rotary_dim)));
+          float sn, cs;
+          sincosf(float(pos) * inv_freq, &sn, &cs);
+          r[u] = x[u] * cs - y[u] * sn;
+          ry[u] = y[u] * cs + x[u] * sn;
+        }
+        *reinterpret_cast<uint4*>(dst + e) = rope_pack(r);
+        *reinterpret_cast<uint4*>(dst + e + half) = rope_pack(ry);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float inv_freq = exp2f(-log2_theta * (2.f * float((e >> 1) + u) / float(rotary_dim)));
+          float sn, cs;
+          sincosf(float(pos) * inv_freq, &sn, &cs);
+          r[2 * u] = x[2 * u] * cs - x[2 * u + 1] * sn;
+          r[2 * u + 1] = x[2 * u + 1] * cs + x[2 * u] * sn;
+        }
+        *reinterpret_cast<uint4*>(dst + e) = rope_pack(r);
+      }
+      continue;
+    }
     if (!interleaved) {
       float cs[8], sn[8];
 #pragma unroll
@@ -822,14 +856,26 @@ extern "C" int tpb_qkv_rope_append(const void* q, const void* k, const void* v, 
                       !((uintptr_t)kcache & 15) && !((uintptr_t)vcache & 15);
   if (vec_ok) {
     const int rot_chunks = interleaved ? rotary_dim / 8 : half_ / 8;
-    const int groups = tpb_rope_head_groups((long long)batch * seq * rot_chunks, q_heads + kv_heads);
-    const int v_groups = tpb_rope_head_groups((long long)batch * seq * (head_dim / 8), kv_heads);
-    const long long per_token = (long long)rot_chunks * groups + (long long)(q_heads + kv_heads) * ((head_dim - rotary_dim) / 8) +
-                                (long long)v_groups * (head_dim / 8);
-    const long long vwork = (long long)batch * seq * per_token;
+    const int heads = q_heads + kv_heads;
+    int groups = tpb_rope_head_groups((long long)batch * seq * rot_chunks, heads);
+    int v_groups = tpb_rope_head_groups((long long)batch * seq * (head_dim / 8), kv_heads);
+    auto threads = [&]() {
+      return (long long)batch * seq * ((long long)rot_chunks * groups + (long long)heads * ((head_dim - rotary_dim) / 8) + (long long)v_groups * (head_dim / 8));
+    };
+    // Registers admit four CTAs per SM, six where a thread has one head.  A launch of more than that, but less than twice that, would take
+    // two rounds for little more than one round of work: twice the heads per thread, up to four, make one round of it (8 + 8 heads of
+    // 128, 1500 tokens: 7.7 -> 6.0 us).
+    const long long round = 148LL * 256 * (groups >= heads ? 6 : 4);
+    if (threads() > round && threads() <= 2 * round) {
+      auto halved = [](int g, int of) { return (of + (g + 1) / 2 - 1) / ((g + 1) / 2) <= 4 ? (g + 1) / 2 : g; };
+      groups = halved(groups, heads);
+      v_groups = halved(v_groups, kv_heads);
+    }
+    const long long vwork = threads();
     long long vgrid = (vwork + 255) / 256;
     if (vgrid > 148 * 32) vgrid = 148 * 32;
-    qkv_rope_append_vec_kernel<<<int(vgrid), 256, 0, s>>>((const bf16*)q, (const bf16*)k, (const bf16*)v, (bf16*)q_out, (bf16*)kcache,
+    auto kernel = groups >= heads ? qkv_rope_append_vec_kernel<true> : qkv_rope_append_vec_kernel<false>;
+    kernel<<<int(vgrid), 256, 0, s>>>((const bf16*)q, (const bf16*)k, (const bf16*)v, (bf16*)q_out, (bf16*)kcache,
                                                           (bf16*)vcache, base_pos, batch, seq, q_heads, kv_heads, groups, v_groups, head_dim,
                                                           rotary_dim, log2f(theta), interleaved, max_seq, q_ld, k_ld, v_ld);
     return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;

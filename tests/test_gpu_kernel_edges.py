@@ -336,6 +336,35 @@ def test_rope_head_groups(heads, tokens, interleaved, rotary):
     assert torch.equal(got[..., rotary:], x[..., rotary:])
 
 
+# one head per thread, several, the step between them and rounds of a launch; rows past the end of the cache
+@pytest.mark.parametrize("heads,kv,d,rotary,interleaved", [(8, 8, 128, 128, False), (12, 3, 64, 64, False), (9, 1, 128, 32, False), (4, 2, 128, 64, True), (32, 32, 128, 128, False)])
+@pytest.mark.parametrize("batch,seq", [(1, 1), (3, 67), (1, 760), (2, 1500), (1, 4000)])
+def test_rotary_append_by_head_groups(heads, kv, d, rotary, interleaved, batch, seq):
+    nat = _native()
+    torch.manual_seed(heads + seq)
+    base, room = 5, seq + 3  # (the last two tokens lie past the end of the cache)
+    qkv = torch.randn(batch * seq, (heads + 2 * kv) * d, device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv.split([heads * d, kv * d, kv * d], dim=1)
+    kc, vc = (torch.full((batch, kv, room, d), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    out = torch.empty(batch * seq, heads * d, device="cuda", dtype=torch.bfloat16)
+    nat.qkv_rope_append(q, k, v, out, kc, vc, torch.tensor([base], device="cuda", dtype=torch.int32), batch, seq, rotary, 10000.0, interleaved=interleaved)
+    pos = torch.arange(base, base + seq, device="cuda")[None].expand(batch, seq)
+    kept = max(0, min(seq, room - base))
+
+    def close(got, x, n):
+        x = x.reshape(batch, seq, n, d)
+        want = OF.apply_rope_ref(x.float(), pos, 10000.0, rotary, interleaved)[:, :kept]
+        # angles up to 4000 rad: 2.4e-4 rad between two fp32 evaluations of the frequency
+        assert (got[:, :kept].float() - want).abs().max().item() <= (2.0 ** -8 * want.abs().max().item() + 5e-3 if kept else 0)
+        assert torch.equal(got[:, :kept, :, rotary:], x[:, :kept, :, rotary:])
+
+    if kept:
+        close(out.view(batch, seq, heads, d), q, heads)
+        close(kc[:, :, base : base + kept].transpose(1, 2), k, kv)
+        assert torch.equal(vc[:, :, base : base + kept].transpose(1, 2), v.reshape(batch, seq, kv, d)[:, :kept])
+    assert bool((kc[:, :, :base] == 7).all()) and bool((vc[:, :, :base] == 7).all())
+
+
 # (vectors of eight from 2^19 elements on)
 @pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (8, 0), (4099, 0), (4096, 1), ((1 << 19) - 1, 0), (1 << 19, 0), ((1 << 19) + 7, 0), (1 << 19, 1)])
 @pytest.mark.parametrize("dtype,gdtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
