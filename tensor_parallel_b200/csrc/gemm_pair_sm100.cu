@@ -7,7 +7,7 @@
 // What bounds it and why pairs: one k-block (64) of a 128 x 256 single-CTA tile takes the tensor core 512 clocks and
 // brings 48 KB into shared memory - 96 bytes per clock and SM, more than the L2 delivers to all SMs at once.  A pair tile
 // of 256 x 256 needs 32 KB per CTA for the same 512 clocks (64 bytes per clock).  Measured against the single-CTA kernel, same
-// results to the bit: 8192 x 32000 x 4096 and its two gradients 1649 -> 1368 us each (1.57 PFLOP/s, cuBLAS burst rate 1.59),
+// results to the bit: 8192 x 32000 x 4096 and its two gradients 1649 -> 1368 us each (1.57 PFLOP/s; cuBLAS in a short run 1.69, in seconds-long loops 1.41),
 // the projections of a 7B layer at 4000 tokens 297 -> 265 us on average, the 4096 x 4096 ones at 8192 tokens 213 -> 177 us.
 //
 // One CTA (192 threads), persistent over the pair's tiles:

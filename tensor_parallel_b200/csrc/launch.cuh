@@ -1,17 +1,19 @@
-// Kernel launch helper.  With TPB_PDL=1 the decode-path kernels are launched with the programmatic-dependent-launch
-// attribute: between two dependent kernels of a CUDA graph lie about 3.7 us on B200 (measured with %globaltimer stamps
-// inside the kernels), part of it launch latency that a successor scheduled ahead of time hides.
-// TPB_PDL is off by default (a decode step on one GPU asks for early launches by itself, kernel by kernel, see `early` in
-// gemm_stream_sm100.cu: those kernels fetch weights before the wait, which the figures below do not include).  Measured on one B200 with the per-rank shapes of a Llama-2-7B decode step: 2.35 vs 2.40 ms at
-// 8-way, 2.96 vs 3.09 ms at 4-way shard shapes, but 4.79 vs 3.91 ms at 2-way and 5.76 vs 5.65 ms unsharded.
+// Kernel launch helper.  A kernel may be launched as a programmatic dependent of its predecessor in the stream: scheduled ahead of time,
+// it hides launch latency (between two dependent kernels of a CUDA graph lie about 3.7 us on B200, measured with %globaltimer stamps
+// inside the kernels) and may fetch what the predecessor does not write.
+// Two ways to ask for it.  `early`, launch by launch: what a decode step on one GPU does; its kernels fetch weights and old cache rows
+// before the wait (gemm_stream_sm100.cu, attn_decode_fused_kernel).  TPB_PDL=1, for every kernel launched through launch_kernel: off by
+// default.  Measured on one B200, without fetches before the wait, with the per-rank shapes of a Llama-2-7B decode step: 2.35 vs
+// 2.40 ms at 8-way, 2.96 vs 3.09 ms at 4-way shard shapes, but 4.79 vs 3.91 ms at 2-way and 5.76 vs 5.65 ms unsharded.
 // Discipline of every such kernel: do the work that does not depend on earlier kernels (barrier init, TMEM
 // allocation), then griddepcontrol.wait, and only THEN griddepcontrol.launch_dependents.  A successor is scheduled
 // once every CTA of this grid has passed that point, i.e. once the whole grid is resident and its predecessor has
 // completed: exactly one kernel is ever scheduled ahead, and its idle CTAs cannot take an SM from a CTA of the grid
 // they wait for.  (Triggering before the wait let a whole chain of future kernels pile up on the SMs and slowed the
-// Llama-7B decode step from 6.4 to 7.9 ms.)  Only the GEMM kernels trigger: measured on B200 a GEMM that follows a GEMM
-// gains about 1 us, whereas successors scheduled into a running attention kernel (many small CTAs, several per SM) end
-// up unevenly spread over the SMs and cost more than the hidden launch latency (+1 to 2 us per attention launch).
+// Llama-7B decode step from 6.4 to 7.9 ms.)  The GEMM kernels trigger always, the decode attention when it is launched early itself: a
+// GEMM that follows a GEMM gains about 1 us, whereas successors that only start ahead of time, scheduled into a running attention kernel
+// (many small CTAs, several per SM), end up unevenly spread over the SMs and cost more than the hidden launch latency (+1 to 2 us per
+// attention launch).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdlib.h>

@@ -211,8 +211,8 @@ __device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_
 
 // Forms for an issue loop that the WHOLE warp walks, with only its `leader` lane issuing.  An MMA takes its descriptors from
 // uniform registers; in code that only the elected lane runs, every operand of every instruction is moved there one by one,
-// and a stream of short MMAs (N <= 64) is then bound by its issue loop (attention backward 4 x 2048, 32 heads of 128, causal: 606 ->
-// 554 us with this form and mask-free common steps, forward 204 -> 194 us).  Descriptors come as 32-bit halves: the high half is
+// and a stream of short MMAs (N <= 64) is then bound by its issue loop (attention 4 x 2048, 32 heads of 128, causal, replayed from a
+// CUDA graph: backward 606 -> 554 us with this form and mask-free common steps, forward 193 -> 161 us).  Descriptors come as 32-bit halves: the high half is
 // a constant of the layout, the low half (address field) advances by plain 32-bit additions.
 constexpr uint32_t DESC_KMAJOR_HI = (1024u >> 4) | (1u << 14) | (2u << 29);  // stride 1024 B, version 1, 128-byte swizzle
 __device__ __forceinline__ uint32_t desc_kmajor_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
