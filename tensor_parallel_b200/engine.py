@@ -581,8 +581,9 @@ class DecoderEngine:
             self._status_tensor().zero_()
             from tensor_parallel_b200.parallel.collectives import TPCollectiveError
 
-            what = {1: "an mbarrier wait", 2: "a wait for a peer GPU"}.get(code, f"status {code}")
-            raise TPCollectiveError(f"{what} timed out inside a kernel; the results of this step are not valid")
+            what = {1: "an mbarrier wait timed out inside a kernel", 2: "a wait for a peer GPU timed out inside a kernel",
+                    3: "a kernel met an index outside its range"}.get(code, f"status {code} from a kernel")
+            raise TPCollectiveError(f"{what}; the results of this step are not valid")
 
     def step_from_host(self, token_ids_host: torch.Tensor, out_host: Optional[torch.Tensor] = None) -> torch.Tensor:
         """One decode step driven from the host: pinned int64 ``[batch]`` ids in, next ids out (pinned).  The kernels'

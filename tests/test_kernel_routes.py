@@ -296,3 +296,19 @@ def test_buckets_that_a_lookup_does_not_take_do_not_reach_the_kernel(monkeypatch
         with pytest.raises((IndexError, RuntimeError)):
             OF.relative_bias(embedding, buckets, 4, 6)
     assert not kernel.taken
+
+
+@needs_library
+@pytest.mark.parametrize("code,words", [(0, None), (1, "timed out"), (2, "peer GPU timed out"), (3, "index outside its range"), (9, "status 9")])
+def test_a_step_says_what_its_kernels_reported(code, words):
+    from tensor_parallel_b200.engine import DecoderEngine
+    from tensor_parallel_b200.parallel.collectives import TPCollectiveError
+
+    status = torch.full((4,), code, dtype=torch.int32)
+    engine = types.SimpleNamespace(status_host=status.clone(), _status_tensor=lambda: status)
+    if words is None:
+        DecoderEngine._raise_on_status(engine)
+    else:
+        with pytest.raises(TPCollectiveError, match=words):
+            DecoderEngine._raise_on_status(engine)
+    assert int(status.sum()) == 0
