@@ -371,8 +371,11 @@ constexpr int FA2_M = 256;
 constexpr int FA2_THREADS = 384;
 constexpr float FA2_RESCALE_LOG2 = 8.f;
 
-// POLY of every 4 pairs of exponentials run on the FMA pipe.  BIAS: the score-bias code exists only where it is needed.
-template <int D, int POLY, bool BIAS>
+// POLY of every 4 pairs of exponentials run on the FMA pipe.  BIAS: the score-bias code exists only where it is needed - 0 none, 1 any bias,
+// loaded in vectors or one by one, 2 bf16 rows in vectors (bias_vector_rows), those of a whole tile ahead.  2 holds 64 registers of raw
+// biases; in one instantiation with 1 they spill there too (2 x 1001, 16 heads of 128, causal, a dense bf16 bias: 296 us, apart 239 us;
+// 4 x 500, 16 heads of 64: 77 and 70 us; fp32 bias of 16 x 512, 32 heads of 64: 282 and 217 us).
+template <int D, int POLY, int BIAS>
 __global__ void __launch_bounds__(FA2_THREADS, 1)
 attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
@@ -550,12 +553,12 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       const bool plain = key0 + FA_N <= p.sk && (!p.causal || key0 + FA_N - 1 <= q0 + t * FA_M + shift);
       // the row's biases of a whole tile, fetched BEFORE the wait for its scores: loaded where they are used, they would add
       // sixteen global round trips to the chain of every tile
-      uint4 bias_raw[BIAS ? FA_N / 8 : 1];
-      const bool ahead = BIAS && plain && p.bias_kind == 2 && p.bias_vec;
+      uint4 bias_raw[BIAS == 2 ? FA_N / 8 : 1];
+      const bool ahead = BIAS == 2 && plain;
       if (ahead) {
         const uint4* src = reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.bias) + bias_row + key0);
 #pragma unroll
-        for (int c = 0; c < FA_N / 8; ++c) bias_raw[BIAS ? c : 0] = __ldg(src + c);
+        for (int c = 0; c < FA_N / 8; ++c) bias_raw[BIAS == 2 ? c : 0] = __ldg(src + c);
       }
       if (*abort_flag || !mbar_wait(&s_full[t], j & 1)) {
         if (!*abort_flag) give_up(STATUS_TIMEOUT_MBAR);
@@ -590,7 +593,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
           tmem_ld_wait();
 #pragma unroll
           for (int c = c0; c < c0 + 32; c += 8) {
-            const uint4 u = bias_raw[BIAS ? c / 8 : 0];
+            const uint4 u = bias_raw[BIAS == 2 ? c / 8 : 0];
             const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -606,16 +609,18 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       } else {
 #pragma unroll
         for (int c0 = 0; c0 < FA_N; c0 += 32) {
+          float bv[4][8];  // (all of a quarter's biases are on their way before the wait for its scores)
+#pragma unroll
+          for (int c = 0; c < 32; c += 8)
+            load_bias8(p.bias, p.bias_kind, bias_row + (long long)(key0 + c0 + c) * p.bias_sk, p.bias_sk, visible - c0 - c, p.bias_vec, bv[c / 8]);
           tmem_ld_x32(s_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(r + c0));
           tmem_ld_wait();
 #pragma unroll
           for (int c = c0; c < c0 + 32; c += 8) {
-            float bv[8];
-            load_bias8(p.bias, p.bias_kind, bias_row + (long long)(key0 + c) * p.bias_sk, p.bias_sk, visible - c, p.bias_vec, bv);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               float sv = c + i < visible ? __uint_as_float(r[c + i]) * p.scale_log2e : -INFINITY;
-              if (c + i < visible) sv += bv[i] * 1.4426950408889634f;
+              if (c + i < visible) sv += bv[(c - c0) / 8][i] * 1.4426950408889634f;
               r[c + i] = __float_as_uint(sv);
               m_tile = fmaxf(m_tile, sv);
             }
@@ -742,7 +747,7 @@ static int fa_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
-template <int D, int POLY, bool BIAS>
+template <int D, int POLY, int BIAS>
 static int fa2_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, dim3 grid, cudaStream_t stream) {
   constexpr size_t smem = size_t(D / 64) * FA_BLOCK_BYTES * 6 + 1024 + 256;
   static std::atomic<bool> configured[64];
@@ -800,8 +805,10 @@ extern "C" int tpb_attn_prefill_sm100(const void* q, const void* k, const void* 
     dim3 grid((sq + FA2_M - 1) / FA2_M, q_heads, batch);
     // one pair of exponentials in four runs as a cubic on the FMA pipe (measured best of 0 / 1 / 2 / 3 in four:
     // 206 / 199 / 205 / 236 us at batch 4, 2048 tokens, 32 heads of 128, causal, before the warp-uniform issue loop: 161 us with it)
-    if (bias) return head_dim == 128 ? fa2_launch<128, 1, true>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, true>(tq, tk, tv, p, grid, s);
-    return head_dim == 128 ? fa2_launch<128, 1, false>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, false>(tq, tk, tv, p, grid, s);
+    if (bias && p.bias_kind == 2 && p.bias_vec)
+      return head_dim == 128 ? fa2_launch<128, 1, 2>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, 2>(tq, tk, tv, p, grid, s);
+    if (bias) return head_dim == 128 ? fa2_launch<128, 1, 1>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, 1>(tq, tk, tv, p, grid, s);
+    return head_dim == 128 ? fa2_launch<128, 1, 0>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, 0>(tq, tk, tv, p, grid, s);
   }
   dim3 grid((sq + FA_M - 1) / FA_M, q_heads, batch);
   return head_dim == 128 ? fa_launch<128>(tq, tk, tv, p, grid, s) : fa_launch<64>(tq, tk, tv, p, grid, s);

@@ -436,8 +436,10 @@ def test_bias_rows_in_vectors_and_one_by_one(sq, sk, layout):
 # head_dim 128 and 64, causal with several key tiles and with a shift, grouped heads, a bias for each batch or for all heads, ragged tiles
 @pytest.mark.parametrize("b,sq,sk,hq,hkv,d,causal,shape", [
     (2, 304, 304, 4, 2, 128, True, (1, 4, 304, 304)), (2, 200, 328, 4, 2, 64, True, (2, 4, 200, 328)), (1, 136, 264, 8, 8, 128, False, (1, 1, 136, 264)),
-    (3, 128, 128, 2, 2, 128, False, (3, 2, 128, 128)), (2, 65, 72, 4, 1, 64, True, (1, 4, 65, 72)), (2, 257, 384, 6, 2, 128, True, (2, 1, 257, 384))])
-def test_dense_bf16_bias_that_travels_with_the_tiles(b, sq, sk, hq, hkv, d, causal, shape):
+    (3, 128, 128, 2, 2, 128, False, (3, 2, 128, 128)), (2, 65, 72, 4, 1, 64, True, (1, 4, 65, 72)), (2, 257, 384, 6, 2, 128, True, (2, 1, 257, 384)),
+    # rows that no vector fits: element by element
+    (1, 301, 303, 4, 2, 128, True, (1, 4, 301, 303)), (2, 150, 260, 2, 2, 64, False, (2, 2, 150, 260))])
+def test_dense_bf16_bias(b, sq, sk, hq, hkv, d, causal, shape):
     torch.manual_seed(sq + sk)
     q = torch.randn(b, sq, hq, d, device="cuda", dtype=torch.bfloat16).requires_grad_()
     k, v = (torch.randn(b, sk, hkv, d, device="cuda", dtype=torch.bfloat16).requires_grad_() for _ in range(2))
