@@ -2,6 +2,8 @@
 
 Every ``csrc/*.cu`` is compiled with ``nvcc -gencode arch=compute_100a,code=sm_100a`` to an object
 file (in parallel) and linked into one shared library with a C ABI, loaded through ``ctypes``.
+``csrc/autograd.cpp`` becomes a
+Python module beside it (host code against torch's headers; it gets the library's entry points from ``ops.native``).
 nvcc cross-compiles without a GPU, so the library can be built on a CPU-only machine and shipped.
 ``python -m tensor_parallel_b200.build`` rebuilds what is out of date.
 """
@@ -18,6 +20,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libtpb200.so"
+AUTOGRAD_PATH = LIB_DIR / "tpb_autograd.so"
 OBJ_DIR = PKG / "build" / "obj"
 
 NVCC_FLAGS = [
@@ -40,6 +43,28 @@ def sources():
 def _newest_header_mtime() -> float:
     headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh"))
     return max((h.stat().st_mtime for h in headers), default=0.0)
+
+
+def build_autograd(force: bool = False) -> Path:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    source = CSRC / "autograd.cpp"
+    newest = max(source.stat().st_mtime, (CSRC / "tpb_api.h").stat().st_mtime)
+    if not force and AUTOGRAD_PATH.exists() and AUTOGRAD_PATH.stat().st_mtime >= newest:
+        return AUTOGRAD_PATH
+    LIB_DIR.mkdir(parents=True, exist_ok=True)
+    cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda_include), str(CSRC)]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={AUTOGRAD_PATH.stem}",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{i}" for i in includes), str(source),
+           *(f"-L{d}" for d in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-o", str(AUTOGRAD_PATH)]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"building {AUTOGRAD_PATH.name} failed: {' '.join(cmd)}\n{proc.stderr}")
+    return AUTOGRAD_PATH
 
 
 def build(force: bool = False, verbose: bool = False, lib_path: Path = None, extra_flags=()) -> Path:
@@ -75,6 +100,8 @@ def build(force: bool = False, verbose: bool = False, lib_path: Path = None, ext
     newest_obj = max(os.path.getmtime(o) for o in objs)
     if force or jobs or not lib_path.exists() or lib_path.stat().st_mtime < newest_obj:
         run([nvcc, "-shared", "-o", str(lib_path), *objs, "-gencode", "arch=compute_100a,code=sm_100a"])
+    if lib_path == LIB_PATH:
+        build_autograd(force)
     return lib_path
 
 

@@ -1,0 +1,226 @@
+// Autograd nodes of the layers whose training calls are bound by the host at ordinary sizes: linear and norms.
+//
+// A small call (100 tokens through a 768 x 3072 projection with bias, forward and backward) keeps the GPU busy for 37 us.  As Python
+// autograd functions over ctypes it took 176 us: each of its launches cost 10 to 20 us of interpreter work, and the backward nodes
+// ran under the interpreter lock on the autograd thread.  The same nodes in C++ enqueue the same kernels, with the same shapes,
+// copies and saved tensors, without entering the interpreter.
+//
+// The module has no link to the kernel library: `bind` receives the entry points of the library that ops/native.py loaded
+// (a variant with index checks, for instance), and the two callbacks that need Python objects.
+#include <torch/extension.h>
+
+#include <c10/cuda/CUDAStream.h>
+
+#include <atomic>
+#include <stdexcept>
+#include <string>
+
+#include "tpb_api.h"
+
+namespace py = pybind11;
+using at::Tensor;
+
+namespace {
+
+struct Library {
+  decltype(&tpb_gemm_plan_ex) plan = nullptr;
+  decltype(&tpb_gemm_bf16_ex) gemm = nullptr;
+  decltype(&tpb_norm_fwd) norm_fwd = nullptr;
+  decltype(&tpb_norm_bwd) norm_bwd = nullptr;
+  decltype(&tpb_norm_bwd_parts) norm_bwd_parts = nullptr;
+};
+Library lib;
+PyObject* error_text = nullptr;     // (code, what) -> message
+PyObject* reserve_slots = nullptr;  // (device index, fp32 elements) -> address of the device's reduction context
+constexpr int MAX_DEVICES = 64;
+std::atomic<tpb_reduce_ctx_t*> contexts[MAX_DEVICES];
+std::atomic<long long> launched{0};
+
+void check(int code, const char* what) {
+  if (code == TPB_OK) return;
+  std::string text = std::string(what) + " failed: " + std::to_string(code);
+  {
+    py::gil_scoped_acquire gil;
+    try {
+      text = py::reinterpret_borrow<py::function>(error_text)(code, what).cast<std::string>();
+    } catch (py::error_already_set& e) {
+      e.discard_as_unraisable("error text of a native kernel");
+    }
+  }
+  throw std::runtime_error(text);
+}
+
+// The reduction context of a device, with at least `elems` fp32 elements per slot.  It lives as long as the process.
+tpb_reduce_ctx_t* context(const Tensor& t, size_t elems) {
+  const int device = t.is_cuda() ? t.get_device() : 0;
+  TORCH_CHECK(device >= 0 && device < MAX_DEVICES, "device index out of range");
+  tpb_reduce_ctx_t* c = contexts[device].load(std::memory_order_acquire);
+  if (c && elems <= c->slot_stride) return c;
+  std::string problem;
+  {
+    py::gil_scoped_acquire gil;
+    try {
+      const auto address = py::reinterpret_borrow<py::function>(reserve_slots)(device, elems).cast<uintptr_t>();
+      c = reinterpret_cast<tpb_reduce_ctx_t*>(address);
+    } catch (py::error_already_set& e) {
+      problem = e.what();
+    }
+  }
+  if (!problem.empty()) throw std::runtime_error(problem);
+  contexts[device].store(c, std::memory_order_release);
+  return c;
+}
+
+void* stream_of(const Tensor& t) {
+  return t.is_cuda() ? static_cast<void*>(c10::cuda::getCurrentCUDAStream().stream()) : nullptr;
+}
+
+Tensor or_undefined(const std::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
+const void* data(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
+
+// TMA needs a unit inner stride, a 16-byte aligned base and a row pitch that is a multiple of 16 bytes; other operands are copied.
+Tensor tma_ready(const Tensor& t) {
+  if (t.stride(1) == 1 && t.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0) return t;
+  const int64_t rows = t.size(0), cols = t.size(1);
+  Tensor view = at::empty({rows, (cols + 7) / 8 * 8}, t.options()).slice(1, 0, cols);
+  view.copy_(t);
+  return view;
+}
+
+// out[tokens, features] = x w^T + bias; x_t / w_t: that operand lies transposed in memory ([k, tokens] / [k, features]).
+Tensor gemm(const Tensor& x_in, const Tensor& w_in, const Tensor& bias, bool x_t, bool w_t) {
+  const Tensor x = tma_ready(x_in), w = tma_ready(w_in);
+  const int64_t tokens = x.size(x_t ? 1 : 0), k = x.size(x_t ? 0 : 1), features = w.size(w_t ? 1 : 0);
+  Tensor out = at::empty({tokens, features}, x.options());
+  tpb_gemm_plan_t plan;
+  check(lib.plan(int(tokens), int(features), int(k), 1, 0, 0, int(x_t || w_t), &plan), "gemm_plan");
+  tpb_reduce_ctx_t* rc = context(x, plan.reduce && !plan.stream ? size_t(tokens) * size_t(out.stride(0)) : 0);
+  tpb_gemm_opts_t opts = {};
+  opts.x_mn = x_t;
+  opts.w_mn = w_t;
+  check(lib.gemm(x.const_data_ptr(), w.const_data_ptr(), out.mutable_data_ptr(), data(bias), nullptr, int(tokens), int(features), int(k), int(x.stride(0)),
+                 int(w.stride(0)), int(out.stride(0)), 0, 1.f, &plan, rc, x_t || w_t ? &opts : nullptr, stream_of(x)),
+        "tpb_gemm_bf16");
+  launched.fetch_add(1, std::memory_order_relaxed);
+  return out;
+}
+
+std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
+  std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = last;
+  return shape;
+}
+
+struct LinearFn : torch::autograd::Function<LinearFn> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_) {
+    const Tensor bias = or_undefined(bias_);
+    const Tensor x2d = x.reshape({-1, x.size(-1)});
+    const Tensor out = gemm(x2d, weight, bias, false, false);
+    ctx->save_for_backward({x2d, weight});
+    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["bias"] = bias.defined();
+    return out.view(with_last(x, weight.size(0)));
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2d = saved[0], &weight = saved[1], &grad = grads[0];
+    const Tensor g = grad.reshape({-1, grad.size(-1)}).to(at::kBFloat16).contiguous();
+    Tensor gx, gw, gb;
+    if (ctx->needs_input_grad(0)) gx = gemm(g, weight, Tensor(), false, true).view(ctx->saved_data["shape"].toIntVector());
+    if (ctx->needs_input_grad(1)) gw = gemm(g, x2d, Tensor(), true, true);
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2))
+      gb = g.sum(at::IntArrayRef{0}, false, at::kFloat).to(grad.scalar_type());  // (summed in fp32 without an fp32 copy of the gradient)
+    return {gx, gw, gb};
+  }
+};
+
+Tensor linear(const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_) {
+  const Tensor bias = or_undefined(bias_);
+  if (at::GradMode::is_enabled() && (x.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad())))
+    return LinearFn::apply(x, weight, bias_);
+  return gemm(x.reshape({-1, x.size(-1)}), weight, bias, false, false).view(with_last(x, weight.size(0)));
+}
+
+int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? 0 : 1; }
+
+// mode 0: RMSNorm, 1: LayerNorm, of bf16 or fp32 rows.
+struct NormFn : torch::autograd::Function<NormFn> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& weight_, const std::optional<Tensor>& bias_,
+                        double eps, int64_t mode) {
+    const Tensor weight = or_undefined(weight_), bias = or_undefined(bias_);
+    const Tensor x2d = x.reshape({-1, x.size(-1)}).contiguous();
+    const Tensor w = weight.defined() ? weight.to(x.scalar_type()).contiguous() : Tensor();
+    const Tensor b = bias.defined() ? bias.to(x.scalar_type()).contiguous() : Tensor();
+    const int64_t rows = x2d.size(0), cols = x2d.size(1);
+    Tensor out = at::empty_like(x2d);
+    Tensor rstd = at::empty({rows}, x2d.options().dtype(at::kFloat));
+    Tensor mean = mode == 1 ? at::empty_like(rstd) : Tensor();
+    check(lib.norm_fwd(x2d.const_data_ptr(), nullptr, data(w), data(b), out.mutable_data_ptr(), nullptr, rstd.data_ptr<float>(),
+                       mean.defined() ? mean.data_ptr<float>() : nullptr, int(rows), int(cols), float(eps), int(mode), dtype_code(x2d), stream_of(x2d)),
+          "tpb_norm_fwd");
+    launched.fetch_add(1, std::memory_order_relaxed);
+    ctx->save_for_backward({x2d, w, rstd, mean});
+    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["mode"] = mode;
+    ctx->saved_data["wdtype"] = weight.defined() ? int64_t(weight.scalar_type()) : int64_t(-1);
+    ctx->saved_data["bdtype"] = bias.defined() ? int64_t(bias.scalar_type()) : int64_t(-1);
+    return out.view(x.sizes());
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2d = saved[0], &w = saved[1], &rstd = saved[2], &mean = saved[3];
+    const int64_t mode = ctx->saved_data["mode"].toInt(), wdtype = ctx->saved_data["wdtype"].toInt(), bdtype = ctx->saved_data["bdtype"].toInt();
+    const Tensor g = grads[0].reshape(x2d.sizes()).to(x2d.scalar_type()).contiguous();
+    const int64_t rows = x2d.size(0), cols = x2d.size(1);
+    Tensor dx = at::empty_like(x2d);
+    // column sums: one fp32 partial row per CTA, added up by a second kernel that writes the gradients in their own dtype
+    const bool has_w = wdtype >= 0, has_b = bdtype >= 0;
+    const bool narrow = has_w && (!has_b || bdtype == wdtype) && wdtype == int64_t(at::kBFloat16);
+    const int parts = lib.norm_bwd_parts(int(rows), int(cols));
+    const auto fp32 = x2d.options().dtype(at::kFloat);
+    const auto as_grad = narrow ? x2d.options().dtype(at::kBFloat16) : fp32;
+    Tensor part_w = has_w ? at::empty({parts, cols}, fp32) : Tensor(), part_b = has_b ? at::empty({parts, cols}, fp32) : Tensor();
+    Tensor dw = has_w ? at::empty({cols}, as_grad) : Tensor(), db = has_b ? at::empty({cols}, as_grad) : Tensor();
+    auto out = [](Tensor& t) { return t.defined() ? t.mutable_data_ptr() : nullptr; };
+    check(lib.norm_bwd(g.const_data_ptr(), x2d.const_data_ptr(), data(w), rstd.const_data_ptr<float>(), mode == 1 ? mean.const_data_ptr<float>() : nullptr,
+                       dx.mutable_data_ptr(), static_cast<float*>(out(part_w)), static_cast<float*>(out(part_b)), out(dw), out(db), int(rows), int(cols),
+                       int(mode), dtype_code(x2d), narrow ? 0 : 1, stream_of(x2d)),
+          "tpb_norm_bwd");
+    launched.fetch_add(has_w || has_b ? 2 : 1, std::memory_order_relaxed);
+    if (has_w) dw = dw.to(at::ScalarType(wdtype));
+    if (has_b) db = db.to(at::ScalarType(bdtype));
+    return {dx.view(ctx->saved_data["shape"].toIntVector()), dw, db, Tensor(), Tensor()};
+  }
+};
+
+Tensor norm(const Tensor& x, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias, double eps, int64_t mode) {
+  return NormFn::apply(x, weight, bias, eps, mode);
+}
+
+template <typename F>
+void entry(F& f, const py::dict& addresses, const char* name) {
+  f = reinterpret_cast<F>(addresses[name].cast<uintptr_t>());
+}
+
+void bind(const py::dict& addresses, py::function text, py::function reserve) {
+  entry(lib.plan, addresses, "tpb_gemm_plan_ex");
+  entry(lib.gemm, addresses, "tpb_gemm_bf16_ex");
+  entry(lib.norm_fwd, addresses, "tpb_norm_fwd");
+  entry(lib.norm_bwd, addresses, "tpb_norm_bwd");
+  entry(lib.norm_bwd_parts, addresses, "tpb_norm_bwd_parts");
+  Py_XDECREF(error_text);
+  Py_XDECREF(reserve_slots);
+  error_text = text.release().ptr();  // (kept for the life of the process, beyond the interpreter's teardown of module globals)
+  reserve_slots = reserve.release().ptr();
+  for (auto& c : contexts) c.store(nullptr, std::memory_order_release);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("bind", &bind);
+  m.def("launches", [] { return launched.load(std::memory_order_relaxed); });
+  const auto unlocked = py::call_guard<py::gil_scoped_release>();
+  m.def("linear", &linear, unlocked);
+  m.def("norm", &norm, unlocked);
+}

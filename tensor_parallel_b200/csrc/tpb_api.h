@@ -114,6 +114,16 @@ int tpb_gemm_allgather_bf16(const void* w, void* out, const void* bias, int toke
                             int ldw, int ld_out, int act, const tpb_gemm_plan_t* plan, const tpb_reduce_ctx_t* rc,
                             const tpb_allgather_ctx_t* ag, void* stream);
 
+// RMSNorm (mode 0) / LayerNorm (mode 1) of [rows, cols] bf16 (dtype 0) or fp32 (dtype 1) rows; cols a multiple of 8.  With `residual`,
+// x + residual is normalised and also written to sum_out.  rstd_out / mean_out (fp32 per row) may be null.
+int tpb_norm_fwd(const void* x, const void* residual, const void* weight, const void* bias, void* out, void* sum_out, float* rstd_out,
+                 float* mean_out, int rows, int cols, float eps, int mode, int dtype, void* stream);
+// Rows of fp32 partials [rows][cols] that part_w / part_b of tpb_norm_bwd hold.
+int tpb_norm_bwd_parts(int rows, int cols);
+// dweight / dbias (either may be null, with its partials) are written, not accumulated; grad_dtype: 0 = bf16, 1 = fp32.
+int tpb_norm_bwd(const void* dy, const void* x, const void* weight, const float* rstd, const float* mean, void* dx, float* part_w,
+                 float* part_b, void* dweight, void* dbias, int rows, int cols, int mode, int dtype, int grad_dtype, void* stream);
+
 // Measurement aids.  tpb_gemm_debug caps the smem ring depth (0 restores the default).  Skipping the MMAs and the
 // kernel-internal %globaltimer trace (tpb_gemm_trace / tpb_gemm_trace_read) exist only in a library built with
 // -DTPB_GEMM_TRACE; in the product build they return TPB_ERR_ARG and the kernels carry no trace code.

@@ -241,7 +241,7 @@ class RankComm:
                                           c_void_p(bias.data_ptr() if bias is not None else 0), tokens, features, k, k,
                                           weight.stride(0), out.stride(0), native.ACT_CODES[act], ctypes.byref(plan),
                                           ctypes.byref(rctx), ctypes.byref(ctx), native._stream()), "tpb_gemm_allgather_bf16")
-        native.launch_count += 1
+        native.count_launches()
         return out
 
     # -- stand-alone collectives on the staging buffers -------------------------------------------
@@ -267,7 +267,7 @@ class RankComm:
                                  self._ptr_arrays["sig"], self._c_epochs, self._c_status, n,
                                  force_algo, self.wait_seconds, mc_in, mc_out, self._ptr_arrays["ll"], local_in,
                                  block_threads, native._stream()), "tpb_collective")
-        native.launch_count += 1
+        native.count_launches()
 
     def all_reduce_staged(self, offset: int, shape, dtype=torch.bfloat16, block_threads: int = 0) -> torch.Tensor:
         """Sum over ranks of the tensor that already lies in the staging-in buffer at byte ``offset`` (a multiple of

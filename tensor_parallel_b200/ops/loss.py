@@ -33,7 +33,7 @@ class _VocabParallelCE(torch.autograd.Function):
         stats = torch.empty(rows, 4, dtype=torch.float32, device=x2d.device)
         check(LIB.tpb_ce_stats(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), rows, cols, logits.stride(0), vocab_start,
                                ignore_index, native._stream()), "tpb_ce_stats")
-        native.launch_count += 1
+        native.count_launches()
         everyone = gather_stats(stats) if gather_stats is not None else stats[None]  # [world, rows, 4]
         gmax = everyone[..., 0].max(dim=0).values
         sumexp = (everyone[..., 1] * torch.exp(everyone[..., 0] - gmax)).sum(dim=0)
@@ -58,7 +58,7 @@ class _VocabParallelCE(torch.autograd.Function):
         scale = (grad_loss.float() / n_valid).reshape(1).contiguous()
         check(LIB.tpb_ce_grad(logits.data_ptr(), labels.data_ptr(), lse.data_ptr(), rows, cols, logits.stride(0), vocab_start,
                               ignore_index, scale.data_ptr(), native._stream()), "tpb_ce_grad")
-        native.launch_count += 1
+        native.count_launches()
         dlogits = logits  # overwritten in place
         gx = gw = None
         if ctx.needs_input_grad[0]:

@@ -7,6 +7,7 @@ fallback to stock PyTorch operators.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import math
 import os
 import threading
@@ -31,8 +32,30 @@ def _load() -> ctypes.CDLL:
     return ctypes.CDLL(str(path))
 
 
+def _load_autograd():
+    if not _build.AUTOGRAD_PATH.exists() or os.environ.get("TPB_REBUILD"):
+        _build.build_autograd()
+    spec = importlib.util.spec_from_file_location(_build.AUTOGRAD_PATH.stem, _build.AUTOGRAD_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 LIB = _load()
-launch_count = 0  # kernels launched through this binding since import (bench.py reports the delta)
+AUTOGRAD = _load_autograd()  # autograd nodes of linear layers and norms in C++ (csrc/autograd.cpp)
+_launches = 0
+
+
+def __getattr__(name):
+    if name == "launch_count":  # kernels launched through this binding since import (bench.py reports the delta)
+        return _launches + AUTOGRAD.launches()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
+def count_launches(n: int = 1):
+    global _launches
+    _launches += n
+
 
 c_void_p, c_int, c_float, c_ll, c_size_t = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_size_t
 
@@ -65,14 +88,18 @@ def device_wait_seconds() -> float:
     return min(float(os.environ.get("TENSOR_PARALLEL_TIMEOUT", "600")), 30.0)
 
 
+def _error_text(code: int, what: str) -> str:
+    detail = ""
+    if code == 3:
+        buf = ctypes.create_string_buffer(256)
+        LIB.tpb_last_cuda_error(buf, 256)
+        detail = f": {buf.value.decode()}"
+    return f"{what} failed: {_ERRORS.get(code, code)}{detail}"
+
+
 def check(code: int, what: str):
     if code != 0:
-        detail = ""
-        if code == 3:
-            buf = ctypes.create_string_buffer(256)
-            LIB.tpb_last_cuda_error(buf, 256)
-            detail = f": {buf.value.decode()}"
-        raise RuntimeError(f"{what} failed: {_ERRORS.get(code, code)}{detail}")
+        raise RuntimeError(_error_text(code, what))
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -153,6 +180,21 @@ def device_state(device: torch.device) -> DeviceState:
         return st
 
 
+def _reserve_slots(index: int, elems: int) -> int:
+    """Address of a device's reduction context with at least ``elems`` fp32 elements per slot (for the C++ autograd nodes)."""
+    state = device_state(torch.device("cuda", index))
+    state.ensure_slots(elems)
+    return ctypes.addressof(state.ctx)
+
+
+def _bind_autograd():
+    names = ("tpb_gemm_plan_ex", "tpb_gemm_bf16_ex", "tpb_norm_fwd", "tpb_norm_bwd", "tpb_norm_bwd_parts")
+    AUTOGRAD.bind({n: ctypes.cast(getattr(LIB, n), c_void_p).value for n in names}, _error_text, _reserve_slots)
+
+
+_bind_autograd()
+
+
 # ------------------------------------------------------------------------------------------------
 # GEMM
 # ------------------------------------------------------------------------------------------------
@@ -215,7 +257,7 @@ def gemm_nt(x2d: torch.Tensor, w: torch.Tensor, bias=None, residual=None, act=No
     indices against; 0 derives it from the shape.  ``early``: the kernel may start, and read ``w``, while the previous kernel
     of the stream is still running (that kernel must not write ``w``); everything else is read after it.  It has no effect on a
     ``w`` that TMA cannot read in place."""
-    global launch_count
+    global _launches
     if x_t:
         k, tokens = x2d.shape
     else:
@@ -247,7 +289,7 @@ def gemm_nt(x2d: torch.Tensor, w: torch.Tensor, bias=None, residual=None, act=No
     check(LIB.tpb_gemm_bf16_ex(_ptr(x2d), _ptr(w), _ptr(out), _ptr(bias), _ptr(residual), tokens, features, k, x2d.stride(0),
                                w.stride(0), out.stride(0), ACT_CODES[act], bias_scale, ctypes.byref(plan), ctypes.byref(ctx),
                                ctypes.byref(opts) if opts is not None else None, _stream()), "tpb_gemm_bf16")
-    launch_count += 1
+    _launches += 1
     return out
 
 
@@ -278,43 +320,15 @@ LIB.tpb_transpose_bf16.argtypes = [c_void_p, c_void_p, c_int, c_int, c_ll, c_ll,
 
 
 def transpose(x2d: torch.Tensor) -> torch.Tensor:
-    global launch_count
+    global _launches
     rows, cols = x2d.shape
     if x2d.stride(1) != 1:
         x2d = x2d.contiguous()
     pitch = (rows + 7) // 8 * 8  # keeps the result usable as a TMA operand
     out = torch.empty(cols, pitch, dtype=x2d.dtype, device=x2d.device)[:, :rows]
     check(LIB.tpb_transpose_bf16(_ptr(x2d), _ptr(out), rows, cols, x2d.stride(0), pitch, _stream()), "tpb_transpose_bf16")
-    launch_count += 1
+    _launches += 1
     return out
-
-
-class _LinearFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias):
-        x2d = x.reshape(-1, x.shape[-1])
-        out = gemm_nt(x2d, weight, bias)
-        ctx.save_for_backward(x2d, weight)
-        ctx.has_bias = bias is not None
-        ctx.x_shape = x.shape
-        return out.view(*x.shape[:-1], weight.shape[0])
-
-    @staticmethod
-    def backward(ctx, grad):
-        x2d, weight = ctx.saved_tensors
-        g2d = grad.reshape(-1, grad.shape[-1])
-        if g2d.dtype != torch.bfloat16:
-            g2d = g2d.to(torch.bfloat16)
-        if not g2d.is_contiguous():
-            g2d = g2d.contiguous()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            gx = linear_dgrad(g2d, weight).view(ctx.x_shape)
-        if ctx.needs_input_grad[1]:
-            gw = linear_wgrad(g2d, x2d)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            gb = g2d.sum(0, dtype=torch.float32).to(grad.dtype)  # (summed in fp32 without an fp32 copy of the gradient)
-        return gx, gw, gb
 
 
 def linear_dgrad(g2d: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -330,10 +344,7 @@ def linear_wgrad(g2d: torch.Tensor, x2d: torch.Tensor) -> torch.Tensor:
 
 
 def linear(x, weight, bias=None):
-    if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)):
-        return _LinearFn.apply(x, weight, bias)
-    x2d = x.reshape(-1, x.shape[-1])
-    return gemm_nt(x2d, weight, bias).view(*x.shape[:-1], weight.shape[0])
+    return AUTOGRAD.linear(x, weight, bias)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -341,7 +352,6 @@ def linear(x, weight, bias=None):
 # ------------------------------------------------------------------------------------------------
 
 LIB.tpb_norm_fwd.argtypes = [c_void_p] * 8 + [c_int, c_int, c_float, c_int, c_int, c_void_p]
-LIB.tpb_norm_bwd.argtypes = [c_void_p] * 10 + [c_int] * 5 + [c_void_p]
 
 
 def norm_supported(x: torch.Tensor) -> bool:
@@ -349,57 +359,23 @@ def norm_supported(x: torch.Tensor) -> bool:
 
 
 def norm_forward(x2d, weight, bias, eps, mode, residual=None, sum_out=None, want_stats=False, out=None):
-    global launch_count
+    global _launches
     rows, cols = x2d.shape
     out = torch.empty_like(x2d) if out is None else out
     rstd = torch.empty(rows, dtype=torch.float32, device=x2d.device) if want_stats else None
     mean = torch.empty(rows, dtype=torch.float32, device=x2d.device) if (want_stats and mode == 1) else None
     check(LIB.tpb_norm_fwd(_ptr(x2d), _ptr(residual), _ptr(weight), _ptr(bias), _ptr(out), _ptr(sum_out), _ptr(rstd), _ptr(mean),
                            rows, cols, eps, mode, _dtype_code(x2d), _stream()), "tpb_norm_fwd")
-    launch_count += 1
+    _launches += 1
     return out, rstd, mean
 
 
-class _NormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, eps, mode):
-        x2d = x.reshape(-1, x.shape[-1]).contiguous()
-        w = None if weight is None else weight.to(x.dtype).contiguous()
-        b = None if bias is None else bias.to(x.dtype).contiguous()
-        out, rstd, mean = norm_forward(x2d, w, b, eps, mode, want_stats=True)
-        ctx.save_for_backward(x2d, w, rstd, mean if mean is not None else rstd)
-        ctx.mode, ctx.shape = mode, x.shape
-        ctx.wdtype = None if weight is None else weight.dtype
-        ctx.bdtype = None if bias is None else bias.dtype
-        return out.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, grad):
-        global launch_count
-        x2d, w, rstd, mean = ctx.saved_tensors
-        g2d = grad.reshape(x2d.shape).to(x2d.dtype).contiguous()
-        rows, cols = x2d.shape
-        dx = torch.empty_like(x2d)
-        # column sums: one fp32 partial row per CTA, added up by a second kernel that writes the gradients in their own dtype
-        has_w, has_b = w is not None, ctx.bdtype is not None
-        gdtype = ctx.wdtype if has_w and (not has_b or ctx.bdtype == ctx.wdtype) and ctx.wdtype == torch.bfloat16 else torch.float32
-        parts = LIB.tpb_norm_bwd_parts(rows, cols)
-        part_w = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_w else None
-        part_b = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_b else None
-        dw = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_w else None
-        db = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_b else None
-        check(LIB.tpb_norm_bwd(_ptr(g2d), _ptr(x2d), _ptr(w), _ptr(rstd), _ptr(mean), _ptr(dx), _ptr(part_w), _ptr(part_b), _ptr(dw), _ptr(db),
-                               rows, cols, ctx.mode, _dtype_code(x2d), int(gdtype == torch.float32), _stream()), "tpb_norm_bwd")
-        launch_count += 2 if has_w or has_b else 1
-        return (dx.view(ctx.shape), None if dw is None else dw.to(ctx.wdtype), None if db is None else db.to(ctx.bdtype), None, None)
-
-
 def rms_norm(x, weight, eps):
-    return _NormFn.apply(x, weight, None, eps, 0)
+    return AUTOGRAD.norm(x, weight, None, eps, 0)
 
 
 def layer_norm(x, weight, bias, eps):
-    return _NormFn.apply(x, weight, bias, eps, 1)
+    return AUTOGRAD.norm(x, weight, bias, eps, 1)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -415,14 +391,14 @@ def rope_supported(x: torch.Tensor) -> bool:
 
 
 def _rope_launch(x, positions, theta, rotary_dim, interleaved, inverse):
-    global launch_count
+    global _launches
     b, s, h, d = x.shape
     xc = x.contiguous()
     out = torch.empty_like(xc)
     pos = positions.to(device=x.device, dtype=torch.int64).expand(b, s).contiguous()
     check(LIB.tpb_rope(_ptr(xc), _ptr(out), _ptr(pos), c_void_p(0), s, b * s, h, d, rotary_dim, theta, int(interleaved), int(inverse),
                        h * d, h * d, _dtype_code(xc), _stream()), "tpb_rope")
-    launch_count += 1
+    _launches += 1
     return out
 
 
@@ -457,7 +433,7 @@ def elementwise_supported(x: torch.Tensor) -> bool:
 
 def act_forward(gate, up, kind: int, out=None):
     """``act(gate) * up`` (``up`` may be None); ``gate`` / ``up`` may be column slices of one wider tensor."""
-    global launch_count
+    global _launches
     cols = gate.shape[-1]
     g2 = gate.reshape(-1, cols) if gate.stride(-1) == 1 else gate.contiguous().view(-1, cols)
     u2 = None if up is None else (up.reshape(-1, cols) if up.stride(-1) == 1 else up.contiguous().view(-1, cols))
@@ -466,7 +442,7 @@ def act_forward(gate, up, kind: int, out=None):
         out = torch.empty(*gate.shape, dtype=gate.dtype, device=gate.device)
     check(LIB.tpb_act_fwd(_ptr(g2), _ptr(u2), _ptr(out), rows, cols, g2.stride(0), 0 if u2 is None else u2.stride(0), kind,
                           _dtype_code(gate), _stream()), "tpb_act_fwd")
-    launch_count += 1
+    _launches += 1
     return out
 
 
@@ -481,7 +457,7 @@ class _ActFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad):
-        global launch_count
+        global _launches
         gate, up = ctx.saved_tensors
         up = up if ctx.has_up else None
         g = grad.to(gate.dtype).contiguous()
@@ -489,7 +465,7 @@ class _ActFn(torch.autograd.Function):
         dup = torch.empty_like(gate) if up is not None else None
         check(LIB.tpb_act_bwd(_ptr(g), _ptr(gate), _ptr(up), _ptr(dgate), _ptr(dup), gate.numel(), ctx.kind, _dtype_code(gate), _stream()),
               "tpb_act_bwd")
-        launch_count += 1
+        _launches += 1
         return dgate, dup, None
 
 
@@ -543,7 +519,7 @@ def _strided_ok(t: torch.Tensor) -> bool:
 def attention_forward(q, k, v, causal, scale, want_lse=False, bias=None, out=None):
     """q ``[B,Sq,Hq,D]``, k / v ``[B,Sk,Hkv,D]`` (any strides with contiguous head_dim) -> ``[B,Sq,Hq,D]``.
     ``bias`` (bf16 / fp32, broadcastable to ``[B,Hq,Sq,Sk]``) is added to the scaled scores; ``-inf`` masks a key."""
-    global launch_count
+    global _launches
     q = q if _strided_ok(q) else q.contiguous()
     k = k if _strided_ok(k) else k.contiguous()
     v = v if _strided_ok(v) else v.contiguous()
@@ -576,7 +552,7 @@ def attention_forward(q, k, v, causal, scale, want_lse=False, bias=None, out=Non
                                         v.stride(0), v.stride(1), v.stride(2), out.stride(0), out.stride(1), out.stride(2),
                                         int(causal), scale, _ptr(bias4), 1 if bias4.dtype == torch.float32 else 0,
                                         strides[0], strides[1], strides[2], strides[3], _stream()), "tpb_attn_prefill_bias")
-    launch_count += 1
+    _launches += 1
     return out, lse
 
 
@@ -594,7 +570,7 @@ def _bias_view(bias):
 def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_dbias=False):
     """Gradients of :func:`attention_forward` (scores are recomputed tile by tile).  With ``bias`` the scores are
     re-biased; ``want_dbias`` also returns the gradient of the bias (fp32, in the bias' own shape)."""
-    global launch_count
+    global _launches
     q, k, v, dout = (t if _strided_ok(t) else t.contiguous() for t in (q, k, v, dout))
     b, sq, hq, d = q.shape
     sk, hkv = k.shape[1], k.shape[2]
@@ -623,7 +599,7 @@ def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_d
                                           dk.stride(0), dk.stride(1), dk.stride(2), int(causal), scale, _ptr(bias4), bias_is_fp32,
                                           bstr[0], bstr[1], bstr[2], bstr[3], _ptr(dbias), _ptr(status), _stream()),
               "tpb_attn_backward_sm100")
-        launch_count += 3
+        _launches += 3
         if want_dbias:
             return dq, dk, dv, dbias.reshape(bias.shape)
         return dq, dk, dv
@@ -635,7 +611,7 @@ def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_d
                                      dk.stride(0), dk.stride(1), dk.stride(2), int(causal), scale, _ptr(bias4),
                                      bias_is_fp32, bstr[0], bstr[1], bstr[2], bstr[3],
                                      _ptr(dbias), _stream()), "tpb_attn_backward")
-    launch_count += 3
+    _launches += 3
     if want_dbias:
         return dq, dk, dv, dbias.reshape(bias.shape)
     return dq, dk, dv
@@ -680,7 +656,7 @@ def attention(q, k, v, causal, bias=None, scale=None):
 
 def attn_decode(q, kcache, vcache, len_ptr, len_add, scale=None, splits=1, workspace=None, out=None):
     """q ``[B,Hq,D]`` against cache ``[B,Hkv,Smax,D]``; the number of valid keys is ``len_ptr[0] + len_add``."""
-    global launch_count
+    global _launches
     b, hq, d = q.shape
     hkv, smax = kcache.shape[1], kcache.shape[2]
     out = torch.empty_like(q) if out is None else out
@@ -693,7 +669,7 @@ def attn_decode(q, kcache, vcache, len_ptr, len_add, scale=None, splits=1, works
     scale = 1.0 / math.sqrt(d) if scale is None else scale
     check(LIB.tpb_attn_decode(_ptr(q), _ptr(kcache), _ptr(vcache), _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(len_ptr), len_add,
                               b, hq, hkv, d, smax, splits, scale, _stream()), "tpb_attn_decode")
-    launch_count += LIB.tpb_last_launches()
+    _launches += LIB.tpb_last_launches()
     return out
 
 
@@ -703,11 +679,11 @@ LIB.tpb_rope_table.argtypes = [c_void_p, c_int, c_int, c_float, c_void_p]
 
 def rope_table(positions: int, rotary_dim: int, theta: float, device) -> torch.Tensor:
     """fp32 ``[positions, rotary_dim // 2, 2]`` table of (cos, sin) rotary angles for :func:`attn_decode_fused`."""
-    global launch_count
+    global _launches
     table = torch.empty(positions, rotary_dim // 2, 2, dtype=torch.float32, device=device)
     with torch.cuda.device(device):
         check(LIB.tpb_rope_table(_ptr(table), positions, rotary_dim, theta, _stream()), "tpb_rope_table")
-    launch_count += 1
+    _launches += 1
     return table
 
 
@@ -718,7 +694,7 @@ def attn_decode_fused(q, k, v, kcache, vcache, pos_ptr, rotary_dim, theta, inter
     ``workspace = (part_o, part_ml, counters)`` with ``counters`` an int32 tensor of at least ``batch * kv_heads`` elements
     zeroed once (``batch * q_heads``: all query-head groups of a KV head share one launch).  ``early``: the kernel may start while
     the previous kernel of the stream is still running and read ``pos_ptr`` and the cached rows, which that kernel must not write."""
-    global launch_count
+    global _launches
     d = kcache.shape[3]
     b, hq, hkv, smax = q.shape[0], q.shape[1] // d, kcache.shape[1], kcache.shape[2]
     out = torch.empty(b, hq, d, dtype=q.dtype, device=q.device) if out is None else out  # (rows may be column slices of a wider buffer)
@@ -735,20 +711,20 @@ def attn_decode_fused(q, k, v, kcache, vcache, pos_ptr, rotary_dim, theta, inter
                                     int(interleaved), q.stride(0), k.stride(0), v.stride(0), _ptr(rope_angles),
                                     out.stride(0) if out.stride(0) != hq * d else 0, 0 if counters is None else counters.numel(), int(early), _stream()),
           "tpb_attn_decode_fused")
-    launch_count += LIB.tpb_last_launches()
+    _launches += LIB.tpb_last_launches()
     return out
 
 
 def qkv_rope_append(q, k, v, q_out, kcache, vcache, base_pos, batch, seq, rotary_dim, theta, interleaved=False):
     """Rotary-embed q / k of ``batch*seq`` new tokens and append k, v to the cache at ``base_pos[0] + s``.
     q / k / v are 2-D views ``[tokens, heads*head_dim]`` (column slices of one fused projection are fine)."""
-    global launch_count
+    global _launches
     d = kcache.shape[3]
     hq, hkv, smax = q.shape[1] // d, kcache.shape[1], kcache.shape[2]
     check(LIB.tpb_qkv_rope_append(_ptr(q), _ptr(k), _ptr(v), _ptr(q_out), _ptr(kcache), _ptr(vcache), _ptr(base_pos), batch, seq,
                                   hq, hkv, d, rotary_dim, theta, int(interleaved), smax, q.stride(0), k.stride(0), v.stride(0),
                                   _stream()), "tpb_qkv_rope_append")
-    launch_count += 1
+    _launches += 1
     return q_out
 
 
@@ -765,21 +741,21 @@ def relative_bias_supported(table: torch.Tensor, queries: int, keys: int) -> boo
 class _RelativeBiasFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, table, buckets, queries, keys):
-        global launch_count
+        global _launches
         n, heads = table.shape
         table = table.contiguous()
         buckets = buckets.to(torch.int64).contiguous()
         out = torch.empty(1, heads, queries, keys, dtype=table.dtype, device=table.device)
         check(LIB.tpb_relative_bias(_ptr(table), _ptr(buckets), _ptr(out), heads, queries, keys, n, _dtype_code(table),
                                     _ptr(device_state(table.device).status), _stream()), "tpb_relative_bias")
-        launch_count += 1
+        _launches += 1
         ctx.save_for_backward(buckets)
         ctx.meta = (n, heads, queries, keys, table.dtype)
         return out
 
     @staticmethod
     def backward(ctx, grad):
-        global launch_count
+        global _launches
         (buckets,) = ctx.saved_tensors
         n, heads, queries, keys, dtype = ctx.meta
         if torch.is_grad_enabled() or OF.transformed(grad):  # a second derivative, or a batch of gradients
@@ -787,7 +763,7 @@ class _RelativeBiasFn(torch.autograd.Function):
         g = grad.to(dtype).contiguous()
         partial = torch.empty(LIB.tpb_relative_bias_parts(queries), n, heads, dtype=torch.float32, device=g.device)
         check(LIB.tpb_relative_bias_bwd(_ptr(g), _ptr(buckets), _ptr(partial), heads, queries, keys, n, _dtype_code(g), _stream()), "tpb_relative_bias_bwd")
-        launch_count += 1
+        _launches += 1
         return partial.sum(0).to(dtype), None, None, None
 
 
@@ -808,14 +784,14 @@ LIB.tpb_cast.argtypes = [c_void_p, c_void_p, c_ll, c_float, c_int, c_void_p]
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor, out=None):
-    global launch_count
+    global _launches
     flat = ids.reshape(-1).to(torch.int64).contiguous()
     cols = table.shape[1]
     if out is None:
         out = torch.empty(flat.numel(), cols, dtype=table.dtype, device=table.device)
     check(LIB.tpb_embedding(_ptr(flat), _ptr(table), _ptr(out), flat.numel(), cols, table.stride(0), out.stride(0), _dtype_code(table),
                             _stream()), "tpb_embedding")
-    launch_count += 1
+    _launches += 1
     return out.view(*ids.shape, cols) if out.shape[0] == flat.numel() and out.is_contiguous() else out
 
 
@@ -825,18 +801,18 @@ LIB.tpb_greedy_pick.argtypes = [c_void_p, c_ll, c_int, c_int, c_void_p, c_void_p
 def greedy_pick(logits: torch.Tensor, next_ids: torch.Tensor, ids: torch.Tensor, pos: torch.Tensor, early: bool = False):
     """End of a greedy decode step in one launch: ``next_ids[:] = ids[:] = logits.argmax(-1)`` (bf16 ``[rows, cols]``, ties and
     NaN like ``torch.argmax``; int64 ids), ``pos[0] += 1`` (int32).  ``early``: see :func:`gemm_nt`."""
-    global launch_count
+    global _launches
     rows, cols = logits.shape
     check(LIB.tpb_greedy_pick(_ptr(logits), logits.stride(0), rows, cols, _ptr(next_ids), _ptr(ids), _ptr(pos), int(early), _stream()),
           "tpb_greedy_pick")
-    launch_count += 1
+    _launches += 1
 
 
 def adamw_step(param, grad, exp_avg, exp_avg_sq, step, lr, beta1, beta2, eps, weight_decay, master=None, grad_scale=1.0):
-    global launch_count
+    global _launches
     check(LIB.tpb_adamw(_ptr(param), _ptr(grad), _ptr(exp_avg), _ptr(exp_avg_sq), _ptr(master), param.numel(), lr, beta1, beta2, eps,
                         weight_decay, step, grad_scale, _dtype_code(param), int(grad.dtype == torch.float32), _stream()), "tpb_adamw")
-    launch_count += 1
+    _launches += 1
 
 
 LIB.tpb_last_cuda_error.argtypes = [ctypes.c_char_p, c_int]

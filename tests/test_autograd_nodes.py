@@ -1,0 +1,217 @@
+"""The C++ autograd nodes of linear layers and norms, on the CPU: the kernels are stood in for by PyTorch on the same memory."""
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+from torch.utils.checkpoint import checkpoint
+
+from tensor_parallel_b200 import build
+
+pytestmark = pytest.mark.skipif(not (build.LIB_PATH.exists() and build.AUTOGRAD_PATH.exists()), reason="native library not built")
+
+_p, _i, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+
+
+def _memory(address, count, dtype):
+    size = torch.empty((), dtype=dtype).element_size()
+    return torch.frombuffer((ctypes.c_char * (count * size)).from_address(address), dtype=dtype)
+
+
+def _matrix(address, rows, cols, pitch, dtype=torch.bfloat16):
+    return _memory(address, (rows - 1) * pitch + cols, dtype).as_strided((rows, cols), (pitch, 1))
+
+
+def _plan(tokens, features, k, world, splits, kbox, flags, plan):
+    return 0
+
+
+def _gemm(x, w, out, bias, residual, tokens, features, k, ldx, ldw, ld_out, act, scale, plan, rc, opts, stream):
+    from tensor_parallel_b200.ops import native
+
+    o = ctypes.cast(opts, ctypes.POINTER(native.GemmOpts)).contents if opts else native.GemmOpts()
+    a = _matrix(x, k, tokens, ldx).t() if o.x_mn else _matrix(x, tokens, k, ldx)
+    b = _matrix(w, k, features, ldw).t() if o.w_mn else _matrix(w, features, k, ldw)
+    y = a.float() @ b.float().t()
+    if bias:
+        y = y + _memory(bias, features, torch.bfloat16).float()
+    _matrix(out, tokens, features, ld_out).copy_(y)
+    return _gemm.code
+
+
+_gemm.code = 0
+
+
+def _norm_fwd(x, residual, weight, bias, out, sum_out, rstd, mean, rows, cols, eps, mode, dtype, stream):
+    dt = torch.float32 if dtype else torch.bfloat16
+    v = _matrix(x, rows, cols, cols, dt).float()
+    m = v.mean(-1) if mode else torch.zeros(rows)
+    r = ((v - m[:, None]).square().mean(-1) + eps).rsqrt()
+    y = (v - m[:, None]) * r[:, None]
+    if weight:
+        y = y * _memory(weight, cols, dt).float()
+    if bias:
+        y = y + _memory(bias, cols, dt).float()
+    _matrix(out, rows, cols, cols, dt).copy_(y)
+    _memory(rstd, rows, torch.float32).copy_(r)
+    if mode:
+        _memory(mean, rows, torch.float32).copy_(m)
+    return 0
+
+
+def _norm_bwd_parts(rows, cols):
+    return 1
+
+
+def _norm_bwd(dy, x, weight, rstd, mean, dx, part_w, part_b, dw, db, rows, cols, mode, dtype, grad_fp32, stream):
+    dt, gt = torch.float32 if dtype else torch.bfloat16, torch.float32 if grad_fp32 else torch.bfloat16
+    g, v = _matrix(dy, rows, cols, cols, dt).float(), _matrix(x, rows, cols, cols, dt).float()
+    r = _memory(rstd, rows, torch.float32)[:, None]
+    xh = (v - _memory(mean, rows, torch.float32)[:, None]) * r if mode else v * r
+    gw = g * _memory(weight, cols, dt).float() if weight else g
+    c1 = gw.mean(-1, keepdim=True) if mode else 0.0
+    _matrix(dx, rows, cols, cols, dt).copy_((gw - c1 - xh * (gw * xh).mean(-1, keepdim=True)) * r)
+    if dw:
+        _memory(dw, cols, gt).copy_((g * xh).sum(0))
+    if db:
+        _memory(db, cols, gt).copy_(g.sum(0))
+    return 0
+
+
+@pytest.fixture
+def nodes():
+    from tensor_parallel_b200.ops import native
+
+    signatures = dict(tpb_gemm_plan_ex=(_plan, [_i] * 7 + [_p]), tpb_gemm_bf16_ex=(_gemm, [_p] * 5 + [_i] * 7 + [_f] + [_p] * 4),
+                      tpb_norm_fwd=(_norm_fwd, [_p] * 8 + [_i, _i, _f, _i, _i, _p]), tpb_norm_bwd=(_norm_bwd, [_p] * 10 + [_i] * 5 + [_p]),
+                      tpb_norm_bwd_parts=(_norm_bwd_parts, [_i, _i]))
+    stubs = {name: ctypes.CFUNCTYPE(_i, *args)(fn) for name, (fn, args) in signatures.items()}
+    context = native.ReduceCtx()
+    native.AUTOGRAD.bind({n: ctypes.cast(s, _p).value for n, s in stubs.items()}, native._error_text, lambda index, elems: ctypes.addressof(context))
+    yield native
+    native._bind_autograd()
+
+
+def _close(got, want):
+    assert got.dtype == want.dtype and got.shape == want.shape
+    assert (got.float() - want.float()).norm() <= 2e-2 * want.float().norm() + 1e-6  # bf16 results of both sides: 2^-8 each, in and out
+
+
+@pytest.mark.parametrize("with_bias", [False, True])
+@pytest.mark.parametrize("frozen", ["", "x", "weight", "bias"])
+@pytest.mark.parametrize("form", ["plain", "three dimensions", "strided", "fp32 gradient", "odd pitch"])
+def test_linear_node(nodes, with_bias, frozen, form):
+    torch.manual_seed(0)
+    inputs = 20 if form == "odd pitch" else 24
+    x = torch.randn(2, 5, inputs, dtype=torch.bfloat16) if form == "three dimensions" else torch.randn(10, inputs, dtype=torch.bfloat16)
+    if form == "strided":
+        x = torch.randn(inputs, 10, dtype=torch.bfloat16).t()
+    leaves = dict(x=x, weight=torch.randn(16, inputs, dtype=torch.bfloat16) * 0.1, bias=torch.randn(16, dtype=torch.bfloat16) if with_bias else None)
+    results = []
+    for call in (nodes.linear, F.linear):
+        t = {n: None if v is None else v.detach().requires_grad_(n != frozen) for n, v in leaves.items()}
+        out = call(t["x"], t["weight"], t["bias"])
+        grad = torch.ones_like(out) + torch.arange(16) / 16
+        if form == "strided":
+            grad = grad.t().contiguous().t()
+        if form == "fp32 gradient":
+            out.float().backward(grad.float())
+        else:
+            out.backward(grad.to(out.dtype))
+        results.append([out.detach()] + [None if v is None else v.grad for v in t.values()])
+    for got, want in zip(*results):
+        assert (got is None) == (want is None)
+        if want is not None:
+            _close(got, want)
+
+
+@pytest.mark.parametrize("mode,dtype,wdtype,with_bias,with_weight", [(0, torch.bfloat16, torch.bfloat16, False, True), (0, torch.float32, torch.float32, False, True),
+                                                                   (1, torch.bfloat16, torch.bfloat16, True, True), (1, torch.float32, torch.bfloat16, True, True),
+                                                                   (1, torch.bfloat16, torch.float32, False, True), (0, torch.bfloat16, None, False, False)])
+def test_norm_node(nodes, mode, dtype, wdtype, with_bias, with_weight):
+    torch.manual_seed(1)
+    x = torch.randn(3, 4, 32, dtype=dtype)
+    w = torch.randn(32, dtype=wdtype) if with_weight else None
+    b = torch.randn(32, dtype=wdtype) if with_bias else None
+    g = torch.randn(3, 4, 32, dtype=dtype)
+    leaves = [None if t is None else t.detach().requires_grad_() for t in (x, w, b)]
+    refs = [None if t is None else t.detach().double().requires_grad_() for t in (x, w, b)]
+    out = nodes.AUTOGRAD.norm(*leaves, 1e-5, mode)
+    out.backward(g)
+    if mode:
+        want = F.layer_norm(refs[0], (32,), refs[1], refs[2], 1e-5)
+    else:
+        want = refs[0] * (refs[0].square().mean(-1, keepdim=True) + 1e-5).rsqrt() * (1 if w is None else refs[1])
+    want.backward(g.double())
+    _close(out.detach(), want.detach().to(dtype))
+    for leaf, ref in zip(leaves, refs):
+        if leaf is not None:
+            _close(leaf.grad, ref.grad.to(leaf.dtype))
+
+
+def _linear_case():
+    torch.manual_seed(2)
+    return torch.randn(6, 16, dtype=torch.bfloat16, requires_grad=True), torch.randn(8, 16, dtype=torch.bfloat16, requires_grad=True)
+
+
+def test_saved_tensors_go_through_the_hooks(nodes):
+    x, w = _linear_case()
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.data_ptr()) or t.clone(), lambda t: t):
+        out = nodes.linear(x, w)
+    assert packed == [x.data_ptr(), w.data_ptr()]
+    out.sum().backward()
+    y = torch.randn(4, 16, requires_grad=True)
+    packed.clear()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.data_ptr()) or t.clone(), lambda t: t):
+        nodes.rms_norm(y, torch.ones(16), 1e-6)
+    assert y.data_ptr() in packed
+
+
+def test_checkpointed_linear(nodes):
+    x, w = _linear_case()
+    checkpoint(lambda t: nodes.linear(t, w).relu(), x, use_reentrant=False).sum().backward()
+    again, w2 = (t.detach().requires_grad_() for t in (x, w))
+    nodes.linear(again, w2).relu().sum().backward()
+    assert torch.equal(x.grad, again.grad) and torch.equal(w.grad, w2.grad)
+
+
+def test_changed_inputs_are_noticed(nodes):
+    x, w = _linear_case()
+    out = nodes.linear(x, w)
+    with torch.no_grad():
+        w.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.sum().backward()
+
+
+@pytest.mark.parametrize("layer", ["linear", "norm"])
+def test_transforms_are_refused(nodes, layer):
+    x, w = _linear_case()
+    call = (lambda t: nodes.linear(t, w)) if layer == "linear" else (lambda t: nodes.rms_norm(t, torch.ones(16, dtype=t.dtype), 1e-6))
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(call)(x.detach()[None])
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: call(t).sum())(x.detach())
+    with pytest.raises(RuntimeError), torch.autograd.forward_ad.dual_level():
+        call(torch.autograd.forward_ad.make_dual(x.detach().requires_grad_(), torch.ones_like(x)))
+    out = call(x)
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(out, x, torch.ones(3, *out.shape, dtype=out.dtype), is_grads_batched=True)
+
+
+def test_nothing_is_recorded_without_gradients(nodes):
+    x, w = _linear_case()
+    with torch.no_grad():
+        assert nodes.linear(x, w).grad_fn is None and nodes.rms_norm(x, None, 1e-6).grad_fn is None
+    assert nodes.linear(x.detach(), w.detach()).grad_fn is None
+
+
+def test_an_error_of_a_kernel_reaches_the_caller(nodes, monkeypatch):
+    x, w = _linear_case()
+    out = nodes.linear(x, w)
+    monkeypatch.setattr(_gemm, "code", 6)
+    with pytest.raises(RuntimeError, match="tpb_gemm_bf16 failed: reduction workspace too small"):
+        nodes.linear(x, w)
+    with pytest.raises(RuntimeError, match="tpb_gemm_bf16 failed: reduction workspace too small"):
+        out.sum().backward()
