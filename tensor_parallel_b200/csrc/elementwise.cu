@@ -7,6 +7,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
 #include "tpb_api.h"
@@ -148,9 +150,10 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T
 // Backward: dx per row; the column sums for dweight / dbias go through one fp32 partial row per CTA, which
 // norm_bwd_reduce_kernel adds up in a fixed order (deterministic, no atomics).  Memory-bound: x and dy are read and dx is
 // written once.  A thread owns 8 columns (a CTA has as many threads as the row has vectors, so that its registers admit 1024
-// threads per SM whatever the width) and walks rows blockIdx.x, + gridDim.x, ... with the column sums in registers; bf16 rows are
-// fetched one ahead, before the block-wide sums of the current row.  RMSNorm 8192 x 4096 bf16: 57 us (3.5 TB/s; 73 us with half as
-// many threads of two vectors each), LayerNorm 1999 x 5120 fp32: 40 us.
+// threads per SM whatever the width) and walks rows blockIdx.x, + gridDim.x, ... with the column sums in registers.  Rows arrive through
+// a ring of private slots in shared memory (cp.async; nobody reads another thread's slot), three rows ahead (fp32: two): one row ahead
+// in registers kept 32 KB per SM in flight, too little for the latency of a loaded memory system.  RMSNorm 8192 x 4096 bf16 63 -> 48 us
+// (4.2 TB/s), 8192 x 8192 122 -> 86; LayerNorm 1999 x 5120 fp32 44 -> 40 us, 8192 x 8192 fp32 201 -> 162; 20 x 4096 5.0 and 5.0.
 constexpr int NORM_BWD_MAXC = 8192;  // 1024 threads
 
 template <typename T> struct Raw8 { uint4 u[sizeof(T) / 2]; };  // 8 elements as they lie in memory
@@ -174,35 +177,112 @@ __device__ __forceinline__ void unpack(const Raw8<float>& r, float (&v)[8]) {
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
 }
 
+// The 8 columns of a thread in 16-byte chunks: bf16 one chunk, fp32 two, which lie blockDim.x chunks apart so that a warp's accesses are
+// contiguous (cp.async goes past L1: chunks side by side would fetch every 32-byte sector twice).
+template <typename T>
+struct RowCols {
+  static constexpr int CHUNKS = sizeof(T) / 2, WIDTH = 16 / sizeof(T);
+  static __device__ __forceinline__ int at(int i) { return (threadIdx.x + i * blockDim.x) * WIDTH; }
+  static __device__ __forceinline__ Raw8<T> load(const T* row, int cols) {
+    Raw8<T> r;
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) r.u[i] = at(i) < cols ? *reinterpret_cast<const uint4*>(row + at(i)) : make_uint4(0, 0, 0, 0);
+    return r;
+  }
+  template <typename O>
+  static __device__ __forceinline__ void store(O* row, int cols, const float (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) {
+      if (at(i) >= cols) continue;
+      if constexpr (CHUNKS == 1) Vec8<O>::store(row + at(0), v);
+      else reinterpret_cast<float4*>(row)[threadIdx.x + i * blockDim.x] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+  }
+};
+
+// Private ring of a thread: STAGES slots of N row slices (8 elements each) in shared memory.  Slots are interleaved by 16-byte chunk, so
+// that a warp's accesses are contiguous.
+template <typename T, int N>
+struct RowRing {
+  static constexpr int STAGES = sizeof(T) == 2 && N == 2 ? 4 : 3;
+  static constexpr int CHUNKS = RowCols<T>::CHUNKS;
+  static size_t bytes(int threads) { return size_t(threads) * STAGES * N * CHUNKS * 16; }
+  uint4* base;
+  __device__ __forceinline__ uint4* slot(int stage, int n, int chunk) const {
+    return base + ((stage * N + n) * CHUNKS + chunk) * blockDim.x + threadIdx.x;
+  }
+  __device__ __forceinline__ void fetch(int stage, int n, const T* row, int cols) const {
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i)
+      if (RowCols<T>::at(i) < cols)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(slot(stage, n, i))), "l"(row + RowCols<T>::at(i)) : "memory");
+  }
+  __device__ __forceinline__ Raw8<T> get(int stage, int n, int cols) const {
+    Raw8<T> r;
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) r.u[i] = RowCols<T>::at(i) < cols ? *slot(stage, n, i) : make_uint4(0, 0, 0, 0);
+    return r;
+  }
+  // one group per row, empty ones included: the row fetched STAGES - 1 groups ago has arrived
+  static __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+  static __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory"); }
+};
+
+// Block-wide sums of two values per row, one barrier per row: `turn` alternates between two sets of warp sums.
+__device__ __forceinline__ void row_sum2(float2 (*warp_sums)[32], int turn, float& a, float& b) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (nw == 1) return;
+  if (lane == 0) warp_sums[turn][warp] = make_float2(a, b);
+  __syncthreads();
+  const float2 w = lane < nw ? warp_sums[turn][lane] : make_float2(0.f, 0.f);
+  a = warp_sum(w.x);
+  b = warp_sum(w.y);
+}
+
 template <typename T, int MODE>
 __global__ void __launch_bounds__(1024)
 norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ weight,
                 const float* __restrict__ rstd_in, const float* __restrict__ mean_in, T* __restrict__ dx,
                 float* __restrict__ part_w, float* __restrict__ part_b, int rows, int cols) {
-  constexpr bool PREFETCH = sizeof(T) == 2;  // (an fp32 row has twice the bytes in flight, and no registers left for another)
-  const int c0 = threadIdx.x * 8;
-  const bool mine = c0 < cols;
+  using Ring = RowRing<T, 2>;
+  extern __shared__ uint4 norm_ring[];
+  __shared__ float2 warp_sums[2][32];
+  const Ring ring{norm_ring};
   float dw_acc[8], db_acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) { dw_acc[j] = 0.f; db_acc[j] = 0.f; }
-  Raw8<T> wr, xr, dr;
-  if (mine && weight) wr = load_raw(weight + c0);
-  auto fetch = [&](int row, Raw8<T>& xo, Raw8<T>& dd) {
-    if (mine) {
-      dd = load_raw(dy + size_t(row) * cols + c0);
-      xo = load_raw(x + size_t(row) * cols + c0);
+  auto fetch = [&](int stage, int row) {
+    if (row < rows) {
+      ring.fetch(stage, 0, dy + size_t(row) * cols, cols);
+      ring.fetch(stage, 1, x + size_t(row) * cols, cols);
     }
+    Ring::commit();
   };
+#pragma unroll
+  for (int i = 0; i < Ring::STAGES - 1; ++i) fetch(i, blockIdx.x + i * gridDim.x);
+  Raw8<T> wr;
+  if (weight) wr = RowCols<T>::load(weight, cols);
   const float inv_n = 1.f / float(cols);
   int row = blockIdx.x;
-  if (row < rows) fetch(row, xr, dr);
-  while (row < rows) {
+  float rstd = 0.f, mean = 0.f;
+  if (row < rows) {
+    rstd = rstd_in[row];
+    if (MODE == 1) mean = mean_in[row];
+  }
+  for (int it = 0; row < rows; ++it) {
     const int next = row + gridDim.x;
-    const float rstd = rstd_in[row], mean = MODE == 1 ? mean_in[row] : 0.f;
-    Raw8<T> xn, dn;
-    if (PREFETCH && next < rows) fetch(next, xn, dn);
+    fetch((it + Ring::STAGES - 1) % Ring::STAGES, row + (Ring::STAGES - 1) * gridDim.x);
+    float rstd_next = 0.f, mean_next = 0.f;
+    if (next < rows) {
+      rstd_next = rstd_in[next];
+      if (MODE == 1) mean_next = mean_in[next];
+    }
+    Ring::wait();
     float s1 = 0.f, s2 = 0.f;  // sum(g), sum(g * xhat)
-    if (mine) {
+    const Raw8<T> dr = ring.get(it % Ring::STAGES, 0, cols), xr = ring.get(it % Ring::STAGES, 1, cols);
+    {
       float d[8], xv[8], w[8];
       unpack(dr, d);
       unpack(xr, xv);
@@ -217,10 +297,10 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
         s2 += g * xh;
       }
     }
-    block_sum2(s1, s2);
+    row_sum2(warp_sums, it & 1, s1, s2);
     const float c1 = MODE == 1 ? s1 * inv_n : 0.f;
     const float c2 = s2 * inv_n;
-    if (mine) {
+    {
       float d[8], xv[8], w[8], o[8];
       unpack(dr, d);
       unpack(xr, xv);
@@ -231,19 +311,69 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
         const float g = weight ? d[j] * w[j] : d[j];
         o[j] = (g - c1 - xh * c2) * rstd;
       }
-      Vec8<T>::store(dx + size_t(row) * cols + c0, o);
-    }
-    if (PREFETCH) {
-      xr = xn;
-      dr = dn;
-    } else if (next < rows) {
-      fetch(next, xr, dr);
+      RowCols<T>::store(dx + size_t(row) * cols, cols, o);
     }
     row = next;
+    rstd = rstd_next;
+    mean = mean_next;
   }
-  if (mine) {
-    if (part_w) Vec8<float>::store(part_w + size_t(blockIdx.x) * cols + c0, dw_acc);
-    if (MODE == 1 && part_b) Vec8<float>::store(part_b + size_t(blockIdx.x) * cols + c0, db_acc);
+  if (part_w) RowCols<T>::store(part_w + size_t(blockIdx.x) * cols, cols, dw_acc);
+  if (MODE == 1 && part_b) RowCols<T>::store(part_b + size_t(blockIdx.x) * cols, cols, db_acc);
+}
+
+// Forward without a residual: rows stream through the same rings; weight and bias stay in registers.  A CTA per row left
+// the weights to be loaded behind the sums, and narrow rows with idle threads.  LayerNorm 8192 x 4096 bf16 41.8 -> 35.0 us, 1999 x 5120
+// fp32 23.1 -> 17.7 us; RMSNorm 1999 x 5120 bf16 13.9 -> 10.8 us, 8192 x 256 9.8 -> 4.3, 8192 x 4096 31.9 and 31.8 (a copy: 22.8).
+// bf16: CTAs for 2048 threads per SM (against 1024: RMSNorm 1999 x 5120 13.2 -> 10.8, 8192 x 8192 59 -> 55 us); fp32: 1024 (2048: RMSNorm
+// 8192 x 4096 46 -> 49, 8192 x 8192 81 -> 95 us).
+template <typename T, int MODE>
+__global__ void __launch_bounds__(1024, sizeof(T) == 2 && MODE == 0 ? 2 : 1)
+norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, const T* __restrict__ bias, T* __restrict__ out,
+                     float* __restrict__ rstd_out, float* __restrict__ mean_out, int rows, int cols, float eps) {
+  using Ring = RowRing<T, 1>;
+  extern __shared__ uint4 norm_ring[];
+  __shared__ float2 warp_sums[2][32];
+  const Ring ring{norm_ring};
+  auto fetch = [&](int stage, int row) {
+    if (row < rows) ring.fetch(stage, 0, x + size_t(row) * cols, cols);
+    Ring::commit();
+  };
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < Ring::STAGES - 1; ++i) fetch(i, blockIdx.x + i * gridDim.x);
+  Raw8<T> wr, br;
+  if (weight) wr = RowCols<T>::load(weight, cols);
+  if (MODE == 1 && bias) br = RowCols<T>::load(bias, cols);
+  const float inv_n = 1.f / float(cols);
+  for (int it = 0, row = blockIdx.x; row < rows; ++it, row += gridDim.x) {
+    fetch((it + Ring::STAGES - 1) % Ring::STAGES, row + (Ring::STAGES - 1) * gridDim.x);
+    Ring::wait();
+    float v[8], s1 = 0.f, s2 = 0.f;
+    unpack(ring.get(it % Ring::STAGES, 0, cols), v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      s1 += v[j];
+      s2 += v[j] * v[j];
+    }
+    row_sum2(warp_sums, it & 1, s1, s2);
+    const float mean = MODE == 1 ? s1 * inv_n : 0.f;
+    const float var = MODE == 1 ? fmaxf(s2 * inv_n - mean * mean, 0.f) : s2 * inv_n;
+    const float rstd = rsqrtf(var + eps);
+    if (threadIdx.x == 0) {
+      if (rstd_out) rstd_out[row] = rstd;
+      if (mean_out) mean_out[row] = mean;
+    }
+    float w[8], b[8], o[8];
+    if (weight) unpack(wr, w);
+    if (MODE == 1 && bias) unpack(br, b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float y = (v[j] - mean) * rstd;
+      if (weight) y *= w[j];
+      if (MODE == 1 && bias) y += b[j];
+      o[j] = y;
+    }
+    RowCols<T>::store(out + size_t(row) * cols, cols, o);
   }
 }
 
@@ -587,6 +717,27 @@ using namespace tpb;
 
 #define TPB_CHECK_LAUNCH() return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA
 
+// Threads of a CTA whose threads own 8 columns each, and CTAs of them that fill an SM, up to 16.
+static inline int norm_row_threads(int cols) { return (cols / 8 + 31) / 32 * 32; }
+static inline int norm_row_ctas(int rows, int cols, int threads_per_sm) {
+  const int per_sm = threads_per_sm / norm_row_threads(cols);
+  const int ctas = 148 * (per_sm > 16 ? 16 : (per_sm < 1 ? 1 : per_sm));
+  return rows < ctas ? rows : ctas;
+}
+
+// Lets a kernel have a ring of the widest row (1024 threads: 192 KB), once per device.
+template <auto KERNEL>
+static bool norm_ring_allowed() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (!done[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024) != cudaSuccess) return false;
+    done[dev].store(true, std::memory_order_release);
+  }
+  return true;
+}
+
 // dtype: 0 = bf16, 1 = fp32.  mode: 0 = RMSNorm, 1 = LayerNorm.
 extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* weight, const void* bias, void* out,
                             void* sum_out, float* rstd_out, float* mean_out, int rows, int cols, float eps, int mode,
@@ -594,6 +745,22 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   if (!x || !out || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_MAXV) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  // (bf16 RMSNorm of rows that are one vector for each of 256 threads: nothing for a ring to add, 2048 x 2048 5.6 us against 5.9)
+  const bool one_each = dtype == 0 && mode == 0 && cols > NORM_THREADS * 4 && cols <= NORM_THREADS * 8;
+  if (!residual && cols <= NORM_BWD_MAXC && !one_each) {
+    const int threads = norm_row_threads(cols);
+    const dim3 grid(norm_row_ctas(rows, cols, dtype == 0 ? 2048 : 1024));
+#define LAUNCH(T, M)                                                                                                                \
+  do {                                                                                                                              \
+    if (!norm_ring_allowed<norm_fwd_rows_kernel<T, M>>()) return TPB_ERR_CUDA;                                                      \
+    launch_kernel(norm_fwd_rows_kernel<T, M>, grid, dim3(threads), RowRing<T, 1>::bytes(threads), s, (const T*)x, (const T*)weight, \
+                  (const T*)bias, (T*)out, rstd_out, mean_out, rows, cols, eps);                                                    \
+  } while (0)
+    if (dtype == 0) { if (mode) LAUNCH(bf16, 1); else LAUNCH(bf16, 0); }
+    else            { if (mode) LAUNCH(float, 1); else LAUNCH(float, 0); }
+#undef LAUNCH
+    TPB_CHECK_LAUNCH();
+  }
 #define LAUNCH3(T, M, V)                                                                                              \
   launch_kernel(norm_fwd_kernel<T, M, V>, dim3(rows), dim3(NORM_THREADS), 0, s, (const T*)x, (const T*)residual, (const T*)weight, \
                 (const T*)bias, (T*)out, (T*)sum_out, rstd_out, mean_out, cols, eps)
@@ -611,14 +778,9 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   TPB_CHECK_LAUNCH();
 }
 
-// Rows of fp32 partials that tpb_norm_bwd needs (= its CTAs): part_w / part_b hold that many rows of `cols` floats.  As many CTAs
-// as 1024 threads per SM make, up to 16 (narrow rows: more partials would cost more than their CTAs bring).
-static inline int norm_bwd_threads(int cols) { return (cols / 8 + 31) / 32 * 32; }
-extern "C" int tpb_norm_bwd_parts(int rows, int cols) {
-  const int per_sm = 1024 / norm_bwd_threads(cols);
-  const int ctas = 148 * (per_sm > 16 ? 16 : (per_sm < 1 ? 1 : per_sm));
-  return rows < ctas ? rows : ctas;
-}
+// Rows of fp32 partials that tpb_norm_bwd needs (= its CTAs): part_w / part_b hold that many rows of `cols` floats.  (More than 16
+// CTAs of narrow rows per SM: more partials would cost more than their CTAs bring.)
+extern "C" int tpb_norm_bwd_parts(int rows, int cols) { return norm_row_ctas(rows, cols, 1024); }
 
 // dweight / dbias (either may be null, with its partials) are written, not accumulated; grad_dtype: 0 = bf16, 1 = fp32.
 extern "C" int tpb_norm_bwd(const void* dy, const void* x, const void* weight, const float* rstd, const float* mean,
@@ -627,11 +789,16 @@ extern "C" int tpb_norm_bwd(const void* dy, const void* x, const void* weight, c
   if (!dy || !x || !dx || !rstd || rows <= 0 || cols <= 0 || (mode && !mean) || (dweight && !part_w) || (dbias && (!part_b || !mode))) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_BWD_MAXC) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  const int grid = tpb_norm_bwd_parts(rows, cols), threads = norm_bwd_threads(cols);
+  const int grid = norm_row_ctas(rows, cols, 1024), threads = norm_row_threads(cols);
   if (!dweight) part_w = nullptr;
   if (!dbias) part_b = nullptr;
-#define LAUNCH(T, M) \
-  norm_bwd_kernel<T, M><<<grid, threads, 0, s>>>((const T*)dy, (const T*)x, (const T*)weight, rstd, mean, (T*)dx, part_w, part_b, rows, cols)
+#define LAUNCH(T, M)                                                                                                                    \
+  do {                                                                                                                                 \
+    const size_t ring = RowRing<T, 2>::bytes(threads);                                                                                 \
+    if (!norm_ring_allowed<norm_bwd_kernel<T, M>>()) return TPB_ERR_CUDA;                                                                \
+    norm_bwd_kernel<T, M><<<grid, threads, ring, s>>>((const T*)dy, (const T*)x, (const T*)weight, rstd, mean, (T*)dx, part_w, part_b, \
+                                                      rows, cols);                                                                     \
+  } while (0)
   if (dtype == 0) { if (mode) LAUNCH(bf16, 1); else LAUNCH(bf16, 0); }
   else            { if (mode) LAUNCH(float, 1); else LAUNCH(float, 0); }
 #undef LAUNCH

@@ -531,3 +531,25 @@ def test_relative_bias_with_a_bucket_out_of_range(bad, dtype):
     out.backward(hit.to(dtype))
     assert emb.weight.grad.abs().max().item() == 0
     nat.device_state(out.device).check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 264), (149, 4096), (1200, 256), (700, 5120), (600, 8192), (5, 8200)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_norm_forward_in_rings_of_rows(dtype, rows, cols, mode):
+    """Fewer rows than CTAs, rings that go round, one warp and 32 per row, and a row too wide for a ring."""
+    nat = _native()
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, cols, device="cuda") * 2 + 0.1).to(dtype)
+    w = (1 + 0.1 * torch.randn(cols, device="cuda")).to(dtype)
+    bias = torch.randn(cols, device="cuda").to(dtype) if mode else None
+    out, rstd, mean = nat.norm_forward(x, w, bias, 1e-6, mode, want_stats=True)
+    xd = x.double()
+    mu = xd.mean(-1, keepdim=True) if mode else torch.zeros(rows, 1, device="cuda", dtype=torch.double)
+    r = ((xd - mu).square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    want = (xd - mu) * r * w.double() + (bias.double() if mode else 0)
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18  # rounding of the result / of fp32 sums over up to 8200 terms
+    assert bool(((out.double() - want).abs() <= rel * (want.abs() + 1)).all())
+    assert bool(((rstd.double() - r[:, 0]).abs() <= 2.0 ** -18 * r[:, 0]).all())
+    if mode:
+        assert bool(((mean.double() - mu[:, 0]).abs() <= 2.0 ** -20).all())
