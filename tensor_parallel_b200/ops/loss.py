@@ -18,6 +18,7 @@ from tensor_parallel_b200.ops import native
 from tensor_parallel_b200.ops.native import LIB, c_float, c_int, c_ll, c_void_p, check
 
 LIB.tpb_ce_stats.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_ll, c_int, c_int, c_void_p]
+LIB.tpb_ce_loss.argtypes = [c_void_p] * 6 + [c_int, c_int, c_int, c_void_p]
 LIB.tpb_ce_grad.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_ll, c_int, c_int, c_void_p, c_void_p]
 
 
@@ -34,14 +35,14 @@ class _VocabParallelCE(torch.autograd.Function):
         check(LIB.tpb_ce_stats(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), rows, cols, logits.stride(0), vocab_start,
                                ignore_index, native._stream()), "tpb_ce_stats")
         native.count_launches()
-        everyone = gather_stats(stats) if gather_stats is not None else stats[None]  # [world, rows, 4]
-        gmax = everyone[..., 0].max(dim=0).values
-        sumexp = (everyone[..., 1] * torch.exp(everyone[..., 0] - gmax)).sum(dim=0)
-        lse = gmax + torch.log(sumexp)
-        target = everyone[..., 2].sum(dim=0)
-        valid = labels != ignore_index
-        n_valid = valid.sum().clamp(min=1)
-        loss = ((lse - target) * valid).sum() / n_valid
+        everyone = gather_stats(stats).float().contiguous() if gather_stats is not None else stats  # [world, rows, 4]
+        lse = torch.empty(rows, dtype=torch.float32, device=x2d.device)
+        partials = torch.empty(LIB.tpb_ce_loss_parts(rows), 2, dtype=torch.float32, device=x2d.device)
+        loss = torch.empty((), dtype=torch.float32, device=x2d.device)
+        n_valid = torch.empty(1, dtype=torch.float32, device=x2d.device)
+        check(LIB.tpb_ce_loss(everyone.data_ptr(), labels.data_ptr(), lse.data_ptr(), partials.data_ptr(), loss.data_ptr(), n_valid.data_ptr(),
+                              everyone.numel() // (4 * rows), rows, ignore_index, native._stream()), "tpb_ce_loss")
+        native.count_launches(2)
         ctx.save_for_backward(x2d, weight, labels, logits, lse, n_valid)
         ctx.meta = (vocab_start, reduce_hidden_grad, ignore_index, hidden.shape)
         return loss
@@ -55,7 +56,7 @@ class _VocabParallelCE(torch.autograd.Function):
             # the loss value is replicated on every rank; its cotangent is the sum over all copies (ranks whose
             # output does not seed the backward pass contribute zero)
             grad_loss = reduce_hidden_grad(grad_loss.float().reshape(1))
-        scale = (grad_loss.float() / n_valid).reshape(1).contiguous()
+        scale = grad_loss.float() / n_valid
         check(LIB.tpb_ce_grad(logits.data_ptr(), labels.data_ptr(), lse.data_ptr(), rows, cols, logits.stride(0), vocab_start,
                               ignore_index, scale.data_ptr(), native._stream()), "tpb_ce_grad")
         native.count_launches()

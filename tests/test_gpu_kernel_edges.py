@@ -553,3 +553,36 @@ def test_norm_forward_in_rings_of_rows(dtype, rows, cols, mode):
     assert bool(((rstd.double() - r[:, 0]).abs() <= 2.0 ** -18 * r[:, 0]).all())
     if mode:
         assert bool(((mean.double() - mu[:, 0]).abs() <= 2.0 ** -20).all())
+
+
+@pytest.mark.parametrize("rows", [1, 255, 257, 8192, 70001])
+@pytest.mark.parametrize("world", [1, 3])
+def test_loss_over_the_statistics_of_several_ranks(rows, world):
+    """One thread per row, one partial per 256 rows; ignored rows, a slice without a finite logit, no row that counts."""
+    _native()
+    from tensor_parallel_b200.ops import loss as L
+
+    torch.manual_seed(rows)
+    stats = torch.randn(world, rows, 4, device="cuda") * 4
+    stats[..., 1] = stats[..., 1].abs() + 1
+    labels = torch.randint(0, 100, (rows,), device="cuda")
+    labels[::3] = -100
+    for ignored in (-100, None):
+        if ignored is None:
+            labels[:] = -100
+        lse, loss, count = torch.empty(rows, device="cuda"), torch.empty((), device="cuda"), torch.empty(1, device="cuda")
+        partials = torch.empty(L.LIB.tpb_ce_loss_parts(rows), 2, device="cuda")
+        L.check(L.LIB.tpb_ce_loss(stats.data_ptr(), labels.data_ptr(), lse.data_ptr(), partials.data_ptr(), loss.data_ptr(), count.data_ptr(), world, rows, -100,
+                                  L.native._stream()), "ce_loss")
+        d = stats.double()
+        want = torch.logsumexp(d[..., 0] + d[..., 1].log(), dim=0)
+        assert bool(((lse.double() - want).abs() <= 2.0 ** -20 * (1 + want.abs())).all())
+        valid = labels != -100
+        shares = (want - d[..., 2].sum(0)) * valid
+        assert count.item() == max(int(valid.sum()), 1)
+        # fp32: the shares' own rounding, and a sum of a few hundred terms deep
+        assert abs(loss.item() - shares.sum().item() / count.item()) <= 2.0 ** -16 * (shares.abs().sum().item() / count.item() + 1e-6)
+    stats[0, 0] = torch.tensor([float("-inf"), float("nan"), 0.0, 0.0])
+    L.check(L.LIB.tpb_ce_loss(stats.data_ptr(), labels.data_ptr(), lse.data_ptr(), partials.data_ptr(), loss.data_ptr(), count.data_ptr(), world, rows, -100,
+                              L.native._stream()), "ce_loss")
+    assert math.isnan(lse[0].item()) and math.isnan(loss.item()) and not lse[1:].isnan().any()
