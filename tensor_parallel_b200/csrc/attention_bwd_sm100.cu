@@ -505,6 +505,508 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
+// The same with 128 streamed rows per step, for head_dim 64 and, without a bias, 128.  Score products of N = 64 (the kernel above) read
+// 6 KB of shared memory per 32 clocks of work and leave the tensor core idle between dependent steps; with N = 128 the accumulators and ONE
+// buffer of S and of dP fill the 512 columns at head_dim 128, so the two are handed over separately and the products interleave:
+//
+//   dK / dV:  dV += P^T dO (n) | S^T (n + 1) | dK += dS^T Q (n) | dP^T (n + 1)        elementwise: P (n) | dS (n) | P (n + 1) ...
+//   dQ     :  S (n + 1), once S (n) has been read | dQ += dS K (n) | dP (n + 1)
+//
+// P^T and dS^T overwrite their own scores; every product is issued behind the one that last read its columns.  Sixteen elementwise warps
+// (8: 521 against 516 us below).  Streamed tiles arrive through two rings, three tiles of the operand that is needed last (Q or K, with the
+// bias) and two of the other.  Shared memory at head_dim 128: 64 KB resident + 160 KB streamed + statistics, which leaves no room for a
+// bias.  What bounds it: shared memory, 192 KB read and 64 KB filled per 2048 clocks of dK / dV products, and fill and drain of a CTA.
+// Whole backward, 4 x 2048 tokens, 32 heads of 128: causal 558 -> 516 us, without a mask 900 -> 801; 2 x 700, 32 / 8 heads 87 -> 85;
+// 1 x 65, 16 heads 15.0 -> 15.3 us.  Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.
+constexpr int BWW_WARPS = 16;                            // elementwise warps
+constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
+constexpr int BWW_T = 128;                               // streamed rows per step
+constexpr int BWW_S1 = 3, BWW_S2 = 2;                    // ring depths: Q (dK / dV) or K (dQ); dO or V
+constexpr int BWW_BARS = 1 + 2 * (BWW_S1 + BWW_S2) + 7;
+constexpr uint32_t BWW_BIAS = BWW_T * BW_R * 2;          // bias elements of one step
+constexpr size_t bww_smem(int d, int bias) {
+  return size_t(2 + BWW_S1 + BWW_S2) * (d / 64) * FA_BLOCK_BYTES + (bias == 2 ? BWW_S1 * BWW_BIAS : 0) + 2 * BWW_T * sizeof(float2) + BWW_BARS * 8 + 16;
+}
+
+template <int D, bool DKV, int BIAS>
+__global__ void __launch_bounds__(BWW_THREADS, 1)
+attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_constant__ CUtensorMap tmap_r2,
+                     const __grid_constant__ CUtensorMap tmap_t1, const __grid_constant__ CUtensorMap tmap_t2,
+                     const __grid_constant__ CUtensorMap tmap_b, const BwParams p) {
+  constexpr int DB = D / 64;
+  constexpr uint32_t TILE = DB * FA_BLOCK_BYTES;  // 128 rows
+  constexpr uint32_t TMEM_COLS = 512, S_COL = 0, DP_COL = BWW_T, ACC0_COL = 2 * BWW_T, ACC1_COL = ACC0_COL + D;
+  constexpr bool RES_TMEM = !DKV || D == 64;  // the resident tiles as tensor-memory operands, where 512 columns leave room
+  constexpr uint32_t RES_COL = ACC0_COL + (DKV ? 2 : 1) * D;
+  static_assert(!RES_TMEM || RES_COL + D <= TMEM_COLS, "tensor memory columns");
+  constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BWW_T, false, false);
+  constexpr uint32_t IDESC_ACC = make_idesc_bf16(BW_R, D, false, true);
+
+  extern __shared__ __align__(1024) uint8_t bww_smem[];
+  uint8_t* smem = bww_smem;
+  if (smem_u32(smem) & 1023) {  // (the swizzle patterns need it, and there is no room to round up)
+    if (threadIdx.x == 0) atomicMax(p.status, STATUS_BAD_ARG);
+    return;
+  }
+  uint8_t* r1_s = smem;
+  uint8_t* r2_s = r1_s + TILE;
+  uint8_t* t1_s = r2_s + TILE;            // [BWW_S1]
+  uint8_t* t2_s = t1_s + BWW_S1 * TILE;   // [BWW_S2]
+  uint8_t* bias_s = t2_s + BWW_S2 * TILE;     // [BWW_S1], BIAS == 2 only
+  float* stat_s = reinterpret_cast<float*>(bias_s + (BIAS == 2 ? BWW_S1 * BWW_BIAS : 0));  // dK / dV, [2 steps]: -lse * log2(e) of 128 streamed queries (-inf = no such query), -delta * scale
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + 4 * BWW_T);
+  uint64_t* r_full = bars;
+  uint64_t* t1_full = bars + 1;
+  uint64_t* t1_empty = t1_full + BWW_S1;
+  uint64_t* t2_full = t1_empty + BWW_S1;
+  uint64_t* t2_empty = t2_full + BWW_S2;
+  uint64_t* s_full = t2_empty + BWW_S2;   // S of the step is there
+  uint64_t* s_done = s_full + 1;          // dK / dV: P is there (over S); dQ: S has been read
+  uint64_t* dp_full = s_done + 1;         // dP of the step is there
+  uint64_t* ds_full = dp_full + 1;        // dS is there (over dP)
+  uint64_t* acc_full = ds_full + 1;
+  uint64_t* res_full = acc_full + 1;      // dQ: the resident tiles are in tensor memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + 1);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int b = blockIdx.z;
+  const int shift = p.sk - p.sq;  // query i may see keys j <= i + shift when causal
+  const int group = p.q_heads / p.kv_heads;
+  int r0, head, kvh, step0, per_head, n_steps;
+  if (DKV) {
+    r0 = blockIdx.x * BW_R;
+    kvh = blockIdx.y;
+    head = kvh * group;
+    const int q_steps = (p.sq + BWW_T - 1) / BWW_T;
+    step0 = p.causal ? max(0, r0 - shift) / BWW_T : 0;
+    per_head = max(0, q_steps - step0);
+    n_steps = per_head * group;
+  } else {
+    r0 = (gridDim.x - 1 - blockIdx.x) * BW_R;
+    head = blockIdx.y;
+    kvh = head / group;
+    int kv_end = p.sk;
+    if (p.causal) kv_end = min(p.sk, r0 + BW_R + shift);
+    step0 = 0;
+    per_head = kv_end > 0 ? (kv_end + BWW_T - 1) / BWW_T : 0;
+    n_steps = per_head;
+  }
+
+  if (threadIdx.x == 0) {
+    prefetch_tmap(&tmap_r1);
+    prefetch_tmap(&tmap_r2);
+    prefetch_tmap(&tmap_t1);
+    prefetch_tmap(&tmap_t2);
+    mbar_init(r_full, 1);
+    for (int s = 0; s < BWW_S1; ++s) {
+      mbar_init(&t1_full[s], 1);
+      mbar_init(&t1_empty[s], 1);
+    }
+    for (int s = 0; s < BWW_S2; ++s) {
+      mbar_init(&t2_full[s], DKV ? 2 : 1);  // the TMA bytes, and for dK / dV the step's statistics written by the producer warp
+      mbar_init(&t2_empty[s], 1);
+    }
+    mbar_init(s_full, 1);
+    mbar_init(s_done, BWW_WARPS);  // one arrival per elementwise warp
+    mbar_init(dp_full, 1);
+    mbar_init(ds_full, BWW_WARPS);
+    mbar_init(acc_full, 1);
+    mbar_init(res_full, BWW_WARPS);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  auto give_up = [&]() {
+    atomicMax(p.status, STATUS_TIMEOUT_MBAR);
+    *abort_flag = 1;
+  };
+
+  if (warp == 0) {
+    // ---------------- TMA producer (the whole warp stays together: all lanes write statistics) ----------------
+    auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row, int h) {
+#pragma unroll
+      for (int d = 0; d < DB; ++d) tma_load_4d(dst + d * FA_BLOCK_BYTES, map, bar, d * 64, row, h, b);
+    };
+    if (n_steps > 0) {
+      if (lane == 0) {
+        mbar_expect_tx(r_full, 2 * TILE);
+        load(r1_s, &tmap_r1, r_full, r0, DKV ? kvh : head);
+        load(r2_s, &tmap_r2, r_full, r0, DKV ? kvh : head);
+      }
+      int g = 0, local = 0;  // query head of the group (dK / dV), step within it
+      for (int n = 0; n < n_steps; ++n) {
+        const int s1 = n % BWW_S1, s2 = n % BWW_S2;
+        bool ok = !*abort_flag && mbar_wait(&t1_empty[s1], ((n / BWW_S1) & 1) ^ 1);
+        const int row0 = (step0 + local) * BWW_T;
+        const int t_head = DKV ? head + g : kvh;
+        if (++local == per_head) { local = 0; ++g; }
+        if (ok && lane == 0) {
+          mbar_expect_tx(&t1_full[s1], TILE + (BIAS == 2 ? BWW_BIAS : 0));
+          load(t1_s + s1 * TILE, &tmap_t1, &t1_full[s1], row0, t_head);
+          if (BIAS == 2) {
+            const int bh = p.b_sh ? (DKV ? t_head : head) : 0, bb = p.b_sb ? b : 0;
+            if (DKV) {  // [128 queries][128 keys]
+              tma_load_4d(bias_s + s1 * BWW_BIAS, &tmap_b, &t1_full[s1], r0, row0, bh, bb);
+            } else {  // two swizzled blocks of [128 queries][64 keys]
+              tma_load_4d(bias_s + s1 * BWW_BIAS, &tmap_b, &t1_full[s1], row0, r0, bh, bb);
+              tma_load_4d(bias_s + s1 * BWW_BIAS + FA_BLOCK_BYTES, &tmap_b, &t1_full[s1], row0 + 64, r0, bh, bb);
+            }
+          }
+        }
+        ok = ok && mbar_wait(&t2_empty[s2], ((n / BWW_S2) & 1) ^ 1);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0 && !*abort_flag) give_up();
+          break;
+        }
+        if (lane == 0) {
+          mbar_expect_tx(&t2_full[s2], TILE);
+          load(t2_s + s2 * TILE, &tmap_t2, &t2_full[s2], row0, t_head);
+        }
+        if (DKV) {
+          float2 st[BWW_T / 32];
+#pragma unroll
+          for (int i = 0; i < BWW_T / 32; ++i) {
+            const int qi = row0 + i * 32 + lane;
+            st[i] = make_float2(-INFINITY, 0.f);
+            if (qi < p.sq) {
+              const long long idx = ((long long)b * p.q_heads + t_head) * p.sq + qi;
+              const float l = __ldg(p.lse + idx);
+              if (l != -INFINITY) st[i].x = -l * 1.4426950408889634f;  // (a query without a visible key has P = 0 everywhere)
+              st[i].y = -__ldg(p.delta + idx) * p.scale;
+            }
+          }
+          // the statistics of step n - 2 are read until its dS is there, which the release of its Q tile tells
+          ok = n < 2 || mbar_wait(&t1_empty[(n - 2) % BWW_S1], ((n - 2) / BWW_S1) & 1);
+          if (!__all_sync(0xffffffffu, ok)) {
+            if (lane == 0 && !*abort_flag) give_up();
+            break;
+          }
+#pragma unroll
+          for (int i = 0; i < BWW_T / 32; ++i) {
+            stat_s[s2 * 2 * BWW_T + i * 32 + lane] = st[i].x;
+            stat_s[(s2 * 2 + 1) * BWW_T + i * 32 + lane] = st[i].y;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&t2_full[s2]);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (the warp stays together, one lane issues: see umma_bf16_lead) ----------------
+    if (n_steps > 0) {
+      const uint32_t leader = elect_one();
+      const uint32_t r1_lo = desc_kmajor_lo(smem_u32(r1_s)), r2_lo = desc_kmajor_lo(smem_u32(r2_s));
+      auto scores = [&](int which, uint32_t tile) {  // S = R1 T1^T (0) or dP = R2 T2^T (1)
+        const uint32_t t_lo = desc_kmajor_lo(tile), col = tmem_base + (which ? DP_COL : S_COL);
+#pragma unroll
+        for (int d = 0; d < DB; ++d) {
+#pragma unroll
+          for (int kk = 0; kk < 64 / 16; ++kk) {
+            const uint32_t off = d * (FA_BLOCK_BYTES >> 4) + kk * 2;
+            if (!RES_TMEM) umma_bf16_lead(leader, col, (which ? r2_lo : r1_lo) + off, t_lo + off, IDESC_S, (d | kk) ? 1u : 0u);
+            else umma_bf16_tmem_a_lead(leader, col, tmem_base + RES_COL + which * (D / 2) + (d * 4 + kk) * 8, t_lo + off, IDESC_S, (d | kk) ? 1u : 0u);
+          }
+        }
+        umma_commit_lead(leader, which ? dp_full : s_full);
+      };
+      auto accumulate = [&](uint32_t acc_col, uint32_t a_col, uint32_t tile, bool first) {
+        const uint32_t t_lo = desc_mnmajor_lo(tile, FA_BLOCK_BYTES);
+#pragma unroll
+        for (int kk = 0; kk < BWW_T / 16; ++kk)  // (the bf16 operand of 32 streamed rows lies in the first half of their own columns)
+          umma_bf16_tmem_a_lead(leader, tmem_base + acc_col, tmem_base + a_col + (kk >> 1) * 32 + (kk & 1) * 8, t_lo + kk * (16 * 128 >> 4), IDESC_ACC,
+                                (!first || kk) ? 1u : 0u);
+      };
+      auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+        const bool there = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+        if (!there && leader) give_up();
+        tc_fence_after();
+        return there;
+      };
+      auto t1_at = [&](int n) { return smem_u32(t1_s + (n % BWW_S1) * TILE); };
+      auto t2_at = [&](int n) { return smem_u32(t2_s + (n % BWW_S2) * TILE); };
+      auto t1_there = [&](int n) { return wait_all(&t1_full[n % BWW_S1], (n / BWW_S1) & 1); };
+      auto t2_there = [&](int n) { return wait_all(&t2_full[n % BWW_S2], (n / BWW_S2) & 1); };
+      bool ok = wait_all(RES_TMEM ? res_full : r_full, 0) && t1_there(0);
+      if (ok) scores(0, t1_at(0));
+      ok = ok && t2_there(0);
+      if (ok) scores(1, t2_at(0));
+      for (int n = 0; ok && n < n_steps; ++n) {
+        const bool more = n + 1 < n_steps;
+        ok = wait_all(s_done, n & 1);
+        if (!ok) break;
+        if (DKV) {
+          accumulate(ACC1_COL, S_COL, t2_at(n), n == 0);
+          umma_commit_lead(leader, &t2_empty[n % BWW_S2]);  // (dP^T of this step has read dO before)
+        }
+        if (more) {
+          ok = t1_there(n + 1);
+          if (!ok) break;
+          scores(0, t1_at(n + 1));
+        }
+        ok = wait_all(ds_full, n & 1);
+        if (!ok) break;
+        accumulate(ACC0_COL, DP_COL, t1_at(n), n == 0);
+        umma_commit_lead(leader, &t1_empty[n % BWW_S1]);
+        if (!DKV) umma_commit_lead(leader, &t2_empty[n % BWW_S2]);
+        if (more) {
+          ok = t2_there(n + 1);
+          if (!ok) break;
+          scores(1, t2_at(n + 1));
+        }
+      }
+      umma_commit_lead(leader, acc_full);
+    }
+  } else {
+    // ---------------- elementwise warps: four threads per TMEM lane, 32 of the step's columns each ----------------
+    constexpr int HC = BWW_T / 4, HD = D / 4;
+    const int quarter = warp & 3;  // TMEM lane quarter this warp may access
+    const int part = (warp - 2) >> 2;
+    const int row = quarter * 32 + lane;
+    const int ri = r0 + row;  // key (DKV) or query
+    const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
+    float my_lse2 = -INFINITY, my_del = 0.f;  // negated
+    if (!DKV && ri < p.sq) {
+      const long long idx = ((long long)b * p.q_heads + head) * p.sq + ri;
+      const float l = __ldg(p.lse + idx);
+      if (l != -INFINITY) my_lse2 = -l * 1.4426950408889634f;
+      my_del = -__ldg(p.delta + idx) * p.scale;
+    }
+    bool alive = true;
+    int g = 0, local = 0;  // as in the producer
+    if (RES_TMEM && n_steps > 0) {
+      // resident tiles: swizzled shared memory -> tensor memory, half a row of one tile per thread
+      if (!mbar_wait(r_full, 0)) {
+        give_up();
+        alive = false;
+      }
+      if (part < 2 * DB) {
+      const uint8_t* block = (part / DB ? r2_s : r1_s) + (part % DB) * FA_BLOCK_BYTES;
+      uint32_t w[32];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint4 u = *reinterpret_cast<const uint4*>(block + row * 128 + ((c ^ (row & 7)) << 4));
+        w[4 * c] = u.x; w[4 * c + 1] = u.y; w[4 * c + 2] = u.z; w[4 * c + 3] = u.w;
+      }
+      __syncwarp();
+      tmem_st_x32(t_lane + RES_COL + part * 32, w);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(res_full);
+    }
+    // every lane learns whether all lanes of its warp saw the barrier complete
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+      const bool there = __all_sync(0xffffffffu, !*abort_flag && mbar_wait(bar, parity));
+      if (!there) {
+        if (lane == 0 && !*abort_flag) give_up();
+        alive = false;
+      }
+      return there;
+    };
+
+    for (int n = 0; alive && n < n_steps; ++n) {
+      const float* neg_lse = stat_s + (n % BWW_S2) * 2 * BWW_T + part * HC;
+      const float* neg_delta = neg_lse + BWW_T;
+      if (DKV && !wait_all(&t2_full[n % BWW_S2], (n / BWW_S2) & 1)) break;
+      if (BIAS == 2 && !wait_all(&t1_full[n % BWW_S1], (n / BWW_S1) & 1)) break;
+      if (!wait_all(s_full, n & 1)) break;
+      tc_fence_after();
+      const int col0 = (step0 + local) * BWW_T + part * HC;  // first query (DKV) or key of my columns
+      const int b_head = DKV ? head + g : head;
+      if (++local == per_head) { local = 0; ++g; }
+      // score bias: element (query, key) = (col0 + c, ri) for dK / dV - there the lanes of a warp own consecutive keys - and
+      // (ri, col0 + c) for dQ, where a thread's columns are consecutive keys of one row and are read eight at a time
+      const long long bias_base = BIAS ? (long long)b * p.b_sb + (long long)b_head * p.b_sh + (long long)ri * (DKV ? p.b_sk : p.b_sq) : 0;
+      const long long bias_step = DKV ? p.b_sq : p.b_sk;  // per column
+      const int col_limit = DKV ? p.sq : p.sk, row_limit = DKV ? p.sk : p.sq;
+      // ---- P = exp(S * scale - lse) ----
+      float pr[HC], bv[8];
+      {
+        uint32_t sv[HC];
+        tmem_ld_x32(t_lane + S_COL + part * HC, sv);
+        tmem_ld_wait();
+        if (!DKV) {  // S may be overwritten
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_done);
+        }
+        // columns [lo, hi) are visible pairs; only steps that touch the diagonal or an end have others (decided per warp)
+        int lo = 0, hi = HC;
+        if (DKV) {
+          if (ri >= p.sk) hi = 0;
+          if (p.causal) lo = max(0, ri - shift - col0);  // query >= key - shift
+        } else {
+          hi = min(HC, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
+        }
+        uint32_t visible = 0xffffffffu;
+        if (lo > 0) visible = lo < HC ? visible << lo : 0u;
+        if (hi < HC) visible = hi > 0 ? visible & (0xffffffffu >> (HC - hi)) : 0u;
+        const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);
+#pragma unroll
+        for (int c = 0; c < HC; c += 4) {
+          const float4 l = DKV ? *reinterpret_cast<const float4*>(neg_lse + c) : make_float4(my_lse2, my_lse2, my_lse2, my_lse2);
+          if (BIAS && (c & 7) == 0) {
+            if (BIAS == 1) {
+              load_bias8(p.bias, p.bias_kind, bias_base + (long long)(col0 + c) * bias_step, bias_step, ri < row_limit ? col_limit - col0 - c : 0,
+                         !DKV && p.bias_vec, bv);
+            } else if (DKV) {  // column = query row of the tile, lanes read consecutive keys
+              const uint8_t* tile = bias_s + (n % BWW_S1) * BWW_BIAS + (part * HC + c) * (BW_R * 2) + row * 2;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) bv[i] = __bfloat162float(*reinterpret_cast<const bf16*>(tile + i * (BW_R * 2)));
+            } else {  // eight keys of this thread's query: one swizzled 16-byte chunk
+              const uint8_t* block = bias_s + (n % BWW_S1) * BWW_BIAS + (part >> 1) * FA_BLOCK_BYTES;
+              const uint4 u = *reinterpret_cast<const uint4*>(block + row * 128 + ((((part & 1) * 4 + (c >> 3)) ^ (row & 7)) << 4));
+              const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                bv[2 * i] = __uint_as_float(w4[i] << 16);
+                bv[2 * i + 1] = __uint_as_float(w4[i] & 0xFFFF0000u);
+              }
+            }
+          }
+          float x0, x1, x2, x3;
+          ffma2(x0, x1, __uint_as_float(sv[c]), __uint_as_float(sv[c + 1]), p.scale_log2e, p.scale_log2e, l.x, l.y);
+          ffma2(x2, x3, __uint_as_float(sv[c + 2]), __uint_as_float(sv[c + 3]), p.scale_log2e, p.scale_log2e, l.z, l.w);
+          if (BIAS) {
+            constexpr float LOG2E = 1.4426950408889634f;
+            ffma2(x0, x1, bv[c & 7], bv[(c & 7) + 1], LOG2E, LOG2E, x0, x1);
+            ffma2(x2, x3, bv[(c & 7) + 2], bv[(c & 7) + 3], LOG2E, LOG2E, x2, x3);
+          }
+          pr[c] = ex2_approx(x0);
+          pr[c + 1] = ex2_approx(x1);
+          pr[c + 2] = ex2_approx(x2);
+          pr[c + 3] = ex2_approx(x3);
+        }
+        if (masked) {
+#pragma unroll
+          for (int c = 0; c < HC; ++c)
+            if (!(visible >> c & 1)) pr[c] = 0.f;
+        }
+      }
+      uint32_t packed[HC / 2];
+      if (DKV) {  // bf16 pairs over the first half of this thread's own columns (nobody else reads or writes those)
+#pragma unroll
+        for (int c = 0; c < HC; c += 2) packed[c >> 1] = pack_bf16x2(pr[c], pr[c + 1]);
+        tmem_st_x16(t_lane + S_COL + part * HC, packed);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_done);
+      }
+      // ---- dS = P * (dP - delta) * scale ----
+      if (!wait_all(dp_full, n & 1)) break;
+      tc_fence_after();
+      uint32_t dv[HC];
+      tmem_ld_x32(t_lane + DP_COL + part * HC, dv);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < HC; c += 4) {
+        const float4 d = DKV ? *reinterpret_cast<const float4*>(neg_delta + c) : make_float4(my_del, my_del, my_del, my_del);
+        float g0, g1, g2, g3;
+        ffma2(g0, g1, __uint_as_float(dv[c]), __uint_as_float(dv[c + 1]), p.scale, p.scale, d.x, d.y);
+        ffma2(g2, g3, __uint_as_float(dv[c + 2]), __uint_as_float(dv[c + 3]), p.scale, p.scale, d.z, d.w);
+        ffma2(g0, g1, g0, g1, pr[c], pr[c + 1], 0.f, 0.f);
+        ffma2(g2, g3, g2, g3, pr[c + 2], pr[c + 3], 0.f, 0.f);
+        if (BIAS && !DKV && p.dbias && ri < row_limit) {
+          // d(bias) = P (dP - delta) = dS / scale; pairs that are masked or out of range contribute nothing
+          const float db[4] = {pr[c] != 0.f ? g0 * p.inv_scale : 0.f, pr[c + 1] != 0.f ? g1 * p.inv_scale : 0.f, pr[c + 2] != 0.f ? g2 * p.inv_scale : 0.f,
+                               pr[c + 3] != 0.f ? g3 * p.inv_scale : 0.f};
+          float* dst = p.dbias + bias_base + (long long)(col0 + c) * bias_step;
+          if (p.bias_vec && col0 + c + 4 <= col_limit) {
+            // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (db[i] != 0.f && col0 + c + i < col_limit) atomicAdd(dst + i * bias_step, db[i]);
+          }
+        }
+        packed[c >> 1] = pack_bf16x2(g0, g1);
+        packed[(c >> 1) + 1] = pack_bf16x2(g2, g3);
+      }
+      tmem_st_x16(t_lane + DP_COL + part * HC, packed);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
+    }
+    // ---- epilogue: accumulators -> bf16 rows in global memory ----
+    if (alive && n_steps > 0 && wait_all(acc_full, 0)) tc_fence_after();
+    if (alive) {
+      const int limit = DKV ? p.sk : p.sq;
+      const int o_head = DKV ? kvh : head;
+#pragma unroll
+      for (int a = 0; a < (DKV ? 2 : 1); ++a) {
+        bf16* base = a == 0 ? p.out0 : p.out1;
+        const long long sb = a == 0 ? p.o0_sb : p.o1_sb, ss = a == 0 ? p.o0_ss : p.o1_ss, sh = a == 0 ? p.o0_sh : p.o1_sh;
+        bf16* orow = base + b * sb + (long long)min(ri, limit - 1) * ss + (long long)o_head * sh + part * HD;
+        const bool vec = (reinterpret_cast<uintptr_t>(orow) & 15) == 0;
+        uint32_t o[HD];
+        if (n_steps > 0) {
+          __syncwarp();
+          const uint32_t at = t_lane + (a == 0 ? ACC0_COL : ACC1_COL) + part * HD;
+          if constexpr (HD == 32) tmem_ld_x32(at, o);
+          else tmem_ld_x16(at, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < HD; ++i) o[i] = 0u;
+        }
+        if (ri < limit) {
+          if (vec) {
+#pragma unroll
+            for (int i = 0; i < HD; i += 8) {
+              uint4 v;
+              v.x = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
+              v.y = pack_bf16x2(__uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
+              v.z = pack_bf16x2(__uint_as_float(o[i + 4]), __uint_as_float(o[i + 5]));
+              v.w = pack_bf16x2(__uint_as_float(o[i + 6]), __uint_as_float(o[i + 7]));
+              *reinterpret_cast<uint4*>(orow + i) = v;
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < HD; i += 2)
+              *reinterpret_cast<uint32_t*>(orow + i) = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
+          }
+        }
+      }
+    }
+  }
+
+  // ---------------- teardown ----------------
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+template <int D, bool DKV, int BIAS>
+static int bw_launch_wide(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& tb,
+                          const BwParams& p, dim3 grid, cudaStream_t stream) {
+  constexpr size_t smem = bww_smem(D, BIAS);
+  static_assert(smem <= 227 * 1024, "shared memory of a CTA");
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(attn_bwd_wide_kernel<D, DKV, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+      return TPB_ERR_CUDA;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  attn_bwd_wide_kernel<D, DKV, BIAS><<<grid, BWW_THREADS, smem, stream>>>(r1, r2, t1, t2, tb, p);
+  return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
+}
+
 template <int D, bool DKV, int BIAS>
 static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& tb, const BwParams& p,
                      dim3 grid, cudaStream_t stream) {
@@ -599,25 +1101,29 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   // a dense bf16 bias travels by TMA (strides and base are multiples of 16 bytes); fp32 ones, unaligned rows and masks that
   // broadcast over the queries are loaded element by element
   const int bias_mode = !bias ? 0 : (p.bias_kind == 2 && p.bias_vec && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0 ? 2 : 1);
+  // the wide kernel has room for everything but a bias at head_dim 128
+  const bool wide = head_dim == 64 || bias_mode == 0;
   CUtensorMap b_kv = q64, b_q = q64;
   if (bias_mode == 2) {
-    rc = bw_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_T, BW_R, false);
+    rc = bw_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, wide ? BWW_T : BW_T, BW_R, false);
     if (rc == TPB_OK) rc = bw_bias_tmap(&b_q, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_R, BW_T, true);
     if (rc != TPB_OK) return rc;
   }
-#define BW_DISPATCH(DKV, R1, R2, T1, T2, TB, GRID)                                                                                        \
-  (head_dim == 128 ? (bias_mode == 0   ? bw_launch<128, DKV, 0>(R1, R2, T1, T2, TB, p, GRID, s)                                           \
-                      : bias_mode == 1 ? bw_launch<128, DKV, 1>(R1, R2, T1, T2, TB, p, GRID, s)                                           \
-                                       : bw_launch<128, DKV, 2>(R1, R2, T1, T2, TB, p, GRID, s))                                          \
-                   : (bias_mode == 0   ? bw_launch<64, DKV, 0>(R1, R2, T1, T2, TB, p, GRID, s)                                            \
-                      : bias_mode == 1 ? bw_launch<64, DKV, 1>(R1, R2, T1, T2, TB, p, GRID, s)                                            \
-                                       : bw_launch<64, DKV, 2>(R1, R2, T1, T2, TB, p, GRID, s)))
-  rc = BW_DISPATCH(true, k128, v128, q64, do64, b_kv, grid_kv);
+  auto launch = [&](auto dkv, const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap* t1, const CUtensorMap* t2, const CUtensorMap& tb, dim3 grid) {
+    constexpr bool DKV = decltype(dkv)::value;
+    if (head_dim == 128)
+      return bias_mode == 0   ? bw_launch_wide<128, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s)
+             : bias_mode == 1 ? bw_launch<128, DKV, 1>(r1, r2, t1[0], t2[0], tb, p, grid, s)
+                              : bw_launch<128, DKV, 2>(r1, r2, t1[0], t2[0], tb, p, grid, s);
+    return bias_mode == 0   ? bw_launch_wide<64, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s)
+           : bias_mode == 1 ? bw_launch_wide<64, DKV, 1>(r1, r2, t1[1], t2[1], tb, p, grid, s)
+                            : bw_launch_wide<64, DKV, 2>(r1, r2, t1[1], t2[1], tb, p, grid, s);
+  };
+  const CUtensorMap qs[2] = {q64, q128}, dos[2] = {do64, do128}, ks[2] = {k64, k128}, vs[2] = {v64, v128};  // steps of 64 and of 128 rows
+  rc = launch(std::true_type{}, k128, v128, qs, dos, b_kv, grid_kv);
   if (rc != TPB_OK) return rc;
   p.out0 = static_cast<bf16*>(dq); p.o0_sb = dq_sb; p.o0_ss = dq_ss; p.o0_sh = dq_sh;
   p.out1 = nullptr;
   p.dbias = dbias;
-  dim3 grid_q((sq + BW_R - 1) / BW_R, q_heads, batch);
-  return BW_DISPATCH(false, q128, do128, k64, v64, b_q, grid_q);
-#undef BW_DISPATCH
+  return launch(std::false_type{}, q128, do128, ks, vs, b_q, dim3((sq + BW_R - 1) / BW_R, q_heads, batch));
 }

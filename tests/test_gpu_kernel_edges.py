@@ -586,3 +586,31 @@ def test_loss_over_the_statistics_of_several_ranks(rows, world):
     L.check(L.LIB.tpb_ce_loss(stats.data_ptr(), labels.data_ptr(), lse.data_ptr(), partials.data_ptr(), loss.data_ptr(), count.data_ptr(), world, rows, -100,
                               L.native._stream()), "ce_loss")
     assert math.isnan(lse[0].item()) and math.isnan(loss.item()) and not lse[1:].isnan().any()
+
+
+@pytest.mark.parametrize("b,sq,sk,hq,hkv,causal", [(1, 1, 1, 1, 1, True), (2, 127, 129, 2, 1, False), (1, 128, 128, 4, 2, True), (1, 129, 257, 6, 2, True),
+                                                   (2, 300, 130, 2, 2, True), (1, 1000, 1000, 3, 1, True), (1, 640, 384, 2, 2, False)])
+def test_attention_backward_in_wide_steps(b, sq, sk, hq, hkv, causal):
+    """head_dim 128 without a bias: 128 streamed rows per step, rings of two and three tiles; ragged ends, more rounds than the rings
+    are deep, grouped heads, queries that see no key (sq > sk, causal)."""
+    nat = _native()
+    torch.manual_seed(sq + sk)
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16).requires_grad_() for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
+    g = torch.randn(b, sq, hq, 128, device="cuda", dtype=torch.bfloat16)
+    nat.attention(q, k, v, causal).backward(g)
+    qr, kr, vr = (t.detach().double() for t in (q, k, v))
+    for t in (qr, kr, vr):
+        t.requires_grad_()
+    kh, vh = (t.repeat_interleave(hq // hkv, 2) for t in (kr, vr))
+    scores = torch.einsum("bqhd,bkhd->bhqk", qr, kh) / math.sqrt(128)
+    if causal:
+        hidden = torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(sk - sq + 1)
+        scores = scores.masked_fill(hidden, -1e300)  # (a row without keys becomes uniform, and is removed again)
+        probs = scores.softmax(-1).masked_fill(hidden, 0.0)
+    else:
+        probs = scores.softmax(-1)
+    torch.einsum("bhqk,bkhd->bqhd", probs, vh).backward(g.double())
+    nat.device_state(q.device).check_status()
+    for got, want in ((q.grad, qr.grad), (k.grad, kr.grad), (v.grad, vr.grad)):
+        # probabilities, dS and results are rounded to bf16 once each (2^-9 relative, independent errors), the output that delta reads too
+        assert (got.double() - want).norm() <= 2.0 ** -7 * want.norm() + 1e-6
