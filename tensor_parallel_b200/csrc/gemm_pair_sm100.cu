@@ -9,6 +9,8 @@
 // of 256 x 256 needs 32 KB per CTA for the same 512 clocks (64 bytes per clock).  Measured against the single-CTA kernel, same
 // results to the bit: 8192 x 32000 x 4096 and its two gradients 1649 -> 1368 us each (1.57 PFLOP/s; cuBLAS in a short run 1.69, in seconds-long loops 1.41),
 // the projections of a 7B layer at 4000 tokens 297 -> 265 us on average, the 4096 x 4096 ones at 8192 tokens 213 -> 177 us.
+// In seconds-long loops the card is at its power limit and every access costs time: results leave in whole 32-byte sectors (8192 x
+// 11008 x 4096 601 -> 571 us, its weight gradient 617 -> 600; 8192 x 4096 x 4096 222 -> 214; 8192 x 2048 x 2048 66 -> 62 us).
 //
 // One CTA (192 threads), persistent over the pair's tiles:
 //   warp 0    : TMA producer of this CTA's operand rows; completion is counted on the LEADER's barrier (no multicast)
@@ -261,6 +263,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const int out_cols = p.act == 5 ? 16 : 32;  // output columns of one 32-column chunk of the product
     const bool vec = (p.ld_out & 7) == 0 && !(reinterpret_cast<uintptr_t>(p.out) & 15) && !(reinterpret_cast<uintptr_t>(p.bias) & 15) &&
                      !(reinterpret_cast<uintptr_t>(p.residual) & 15);
+    const bool sectors = vec && (p.ld_out & 15) == 0 && !(reinterpret_cast<uintptr_t>(p.out) & 31);
     uint32_t local = 0;
     for (int t = pair; t < tiles; t += pairs, ++local) {
       int mt, nt;
@@ -331,12 +334,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           }
           if (TPB_IN_BOUNDS(base + out_cols <= p.out_elems, p.status)) {
-            uint4* op = reinterpret_cast<uint4*>(p.out + base);
+            uint32_t w[16];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if (q * 8 < out_cols)
-                op[q] = make_uint4(pack_bf16x2(v[8 * q], v[8 * q + 1]), pack_bf16x2(v[8 * q + 2], v[8 * q + 3]),
-                                   pack_bf16x2(v[8 * q + 4], v[8 * q + 5]), pack_bf16x2(v[8 * q + 6], v[8 * q + 7]));
+            for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+            if (sectors) {
+              st_global_v8(p.out + base, w);
+              if (out_cols == 32) st_global_v8(p.out + base + 16, w + 8);
+            } else {
+              uint4* op = reinterpret_cast<uint4*>(p.out + base);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                if (q * 8 < out_cols) op[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+              }
             }
           }
         } else if (p.act == 5) {  // (the feature count is a multiple of 32: only the vector path's alignment can be missing)

@@ -420,6 +420,14 @@ __device__ __forceinline__ uint4 ld_after_wait_v4(const void* p) {
   return v;
 }
 
+// One whole 32-byte sector (32-byte aligned).  Where every lane writes a row of its own, 16-byte stores reach L2 as halves of sectors, an
+// access each.
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float(static_cast<uint32_t>(b) << 16); }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
