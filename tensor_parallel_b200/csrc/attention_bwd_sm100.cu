@@ -951,6 +951,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         const long long sb = a == 0 ? p.o0_sb : p.o1_sb, ss = a == 0 ? p.o0_ss : p.o1_ss, sh = a == 0 ? p.o0_sh : p.o1_sh;
         bf16* orow = base + b * sb + (long long)min(ri, limit - 1) * ss + (long long)o_head * sh + part * HD;
         const bool vec = (reinterpret_cast<uintptr_t>(orow) & 15) == 0;
+        const bool sectors = (reinterpret_cast<uintptr_t>(orow) & 31) == 0;
         uint32_t o[HD];
         if (n_steps > 0) {
           __syncwarp();
@@ -963,7 +964,13 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
           for (int i = 0; i < HD; ++i) o[i] = 0u;
         }
         if (ri < limit) {
-          if (vec) {
+          if (sectors) {
+            uint32_t w[HD / 2];
+#pragma unroll
+            for (int i = 0; i < HD / 2; ++i) w[i] = pack_bf16x2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
+#pragma unroll
+            for (int i = 0; i < HD / 2; i += 8) st_global_v8(orow + 2 * i, w + i);
+          } else if (vec) {
 #pragma unroll
             for (int i = 0; i < HD; i += 8) {
               uint4 v;

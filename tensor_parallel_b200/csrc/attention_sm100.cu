@@ -694,6 +694,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       bf16* orow = p.out + b * p.o_sb + (long long)min(qi, p.sq - 1) * p.o_ss + (long long)h * p.o_sh;
       const bool vec = (reinterpret_cast<uintptr_t>(orow) & 15) == 0;
+      const bool sectors = (reinterpret_cast<uintptr_t>(orow) & 31) == 0;
 #pragma unroll
       for (int c = 0; c < D; c += 32) {
         uint32_t o[32];
@@ -705,7 +706,13 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
           for (int i = 0; i < 32; ++i) o[i] = 0u;
         }
         if (qi < p.sq) {
-          if (vec) {
+          if (sectors) {
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+            st_global_v8(orow + c, w);
+            st_global_v8(orow + c + 16, w + 8);
+          } else if (vec) {
 #pragma unroll
             for (int i = 0; i < 32; i += 8) {
               uint4 v;
