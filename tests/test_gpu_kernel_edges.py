@@ -614,3 +614,30 @@ def test_attention_backward_in_wide_steps(b, sq, sk, hq, hkv, causal):
     for got, want in ((q.grad, qr.grad), (k.grad, kr.grad), (v.grad, vr.grad)):
         # probabilities, dS and results are rounded to bf16 once each (2^-9 relative, independent errors), the output that delta reads too
         assert (got.double() - want).norm() <= 2.0 ** -7 * want.norm() + 1e-6
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (10, 2, 64), (16, 1, 64), (34, 2, 128), (12, 3, 128)])
+@pytest.mark.parametrize("ctx", [0, 15, 16, 129, 700])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_decode_attention_of_grouped_heads(hq, hkv, d, ctx, splits):
+    """Four and more query heads per KV head: groups that leave rows of the MMA empty, fill them, need a second group; no cached key, a
+    tile of 16 keys less one, a whole one, rings that go round, splits without a key, rows of non-zero data behind the cache's end."""
+    nat = _native()
+    torch.manual_seed(hq + ctx)
+    b, smax = 3, 720
+    kc, vc = (torch.randn(b, hkv, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    vc[:, :, ctx + 1:] = float("inf")  # (what lies behind the newest key is never used)
+    qkv = torch.randn(b, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+    at = torch.tensor([ctx], device="cuda", dtype=torch.int32)
+    out = nat.attn_decode_fused(q, k, v, kc, vc, at, d, 10000.0, splits=splits)
+    rot = lambda x, heads: OF.apply_rope_ref(x.reshape(b, 1, heads, d).float(), at.long().view(1, 1).expand(b, 1), 10000.0)[:, 0]
+    assert torch.equal(vc[:, :, ctx], v.reshape(b, hkv, d))
+    assert bool(((kc[:, :, ctx].double() - rot(k, hkv).double()).abs() <= 2.0 ** -7 * rot(k, hkv).abs() + 1e-3).all())
+    qr = rot(q, hq).to(torch.bfloat16).double()
+    kd, vd = (t[:, :, : ctx + 1].double().repeat_interleave(hq // hkv, 1) for t in (kc, vc))
+    probs = (torch.einsum("bhd,bhnd->bhn", qr, kd) / math.sqrt(d)).softmax(-1)
+    want = torch.einsum("bhn,bhnd->bhd", probs, vd)
+    # the result's rounding, and that of the rotated query (half a unit of 2^-8, either way) in a handful of its elements
+    err = (out.view(b, hq, d).double() - want).abs()
+    assert bool((err <= 2.0 ** -7 * want.abs() + 2.0 ** -7 * want.abs().amax(-1, keepdim=True) + 1e-4).all()), err.max()
