@@ -745,9 +745,12 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   if (!x || !out || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_MAXV) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  // (bf16 RMSNorm of rows that are one vector for each of 256 threads: nothing for a ring to add, 2048 x 2048 5.6 us against 5.9)
-  const bool one_each = dtype == 0 && mode == 0 && cols > NORM_THREADS * 4 && cols <= NORM_THREADS * 8;
-  if (!residual && cols <= NORM_BWD_MAXC && !one_each) {
+  // A CTA per row is as good, and better with many rows, where RMSNorm rows fill its 256 threads: 2048 x 2048 bf16 5.6 us (ring 5.9), 32768 x
+  // 4096 bf16 107 (117), fp32 169 (192), 16384 x 2048 fp32 45 (48); with fewer rows 2048 x 2048 fp32 8.4 (6.6), 20 x 4096 2.8 (2.5); rows
+  // that leave threads idle: 1999 x 5120 bf16 13.9 (10.8).
+  const bool filled = (cols > NORM_THREADS * 6 && cols <= NORM_THREADS * 8) || (cols > NORM_THREADS * 12 && cols <= NORM_THREADS * 16);
+  const bool one_cta = mode == 0 && filled && rows >= (dtype == 0 ? 2048 : 8192);
+  if (!residual && cols <= NORM_BWD_MAXC && !one_cta) {
     const int threads = norm_row_threads(cols);
     const dim3 grid(norm_row_ctas(rows, cols, dtype == 0 ? 2048 : 1024));
 #define LAUNCH(T, M)                                                                                                                \
