@@ -666,7 +666,8 @@ struct GqaShape {
   static constexpr int WARPS = D == 64 ? 8 : 4, THREADS = WARPS * 32, STAGES = 3, KEYS = 16;
   static constexpr int TILE = KEYS * D;                                                  // elements of K or V of one stage
   static constexpr size_t RING = size_t(WARPS) * STAGES * 2 * TILE * sizeof(bf16);      // 96 KB: two CTAs per SM
-  static_assert(RING >= size_t(WARPS) * 16 * D * sizeof(float), "the warps' outputs are merged in the ring");
+  static constexpr int OUT_LD = D + 8;  // fp32 row pitch of the warps' outputs, which are merged in the ring (rows on different banks)
+  static_assert(RING >= size_t(WARPS) * 16 * OUT_LD * sizeof(float), "the warps' outputs fit the ring");
 };
 
 template <int D>
@@ -727,36 +728,55 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
   }
   static_assert(D <= S::THREADS, "one element of v per thread");
   const float v_new = threadIdx.x < D ? bf16_bits_to_float(ld_after_wait_u16(v + b * v_ld + (long long)kvh * D + threadIdx.x)) : 0.f;
-  for (int i = threadIdx.x; i < (heads + 1) * (D / 2); i += S::THREADS) {
-    const int hsel = i / (D / 2), pr = i % (D / 2);
-    const bool is_k = hsel == heads;
-    const bf16* src = is_k ? k + b * k_ld + (long long)kvh * D : q + b * q_ld + (long long)(kvh * g_total + g_offset + hsel) * D;
-    auto put = [&](int e, float x) {
-      if (is_k) knew_s[e] = __bfloat162float(__float2bfloat16(x));
-      else tile_ptr<D>(q_s, hsel, e >> 3)[e & 7] = __float2bfloat16(x);
-    };
-    if (pr < half) {
-      const int ia = interleaved ? 2 * pr : pr;
-      const int ib = interleaved ? 2 * pr + 1 : pr + half;
-      float sn, cs;
-      if (rope_table) {
-        const float2 t = __ldg(rope_table + (long long)pos * half + pr);
-        cs = t.x;
-        sn = t.y;
+  // element pairs (D / 2 per head, the key last), four per thread on their way at once
+  constexpr int PAIRS = 4;
+  for (int i0 = threadIdx.x; i0 < (heads + 1) * (D / 2); i0 += PAIRS * S::THREADS) {
+    float x[PAIRS], y[PAIRS], cs[PAIRS], sn[PAIRS];
+    int ea[PAIRS], eb[PAIRS];
+#pragma unroll
+    for (int u = 0; u < PAIRS; ++u) {
+      const int i = i0 + u * S::THREADS;
+      const int hsel = i / (D / 2), pr = i % (D / 2);
+      if (hsel > heads) break;
+      const bf16* src = hsel == heads ? k + b * k_ld + (long long)kvh * D : q + b * q_ld + (long long)(kvh * g_total + g_offset + hsel) * D;
+      if (pr < half) {
+        ea[u] = interleaved ? 2 * pr : pr;
+        eb[u] = interleaved ? 2 * pr + 1 : pr + half;
+        if (rope_table) {
+          const float2 t = __ldg(rope_table + (long long)pos * half + pr);
+          cs[u] = t.x;
+          sn[u] = t.y;
+        } else {
+          const float inv_freq = exp2f(-log2_theta * (2.f * float(pr) / float(rotary_dim)));
+          sincosf(float(pos) * inv_freq, &sn[u], &cs[u]);
+        }
       } else {
-        const float inv_freq = exp2f(-log2_theta * (2.f * float(pr) / float(rotary_dim)));
-        sincosf(float(pos) * inv_freq, &sn, &cs);
+        ea[u] = rotary_dim + 2 * (pr - half);
+        eb[u] = ea[u] + 1;
       }
-      const float x = bf16_bits_to_float(ld_after_wait_u16(src + ia)), y = bf16_bits_to_float(ld_after_wait_u16(src + ib));
-      put(ia, x * cs - y * sn);
-      put(ib, y * cs + x * sn);
-    } else {
-      const int e = rotary_dim + 2 * (pr - half);
-      put(e, bf16_bits_to_float(ld_after_wait_u16(src + e)));
-      put(e + 1, bf16_bits_to_float(ld_after_wait_u16(src + e + 1)));
+      x[u] = bf16_bits_to_float(ld_after_wait_u16(src + ea[u]));
+      y[u] = bf16_bits_to_float(ld_after_wait_u16(src + eb[u]));
+    }
+#pragma unroll
+    for (int u = 0; u < PAIRS; ++u) {
+      const int hsel = (i0 + u * S::THREADS) / (D / 2);
+      if (hsel > heads) break;
+      float ra = x[u], rb = y[u];
+      if ((i0 + u * S::THREADS) % (D / 2) < half) {
+        ra = x[u] * cs[u] - y[u] * sn[u];
+        rb = y[u] * cs[u] + x[u] * sn[u];
+      }
+      if (hsel == heads) {
+        knew_s[ea[u]] = __bfloat162float(__float2bfloat16(ra));
+        knew_s[eb[u]] = __bfloat162float(__float2bfloat16(rb));
+      } else {
+        tile_ptr<D>(q_s, hsel, ea[u] >> 3)[ea[u] & 7] = __float2bfloat16(ra);
+        tile_ptr<D>(q_s, hsel, eb[u] >> 3)[eb[u] & 7] = __float2bfloat16(rb);
+      }
     }
   }
-  for (int i = heads * D + threadIdx.x; i < 16 * D; i += S::THREADS) tile_ptr<D>(q_s, i / D, (i % D) >> 3)[i & 7] = __float2bfloat16(0.f);
+  for (int i = heads * (D / 8) + threadIdx.x; i < 16 * (D / 8); i += S::THREADS)
+    *reinterpret_cast<uint4*>(tile_ptr<D>(q_s, i / (D / 8), i % (D / 8))) = make_uint4(0, 0, 0, 0);
   if (threadIdx.x < D) vnew_s[threadIdx.x] = v_new;
   __syncthreads();
   if (owns_new && blockIdx.z == 0) {  // persist the new key / value for later steps
@@ -866,29 +886,46 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
   __syncthreads();  // every ring has been read
   float* red_o = reinterpret_cast<float*>(dec_ring);  // [warp][16 heads][D]
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n)
+  for (int hh = 0; hh < 2; ++hh) {
+    if (g + 8 * hh >= heads) continue;
 #pragma unroll
-    for (int hh = 0; hh < 2; ++hh)
-      *reinterpret_cast<float2*>(red_o + (warp * 16 + g + 8 * hh) * D + n * 8 + 2 * t4) = make_float2(o[n][2 * hh], o[n][2 * hh + 1]);
+    for (int n = 0; n < D / 8; ++n)
+      *reinterpret_cast<float2*>(red_o + (warp * 16 + g + 8 * hh) * S::OUT_LD + n * 8 + 2 * t4) = make_float2(o[n][2 * hh], o[n][2 * hh + 1]);
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < heads * D; i += S::THREADS) {
-    const int h = i / D, d = i % D;
+  // four elements per thread: a group of four heads of 128 is one round of the CTA
+  auto store = [&](int qh, int d, float4 x, float ll) {
+    bf16* dst = out + (long long)b * out_ld + (long long)qh * D + d;
+    dst[0] = __float2bfloat16(ll > 0.f ? x.x / ll : 0.f);
+    dst[1] = __float2bfloat16(ll > 0.f ? x.y / ll : 0.f);
+    dst[2] = __float2bfloat16(ll > 0.f ? x.z / ll : 0.f);
+    dst[3] = __float2bfloat16(ll > 0.f ? x.w / ll : 0.f);
+  };
+  auto add = [](float4& acc, const float4& x, float c) {
+    acc.x += x.x * c;
+    acc.y += x.y * c;
+    acc.z += x.z * c;
+    acc.w += x.w * c;
+  };
+  for (int i = threadIdx.x; i < heads * (D / 4); i += S::THREADS) {
+    const int h = i / (D / 4), d = i % (D / 4) * 4;
     float mm = -INFINITY;
 #pragma unroll
     for (int w = 0; w < S::WARPS; ++w) mm = fmaxf(mm, red_m[w][h]);
-    float ll = 0.f, oo = 0.f;
+    float ll = 0.f;
+    float4 oo = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < S::WARPS; ++w) {
       const float c = red_m[w][h] == -INFINITY ? 0.f : exp2f(red_m[w][h] - mm);
       ll += red_l[w][h] * c;
-      oo += red_o[(w * 16 + h) * D + d] * c;
+      add(oo, *reinterpret_cast<const float4*>(red_o + (w * 16 + h) * S::OUT_LD + d), c);
     }
     const int qh = kvh * g_total + g_offset + h;
     const long long row = (long long)b * q_heads + qh;
     if (splits == 1) {
-      out[(long long)b * out_ld + (long long)qh * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
+      store(qh, d, oo, ll);
     } else {
-      part_o[(row * splits + split) * D + d] = oo;
+      *reinterpret_cast<float4*>(part_o + (row * splits + split) * D + d) = oo;
       if (d == 0) { part_ml[(row * splits + split) * 2] = mm; part_ml[(row * splits + split) * 2 + 1] = ll; }
     }
   }
@@ -905,37 +942,38 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  for (int i = threadIdx.x; i < heads * D; i += S::THREADS) {
-    const int g = i / D, d = i % D;
-    const long long row = (long long)b * q_heads + kvh * g_total + g_offset + g;
-    // all loads of a batch of 8 splits are issued before the first one is used (each dependent load would cost a
-    // full memory round trip); batches are folded with the running (max, sum, output) like one more online-softmax step
-    float mm = -INFINITY, ll = 0.f, oo = 0.f;
+  for (int i = threadIdx.x; i < heads * (D / 4); i += S::THREADS) {
+    const int h = i / (D / 4), d = i % (D / 4) * 4;
+    const int qh = kvh * g_total + g_offset + h;
+    const long long row = (long long)b * q_heads + qh;
+    // (all loads of a batch of eight splits before the first use, as in attn_decode_fused_kernel)
+    float mm = -INFINITY, ll = 0.f;
+    float4 oo = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s0 = 0; s0 < splits; s0 += 8) {
-      float ms[8], ls[8], os[8];
+      float2 ml[8];
+      float4 os[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const bool live = s0 + q < splits;
-        const long long pr = row * splits + s0 + q;
-        ms[q] = live ? __ldcg(part_ml + pr * 2) : -INFINITY;
-        ls[q] = live ? __ldcg(part_ml + pr * 2 + 1) : 0.f;
-        os[q] = live ? __ldcg(part_o + pr * D + d) : 0.f;
+      for (int q8 = 0; q8 < 8; ++q8) {
+        const bool live = s0 + q8 < splits;
+        const long long pr = row * splits + s0 + q8;
+        ml[q8] = live ? make_float2(__ldcg(part_ml + pr * 2), __ldcg(part_ml + pr * 2 + 1)) : make_float2(-INFINITY, 0.f);
+        os[q8] = live ? __ldcg(reinterpret_cast<const float4*>(part_o + pr * D + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       float m_new = mm;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) m_new = fmaxf(m_new, ms[q]);
+      for (int q8 = 0; q8 < 8; ++q8) m_new = fmaxf(m_new, ml[q8].x);
       const float c_old = mm == -INFINITY ? 0.f : exp2f(mm - m_new);
       ll *= c_old;
-      oo *= c_old;
+      oo = make_float4(oo.x * c_old, oo.y * c_old, oo.z * c_old, oo.w * c_old);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float c = ms[q] == -INFINITY ? 0.f : exp2f(ms[q] - m_new);
-        ll += ls[q] * c;
-        oo += os[q] * c;
+      for (int q8 = 0; q8 < 8; ++q8) {
+        const float c = ml[q8].x == -INFINITY ? 0.f : exp2f(ml[q8].x - m_new);
+        ll += ml[q8].y * c;
+        add(oo, os[q8], c);
       }
       mm = m_new;
     }
-    out[(long long)b * out_ld + (long long)(kvh * g_total + g_offset + g) * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
+    store(qh, d, oo, ll);
   }
 }
 
@@ -1313,10 +1351,10 @@ extern "C" int tpb_attn_decode_fused(const void* q, const void* k, const void* v
   const float l2t = log2f(theta);
   int done = 0, launches = 0;
   // four heads and more fill a quarter and more of the rows of an MMA; below that the rows that would be empty cost more than they bring
-  const bool tensor = g_total >= 4;
+  const bool tensor = g_total >= 4 && !(reinterpret_cast<uintptr_t>(part_o) & 15);
   while (done < g_total) {
     const int left = g_total - done;
-    const int gnow = tensor ? 16 : (left >= 2 ? 2 : 1);
+    const int gnow = tensor ? 16 : (left >= 2 ? 2 : 1);  // (larger groups come here only with partials off a 16-byte boundary)
     // groups share one launch (grid z) when the caller's counter array has a counter for each of them
     int reps = tensor ? (left + 15) / 16 : left / gnow;
     if (splits > 1 && (long long)batch * kv_heads * reps > counter_elems) reps = 1;

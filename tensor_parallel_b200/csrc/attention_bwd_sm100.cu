@@ -516,8 +516,8 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 // (8: 521 against 516 us below).  Streamed tiles arrive through two rings, three tiles of the operand that is needed last (Q or K, with the
 // bias) and two of the other.  Shared memory at head_dim 128: 64 KB resident + 160 KB streamed + statistics, which leaves no room for a
 // bias.  What bounds it: shared memory, 192 KB read and 64 KB filled per 2048 clocks of dK / dV products, and fill and drain of a CTA.
-// Whole backward, 4 x 2048 tokens, 32 heads of 128: causal 558 -> 516 us, without a mask 900 -> 801; 2 x 700, 32 / 8 heads 87 -> 85;
-// 1 x 65, 16 heads 15.0 -> 15.3 us.  Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.
+// Whole backward, 4 x 2048 tokens, 32 heads of 128: causal 558 -> 501 us, without a mask 884 -> 793; 1 x 1000 76 -> 74 us.
+// Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.
 constexpr int BWW_WARPS = 16;                            // elementwise warps
 constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
 constexpr int BWW_T = 128;                               // streamed rows per step
@@ -1118,8 +1118,12 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   }
   auto launch = [&](auto dkv, const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap* t1, const CUtensorMap* t2, const CUtensorMap& tb, dim3 grid) {
     constexpr bool DKV = decltype(dkv)::value;
+    // a streamed sequence that ends in the first half of a step: over a few steps the empty half costs more than wide steps bring (2 x 700,
+    // 32 heads: 82 us in steps of 64, 85 in steps of 128; 1 x 1000: 76 and 74)
+    const int streamed = DKV ? sq : sk, rest = streamed % BWW_T;
+    const bool narrow = streamed < 1024 && rest > 0 && rest <= BW_T;
     if (head_dim == 128)
-      return bias_mode == 0   ? bw_launch_wide<128, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s)
+      return bias_mode == 0   ? (narrow ? bw_launch<128, DKV, 0>(r1, r2, t1[0], t2[0], tb, p, grid, s) : bw_launch_wide<128, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s))
              : bias_mode == 1 ? bw_launch<128, DKV, 1>(r1, r2, t1[0], t2[0], tb, p, grid, s)
                               : bw_launch<128, DKV, 2>(r1, r2, t1[0], t2[0], tb, p, grid, s);
     return bias_mode == 0   ? bw_launch_wide<64, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s)
