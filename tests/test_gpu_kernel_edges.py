@@ -620,8 +620,8 @@ def test_attention_backward_in_wide_steps(b, sq, sk, hq, hkv, causal):
 @pytest.mark.parametrize("ctx", [0, 15, 16, 129, 700])
 @pytest.mark.parametrize("splits", [1, 3])
 def test_decode_attention_of_grouped_heads(hq, hkv, d, ctx, splits):
-    """Four and more query heads per KV head: groups that leave rows of the MMA empty, fill them, need a second group; no cached key, a
-    tile of 16 keys less one, a whole one, rings that go round, splits without a key, rows of non-zero data behind the cache's end."""
+    """Four and more query heads per KV head: one whole group, several, a remainder in groups of its own; no cached key, a few, rings that
+    go round, splits without a key, rows of non-zero data behind the cache's end."""
     nat = _native()
     torch.manual_seed(hq + ctx)
     b, smax = 3, 720
@@ -640,4 +640,85 @@ def test_decode_attention_of_grouped_heads(hq, hkv, d, ctx, splits):
     want = torch.einsum("bhn,bhnd->bhd", probs, vd)
     # the result's rounding, and that of the rotated query (half a unit of 2^-8, either way) in a handful of its elements
     err = (out.view(b, hq, d).double() - want).abs()
+    assert bool((err <= 2.0 ** -7 * want.abs() + 2.0 ** -7 * want.abs().amax(-1, keepdim=True) + 1e-4).all()), err.max()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(2, 2, 128), (8, 1, 64), (16, 1, 64), (8, 2, 128)])
+@pytest.mark.parametrize("splits", [2, 3])
+def test_decode_attention_keeps_its_partial_results_in_32_bits(hq, hkv, d, splits):
+    """Scores, probabilities and sums of a split stay fp32: its maximum, sum and unnormalised output, as they lie in the workspace."""
+    nat = _native()
+    torch.manual_seed(hq + d)
+    b, ctx, smax = 2, 1000, 1024
+    kc, vc = (torch.randn(b, hkv, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    qkv = torch.randn(b, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+    part_o, part_ml = torch.empty(b, hq, splits, d, device="cuda"), torch.empty(b, hq, splits, 2, device="cuda")
+    counters = torch.zeros(b * hq, dtype=torch.int32, device="cuda")
+    nat.attn_decode_fused(q, k, v, kc, vc, torch.tensor([ctx], device="cuda", dtype=torch.int32), 0, 10000.0, splits=splits, workspace=(part_o, part_ml, counters))
+    kd, vd = (t[:, :, : ctx + 1].double().repeat_interleave(hq // hkv, 1) for t in (kc, vc))
+    scores = torch.einsum("bhd,bhnd->bhn", q.reshape(b, hq, d).double(), kd) / math.sqrt(d) * math.log2(math.e)
+    chunk = -(-(ctx + 1) // splits)
+    for i in range(splits):
+        at = slice(i * chunk, (i + 1) * chunk)
+        top = scores[..., at].amax(-1)
+        p = (scores[..., at] - top[..., None]).exp2()
+        assert bool(((part_ml[:, :, i, 0].double() - top).abs() <= 2.0 ** -20 * (1 + top.abs())).all())
+        # A score is a sum of d products in fp32: a few roundings of at most 2^-24 of its magnitude (4 or so), independent from key to key, and
+        # the same again from the maximum, which is common to all keys: below 1e-6 of both results.  Probabilities of 17 bits exceed it.
+        for got, want in ((part_ml[:, :, i, 1], p.sum(-1)), (part_o[:, :, i], torch.einsum("bhn,bhnd->bhd", p, vd[:, :, at]))):
+            assert (got.double() - want).norm() <= 1e-6 * want.norm()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (16, 1, 64), (2, 2, 64)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_decode_attention_of_infinite_values(hq, hkv, d, splits):
+    """An infinite cached value gives an infinite element of the output (its probability is above zero), and no NaN anywhere."""
+    nat = _native()
+    torch.manual_seed(hq + d)
+    b, ctx, smax = 2, 300, 320
+    kc, vc = (torch.randn(b, hkv, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    vc[:, :, 17, 3] = float("inf")
+    vc[:, :, 250, 5] = float("-inf")
+    qkv = torch.randn(b, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+    out = nat.attn_decode_fused(q, k, v, kc, vc, torch.tensor([ctx], device="cuda", dtype=torch.int32), d, 10000.0, splits=splits).view(b, hq, d)
+    want = torch.zeros_like(out, dtype=torch.float32)
+    want[..., 3], want[..., 5] = float("inf"), float("-inf")
+    assert torch.equal(out.float().nan_to_num(nan=7.0, posinf=1e9, neginf=-1e9).abs() >= 1e9, want.abs() > 0)
+    assert bool((out[..., 3] == float("inf")).all() and (out[..., 5] == float("-inf")).all()) and not out.isnan().any()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(2, 2, 128), (2, 1, 64), (4, 1, 128), (8, 1, 64), (6, 2, 128)])
+@pytest.mark.parametrize("rotary_dim", [0, 32, None])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("table", [False, True])
+def test_decode_attention_rotary_forms(hq, hkv, d, rotary_dim, interleaved, table):
+    """Partial rotary spans, an untouched rest, interleaved pairs, none at all; angles computed and looked up."""
+    nat = _native()
+    rotary_dim = d if rotary_dim is None else rotary_dim
+    torch.manual_seed(hq + d + rotary_dim)
+    b, ctx, smax = 2, 150, 160
+    kc, vc = (torch.randn(b, hkv, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    qkv = torch.randn(b, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+    at = torch.tensor([ctx], device="cuda", dtype=torch.int32)
+    angles = nat.rope_table(smax, rotary_dim, 10000.0, torch.device("cuda", 0)) if table and rotary_dim else None
+    outs = []
+    for early in (False, True):
+        k2, v2 = kc.clone(), vc.clone()
+        torch.cuda.synchronize()
+        out = nat.attn_decode_fused(q, k, v, k2, v2, at, rotary_dim, 10000.0, interleaved=interleaved, splits=2, rope_angles=angles, early=early)
+        outs.append((out, k2, v2))
+    assert all(torch.equal(x, y) for x, y in zip(*outs))
+    rot = lambda x, heads: OF.apply_rope_ref(x.reshape(b, 1, heads, d), at.long().view(1, 1).expand(b, 1), 10000.0, rotary_dim, interleaved)[:, 0] if rotary_dim else x.reshape(b, heads, d)
+    assert torch.equal(v2[:, :, ctx], v.reshape(b, hkv, d))
+    # the angle of position 150 has an fp32 error of a few 2^-17, then one bf16 rounding: half a unit, either way
+    assert bool(((k2[:, :, ctx].double() - rot(k, hkv).double()).abs() <= 2.0 ** -7 * rot(k, hkv).double().abs() + 1e-3).all())
+    assert torch.equal(k2[:, :, ctx, rotary_dim:], k.reshape(b, hkv, d)[..., rotary_dim:])
+    qr = rot(q, hq).double()
+    kd, vd = (t[:, :, : ctx + 1].double().repeat_interleave(hq // hkv, 1) for t in (k2, v2))
+    want = torch.einsum("bhn,bhnd->bhd", (torch.einsum("bhd,bhnd->bhn", qr, kd) / math.sqrt(d)).softmax(-1), vd)
+    err = (out.view(b, hq, d).double() - want).abs()
+    # the result's rounding, and that of the rotated query (half a unit of 2^-8, either way) in a handful of its elements
     assert bool((err <= 2.0 ** -7 * want.abs() + 2.0 ** -7 * want.abs().amax(-1, keepdim=True) + 1e-4).all()), err.max()
