@@ -7,9 +7,10 @@
 //   dS = P * (dP - delta) * scale      delta[i] = sum_d out[i, d] * dout[i, d]
 //   dQ = dS K                          dK = dS^T Q
 //
-// Two launches of ONE kernel template, both free of atomics and therefore deterministic (the optional bias gradient is the
-// exception: fp32 atomic adds).  A CTA keeps 128 "resident"
-// rows (the TMEM lanes) and streams the other sequence through in steps of 64 rows (TMEM columns):
+// Two launches, dK / dV and dQ, both free of atomics and therefore deterministic (the optional bias gradient is the exception: fp32
+// atomic adds).  A CTA keeps 128 "resident" rows (the TMEM lanes) and streams the other sequence through.  There are two kernels, each a
+// template of both launches: attn_bwd_tcgen05_kernel streams 64 rows per step (described here), attn_bwd_wide_kernel 128 (described
+// there); step_rows below says which launch takes which.
 //
 //   dK / dV (DKV = true) : resident = 128 keys of one KV head (K and V tiles), streamed = queries (Q and dO, over all
 //                          query heads of the group):  S^T = K Q^T and dP^T = V dO^T land in TMEM with a key per lane,
@@ -74,7 +75,7 @@ struct BwParams {
 // BIAS: the score-bias code exists only in the instantiations that need it.  1: elements are loaded by the threads that use them;
 // 2: a dense bf16 bias whose rows TMA can address travels with the streamed tiles, [64 queries][128 keys] (dK / dV) or
 // [128 queries][64 keys] (dQ) per step, so that no elementwise warp ever waits for a global load (16 x 512 tokens, 32 heads of 64,
-// one bias for all batches: dK / dV 1093 -> 205 us, dQ 316 -> 231 us).
+// one bias for all batches, in steps of 64 rows: dK / dV 1093 -> 205 us, dQ 316 -> 231 us).
 template <int D, bool DKV, int BIAS>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_constant__ CUtensorMap tmap_r2,
@@ -86,8 +87,8 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   constexpr uint32_t TMEM_COLS = 512;
   constexpr uint32_t S_COL0 = 0, DP_COL0 = 2 * BW_T, ACC0_COL = 4 * BW_T, ACC1_COL = 4 * BW_T + D;
   // The resident tiles as tensor-memory A operands where 512 columns leave room for them (all of dQ, dK / dV at head_dim 64): from
-  // shared memory, a score MMA of 128 x 64 x 16 reads 6 KB for 32 clocks of work and is bound by that (dQ of 4 x 2048, 32 heads of
-  // 128, causal: 248 -> 233 us; whole backward of 16 x 512, 32 heads of 64: 291 -> 273 us).
+  // shared memory, a score MMA of 128 x 64 x 16 reads 6 KB for 32 clocks of work and is bound by that (in this kernel, dQ of 4 x 2048, 32
+  // heads of 128, causal: 248 -> 233 us; whole backward of 16 x 512, 32 heads of 64: 291 -> 273 us).
   constexpr bool RES_TMEM = !DKV || D == 64;
   constexpr uint32_t RES_COL0 = ACC0_COL + (DKV ? 2 : 1) * D;  // resident 1, then resident 2: D / 2 columns each (two bf16 per column)
   static_assert(!RES_TMEM || RES_COL0 + D <= TMEM_COLS, "tensor memory columns");
@@ -505,7 +506,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// The same with 128 streamed rows per step, for head_dim 64 and, without a bias, 128.  Score products of N = 64 (the kernel above) read
+// The same with 128 streamed rows per step, for head_dim 64 and, without a bias, 128, where step_rows below says so.  Score products of N = 64 (the kernel above) read
 // 6 KB of shared memory per 32 clocks of work and leave the tensor core idle between dependent steps; with N = 128 the accumulators and ONE
 // buffer of S and of dP fill the 512 columns at head_dim 128, so the two are handed over separately and the products interleave:
 //
@@ -517,7 +518,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 // bias) and two of the other.  Shared memory at head_dim 128: 64 KB resident + 160 KB streamed + statistics, which leaves no room for a
 // bias.  What bounds it: shared memory, 192 KB read and 64 KB filled per 2048 clocks of dK / dV products, and fill and drain of a CTA.
 // Whole backward, 4 x 2048 tokens, 32 heads of 128: causal 558 -> 501 us, without a mask 884 -> 793; 1 x 1000 76 -> 74 us.
-// Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.
+// Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.  Short and ragged sequences: step_rows.
 constexpr int BWW_WARPS = 16;                            // elementwise warps
 constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
 constexpr int BWW_T = 128;                               // streamed rows per step
@@ -1031,6 +1032,27 @@ static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtenso
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
+// Streamed rows per step of a launch, 64 or 128: which kernel it takes.  bias_mode as BIAS above; heads: of the launch's grid (KV heads for
+// dK / dV).  What decides is how many rows of the last step are empty, in every product and elementwise pass, against what a step costs.
+// Times are of whole backwards, both launches in steps of 64 / of 128 rows, in us, causal where no bias is named.
+//   head_dim 128 with a bias: 64, the wide rings leave no room for it.
+//   head_dim 128: 64 for a sequence that ends in the first half of its first, second or third wide step (32 heads: 1 x 33 12.2 / 13.4, 8 x 150
+//   52.7 / 54.8, 2 x 300 32.0 / 33.2); from the fourth on wide steps win all the same (2 x 420 41.9 / 41.2, 4 x 700 133 / 128).
+//   head_dim 64, the same line (32 heads: 4 x 33 12.5 / 14.8, 8 x 150 38.6 / 44.4, 8 x 300 65.4 / 73.3), and with 64 heads x batches and more, where
+//   two CTAs of the 64-row kernel share an SM, up to the fifth (32 heads: 2 x 420 33.9 / 34.8, 16 x 420 191 / 202, 2 x 576 3 % and
+//   1 x 576 -4 %; 4 x 420, 12 heads 33.5 / 30.9).  At six steps either may be 3 % ahead.
+//   head_dim 64, one or two whole steps of very many heads: fill and drain of a CTA count (32 heads: 16 x 100 38.6 / 40.9, 4 x 100 14.2 / 14.2).
+//   head_dim 64 with a bias: 64 only for up to 64 rows (32 heads: 4 x 64 10 %, with a padding mask 7 % longer in wide steps); beyond, the wide
+//   kernel's warps, twice as many per bias element, decide (4 x 300 0.79 of the time, 2 x 900 0.71, with a mask 0.76 and 0.64).
+static int step_rows(int head_dim, int bias_mode, int streamed, int heads, int batch) {
+  const bool half = streamed % BWW_T > 0 && streamed % BWW_T <= BW_T;
+  if (head_dim == 128) return bias_mode || (half && streamed < 3 * BWW_T) ? BW_T : BWW_T;
+  if (bias_mode) return streamed <= BW_T ? BW_T : BWW_T;
+  const long long rows = (long long)heads * batch;
+  if (half) return streamed < 3 * BWW_T || (streamed < 5 * BWW_T && rows >= 64) ? BW_T : BWW_T;
+  return streamed <= 2 * BWW_T && rows >= 256 ? BW_T : BWW_T;
+}
+
 // Tensor map over a bf16 score bias [batch or 1][heads or 1][sq][sk] (keys contiguous); box = [rows queries][keys].
 static int bw_bias_tmap(CUtensorMap* map, const void* bias, int batch, int heads, int sq, int sk, long long sb, long long sh, long long sqs, int rows,
                         int keys, bool swizzled) {
@@ -1049,6 +1071,9 @@ static int bw_bias_tmap(CUtensorMap* map, const void* bias, int batch, int heads
 }  // namespace tpb
 
 using namespace tpb;
+
+// Rows per step (64 or 128) of a launch of tpb_attn_backward_sm100 that streams `streamed` rows; bias: 0 none, 1 element by element, 2 by TMA.
+extern "C" int tpb_attn_backward_step_rows(int head_dim, int bias, int streamed, int heads, int batch) { return step_rows(head_dim, bias, streamed, heads, batch); }
 
 // Same contract as tpb_attn_backward_bias (strides in elements, head_dim contiguous; bias strides of 0 broadcast; dbias is fp32 with
 // the bias' strides, zero-initialised; `delta` is a [batch][q_heads][sq] fp32
@@ -1108,27 +1133,24 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   // a dense bf16 bias travels by TMA (strides and base are multiples of 16 bytes); fp32 ones, unaligned rows and masks that
   // broadcast over the queries are loaded element by element
   const int bias_mode = !bias ? 0 : (p.bias_kind == 2 && p.bias_vec && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0 ? 2 : 1);
-  // the wide kernel has room for everything but a bias at head_dim 128
-  const bool wide = head_dim == 64 || bias_mode == 0;
+  const int kv_rows = step_rows(head_dim, bias_mode, sq, kv_heads, batch), q_rows = step_rows(head_dim, bias_mode, sk, q_heads, batch);
   CUtensorMap b_kv = q64, b_q = q64;
-  if (bias_mode == 2) {
-    rc = bw_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, wide ? BWW_T : BW_T, BW_R, false);
+  if (bias_mode == 2) {  // (a wide dQ step takes two boxes)
+    rc = bw_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, kv_rows, BW_R, false);
     if (rc == TPB_OK) rc = bw_bias_tmap(&b_q, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_R, BW_T, true);
     if (rc != TPB_OK) return rc;
   }
   auto launch = [&](auto dkv, const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap* t1, const CUtensorMap* t2, const CUtensorMap& tb, dim3 grid) {
     constexpr bool DKV = decltype(dkv)::value;
-    // a streamed sequence that ends in the first half of a step: over a few steps the empty half costs more than wide steps bring (2 x 700,
-    // 32 heads: 82 us in steps of 64, 85 in steps of 128; 1 x 1000: 76 and 74)
-    const int streamed = DKV ? sq : sk, rest = streamed % BWW_T;
-    const bool narrow = streamed < 1024 && rest > 0 && rest <= BW_T;
-    if (head_dim == 128)
-      return bias_mode == 0   ? (narrow ? bw_launch<128, DKV, 0>(r1, r2, t1[0], t2[0], tb, p, grid, s) : bw_launch_wide<128, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s))
-             : bias_mode == 1 ? bw_launch<128, DKV, 1>(r1, r2, t1[0], t2[0], tb, p, grid, s)
-                              : bw_launch<128, DKV, 2>(r1, r2, t1[0], t2[0], tb, p, grid, s);
-    return bias_mode == 0   ? bw_launch_wide<64, DKV, 0>(r1, r2, t1[1], t2[1], tb, p, grid, s)
-           : bias_mode == 1 ? bw_launch_wide<64, DKV, 1>(r1, r2, t1[1], t2[1], tb, p, grid, s)
-                            : bw_launch_wide<64, DKV, 2>(r1, r2, t1[1], t2[1], tb, p, grid, s);
+    const bool wide = (DKV ? kv_rows : q_rows) == BWW_T;
+#define BW_ONE(D, BIAS)                                                                  \
+  (wide ? bw_launch_wide<D, DKV, BIAS>(r1, r2, t1[1], t2[1], tb, p, grid, s)             \
+        : bw_launch<D, DKV, BIAS>(r1, r2, t1[0], t2[0], tb, p, grid, s))
+    if (head_dim == 64) return bias_mode == 0 ? BW_ONE(64, 0) : bias_mode == 1 ? BW_ONE(64, 1) : BW_ONE(64, 2);
+    return bias_mode == 0   ? BW_ONE(128, 0)
+           : bias_mode == 1 ? bw_launch<128, DKV, 1>(r1, r2, t1[0], t2[0], tb, p, grid, s)
+                            : bw_launch<128, DKV, 2>(r1, r2, t1[0], t2[0], tb, p, grid, s);
+#undef BW_ONE
   };
   const CUtensorMap qs[2] = {q64, q128}, dos[2] = {do64, do128}, ks[2] = {k64, k128}, vs[2] = {v64, v128};  // steps of 64 and of 128 rows
   rc = launch(std::true_type{}, k128, v128, qs, dos, b_kv, grid_kv);

@@ -591,8 +591,9 @@ def test_loss_over_the_statistics_of_several_ranks(rows, world):
 @pytest.mark.parametrize("b,sq,sk,hq,hkv,causal", [(1, 1, 1, 1, 1, True), (2, 127, 129, 2, 1, False), (1, 128, 128, 4, 2, True), (1, 129, 257, 6, 2, True),
                                                    (2, 300, 130, 2, 2, True), (1, 1000, 1000, 3, 1, True), (1, 640, 384, 2, 2, False)])
 def test_attention_backward_in_wide_steps(b, sq, sk, hq, hkv, causal):
-    """head_dim 128 without a bias: 128 streamed rows per step, rings of two and three tiles; ragged ends, more rounds than the rings
-    are deep, grouped heads, queries that see no key (sq > sk, causal)."""
+    """head_dim 128 without a bias, few steps: the launches that stream at least 65 of the last 128 rows take the kernel of 128 rows per step,
+    those that end in a first half the one of 64; ragged ends, more rounds than the rings are deep, grouped heads, queries that see no key
+    (sq > sk, causal).  (Which launch takes which: test_attention_backward_by_step.)"""
     nat = _native()
     torch.manual_seed(sq + sk)
     q, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16).requires_grad_() for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
@@ -722,3 +723,58 @@ def test_decode_attention_rotary_forms(hq, hkv, d, rotary_dim, interleaved, tabl
     err = (out.view(b, hq, d).double() - want).abs()
     # the result's rounding, and that of the rotated query (half a unit of 2^-8, either way) in a handful of its elements
     assert bool((err <= 2.0 ** -7 * want.abs() + 2.0 ** -7 * want.abs().amax(-1, keepdim=True) + 1e-4).all()), err.max()
+
+
+def _backward_rows(d, bias_mode, streamed, heads, batch):
+    return _native().LIB.tpb_attn_backward_step_rows(d, bias_mode, streamed, heads, batch)
+
+
+# rows per step of the dK / dV launch (which streams the queries) and of the dQ launch (which streams the keys), without a bias
+@pytest.mark.parametrize("d,b,sq,sk,hq,hkv,causal,rows", [
+    # last wide steps of one row and of 64, more steps than either ring is deep; grouped heads; queries without a key (sq > sk), empty dQ steps
+    (128, 1, 1025, 1025, 2, 1, True, (128, 128)), (128, 1, 1088, 1025, 3, 3, False, (128, 128)), (128, 2, 384, 250, 4, 2, True, (128, 128)),
+    (128, 1, 512, 100, 2, 2, True, (128, 128)), (128, 1, 65, 385, 2, 1, True, (128, 128)), (128, 2, 448, 449, 2, 2, True, (128, 128)),
+    (64, 1, 449, 449, 4, 2, True, (128, 128)), (64, 1, 385, 700, 3, 1, False, (128, 128)), (64, 2, 384, 250, 4, 2, True, (128, 128)),
+    (64, 1, 1025, 1088, 2, 2, True, (128, 128)), (64, 2, 100, 128, 2, 1, False, (128, 128)),
+    # steps of 64: one short or whole one, a few that end in a first half, one launch of each kind, many heads.  (Two keys at least: with
+    # one, the gradients of query and key are zero, and what a kernel returns is the rounding of dP - delta, 2^-24 of its d terms, with no
+    # want.grad to hold it against.)
+    (128, 2, 1, 33, 2, 1, True, (64, 64)), (128, 1, 300, 129, 4, 2, True, (64, 64)), (128, 2, 64, 200, 2, 2, False, (64, 128)),
+    (64, 2, 1, 2, 2, 1, True, (64, 64)), (64, 1, 64, 33, 4, 1, True, (64, 64)), (64, 2, 150, 320, 2, 2, True, (64, 64)), (64, 1, 200, 257, 4, 2, False, (128, 64)),
+    (64, 8, 400, 576, 16, 8, True, (64, 64)), (64, 16, 100, 193, 32, 16, True, (64, 64)), (64, 16, 256, 65, 16, 16, True, (64, 64))])
+@pytest.mark.parametrize("bias", ["none", "dense", "rows off 16 bytes", "padding"])
+def test_attention_backward_by_step(d, b, sq, sk, hq, hkv, causal, rows, bias):
+    """Both kernels of the backward against 64 bits, at the edges of their steps and rings, and of the rule that chooses between them."""
+    if bias != "none" and b * hq * sq * sk > 1 << 24:
+        pytest.skip("the rule for many heads concerns calls without a bias")
+    nat = _native()
+    torch.manual_seed(sq + sk + d)
+    assert rows == (_backward_rows(d, 0, sq, hkv, b), _backward_rows(d, 0, sk, hq, b))
+    for mode in (1, 2):
+        assert _backward_rows(d, mode, sq, hkv, b) == (64 if d == 128 or sq <= 64 else 128)
+    q, k, v = (torch.randn(b, s, h, d, device="cuda", dtype=torch.bfloat16).requires_grad_() for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
+    g = torch.randn(b, sq, hq, d, device="cuda", dtype=torch.bfloat16)
+    if bias == "none":
+        leaf = added = None
+    elif bias == "padding":
+        leaf = added = torch.zeros(b, 1, 1, sk, device="cuda", dtype=torch.bfloat16)
+        leaf[0, :, :, sk - sk // 3:] = -math.inf
+    else:  # rows of a multiple of eight keys travel by TMA, others element by element
+        pitch = (sk + 7) // 8 * 8 + (0 if bias == "dense" else 1)
+        leaf = torch.randn(1, hq, sq, pitch, device="cuda", dtype=torch.bfloat16)
+        added = leaf[..., :sk].detach().requires_grad_()
+    nat.attention(q, k, v, causal, added).backward(g)
+    ref = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    kh, vh = (t.repeat_interleave(hq // hkv, 2) for t in ref[1:])
+    scores = torch.einsum("bqhd,bkhd->bhqk", ref[0], kh) / math.sqrt(d)
+    if added is not None:
+        ref.append(added.detach().double().requires_grad_())
+        scores = scores + ref[3]
+    hidden = torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(sk - sq + 1) if causal else torch.zeros(sq, sk, dtype=torch.bool, device="cuda")
+    unseen = hidden | (scores.detach() == -math.inf)
+    probs = scores.masked_fill(unseen, -1e300).softmax(-1).masked_fill(unseen, 0.0)  # (a row without keys becomes uniform, and is removed again)
+    torch.einsum("bhqk,bkhd->bqhd", probs, vh).backward(g.double())
+    nat.device_state(q.device).check_status()
+    for got, want in zip([q, k, v] + ([added] if added is not None and added.requires_grad else []), ref):
+        # probabilities, dS and results are rounded to bf16 once each (2^-9 relative, independent errors), the output that delta reads too
+        assert (got.grad.double() - want.grad).norm() <= 2.0 ** -7 * want.grad.norm() + 1e-6
