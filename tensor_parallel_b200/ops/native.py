@@ -343,7 +343,36 @@ def linear_wgrad(g2d: torch.Tensor, x2d: torch.Tensor) -> torch.Tensor:
     return gemm_nt(g2d, x2d, x_t=True, w_t=True)
 
 
+class _LinearFn(torch.autograd.Function):
+    """The node of :func:`linear` where it has to be a Python function: ``torch.jit.trace`` records calls of these (a C++ node leaves
+    nothing in the graph but the allocation of its result)."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias):
+        x2d = x.reshape(-1, x.shape[-1])
+        out = gemm_nt(x2d, weight, bias)
+        ctx.save_for_backward(x2d, weight)
+        ctx.has_bias = bias is not None
+        ctx.x_shape = x.shape
+        return out.view(*x.shape[:-1], weight.shape[0])
+
+    @staticmethod
+    def backward(ctx, grad):
+        x2d, weight = ctx.saved_tensors
+        g2d = grad.reshape(-1, grad.shape[-1]).to(torch.bfloat16).contiguous()
+        gx = gw = gb = None
+        if ctx.needs_input_grad[0]:
+            gx = linear_dgrad(g2d, weight).view(ctx.x_shape)
+        if ctx.needs_input_grad[1]:
+            gw = linear_wgrad(g2d, x2d)
+        if ctx.has_bias and ctx.needs_input_grad[2]:
+            gb = g2d.sum(0, dtype=torch.float32).to(grad.dtype)  # (summed in fp32 without an fp32 copy of the gradient)
+        return gx, gw, gb
+
+
 def linear(x, weight, bias=None):
+    if torch.jit.is_tracing():
+        return _LinearFn.apply(x, weight, bias)
     return AUTOGRAD.linear(x, weight, bias)
 
 
@@ -352,6 +381,7 @@ def linear(x, weight, bias=None):
 # ------------------------------------------------------------------------------------------------
 
 LIB.tpb_norm_fwd.argtypes = [c_void_p] * 8 + [c_int, c_int, c_float, c_int, c_int, c_void_p]
+LIB.tpb_norm_bwd.argtypes = [c_void_p] * 10 + [c_int] * 5 + [c_void_p]
 
 
 def norm_supported(x: torch.Tensor) -> bool:
@@ -370,12 +400,54 @@ def norm_forward(x2d, weight, bias, eps, mode, residual=None, sum_out=None, want
     return out, rstd, mean
 
 
+class _NormFn(torch.autograd.Function):
+    """The node of the norms where it has to be a Python function (see :class:`_LinearFn`)."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps, mode):
+        x2d = x.reshape(-1, x.shape[-1]).contiguous()
+        w = None if weight is None else weight.to(x.dtype).contiguous()
+        b = None if bias is None else bias.to(x.dtype).contiguous()
+        out, rstd, mean = norm_forward(x2d, w, b, eps, mode, want_stats=True)
+        ctx.save_for_backward(x2d, w, rstd, mean if mean is not None else rstd)
+        ctx.mode, ctx.shape = mode, x.shape
+        ctx.wdtype = None if weight is None else weight.dtype
+        ctx.bdtype = None if bias is None else bias.dtype
+        return out.view(x.shape)
+
+    @staticmethod
+    def backward(ctx, grad):
+        global _launches
+        x2d, w, rstd, mean = ctx.saved_tensors
+        g2d = grad.reshape(x2d.shape).to(x2d.dtype).contiguous()
+        rows, cols = x2d.shape
+        dx = torch.empty_like(x2d)
+        # column sums: one fp32 partial row per CTA, added up by a second kernel that writes the gradients in their own dtype
+        has_w, has_b = w is not None, ctx.bdtype is not None
+        gdtype = ctx.wdtype if has_w and (not has_b or ctx.bdtype == ctx.wdtype) and ctx.wdtype == torch.bfloat16 else torch.float32
+        parts = LIB.tpb_norm_bwd_parts(rows, cols)
+        part_w = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_w else None
+        part_b = torch.empty(parts, cols, dtype=torch.float32, device=x2d.device) if has_b else None
+        dw = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_w else None
+        db = torch.empty(cols, dtype=gdtype, device=x2d.device) if has_b else None
+        check(LIB.tpb_norm_bwd(_ptr(g2d), _ptr(x2d), _ptr(w), _ptr(rstd), _ptr(mean), _ptr(dx), _ptr(part_w), _ptr(part_b), _ptr(dw), _ptr(db),
+                               rows, cols, ctx.mode, _dtype_code(x2d), int(gdtype == torch.float32), _stream()), "tpb_norm_bwd")
+        _launches += 2 if has_w or has_b else 1
+        return (dx.view(ctx.shape), None if dw is None else dw.to(ctx.wdtype), None if db is None else db.to(ctx.bdtype), None, None)
+
+
+def _norm(x, weight, bias, eps, mode):
+    if torch.jit.is_tracing():
+        return _NormFn.apply(x, weight, bias, eps, mode)
+    return AUTOGRAD.norm(x, weight, bias, eps, mode)
+
+
 def rms_norm(x, weight, eps):
-    return AUTOGRAD.norm(x, weight, None, eps, 0)
+    return _norm(x, weight, None, eps, 0)
 
 
 def layer_norm(x, weight, bias, eps):
-    return AUTOGRAD.norm(x, weight, bias, eps, 1)
+    return _norm(x, weight, bias, eps, 1)
 
 
 # ------------------------------------------------------------------------------------------------

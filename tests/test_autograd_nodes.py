@@ -1,5 +1,6 @@
 """The C++ autograd nodes of linear layers and norms, on the CPU: the kernels are stood in for by PyTorch on the same memory."""
 import ctypes
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -90,6 +91,20 @@ def nodes():
     native.AUTOGRAD.bind({n: ctypes.cast(s, _p).value for n, s in stubs.items()}, native._error_text, lambda index, elems: ctypes.addressof(context))
     yield native
     native._bind_autograd()
+
+
+@pytest.fixture
+def python_nodes(nodes, monkeypatch):
+    """The Python autograd functions too run on the stand-ins."""
+    types = dict(tpb_gemm_plan_ex=(_plan, [_i] * 7 + [_p]), tpb_gemm_bf16_ex=(_gemm, [_p] * 5 + [_i] * 7 + [_f] + [_p] * 4),
+                 tpb_norm_fwd=(_norm_fwd, [_p] * 8 + [_i, _i, _f, _i, _i, _p]), tpb_norm_bwd=(_norm_bwd, [_p] * 10 + [_i] * 5 + [_p]),
+                 tpb_norm_bwd_parts=(_norm_bwd_parts, [_i, _i]))
+    library = SimpleNamespace(**{name: ctypes.CFUNCTYPE(_i, *args)(fn) for name, (fn, args) in types.items()})
+    monkeypatch.setattr(nodes, "LIB", library)
+    monkeypatch.setattr(nodes, "gemm_plan", lambda *a, **k: nodes.GemmPlan())
+    monkeypatch.setattr(nodes, "device_state", lambda device: SimpleNamespace(ctx=nodes.ReduceCtx()))
+    monkeypatch.setattr(nodes, "_stream", lambda: None)
+    return nodes
 
 
 def _close(got, want):
@@ -215,3 +230,40 @@ def test_an_error_of_a_kernel_reaches_the_caller(nodes, monkeypatch):
         nodes.linear(x, w)
     with pytest.raises(RuntimeError, match="tpb_gemm_bf16 failed: reduction workspace too small"):
         out.sum().backward()
+
+
+class _Layer(torch.nn.Module):
+    def __init__(self, nodes, kind, learned, dtype=torch.bfloat16):
+        super().__init__()
+        self.nodes, self.kind = nodes, kind
+        torch.manual_seed(4)
+        self.weight = torch.nn.Parameter(torch.randn(*((8, 16) if kind == "linear" else (16,)), dtype=dtype), requires_grad=learned)
+        self.bias = torch.nn.Parameter(torch.randn(8 if kind == "linear" else 16, dtype=dtype), requires_grad=learned)
+
+    def forward(self, x):
+        if self.kind == "linear":
+            return self.nodes.linear(x, self.weight, self.bias)
+        if self.kind == "rms":
+            return self.nodes.rms_norm(x, self.weight, 1e-6)
+        return self.nodes.layer_norm(x, self.weight, self.bias, 1e-6)
+
+
+@pytest.mark.parametrize("kind", ["linear", "rms", "layer"])
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("grad_mode", [False, True])
+def test_a_traced_layer_computes(python_nodes, kind, learned, grad_mode):
+    """On inputs that it was not traced with, and of another number of rows; gradients flow where they did when it was traced."""
+    layer = _Layer(python_nodes, kind, learned)
+    x = torch.randn(3, 16, dtype=torch.bfloat16)
+    with torch.set_grad_enabled(grad_mode):
+        traced = torch.jit.trace(layer, x)
+        for rows in (3, 5):
+            y = torch.randn(rows, 16, dtype=torch.bfloat16)
+            assert torch.equal(traced(y), layer(y))
+    if grad_mode and learned:
+        traced(y).sum().backward()
+        grads = [p.grad for p in layer.parameters()]
+        layer.zero_grad()
+        layer(y).sum().backward()
+        for got, p in zip(grads, layer.parameters()):
+            assert (got is None) == (p.grad is None) and (got is None or torch.equal(got, p.grad))
