@@ -58,9 +58,12 @@ def build_autograd(force: bool = False) -> Path:
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
     includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda_include), str(CSRC)]
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={AUTOGRAD_PATH.stem}",
+    # the host compiler that nvcc takes, and the C++ runtime that torch has loaded: in a module with a runtime of its own (a compiler that links it
+    # statically), an exception that carries a message of torch's crashes the process
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={AUTOGRAD_PATH.stem}",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{i}" for i in includes), str(source),
-           *(f"-L{d}" for d in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-o", str(AUTOGRAD_PATH)]
+           *(f"-L{d}" for d in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-l:libstdc++.so.6",
+           "-o", str(AUTOGRAD_PATH)]
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError(f"building {AUTOGRAD_PATH.name} failed: {' '.join(cmd)}\n{proc.stderr}")

@@ -267,3 +267,8 @@ def test_a_traced_layer_computes(python_nodes, kind, learned, grad_mode):
         layer(y).sum().backward()
         for got, p in zip(grads, layer.parameters()):
             assert (got is None) == (p.grad is None) and (got is None or torch.equal(got, p.grad))
+
+
+def test_the_module_shares_the_cpp_runtime_of_torch():
+    """With a runtime of its own, a failed check inside the module ended the process instead of raising."""
+    assert b"\0libstdc++.so.6\0" in build.AUTOGRAD_PATH.read_bytes()
