@@ -89,8 +89,12 @@ Tensor tma_ready(const Tensor& t) {
 
 // out[tokens, features] = x w^T + bias; x_t / w_t: that operand lies transposed in memory ([k, tokens] / [k, features]).
 Tensor gemm(const Tensor& x_in, const Tensor& w_in, const Tensor& bias, bool x_t, bool w_t) {
+  if (x_in.scalar_type() != at::kBFloat16 || w_in.scalar_type() != at::kBFloat16)  // (the kernel takes its operands' element size for granted)
+    throw py::type_error("native GEMMs take bf16 operands, got " + std::string(at::toString(x_in.scalar_type())) + " and " + at::toString(w_in.scalar_type()));
+  const int64_t tokens = x_in.size(x_t ? 1 : 0), k = x_in.size(x_t ? 0 : 1), features = w_in.size(w_t ? 1 : 0);
+  TORCH_CHECK(x_in.dim() == 2 && w_in.dim() == 2 && w_in.size(w_t ? 0 : 1) == k, "operands of a native GEMM of ", x_in.sizes(), " and ", w_in.sizes(),
+              " do not contract");
   const Tensor x = tma_ready(x_in), w = tma_ready(w_in);
-  const int64_t tokens = x.size(x_t ? 1 : 0), k = x.size(x_t ? 0 : 1), features = w.size(w_t ? 1 : 0);
   Tensor out = at::empty({tokens, features}, x.options());
   tpb_gemm_plan_t plan;
   check(lib.plan(int(tokens), int(features), int(k), 1, 0, 0, int(x_t || w_t), &plan), "gemm_plan");
@@ -141,13 +145,18 @@ Tensor linear(const Tensor& x, const Tensor& weight, const std::optional<Tensor>
   return gemm(x.reshape({-1, x.size(-1)}), weight, bias, false, false).view(with_last(x, weight.size(0)));
 }
 
-int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? 0 : 1; }
+int dtype_code(const Tensor& t) {
+  if (t.scalar_type() == at::kBFloat16) return 0;
+  if (t.scalar_type() == at::kFloat) return 1;
+  throw py::type_error("native kernels take bf16 or fp32 tensors, got " + std::string(at::toString(t.scalar_type())));
+}
 
 // mode 0: RMSNorm, 1: LayerNorm, of bf16 or fp32 rows.
 struct NormFn : torch::autograd::Function<NormFn> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& weight_, const std::optional<Tensor>& bias_,
                         double eps, int64_t mode) {
     const Tensor weight = or_undefined(weight_), bias = or_undefined(bias_);
+    const int dtype = dtype_code(x);
     const Tensor x2d = x.reshape({-1, x.size(-1)}).contiguous();
     const Tensor w = weight.defined() ? weight.to(x.scalar_type()).contiguous() : Tensor();
     const Tensor b = bias.defined() ? bias.to(x.scalar_type()).contiguous() : Tensor();
@@ -156,7 +165,7 @@ struct NormFn : torch::autograd::Function<NormFn> {
     Tensor rstd = at::empty({rows}, x2d.options().dtype(at::kFloat));
     Tensor mean = mode == 1 ? at::empty_like(rstd) : Tensor();
     check(lib.norm_fwd(x2d.const_data_ptr(), nullptr, data(w), data(b), out.mutable_data_ptr(), nullptr, rstd.data_ptr<float>(),
-                       mean.defined() ? mean.data_ptr<float>() : nullptr, int(rows), int(cols), float(eps), int(mode), dtype_code(x2d), stream_of(x2d)),
+                       mean.defined() ? mean.data_ptr<float>() : nullptr, int(rows), int(cols), float(eps), int(mode), dtype, stream_of(x2d)),
           "tpb_norm_fwd");
     launched.fetch_add(1, std::memory_order_relaxed);
     ctx->save_for_backward({x2d, w, rstd, mean});

@@ -272,3 +272,28 @@ def test_a_traced_layer_computes(python_nodes, kind, learned, grad_mode):
 def test_the_module_shares_the_cpp_runtime_of_torch():
     """With a runtime of its own, a failed check inside the module ended the process instead of raising."""
     assert b"\0libstdc++.so.6\0" in build.AUTOGRAD_PATH.read_bytes()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float64, torch.int32])
+def test_other_types_are_refused_before_a_kernel_is_called(nodes, dtype):
+    """The kernels would take 2-byte elements for 4-byte ones, past the end of the tensors."""
+    x, w = torch.ones(4, 8).to(dtype), torch.ones(8).to(dtype)
+    before = nodes.launch_count
+    with pytest.raises(TypeError, match="bf16 or fp32"):
+        nodes.rms_norm(x, w, 1e-6)
+    with pytest.raises(TypeError, match="bf16 or fp32"):
+        nodes.layer_norm(x, None, None, 1e-6)
+    with pytest.raises(TypeError, match="bf16 operands"):
+        nodes.linear(x, torch.ones(16, 8, dtype=torch.bfloat16))
+    with pytest.raises(TypeError, match="bf16 operands"):
+        nodes.linear(torch.ones(4, 8, dtype=torch.bfloat16), torch.ones(16, 8).to(dtype))
+    assert nodes.launch_count == before
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("weight", [(16, 6), (16, 10), (16,), (1, 16, 8)])
+def test_operands_that_do_not_contract_are_refused(nodes, weight, grad):
+    before = nodes.launch_count
+    with pytest.raises((RuntimeError, IndexError)):
+        nodes.linear(torch.ones(4, 8, dtype=torch.bfloat16, requires_grad=grad), torch.ones(*weight, dtype=torch.bfloat16))
+    assert nodes.launch_count == before
