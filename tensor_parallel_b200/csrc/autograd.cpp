@@ -228,6 +228,7 @@ void bind(const py::dict& addresses, py::function text, py::function reserve) {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bind", &bind);
+  m.def("layout", [] { return TPB_API_LAYOUT; });  // of the structures that it hands to the library it is bound to
   m.def("launches", [] { return launched.load(std::memory_order_relaxed); });
   const auto unlocked = py::call_guard<py::gil_scoped_release>();
   m.def("linear", &linear, unlocked);

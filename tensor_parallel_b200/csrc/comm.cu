@@ -303,6 +303,8 @@ extern "C" int tpb_ipc_open_handle(const void* handle64, void** out_ptr) {
 }
 extern "C" int tpb_ipc_close_handle(void* ptr) { return cudaIpcCloseMemHandle(ptr) == cudaSuccess ? TPB_OK : TPB_ERR_CUDA; }
 
+extern "C" unsigned long long tpb_api_layout(void) { return TPB_API_LAYOUT; }
+
 extern "C" int tpb_last_cuda_error(char* buf, int len) {
   const char* s = cudaGetErrorString(cudaGetLastError());
   strncpy(buf, s, len - 1);

@@ -124,6 +124,11 @@ int tpb_norm_bwd_parts(int rows, int cols);
 int tpb_norm_bwd(const void* dy, const void* x, const void* weight, const float* rstd, const float* mean, void* dx, float* part_w,
                  float* part_b, void* dweight, void* dbias, int rows, int cols, int mode, int dtype, int grad_dtype, void* stream);
 
+// Sizes of the structures above as this library was built, one byte-count per 16 bits (plan, reduction context, options), for callers that
+// are built apart from it.
+#define TPB_API_LAYOUT ((unsigned long long)sizeof(tpb_gemm_plan_t) | (unsigned long long)sizeof(tpb_reduce_ctx_t) << 16 | (unsigned long long)sizeof(tpb_gemm_opts_t) << 32)
+unsigned long long tpb_api_layout(void);
+
 // Measurement aids.  tpb_gemm_debug caps the smem ring depth (0 restores the default).  Skipping the MMAs and the
 // kernel-internal %globaltimer trace (tpb_gemm_trace / tpb_gemm_trace_read) exist only in a library built with
 // -DTPB_GEMM_TRACE; in the product build they return TPB_ERR_ARG and the kernels carry no trace code.

@@ -11,6 +11,7 @@ import importlib.util
 import math
 import os
 import threading
+import warnings
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -32,23 +33,33 @@ def _load() -> ctypes.CDLL:
     return ctypes.CDLL(str(path))
 
 
-def _load_autograd():
-    if not _build.AUTOGRAD_PATH.exists() or os.environ.get("TPB_REBUILD"):
-        _build.build_autograd()
-    spec = importlib.util.spec_from_file_location(_build.AUTOGRAD_PATH.stem, _build.AUTOGRAD_PATH)
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
+def _load_autograd(lib):
+    """The module of C++ autograd nodes, or None (with a warning) where none fits: no compiler for a tree that came without it, or a
+    library variant from before it.  The Python nodes then launch the same kernels."""
+    try:
+        if not _build.AUTOGRAD_PATH.exists() or os.environ.get("TPB_REBUILD"):
+            _build.build_autograd()
+        spec = importlib.util.spec_from_file_location(_build.AUTOGRAD_MODULE, _build.AUTOGRAD_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        lib.tpb_api_layout.restype = ctypes.c_ulonglong
+        layout = lib.tpb_api_layout()
+    except (RuntimeError, OSError, ImportError, AttributeError) as e:
+        warnings.warn(f"linear layers and norms run on Python autograd functions, which cost more host time: {e}", RuntimeWarning)
+        return None
+    if layout != module.layout():
+        raise RuntimeError(f"the native library and {_build.AUTOGRAD_PATH.name} disagree about the structures they share: rebuild both")
     return module
 
 
 LIB = _load()
-AUTOGRAD = _load_autograd()  # autograd nodes of linear layers and norms in C++ (csrc/autograd.cpp)
+AUTOGRAD = _load_autograd(LIB)  # autograd nodes of linear layers and norms in C++ (csrc/autograd.cpp)
 _launches = 0
 
 
 def __getattr__(name):
     if name == "launch_count":  # kernels launched through this binding since import (bench.py reports the delta)
-        return _launches + AUTOGRAD.launches()
+        return _launches + (0 if AUTOGRAD is None else AUTOGRAD.launches())
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
@@ -192,7 +203,8 @@ def _bind_autograd():
     AUTOGRAD.bind({n: ctypes.cast(getattr(LIB, n), c_void_p).value for n in names}, _error_text, _reserve_slots)
 
 
-_bind_autograd()
+if AUTOGRAD is not None:
+    _bind_autograd()
 
 
 # ------------------------------------------------------------------------------------------------
@@ -344,8 +356,8 @@ def linear_wgrad(g2d: torch.Tensor, x2d: torch.Tensor) -> torch.Tensor:
 
 
 class _LinearFn(torch.autograd.Function):
-    """The node of :func:`linear` where it has to be a Python function: ``torch.jit.trace`` records calls of these (a C++ node leaves
-    nothing in the graph but the allocation of its result)."""
+    """The node of :func:`linear` where it has to be a Python function: without the C++ module, and under ``torch.jit.trace``, which records
+    calls of these (a C++ node leaves nothing in the graph but the allocation of its result)."""
 
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -371,7 +383,7 @@ class _LinearFn(torch.autograd.Function):
 
 
 def linear(x, weight, bias=None):
-    if torch.jit.is_tracing():
+    if AUTOGRAD is None or torch.jit.is_tracing():
         return _LinearFn.apply(x, weight, bias)
     return AUTOGRAD.linear(x, weight, bias)
 
@@ -437,7 +449,7 @@ class _NormFn(torch.autograd.Function):
 
 
 def _norm(x, weight, bias, eps, mode):
-    if torch.jit.is_tracing():
+    if AUTOGRAD is None or torch.jit.is_tracing():
         return _NormFn.apply(x, weight, bias, eps, mode)
     return AUTOGRAD.norm(x, weight, bias, eps, mode)
 

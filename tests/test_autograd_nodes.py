@@ -1,5 +1,9 @@
 """The C++ autograd nodes of linear layers and norms, on the CPU: the kernels are stood in for by PyTorch on the same memory."""
 import ctypes
+import sysconfig
+import time
+from concurrent.futures import ThreadPoolExecutor
+from pathlib import Path
 from types import SimpleNamespace
 
 import pytest
@@ -297,3 +301,79 @@ def test_operands_that_do_not_contract_are_refused(nodes, weight, grad):
     with pytest.raises((RuntimeError, IndexError)):
         nodes.linear(torch.ones(4, 8, dtype=torch.bfloat16, requires_grad=grad), torch.ones(*weight, dtype=torch.bfloat16))
     assert nodes.launch_count == before
+
+
+@pytest.fixture
+def compiler(monkeypatch, tmp_path):
+    """A module path of its own and a compiler that writes what it was told to, slowly."""
+    calls = []
+
+    def run(cmd, **kwargs):
+        target = Path(cmd[cmd.index("-o") + 1])
+        calls.append(target)
+        target.write_bytes(b"half")
+        time.sleep(0.1)
+        target.write_bytes(b"whole")
+        return SimpleNamespace(returncode=run.code, stderr="refused", stdout="")
+
+    run.code = 0
+    monkeypatch.setattr(build, "LIB_DIR", tmp_path)
+    monkeypatch.setattr(build, "AUTOGRAD_PATH", tmp_path / build.AUTOGRAD_PATH.name)
+    monkeypatch.setattr(build.subprocess, "run", run)
+    monkeypatch.setattr(build, "_nvcc", lambda: "/usr/local/cuda/bin/nvcc")
+    return SimpleNamespace(calls=calls, run=run)
+
+
+def test_the_module_is_named_after_what_it_fits():
+    assert torch.__version__ in build.AUTOGRAD_PATH.name and sysconfig.get_config_var("SOABI") in build.AUTOGRAD_PATH.name
+
+
+def test_processes_that_build_at_once_take_turns(compiler):
+    """No reader sees half a file, and one of them compiles for all.  (The lock of an open file excludes threads as it does processes.)"""
+    seen = []
+    with ThreadPoolExecutor(4) as pool:
+        jobs = [pool.submit(build.build_autograd) for _ in range(4)]
+        while not all(j.done() for j in jobs):
+            if build.AUTOGRAD_PATH.exists():
+                seen.append(build.AUTOGRAD_PATH.read_bytes())
+        assert {j.result() for j in jobs} == {build.AUTOGRAD_PATH}
+    assert len(compiler.calls) == 1 and compiler.calls[0] != build.AUTOGRAD_PATH
+    assert set(seen) <= {b"whole"} and build.AUTOGRAD_PATH.read_bytes() == b"whole"
+
+
+def test_a_failed_build_leaves_the_module_as_it_was(compiler):
+    build.AUTOGRAD_PATH.write_bytes(b"before")
+    compiler.run.code = 1
+    with pytest.raises(RuntimeError, match="refused"):
+        build.build_autograd(force=True)
+    assert build.AUTOGRAD_PATH.read_bytes() == b"before" and [p.name for p in build.LIB_DIR.iterdir() if p.suffix == ".part"] == []
+
+
+def test_a_variant_of_the_library_brings_the_module_up_to_date(compiler, tmp_path):
+    build.build(lib_path=tmp_path / "variant" / "libvariant.so")
+    assert build.AUTOGRAD_PATH.read_bytes() == b"whole"
+
+
+def test_without_a_compiler_the_python_nodes_serve(python_nodes, monkeypatch, tmp_path):
+    nodes = python_nodes
+    results = []
+    for module in (nodes.AUTOGRAD, None):
+        if module is None:
+            monkeypatch.setattr(build, "AUTOGRAD_PATH", tmp_path / "absent.so")
+            monkeypatch.setattr(build.subprocess, "run", lambda *a, **k: (_ for _ in ()).throw(FileNotFoundError("g++")))
+            monkeypatch.setattr(build, "LIB_DIR", tmp_path)
+            with pytest.warns(RuntimeWarning, match="Python autograd functions"):
+                monkeypatch.setattr(nodes, "AUTOGRAD", nodes._load_autograd(nodes.LIB))
+            assert nodes.AUTOGRAD is None and nodes.launch_count > 0
+        x, w = _linear_case()
+        bias = torch.linspace(-1, 1, 8, dtype=torch.bfloat16).requires_grad_()
+        out = nodes.layer_norm(nodes.linear(x, w, bias), bias, bias, 1e-5)
+        out.sum().backward()
+        results.append([out.detach(), x.grad, w.grad, bias.grad])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_a_library_of_another_layout_is_refused(nodes):
+    library = SimpleNamespace(tpb_api_layout=ctypes.CFUNCTYPE(ctypes.c_ulonglong)(lambda: nodes.AUTOGRAD.layout() + 1))
+    with pytest.raises(RuntimeError, match="rebuild"):
+        nodes._load_autograd(library)
