@@ -10,7 +10,9 @@ import ctypes
 import importlib.util
 import math
 import os
+import sys
 import threading
+import types
 import warnings
 from typing import Dict, Optional, Tuple
 
@@ -57,10 +59,18 @@ AUTOGRAD = _load_autograd(LIB)  # autograd nodes of linear layers and norms in C
 _launches = 0
 
 
-def __getattr__(name):
-    if name == "launch_count":  # kernels launched through this binding since import (bench.py reports the delta)
-        return _launches + (0 if AUTOGRAD is None else AUTOGRAD.launches())
-    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+class _Module(types.ModuleType):
+    @property
+    def launch_count(self):
+        """Kernels launched through this binding since import, or since it was last set (bench.py reports the delta)."""
+        return self._launches + (0 if self.AUTOGRAD is None else self.AUTOGRAD.launches())
+
+    @launch_count.setter
+    def launch_count(self, value):
+        self._launches += value - self.launch_count
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 def count_launches(n: int = 1):

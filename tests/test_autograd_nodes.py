@@ -377,3 +377,14 @@ def test_a_library_of_another_layout_is_refused(nodes):
     library = SimpleNamespace(tpb_api_layout=ctypes.CFUNCTYPE(ctypes.c_ulonglong)(lambda: nodes.AUTOGRAD.layout() + 1))
     with pytest.raises(RuntimeError, match="rebuild"):
         nodes._load_autograd(library)
+
+
+def test_the_launch_count_can_be_set(nodes):
+    x, w = _linear_case()
+    nodes.launch_count = 0
+    nodes.linear(x, w)
+    assert nodes.launch_count == 1
+    nodes.launch_count += 4
+    nodes.count_launches(2)
+    nodes.linear(x, w)
+    assert nodes.launch_count == 8
