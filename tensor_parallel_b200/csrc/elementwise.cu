@@ -245,7 +245,7 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(1024)
 norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ weight,
                 const float* __restrict__ rstd_in, const float* __restrict__ mean_in, T* __restrict__ dx,
-                float* __restrict__ part_w, float* __restrict__ part_b, int rows, int cols) {
+                float* __restrict__ part_w, float* __restrict__ part_b, unsigned rows, int cols) {
   using Ring = RowRing<T, 2>;
   extern __shared__ uint4 norm_ring[];
   __shared__ float2 warp_sums[2][32];
@@ -253,7 +253,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
   float dw_acc[8], db_acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) { dw_acc[j] = 0.f; db_acc[j] = 0.f; }
-  auto fetch = [&](int stage, int row) {
+  auto fetch = [&](int stage, unsigned row) {  // (rows unsigned: the row after the last may be beyond 2^31)
     if (row < rows) {
       ring.fetch(stage, 0, dy + size_t(row) * cols, cols);
       ring.fetch(stage, 1, x + size_t(row) * cols, cols);
@@ -265,14 +265,14 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
   Raw8<T> wr;
   if (weight) wr = RowCols<T>::load(weight, cols);
   const float inv_n = 1.f / float(cols);
-  int row = blockIdx.x;
+  unsigned row = blockIdx.x;
   float rstd = 0.f, mean = 0.f;
   if (row < rows) {
     rstd = rstd_in[row];
     if (MODE == 1) mean = mean_in[row];
   }
   for (int it = 0; row < rows; ++it) {
-    const int next = row + gridDim.x;
+    const unsigned next = row + gridDim.x;
     fetch((it + Ring::STAGES - 1) % Ring::STAGES, row + (Ring::STAGES - 1) * gridDim.x);
     float rstd_next = 0.f, mean_next = 0.f;
     if (next < rows) {
@@ -329,12 +329,12 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
 template <typename T, int MODE>
 __global__ void __launch_bounds__(1024, sizeof(T) == 2 && MODE == 0 ? 2 : 1)
 norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, const T* __restrict__ bias, T* __restrict__ out,
-                     float* __restrict__ rstd_out, float* __restrict__ mean_out, int rows, int cols, float eps) {
+                     float* __restrict__ rstd_out, float* __restrict__ mean_out, unsigned rows, int cols, float eps) {
   using Ring = RowRing<T, 1>;
   extern __shared__ uint4 norm_ring[];
   __shared__ float2 warp_sums[2][32];
   const Ring ring{norm_ring};
-  auto fetch = [&](int stage, int row) {
+  auto fetch = [&](int stage, unsigned row) {
     if (row < rows) ring.fetch(stage, 0, x + size_t(row) * cols, cols);
     Ring::commit();
   };
@@ -345,7 +345,8 @@ norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, cons
   if (weight) wr = RowCols<T>::load(weight, cols);
   if (MODE == 1 && bias) br = RowCols<T>::load(bias, cols);
   const float inv_n = 1.f / float(cols);
-  for (int it = 0, row = blockIdx.x; row < rows; ++it, row += gridDim.x) {
+  int it = 0;
+  for (unsigned row = blockIdx.x; row < rows; ++it, row += gridDim.x) {
     fetch((it + Ring::STAGES - 1) % Ring::STAGES, row + (Ring::STAGES - 1) * gridDim.x);
     Ring::wait();
     float v[8], s1 = 0.f, s2 = 0.f;
@@ -757,7 +758,7 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   do {                                                                                                                              \
     if (!norm_ring_allowed<norm_fwd_rows_kernel<T, M>>()) return TPB_ERR_CUDA;                                                      \
     launch_kernel(norm_fwd_rows_kernel<T, M>, grid, dim3(threads), RowRing<T, 1>::bytes(threads), s, (const T*)x, (const T*)weight, \
-                  (const T*)bias, (T*)out, rstd_out, mean_out, rows, cols, eps);                                                    \
+                  (const T*)bias, (T*)out, rstd_out, mean_out, unsigned(rows), cols, eps);                                          \
   } while (0)
     if (dtype == 0) { if (mode) LAUNCH(bf16, 1); else LAUNCH(bf16, 0); }
     else            { if (mode) LAUNCH(float, 1); else LAUNCH(float, 0); }

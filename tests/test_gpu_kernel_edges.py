@@ -778,3 +778,19 @@ def test_attention_backward_by_step(d, b, sq, sk, hq, hkv, causal, rows, bias):
     for got, want in zip([q, k, v] + ([added] if added is not None and added.requires_grad else []), ref):
         # probabilities, dS and results are rounded to bf16 once each (2^-9 relative, independent errors), the output that delta reads too
         assert (got.grad.double() - want.grad).norm() <= 2.0 ** -7 * want.grad.norm() + 1e-6
+
+
+def test_norm_of_as_many_rows_as_an_int_counts():
+    """2^31 - 1 narrow rows: the rows fetched ahead of the last ones have numbers that no int holds."""
+    rows, cols = 2 ** 31 - 1, 8
+    if torch.cuda.mem_get_info()[0] < 80e9:
+        pytest.skip("needs 70 GB")
+    nat = _native()
+    x = torch.empty(rows, cols, device="cuda", dtype=torch.bfloat16)
+    x[:-5000] = 1.0
+    x[-5000:] = torch.randn(5000, cols, device="cuda")
+    out = nat.norm_forward(x, None, None, 1e-6, 1)[0]
+    assert bool((out[-5000:].double() - torch.nn.functional.layer_norm(x[-5000:].double(), (cols,), eps=1e-6)).abs().max() <= 2.0 ** -6)  # bf16 results below 4
+    assert not bool(out[: 1 << 20].any()) and not bool(out[1 << 30 : (1 << 30) + (1 << 20)].any())
+    del x, out
+    torch.cuda.empty_cache()
