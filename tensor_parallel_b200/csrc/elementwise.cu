@@ -378,6 +378,60 @@ norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, cons
   }
 }
 
+// fp32 RMSNorm of many rows: a CTA per row, faster than rings from about 8192 rows on (see tpb_norm_fwd: 32768 x 4096 192 -> 159 us, 6.8 TB/s, HBM), with
+// the sums of a row added up in the order of norm_fwd_rows_kernel, so that a row's result does not depend on how many others came with it: thread t stands for threads t, t + 256,
+// ... of a ring CTA (`ring_threads`, a multiple of 32), which own the same columns and end up in the same place among the warps' sums.
+template <int MAXV>
+__global__ void __launch_bounds__(NORM_THREADS)
+norm_fwd_row_kernel(const float* __restrict__ x, const float* __restrict__ weight, float* __restrict__ out, float* __restrict__ rstd_out,
+                    float* __restrict__ mean_out, int cols, int ring_threads, float eps) {
+  __shared__ float warp_sums[MAXV * NORM_THREADS / 32];
+  pdl_wait();
+  const size_t row = blockIdx.x;
+  const float* xr = x + row * cols;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = ring_threads >> 5;
+  auto column = [&](int i, int chunk) { return (int(threadIdx.x) + i * NORM_THREADS + chunk * ring_threads) * 4; };
+  float v[MAXV][8];
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const bool live = threadIdx.x + i * NORM_THREADS < ring_threads;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float4 f = live && column(i, c) < cols ? *reinterpret_cast<const float4*>(xr + column(i, c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[i][4 * c] = f.x; v[i][4 * c + 1] = f.y; v[i][4 * c + 2] = f.z; v[i][4 * c + 3] = f.w;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += v[i][j] * v[i][j];
+    s = warp_sum(s);
+    if (lane == 0) warp_sums[warp + i * (NORM_THREADS / 32)] = s;
+  }
+  __syncthreads();
+  const float total = warp_sum(lane < warps ? warp_sums[lane] : 0.f);
+  const float rstd = rsqrtf(total * (1.f / float(cols)) + eps);
+  if (threadIdx.x == 0) {
+    if (rstd_out) rstd_out[row] = rstd;
+    if (mean_out) mean_out[row] = 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    if (threadIdx.x + i * NORM_THREADS >= ring_threads) continue;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (column(i, c) >= cols) continue;
+      float4 o = make_float4(v[i][4 * c] * rstd, v[i][4 * c + 1] * rstd, v[i][4 * c + 2] * rstd, v[i][4 * c + 3] * rstd);
+      if (weight) {
+        const float4 w = *reinterpret_cast<const float4*>(weight + column(i, c));
+        o = make_float4(o.x * w.x, o.y * w.y, o.z * w.z, o.w * w.w);
+      }
+      *reinterpret_cast<float4*>(out + row * cols + column(i, c)) = o;
+    }
+  }
+}
+
 // out[c] = sum over parts of part[p][c] (blockIdx.y: 0 = weight, 1 = bias).  32 columns x 32 rows of partials per step, so that
 // every partial row's loads are independent; the summation order depends on the number of partials only.
 template <typename O>
@@ -746,11 +800,20 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   if (!x || !out || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_MAXV) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  // A CTA per row is as good, and better with many rows, where RMSNorm rows fill its 256 threads: 2048 x 2048 bf16 5.6 us (ring 5.9), 32768 x
-  // 4096 bf16 107 (117), fp32 169 (192), 16384 x 2048 fp32 45 (48); with fewer rows 2048 x 2048 fp32 8.4 (6.6), 20 x 4096 2.8 (2.5); rows
-  // that leave threads idle: 1999 x 5120 bf16 13.9 (10.8).
+  // A CTA per row instead of rings where RMSNorm rows fill its 256 threads, by width and type alone where the two add a row up in different orders.
+  // bf16: 600 x 4096 3.2 us (ring 4.2), 1000 x 2048 3.2 (3.7), 32768 x 4096 106 (107); 20 x 4096 2.6 (2.5), 2048 x 4096 10.2 (9.4).  fp32, both in the same
+  // order: 8192 x 4096 43.1 (47.7), 16384 x 2048 41.6 (48.2), 32768 x 4096 159 (192); fewer rows 4000 x 4096 25.5 (22.6), 1000 x 2048 5.0 (4.4).  Rows that
+  // leave threads idle: 1999 x 5120 bf16 13.9 (10.8).
   const bool filled = (cols > NORM_THREADS * 6 && cols <= NORM_THREADS * 8) || (cols > NORM_THREADS * 12 && cols <= NORM_THREADS * 16);
-  const bool one_cta = mode == 0 && filled && rows >= (dtype == 0 ? 2048 : 8192);
+  const bool one_cta = mode == 0 && filled && (dtype == 0 || rows >= 8192);
+  if (!residual && one_cta && dtype == 1) {
+#define LAUNCH(V)                                                                                                                          \
+  launch_kernel(norm_fwd_row_kernel<V>, dim3(rows), dim3(NORM_THREADS), 0, s, (const float*)x, (const float*)weight, (float*)out, rstd_out, \
+                mean_out, cols, norm_row_threads(cols), eps)
+    if (cols <= NORM_THREADS * 8) LAUNCH(1); else LAUNCH(2);
+#undef LAUNCH
+    TPB_CHECK_LAUNCH();
+  }
   if (!residual && cols <= NORM_BWD_MAXC && !one_cta) {
     const int threads = norm_row_threads(cols);
     const dim3 grid(norm_row_ctas(rows, cols, dtype == 0 ? 2048 : 1024));
