@@ -321,11 +321,9 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
   if (MODE == 1 && part_b) RowCols<T>::store(part_b + size_t(blockIdx.x) * cols, cols, db_acc);
 }
 
-// Forward without a residual: rows stream through the same rings; weight and bias stay in registers.  A CTA per row left
-// the weights to be loaded behind the sums, and narrow rows with idle threads.  LayerNorm 8192 x 4096 bf16 41.8 -> 35.0 us, 1999 x 5120
-// fp32 23.1 -> 17.7 us; RMSNorm 1999 x 5120 bf16 13.9 -> 10.8 us, 8192 x 256 9.8 -> 4.3, 8192 x 4096 31.9 and 31.8 (a copy: 22.8).
-// bf16: CTAs for 2048 threads per SM (against 1024: RMSNorm 1999 x 5120 13.2 -> 10.8, 8192 x 8192 59 -> 55 us); fp32: 1024 (2048: RMSNorm
-// 8192 x 4096 46 -> 49, 8192 x 8192 81 -> 95 us).
+// Forward without a residual: rows stream through the same rings; weight and bias stay in registers.  For narrow rows, which left threads of a
+// CTA per row idle, fp32 rows, and few rows (norm_takes_row_cta).  LayerNorm 1999 x 5120 fp32 23.1 -> 17.7 us, 8192 x 1024 bf16 17.5 -> 10.7; RMSNorm
+// 8192 x 256 bf16 11.3 -> 4.8.  bf16: CTAs for 2048 threads per SM; fp32: 1024 (2048: RMSNorm 8192 x 4096 46 -> 49, 8192 x 8192 81 -> 95 us).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(1024, sizeof(T) == 2 && MODE == 0 ? 2 : 1)
 norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, const T* __restrict__ bias, T* __restrict__ out,
@@ -378,56 +376,71 @@ norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, cons
   }
 }
 
-// fp32 RMSNorm of many rows: a CTA per row, faster than rings from about 8192 rows on (see tpb_norm_fwd: 32768 x 4096 192 -> 159 us, 6.8 TB/s, HBM), with
-// the sums of a row added up in the order of norm_fwd_rows_kernel, so that a row's result does not depend on how many others came with it: thread t stands for threads t, t + 256,
-// ... of a ring CTA (`ring_threads`, a multiple of 32), which own the same columns and end up in the same place among the warps' sums.
-template <int MAXV>
+// A CTA per row, with the row added up in the order of norm_fwd_rows_kernel, so that its result does not depend on which of the two a call takes:
+// thread t stands for threads t, t + 256, ... of a ring CTA (`ring_threads`, a multiple of 32), which own the same columns and end up in the
+// same place among the warps' sums.  Several rows per SM in flight, each in registers, no row waits for another's barrier; where the lines lie:
+// norm_takes_row_cta.  RMSNorm bf16 4000 x 5120, input in L2 / in memory: 13.7 / 17.6 us (rings 18.4 / 19.4; rows in one CTA that loads the next row
+// only when it is done 17.4 / 25.0); LayerNorm bf16 4000 x 4096 14.0 / 18.1 (17.6 / 18.9); 8192 x 8192 56 us, 4.8 TB/s (70).
+template <typename T, int MODE, int MAXV>
 __global__ void __launch_bounds__(NORM_THREADS)
-norm_fwd_row_kernel(const float* __restrict__ x, const float* __restrict__ weight, float* __restrict__ out, float* __restrict__ rstd_out,
+norm_fwd_row_kernel(const T* __restrict__ x, const T* __restrict__ weight, const T* __restrict__ bias, T* __restrict__ out, float* __restrict__ rstd_out,
                     float* __restrict__ mean_out, int cols, int ring_threads, float eps) {
-  __shared__ float warp_sums[MAXV * NORM_THREADS / 32];
+  constexpr int CHUNKS = RowCols<T>::CHUNKS, WIDTH = RowCols<T>::WIDTH;
+  __shared__ float2 warp_sums[MAXV * NORM_THREADS / 32];
   pdl_wait();
-  const size_t row = blockIdx.x;
-  const float* xr = x + row * cols;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = ring_threads >> 5;
-  auto column = [&](int i, int chunk) { return (int(threadIdx.x) + i * NORM_THREADS + chunk * ring_threads) * 4; };
+  const size_t at = size_t(blockIdx.x) * cols;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto column = [&](int i, int chunk) { return (int(threadIdx.x) + i * NORM_THREADS + chunk * ring_threads) * WIDTH; };
+  auto mine = [&](int i, int chunk) { return int(threadIdx.x) + i * NORM_THREADS < ring_threads && column(i, chunk) < cols; };
+  auto load = [&](const T* row, int i, float (&f)[8]) {
+    Raw8<T> r;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) r.u[c] = mine(i, c) ? *reinterpret_cast<const uint4*>(row + column(i, c)) : make_uint4(0, 0, 0, 0);
+    unpack(r, f);
+  };
   float v[MAXV][8];
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const bool live = threadIdx.x + i * NORM_THREADS < ring_threads;
+  for (int i = 0; i < MAXV; ++i) load(x + at, i, v[i]);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const float4 f = live && column(i, c) < cols ? *reinterpret_cast<const float4*>(xr + column(i, c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[i][4 * c] = f.x; v[i][4 * c + 1] = f.y; v[i][4 * c + 2] = f.z; v[i][4 * c + 3] = f.w;
+  for (int i = 0; i < MAXV; ++i) {
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      s1 += v[i][j];
+      s2 += v[i][j] * v[i][j];
     }
-  }
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    float s = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s += v[i][j] * v[i][j];
-    s = warp_sum(s);
-    if (lane == 0) warp_sums[warp + i * (NORM_THREADS / 32)] = s;
+    s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    if (lane == 0) warp_sums[warp + i * (NORM_THREADS / 32)] = make_float2(s1, s2);
   }
   __syncthreads();
-  const float total = warp_sum(lane < warps ? warp_sums[lane] : 0.f);
-  const float rstd = rsqrtf(total * (1.f / float(cols)) + eps);
+  const float2 sums = lane < ring_threads >> 5 ? warp_sums[lane] : make_float2(0.f, 0.f);
+  const float s1 = warp_sum(sums.x), s2 = warp_sum(sums.y);
+  const float inv_n = 1.f / float(cols);
+  const float mean = MODE == 1 ? s1 * inv_n : 0.f;
+  const float var = MODE == 1 ? fmaxf(s2 * inv_n - mean * mean, 0.f) : s2 * inv_n;
+  const float rstd = rsqrtf(var + eps);
   if (threadIdx.x == 0) {
-    if (rstd_out) rstd_out[row] = rstd;
-    if (mean_out) mean_out[row] = 0.f;
+    if (rstd_out) rstd_out[blockIdx.x] = rstd;
+    if (mean_out) mean_out[blockIdx.x] = mean;
   }
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
-    if (threadIdx.x + i * NORM_THREADS >= ring_threads) continue;
+    float w[8], b[8], o[8];
+    if (weight) load(weight, i, w);
+    if (MODE == 1 && bias) load(bias, i, b);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      if (column(i, c) >= cols) continue;
-      float4 o = make_float4(v[i][4 * c] * rstd, v[i][4 * c + 1] * rstd, v[i][4 * c + 2] * rstd, v[i][4 * c + 3] * rstd);
-      if (weight) {
-        const float4 w = *reinterpret_cast<const float4*>(weight + column(i, c));
-        o = make_float4(o.x * w.x, o.y * w.y, o.z * w.z, o.w * w.w);
-      }
-      *reinterpret_cast<float4*>(out + row * cols + column(i, c)) = o;
+    for (int j = 0; j < 8; ++j) {
+      float y = (v[i][j] - mean) * rstd;
+      if (weight) y *= w[j];
+      if (MODE == 1 && bias) y += b[j];
+      o[j] = y;
+    }
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      if (!mine(i, c)) continue;
+      if constexpr (CHUNKS == 1) Vec8<T>::store(out + at + column(i, 0), o);
+      else *reinterpret_cast<float4*>(out + at + column(i, c)) = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
     }
   }
 }
@@ -780,6 +793,26 @@ static inline int norm_row_ctas(int rows, int cols, int threads_per_sm) {
   return rows < ctas ? rows : ctas;
 }
 
+// Widths whose rows (nearly) fill 256 threads with one or two vectors each.
+static inline bool norm_filled(int cols) { return (cols > NORM_THREADS * 6 && cols <= NORM_THREADS * 8) || (cols > NORM_THREADS * 12 && cols <= NORM_THREADS * 16); }
+
+// norm_fwd_row_kernel (true) or norm_fwd_rows_kernel for a forward without a residual, which give the same bits.  Times in us as row / ring, "hot"
+// with the input in L2, as the kernel before leaves it, "cold" with it in memory.
+static inline bool norm_takes_row_cta(int rows, int cols, int mode, int dtype) {
+  // fp32: RMSNorm of many rows that fill the threads (8192 x 4096 43.1 / 47.7, 16384 x 2048 41.6 / 48.2, 32768 x 4096 159 / 192; 4000 x 4096 25.5 / 22.6)
+  if (dtype == 1) return mode == 0 && norm_filled(cols) && rows >= 8192;
+  // one row per SM: the ring kernel's CTA has more threads for it (LayerNorm 100 x 8192 4.1 / 3.2, 20 x 4096 2.8 / 2.4)
+  if (cols > 1536 && rows <= 148) return false;
+  // wide rows: RMSNorm 2000 x 5120 hot 7.4 / 10.2, cold 10.6 / 11.0; 2000 x 3072 6.3 / 7.5, 8.3 / 7.9; LayerNorm 2000 x 4096 8.1 / 10.2, 10.7 / 11.4; 1000 x
+  // 8192 9.0 / 11.0, 11.4 / 12.8.  But 4000 x 2560 10.2 / 10.4, 13.0 / 10.8, LayerNorm 4000 x 3072 13.4 / 13.5, 16.5 / 15.9: rings
+  if (cols > 3072 || (mode == 0 && cols > 2560)) return true;
+  // middle widths: hot faster, cold slower (RMSNorm 4000 x 1536 6.8 / 7.5, 8.6 / 7.7; LayerNorm 4000 x 2048 9.2 / 10.1, 11.6 / 11.0), so by whether
+  // input and output can be hot
+  if (mode == 0 ? cols > 1024 && cols <= 1536 : cols > 1536 && cols <= 2048) return (long long)rows * cols <= 1 << 24;
+  // narrow RMSNorm rows that are all resident at once (300 x 768 2.15 / 2.31, 1000 x 512 2.55 / 2.64; 2000 x 768 4.1 / 3.2, 300 x 256 2.2 / 2.2)
+  return mode == 0 && cols > 256 && cols <= 1024 && rows <= 8 * 148;
+}
+
 // Lets a kernel have a ring of the widest row (1024 threads: 192 KB), once per device.
 template <auto KERNEL>
 static bool norm_ring_allowed() {
@@ -800,17 +833,23 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   if (!x || !out || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_MAXV) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  // A CTA per row instead of rings where RMSNorm rows fill its 256 threads, by width and type alone where the two add a row up in different orders.
-  // bf16: 600 x 4096 3.2 us (ring 4.2), 1000 x 2048 3.2 (3.7), 32768 x 4096 106 (107); 20 x 4096 2.6 (2.5), 2048 x 4096 10.2 (9.4).  fp32, both in the same
-  // order: 8192 x 4096 43.1 (47.7), 16384 x 2048 41.6 (48.2), 32768 x 4096 159 (192); fewer rows 4000 x 4096 25.5 (22.6), 1000 x 2048 5.0 (4.4).  Rows that
-  // leave threads idle: 1999 x 5120 bf16 13.9 (10.8).
-  const bool filled = (cols > NORM_THREADS * 6 && cols <= NORM_THREADS * 8) || (cols > NORM_THREADS * 12 && cols <= NORM_THREADS * 16);
-  const bool one_cta = mode == 0 && filled && (dtype == 0 || rows >= 8192);
-  if (!residual && one_cta && dtype == 1) {
-#define LAUNCH(V)                                                                                                                          \
-  launch_kernel(norm_fwd_row_kernel<V>, dim3(rows), dim3(NORM_THREADS), 0, s, (const float*)x, (const float*)weight, (float*)out, rstd_out, \
+  // bf16 RMSNorm rows that fill 256 threads: a CTA per row in an order of its own whatever their number (600 x 4096 3.3 us, ring 4.4; 1000 x 2048 3.2
+  // and 3.7; 32768 x 4096 106 and 107; 20 x 4096 2.7 and 2.4; 2048 x 4096 10.2 and 9.3)
+  const bool one_cta = mode == 0 && norm_filled(cols) && dtype == 0;
+  if (!residual && !one_cta && cols <= NORM_BWD_MAXC && norm_takes_row_cta(rows, cols, mode, dtype)) {
+#define LAUNCH(T, M, V)                                                                                                                        \
+  launch_kernel(norm_fwd_row_kernel<T, M, V>, dim3(rows), dim3(NORM_THREADS), 0, s, (const T*)x, (const T*)weight, (const T*)bias, (T*)out, rstd_out, \
                 mean_out, cols, norm_row_threads(cols), eps)
-    if (cols <= NORM_THREADS * 8) LAUNCH(1); else LAUNCH(2);
+#define LAUNCH_V(T, M)                                                                                                  \
+  do {                                                                                                                  \
+    if (cols <= NORM_THREADS * 8) LAUNCH(T, M, 1);                                                                      \
+    else if (cols <= NORM_THREADS * 16) LAUNCH(T, M, 2);                                                                \
+    else if constexpr (sizeof(T) == 2) { if (cols <= NORM_THREADS * 24) LAUNCH(T, M, 3); else LAUNCH(T, M, 4); }        \
+  } while (0)
+    if (dtype == 1) LAUNCH_V(float, 0);
+    else if (mode) LAUNCH_V(bf16, 1);
+    else LAUNCH_V(bf16, 0);
+#undef LAUNCH_V
 #undef LAUNCH
     TPB_CHECK_LAUNCH();
   }

@@ -797,21 +797,22 @@ def test_norm_of_as_many_rows_as_an_int_counts():
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("cols", [8, 264, 1536, 1544, 1800, 2048, 3080, 3584, 4096, 5120])
+@pytest.mark.parametrize("cols", [8, 264, 776, 1024, 1536, 1544, 1800, 2048, 2568, 3072, 3080, 3584, 4096, 4104, 5120, 6152, 8192])
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("with_weight", [False, True])
 def test_norm_of_a_row_does_not_depend_on_the_others(dtype, cols, mode, with_weight):
     """The same bits for a row alone, among few, and among as many as take another kernel."""
     nat = _native()
     torch.manual_seed(cols)
-    x = (torch.randn(8200, cols, device="cuda") * 2 + 0.1).to(dtype)
+    x = (torch.randn(16000, cols, device="cuda") * 2 + 0.1).to(dtype)
     w = torch.randn(cols, device="cuda").to(dtype) if with_weight else None
-    out, rstd, mean = nat.norm_forward(x, w, None, 1e-6, mode, want_stats=True)
-    for first, count in ((0, 1), (5, 20), (100, 700), (8, 2048), (1, 8191), (8, 8192)):
-        part, r, m = nat.norm_forward(x[first : first + count], w, None, 1e-6, mode, want_stats=True)
+    b = torch.randn(cols, device="cuda").to(dtype) if with_weight and mode else None
+    out, rstd, mean = nat.norm_forward(x, w, b, 1e-6, mode, want_stats=True)
+    for first, count in ((0, 1), (5, 20), (3, 148), (9, 149), (100, 700), (7, 1184), (7, 1185), (8, 2048), (1, 8191), (8, 8192)):
+        part, r, m = nat.norm_forward(x[first : first + count], w, b, 1e-6, mode, want_stats=True)
         assert torch.equal(part, out[first : first + count]) and torch.equal(r, rstd[first : first + count])
         assert mean is None or torch.equal(m, mean[first : first + count])
-    assert (out[:64].double() - _norm_double(x[:64], w, mode)).norm() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * out[:64].double().norm()
+    assert (out[:64].double() - _norm_double(x[:64], w, mode) - (0 if b is None else b.double())).norm() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * out[:64].double().norm()
 
 
 def _norm_double(x, w, mode):
