@@ -160,9 +160,10 @@ class DeviceState:
         self.slots: Optional[torch.Tensor] = None
         self.slot_stride = 0
         self.ctx = ReduceCtx()
-        self._refresh()
+        self._growing = threading.Lock()
+        self._refresh(0)
 
-    def _refresh(self):
+    def _refresh(self, slot_stride: int):
         ctx = self.ctx
         ctx.world, ctx.rank = 1, 0
         ctx.slots[0] = self.slots.data_ptr() if self.slots is not None else 0
@@ -170,15 +171,18 @@ class DeviceState:
         ctx.expected = self.expected.data_ptr()
         ctx.split_counters = self.split_counters.data_ptr()
         ctx.status = self.status.data_ptr()
-        ctx.slot_stride = self.slot_stride
         ctx.max_slots, ctx.max_tiles = MAX_SLOTS, MAX_TILES
+        ctx.slot_stride = self.slot_stride = slot_stride  # (last: whoever sees it finds the rest in place)
 
     def ensure_slots(self, elems: int):
         """Grow-only; growing replaces the buffer, so warm shapes up before capturing a CUDA graph."""
-        if elems > self.slot_stride:
-            self.slot_stride = max(elems, 1 << 20)
-            self.slots = torch.empty(MAX_SLOTS * self.slot_stride, dtype=torch.float32, device=self.device)
-            self._refresh()
+        if elems <= self.slot_stride:
+            return
+        with self._growing:
+            if elems > self.slot_stride:
+                stride = max(elems, 1 << 20)
+                self.slots = torch.empty(MAX_SLOTS * stride, dtype=torch.float32, device=self.device)
+                self._refresh(stride)
 
     def check_status(self):
         code = int(self.status[0].item())

@@ -388,3 +388,24 @@ def test_the_launch_count_can_be_set(nodes):
     nodes.count_launches(2)
     nodes.linear(x, w)
     assert nodes.launch_count == 8
+
+
+def test_threads_that_need_the_workspace_at_once(monkeypatch):
+    """The nodes run without the interpreter lock, several threads at a time: who finds the workspace large enough finds its address too."""
+    from tensor_parallel_b200.ops import native
+
+    state, empty = native.DeviceState(torch.device("cpu")), torch.empty
+
+    def slow(*args, **kwargs):
+        time.sleep(0.05)
+        return empty(*args, **kwargs)
+
+    monkeypatch.setattr(torch, "empty", slow)
+
+    def reserve(elems):
+        state.ensure_slots(elems)
+        return state.ctx.slot_stride >= elems and state.ctx.slots[0] == state.slots.data_ptr()
+
+    with ThreadPoolExecutor(4) as pool:
+        assert all(pool.map(reserve, [1000] * 4))
+        assert all(pool.map(reserve, [1 << 21, 1 << 20, 1 << 21, 1000]))
