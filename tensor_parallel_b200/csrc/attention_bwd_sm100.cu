@@ -72,6 +72,72 @@ struct BwParams {
   uint32_t* status;
 };
 
+// ---- what the elementwise warps of both kernels do with 32 columns (streamed rows) of one TMEM lane (resident row) ----
+
+// Bits of the columns from col0 on that are visible pairs with resident row ri; only steps that touch the diagonal or an end have any cleared.
+template <bool DKV>
+__device__ __forceinline__ uint32_t bw_visible(const BwParams& p, int ri, int shift, int col0) {
+  int lo = 0, hi = 32;  // columns [lo, hi) are
+  if (DKV) {
+    if (ri >= p.sk) hi = 0;
+    if (p.causal) lo = max(0, ri - shift - col0);  // query >= key - shift
+  } else {
+    hi = min(32, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
+  }
+  uint32_t visible = 0xffffffffu;
+  if (lo > 0) visible = lo < 32 ? visible << lo : 0u;
+  if (hi < 32) visible = hi > 0 ? visible & (0xffffffffu >> (32 - hi)) : 0u;
+  return visible;
+}
+
+// Eight score biases of resident row `row` from column `col` of a step on, out of the step's tile in shared memory.
+template <bool DKV>
+__device__ __forceinline__ void bw_bias8(const uint8_t* tile, int row, int col, float (&v)[8]) {
+  if (DKV) {  // column = query row of the tile, lanes read consecutive keys
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __bfloat162float(*reinterpret_cast<const bf16*>(tile + (col + i) * (BW_R * 2) + row * 2));
+  } else {  // eight keys of this thread's query: one swizzled 16-byte chunk of a block of 64 keys
+    const uint4 u = *reinterpret_cast<const uint4*>(tile + (col >> 6) * FA_BLOCK_BYTES + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4));
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+  }
+}
+
+// Adds the bias gradients of keys col to col + 3 of one query.
+__device__ __forceinline__ void bw_add_dbias(const BwParams& p, long long bias_base, int col, const float (&db)[4]) {
+  float* dst = p.dbias + bias_base + (long long)col * p.b_sk;
+  if (p.bias_vec && col + 4 <= p.sk) {
+    // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (db[i] != 0.f && col + i < p.sk) atomicAdd(dst + i * p.b_sk, db[i]);
+  }
+}
+
+// N accumulator columns as bf16: whole 32-byte sectors, 16 bytes or pairs, as the address allows.
+template <int N>
+__device__ __forceinline__ void bw_store_row(bf16* dst, const uint32_t (&o)[N]) {
+  uint32_t w[N / 2];
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) w[i] = pack_bf16x2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
+  if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
+#pragma unroll
+    for (int i = 0; i < N / 2; i += 8) st_global_v8(dst + 2 * i, w + i);
+  } else if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < N / 2; i += 4) *reinterpret_cast<uint4*>(dst + 2 * i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) *reinterpret_cast<uint32_t*>(dst + 2 * i) = w[i];
+  }
+}
+
 // BIAS: the score-bias code exists only in the instantiations that need it.  1: elements are loaded by the threads that use them;
 // 2: a dense bf16 bias whose rows TMA can address travels with the streamed tiles, [64 queries][128 keys] (dK / dV) or
 // [128 queries][64 keys] (dQ) per step, so that no elementwise warp ever waits for a global load (16 x 512 tokens, 32 heads of 64,
@@ -355,19 +421,8 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
       tmem_ld_x32(t_lane + S_COL0 + buf * BW_T + half * HC, sv);
       tmem_ld_x32(t_lane + DP_COL0 + buf * BW_T + half * HC, dv);
       tmem_ld_wait();
-      // columns [lo, hi) of mine are visible pairs
-      int lo = 0, hi = HC;
-      if (DKV) {
-        if (ri >= p.sk) hi = 0;
-        if (p.causal) lo = max(0, ri - shift - col0);  // query >= key - shift
-      } else {
-        hi = min(HC, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
-      }
-      // ... as bits; only steps that touch the diagonal or an end have any cleared (decided per warp: the common loop has no masks)
-      uint32_t visible = 0xffffffffu;
-      if (lo > 0) visible = lo < HC ? visible << lo : 0u;
-      if (hi < HC) visible = hi > 0 ? visible & (0xffffffffu >> (HC - hi)) : 0u;
-      const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);
+      const uint32_t visible = bw_visible<DKV>(p, ri, shift, col0);
+      const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);  // (per warp: the common loop has no masks)
       // score bias: element (query, key) = (col0 + c, ri) for dK / dV - there the lanes of a warp own consecutive keys - and
       // (ri, col0 + c) for dQ, where a thread's columns are consecutive keys of one row and are read eight at a time
       const long long bias_base = BIAS ? (long long)b * p.b_sb + (long long)b_head * p.b_sh + (long long)ri * (DKV ? p.b_sk : p.b_sq) : 0;
@@ -387,22 +442,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
             l0 = l1 = my_lse2;
             d0 = d1 = my_del;
           }
-          if (BIAS == 2 && (c & 7) == 0) {
-            const uint8_t* tile = bias_s + s * BW_BIAS_BYTES;
-            if (DKV) {  // column = query row of the tile, lanes read consecutive keys
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                bv[i] = __bfloat162float(*reinterpret_cast<const bf16*>(tile + (half * HC + c + i) * (BW_R * 2) + row * 2));
-            } else {  // eight keys of this thread's query: one swizzled 16-byte chunk
-              const uint4 u = *reinterpret_cast<const uint4*>(tile + row * 128 + ((((half * HC + c) >> 3) ^ (row & 7)) << 4));
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                bv[2 * i] = __uint_as_float(w[i] << 16);
-                bv[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-              }
-            }
-          }
+          if (BIAS == 2 && (c & 7) == 0) bw_bias8<DKV>(bias_s + s * BW_BIAS_BYTES, row, half * HC + c, bv);
           if (BIAS == 1 && (c & 7) == 0)
             load_bias8(p.bias, p.bias_kind, bias_base + (long long)(col0 + c) * bias_step, bias_step, ri < row_limit ? col_limit - col0 - c : 0,
                        !DKV && p.bias_vec, bv);
@@ -423,18 +463,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
           if (BIAS && !DKV && p.dbias) {  // d(bias) = P (dP - delta) = dS / scale; pairs that are masked or out of range contribute nothing
             db[c & 3] = p0 != 0.f ? g0 * p.inv_scale : 0.f;
             db[(c & 3) + 1] = p1 != 0.f ? g1 * p.inv_scale : 0.f;
-            if ((c & 3) == 2 && ri < row_limit) {
-              const int c4 = c - 2;
-              float* dst = p.dbias + bias_base + (long long)(col0 + c4) * bias_step;
-              if (p.bias_vec && col0 + c4 + 4 <= col_limit) {
-                // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
-              } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                  if (db[i] != 0.f && col0 + c4 + i < col_limit) atomicAdd(dst + i * bias_step, db[i]);
-              }
-            }
+            if ((c & 3) == 2 && ri < row_limit) bw_add_dbias(p, bias_base, col0 + c - 2, db);
           }
           if (DKV) pp[c >> 1] = pack_bf16x2(p0, p1);
           ds[c >> 1] = pack_bf16x2(g0, g1);
@@ -467,7 +496,6 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
         bf16* base = a == 0 ? p.out0 : p.out1;
         const long long sb = a == 0 ? p.o0_sb : p.o1_sb, ss = a == 0 ? p.o0_ss : p.o1_ss, sh = a == 0 ? p.o0_sh : p.o1_sh;
         bf16* orow = base + b * sb + (long long)min(ri, limit - 1) * ss + (long long)o_head * sh + half * HD;
-        const bool vec = (reinterpret_cast<uintptr_t>(orow) & 15) == 0;
 #pragma unroll
         for (int c = 0; c < HD; c += 32) {
           uint32_t o[32];
@@ -478,23 +506,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[i] = 0u;
           }
-          if (ri < limit) {
-            if (vec) {
-#pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                uint4 v;
-                v.x = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-                v.y = pack_bf16x2(__uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
-                v.z = pack_bf16x2(__uint_as_float(o[i + 4]), __uint_as_float(o[i + 5]));
-                v.w = pack_bf16x2(__uint_as_float(o[i + 6]), __uint_as_float(o[i + 7]));
-                *reinterpret_cast<uint4*>(orow + c + i) = v;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; i += 2)
-                *reinterpret_cast<uint32_t*>(orow + c + i) = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-            }
-          }
+          if (ri < limit) bw_store_row(orow + c, o);
         }
       }
     }
@@ -791,15 +803,15 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         alive = false;
       }
       if (part < 2 * DB) {
-      const uint8_t* block = (part / DB ? r2_s : r1_s) + (part % DB) * FA_BLOCK_BYTES;
-      uint32_t w[32];
+        const uint8_t* block = (part / DB ? r2_s : r1_s) + (part % DB) * FA_BLOCK_BYTES;
+        uint32_t w[32];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint4 u = *reinterpret_cast<const uint4*>(block + row * 128 + ((c ^ (row & 7)) << 4));
-        w[4 * c] = u.x; w[4 * c + 1] = u.y; w[4 * c + 2] = u.z; w[4 * c + 3] = u.w;
-      }
-      __syncwarp();
-      tmem_st_x32(t_lane + RES_COL + part * 32, w);
+        for (int c = 0; c < 8; ++c) {
+          const uint4 u = *reinterpret_cast<const uint4*>(block + row * 128 + ((c ^ (row & 7)) << 4));
+          w[4 * c] = u.x; w[4 * c + 1] = u.y; w[4 * c + 2] = u.z; w[4 * c + 3] = u.w;
+        }
+        __syncwarp();
+        tmem_st_x32(t_lane + RES_COL + part * 32, w);
       }
       tmem_st_wait();
       tc_fence_before();
@@ -842,18 +854,8 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
           __syncwarp();
           if (lane == 0) mbar_arrive(s_done);
         }
-        // columns [lo, hi) are visible pairs; only steps that touch the diagonal or an end have others (decided per warp)
-        int lo = 0, hi = HC;
-        if (DKV) {
-          if (ri >= p.sk) hi = 0;
-          if (p.causal) lo = max(0, ri - shift - col0);  // query >= key - shift
-        } else {
-          hi = min(HC, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
-        }
-        uint32_t visible = 0xffffffffu;
-        if (lo > 0) visible = lo < HC ? visible << lo : 0u;
-        if (hi < HC) visible = hi > 0 ? visible & (0xffffffffu >> (HC - hi)) : 0u;
-        const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);
+        const uint32_t visible = bw_visible<DKV>(p, ri, shift, col0);
+        const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);  // (per warp)
 #pragma unroll
         for (int c = 0; c < HC; c += 4) {
           const float4 l = DKV ? *reinterpret_cast<const float4*>(neg_lse + c) : make_float4(my_lse2, my_lse2, my_lse2, my_lse2);
@@ -861,19 +863,8 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
             if (BIAS == 1) {
               load_bias8(p.bias, p.bias_kind, bias_base + (long long)(col0 + c) * bias_step, bias_step, ri < row_limit ? col_limit - col0 - c : 0,
                          !DKV && p.bias_vec, bv);
-            } else if (DKV) {  // column = query row of the tile, lanes read consecutive keys
-              const uint8_t* tile = bias_s + (n % BWW_S1) * BWW_BIAS + (part * HC + c) * (BW_R * 2) + row * 2;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) bv[i] = __bfloat162float(*reinterpret_cast<const bf16*>(tile + i * (BW_R * 2)));
-            } else {  // eight keys of this thread's query: one swizzled 16-byte chunk
-              const uint8_t* block = bias_s + (n % BWW_S1) * BWW_BIAS + (part >> 1) * FA_BLOCK_BYTES;
-              const uint4 u = *reinterpret_cast<const uint4*>(block + row * 128 + ((((part & 1) * 4 + (c >> 3)) ^ (row & 7)) << 4));
-              const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                bv[2 * i] = __uint_as_float(w4[i] << 16);
-                bv[2 * i + 1] = __uint_as_float(w4[i] & 0xFFFF0000u);
-              }
+            } else {
+              bw_bias8<DKV>(bias_s + (n % BWW_S1) * BWW_BIAS, row, part * HC + c, bv);
             }
           }
           float x0, x1, x2, x3;
@@ -923,15 +914,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
           // d(bias) = P (dP - delta) = dS / scale; pairs that are masked or out of range contribute nothing
           const float db[4] = {pr[c] != 0.f ? g0 * p.inv_scale : 0.f, pr[c + 1] != 0.f ? g1 * p.inv_scale : 0.f, pr[c + 2] != 0.f ? g2 * p.inv_scale : 0.f,
                                pr[c + 3] != 0.f ? g3 * p.inv_scale : 0.f};
-          float* dst = p.dbias + bias_base + (long long)(col0 + c) * bias_step;
-          if (p.bias_vec && col0 + c + 4 <= col_limit) {
-            // the batches (and whatever else the bias broadcasts over) add into one buffer: four keys per reduction
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(db[0]), "f"(db[1]), "f"(db[2]), "f"(db[3]) : "memory");
-          } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (db[i] != 0.f && col0 + c + i < col_limit) atomicAdd(dst + i * bias_step, db[i]);
-          }
+          bw_add_dbias(p, bias_base, col0 + c, db);
         }
         packed[c >> 1] = pack_bf16x2(g0, g1);
         packed[(c >> 1) + 1] = pack_bf16x2(g2, g3);
@@ -952,8 +935,6 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         bf16* base = a == 0 ? p.out0 : p.out1;
         const long long sb = a == 0 ? p.o0_sb : p.o1_sb, ss = a == 0 ? p.o0_ss : p.o1_ss, sh = a == 0 ? p.o0_sh : p.o1_sh;
         bf16* orow = base + b * sb + (long long)min(ri, limit - 1) * ss + (long long)o_head * sh + part * HD;
-        const bool vec = (reinterpret_cast<uintptr_t>(orow) & 15) == 0;
-        const bool sectors = (reinterpret_cast<uintptr_t>(orow) & 31) == 0;
         uint32_t o[HD];
         if (n_steps > 0) {
           __syncwarp();
@@ -965,29 +946,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
 #pragma unroll
           for (int i = 0; i < HD; ++i) o[i] = 0u;
         }
-        if (ri < limit) {
-          if (sectors) {
-            uint32_t w[HD / 2];
-#pragma unroll
-            for (int i = 0; i < HD / 2; ++i) w[i] = pack_bf16x2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1]));
-#pragma unroll
-            for (int i = 0; i < HD / 2; i += 8) st_global_v8(orow + 2 * i, w + i);
-          } else if (vec) {
-#pragma unroll
-            for (int i = 0; i < HD; i += 8) {
-              uint4 v;
-              v.x = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-              v.y = pack_bf16x2(__uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
-              v.z = pack_bf16x2(__uint_as_float(o[i + 4]), __uint_as_float(o[i + 5]));
-              v.w = pack_bf16x2(__uint_as_float(o[i + 6]), __uint_as_float(o[i + 7]));
-              *reinterpret_cast<uint4*>(orow + i) = v;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < HD; i += 2)
-              *reinterpret_cast<uint32_t*>(orow + i) = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-          }
-        }
+        if (ri < limit) bw_store_row(orow, o);
       }
     }
   }
@@ -1039,10 +998,10 @@ static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtenso
 //   head_dim 128 with a bias: 64, the wide rings leave no room for it.
 //   head_dim 128: 64 for a sequence that ends in the first half of its first, second or third wide step (32 heads: 1 x 33 12.2 / 13.4, 8 x 150
 //   52.7 / 54.8, 2 x 300 32.0 / 33.2); from the fourth on wide steps win all the same (2 x 420 41.9 / 41.2, 4 x 700 133 / 128).
-//   head_dim 64, the same line (32 heads: 4 x 33 12.5 / 14.8, 8 x 150 38.6 / 44.4, 8 x 300 65.4 / 73.3), and with 64 heads x batches and more, where
-//   two CTAs of the 64-row kernel share an SM, up to the fifth (32 heads: 2 x 420 33.9 / 34.8, 16 x 420 191 / 202, 2 x 576 3 % and
+//   head_dim 64, the same line (32 heads: 4 x 33 12.5 / 14.8, 8 x 150 38.6 / 44.4, 8 x 300 65.4 / 73.3), and with 64 heads x batches and more, several
+//   rounds of CTAs, up to the fifth (32 heads: 2 x 420 33.9 / 34.8, 16 x 420 191 / 202, 2 x 576 3 % and
 //   1 x 576 -4 %; 4 x 420, 12 heads 33.5 / 30.9).  At six steps either may be 3 % ahead.
-//   head_dim 64, one or two whole steps of very many heads: fill and drain of a CTA count (32 heads: 16 x 100 38.6 / 40.9, 4 x 100 14.2 / 14.2).
+//   head_dim 64, one or two whole steps of very many heads: the smaller CTA's shorter fill and drain, many times over (32 heads: 16 x 100 38.6 / 40.9, 4 x 100 14.2 / 14.2).
 //   head_dim 64 with a bias: 64 only for up to 64 rows (32 heads: 4 x 64 10 %, with a padding mask 7 % longer in wide steps); beyond, the wide
 //   kernel's warps, twice as many per bias element, decide (4 x 300 0.79 of the time, 2 x 900 0.71, with a mask 0.76 and 0.64).
 static int step_rows(int head_dim, int bias_mode, int streamed, int heads, int batch) {
