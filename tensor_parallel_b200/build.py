@@ -87,10 +87,11 @@ def build_autograd(force: bool = False) -> Path:
     return AUTOGRAD_PATH
 
 
-def build(force: bool = False, verbose: bool = False, lib_path: Path = None, extra_flags=()) -> Path:
+def build(force: bool = False, verbose: bool = False, lib_path: Path = None, extra_flags=(), autograd: bool = True) -> Path:
     """Builds what is out of date.  ``lib_path`` / ``extra_flags`` make a variant of the library somewhere else (its
     objects live beside it), e.g. ``-DTPB_GEMM_TRACE`` for the kernel-internal phase trace or ``-DTPB_BOUNDS`` for the
-    in-kernel bounds checks; ``TPB_LIB_PATH`` makes ``ops.native`` load such a variant."""
+    in-kernel bounds checks; ``TPB_LIB_PATH`` makes ``ops.native`` load such a variant.  ``autograd=False`` leaves the autograd module alone,
+    which needs the headers of Python and torch."""
     nvcc = _nvcc()
     lib_path = Path(lib_path) if lib_path is not None else LIB_PATH
     obj_dir = OBJ_DIR if lib_path == LIB_PATH else lib_path.parent / (lib_path.stem + "_obj")
@@ -120,7 +121,8 @@ def build(force: bool = False, verbose: bool = False, lib_path: Path = None, ext
     newest_obj = max(os.path.getmtime(o) for o in objs)
     if force or jobs or not lib_path.exists() or lib_path.stat().st_mtime < newest_obj:
         run([nvcc, "-shared", "-o", str(lib_path), *objs, "-gencode", "arch=compute_100a,code=sm_100a"])
-    build_autograd(force and lib_path == LIB_PATH)  # (it serves every variant of the library)
+    if autograd:
+        build_autograd(force and lib_path == LIB_PATH)  # (it serves every variant of the library)
     return lib_path
 
 

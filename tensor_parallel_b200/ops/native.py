@@ -31,7 +31,7 @@ def _load() -> ctypes.CDLL:
         return ctypes.CDLL(variant)
     path = _build.LIB_PATH
     if not path.exists() or os.environ.get("TPB_REBUILD"):
-        _build.build()  # explicit rebuilds otherwise: python -m tensor_parallel_b200.build
+        _build.build(autograd=False)  # explicit rebuilds otherwise: python -m tensor_parallel_b200.build
     return ctypes.CDLL(str(path))
 
 

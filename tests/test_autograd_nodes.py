@@ -373,6 +373,18 @@ def test_without_a_compiler_the_python_nodes_serve(python_nodes, monkeypatch, tm
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
+def test_an_import_that_builds_the_library_does_without_the_module(compiler, monkeypatch, tmp_path):
+    """Where its headers are missing, the library is built and loaded all the same."""
+    from tensor_parallel_b200.ops import native
+
+    monkeypatch.setattr(build, "LIB_PATH", tmp_path / "libnew.so")
+    monkeypatch.setattr(build, "OBJ_DIR", tmp_path / "obj")
+    monkeypatch.setattr(build, "build_autograd", lambda *a: (_ for _ in ()).throw(RuntimeError("Python.h: No such file")))
+    monkeypatch.setattr(native.ctypes, "CDLL", lambda path: path)
+    monkeypatch.delenv("TPB_LIB_PATH", raising=False)
+    assert native._load() == str(tmp_path / "libnew.so")
+
+
 def test_a_library_of_another_layout_is_refused(nodes):
     library = SimpleNamespace(tpb_api_layout=ctypes.CFUNCTYPE(ctypes.c_ulonglong)(lambda: nodes.AUTOGRAD.layout() + 1))
     with pytest.raises(RuntimeError, match="rebuild"):
