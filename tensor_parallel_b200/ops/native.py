@@ -397,7 +397,7 @@ class _LinearFn(torch.autograd.Function):
 
 
 def linear(x, weight, bias=None):
-    if AUTOGRAD is None or torch.jit.is_tracing():
+    if AUTOGRAD is None or torch._C._is_tracing():
         return _LinearFn.apply(x, weight, bias)
     return AUTOGRAD.linear(x, weight, bias)
 
@@ -463,7 +463,7 @@ class _NormFn(torch.autograd.Function):
 
 
 def _norm(x, weight, bias, eps, mode):
-    if AUTOGRAD is None or torch.jit.is_tracing():
+    if AUTOGRAD is None or torch._C._is_tracing():
         return _NormFn.apply(x, weight, bias, eps, mode)
     return AUTOGRAD.norm(x, weight, bias, eps, mode)
 
