@@ -530,7 +530,7 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 // bias) and two of the other.  Shared memory at head_dim 128: 64 KB resident + 160 KB streamed + statistics, which leaves no room for a
 // bias.  What bounds it: the chain of a step, S -> P -> dV and dP -> dS -> dK through one buffer each, and fill and drain of a CTA; the tensor pipe is active
 // for 47 % (dQ 50 %) of the causal launch below.  (Next would be shared memory: 192 KB read and 64 KB filled per 2048 clocks of dK / dV products.)
-// Whole backward, 4 x 2048 tokens, 32 heads of 128: causal 558 -> 501 us, without a mask 884 -> 793; 1 x 1000 76 -> 74 us.
+// Whole backward, 32 heads of 128: 4 x 2048 causal 558 -> 507 us, 2 x 2080 344 -> 323, without a mask 560 -> 518; 1 x 1000 65.7 -> 61.3.
 // Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.  Short and ragged sequences: step_rows.
 constexpr int BWW_WARPS = 16;                            // elementwise warps
 constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
