@@ -654,6 +654,387 @@ attn_decode_fused_kernel(const bf16* q, const bf16* k, const bf16* v,
   }
 }
 
+// The same step for four or more query heads per KV head, on tensor cores: the heads of a group are the rows of an m16n8k16 MMA, keys
+// (for the scores) and head elements (for the output) its columns.  Head by head on the CUDA cores, every key costs about 45 instructions
+// per query head and four keys, and the kernel above is bound by them (16 sequences x 1024 keys, 128 / 8 heads of 64: 57 us for 34 MB).
+// A warp takes 16 keys per iteration from a ring of its own (cp.async; keys past the end arrive as zeros, the new key is put into its row of
+// the last tile), keeps its own running maximum and sum, and the warps' results are merged at the end.  Nothing is held in fewer bits
+// than on the CUDA cores: q, K and V are bf16 numbers as they are, and a probability enters as the exact sum of three bf16 numbers (8 bits
+// each, fp32 has 24), in three MMAs.  Only where a result is not finite - 0 * inf in one of the three parts is NaN - the CTA does its keys
+// again on the CUDA cores.  Partial results against 64 bits, 16 heads of 64, 30 / 1000 / 4000 keys: 1.2 / 2.2 / 2.8e-7 of the result on the CUDA
+// cores, 1.0 / 1.8 / 2.1e-7 here (two bf16 numbers per probability: 2e-6).  Replayed from a CUDA graph, caches in memory: 16 x 1024 keys, 128 / 8 heads of
+// 64 57 -> 13 us; 8 x 2048, 32 / 8 heads of 128 54 -> 22 us; 16 x 2048, 40 / 10 heads of 128 165 -> 48 us; 20 keys, 128 / 8 heads of 64 9.7 -> 7.4 us, four
+// heads of 64 6.0 -> 5.3 us, 8 x 60 keys of them 6.4 -> 6.7 us (the worst of 100 shapes).
+template <int D>
+struct GqaShape {
+  static constexpr int WARPS = D == 64 ? 8 : 4, THREADS = WARPS * 32, STAGES = 3, KEYS = 16;
+  static constexpr int TILE = KEYS * D;                                                  // elements of K or V of one stage
+  static constexpr size_t RING = size_t(WARPS) * STAGES * 2 * TILE * sizeof(bf16);      // 96 KB: two CTAs per SM
+  static constexpr int OUT_LD = D + 8;  // fp32 row pitch of the warps' outputs, which are merged in the ring (rows on different banks)
+  static_assert(RING >= size_t(WARPS) * 16 * OUT_LD * sizeof(float), "the warps' outputs fit the ring");
+};
+
+template <int D>
+__global__ void __launch_bounds__(GqaShape<D>::THREADS, 2)
+attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __restrict__ kcache, bf16* __restrict__ vcache, bf16* __restrict__ out,
+                       float* __restrict__ part_o, float* __restrict__ part_ml, uint32_t* __restrict__ counters, const int* __restrict__ pos_ptr,
+                       int q_heads, int kv_heads, int g_total, int g_offset, int max_seq, int splits, float scale_log2e, int rotary_dim,
+                       float log2_theta, int interleaved, long long q_ld, long long k_ld, long long v_ld, const float2* __restrict__ rope_table,
+                       long long out_ld, int early) {
+  using S = GqaShape<D>;
+  if (!early) pdl_wait();  // (see attn_decode_fused_kernel)
+  const int bh = blockIdx.x;
+  const int b = bh / kv_heads, kvh = bh % kv_heads;
+  const int split = blockIdx.y;
+  g_offset += blockIdx.z * 16;
+  const int heads = min(16, g_total - g_offset);
+  counters += (size_t)blockIdx.z * gridDim.x;
+  const int pos = pos_ptr[0];
+  const int len = min(pos + 1, max_seq);
+  const int chunk = (len + splits - 1) / splits;
+  const int k0 = split * chunk, k1 = min(len, k0 + chunk);
+  const bool owns_new = pos < max_seq && pos >= k0 && pos < k1;
+  const int k1_cache = owns_new ? pos : k1;  // keys taken from the cache
+
+  extern __shared__ uint4 dec_ring[];
+  __shared__ __align__(16) bf16 q_s[16 * D];
+  __shared__ __align__(16) bf16 knew_s[D], vnew_s[D];
+  __shared__ float red_m[S::WARPS][16], red_l[S::WARPS][16];
+  __shared__ uint32_t is_last;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = rotary_dim >> 1;
+  bf16* ring = reinterpret_cast<bf16*>(dec_ring) + warp * S::STAGES * 2 * S::TILE;
+  const bf16* kbase = kcache + (long long)bh * max_seq * D;
+  const bf16* vbase = vcache + (long long)bh * max_seq * D;
+  auto issue = [&](int stage, int key0) {
+    constexpr int CH = D / 8;
+    bf16* kt = ring + stage * 2 * S::TILE;
+#pragma unroll
+    for (int i = 0; i < S::KEYS * CH / 32; ++i) {
+      const int r = (i * 32 + lane) / CH, c = (i * 32 + lane) % CH;
+      const bool ok = key0 + r < k1_cache;
+      const long long off = (long long)(ok ? key0 + r : 0) * D + c * 8;
+      cp_async16(tile_ptr<D>(kt, r, c), kbase + off, ok);
+      cp_async16(tile_ptr<D>(kt + S::TILE, r, c), vbase + off, ok);
+    }
+    cp_async_commit();
+  };
+  constexpr int STEP = S::WARPS * S::KEYS;
+  int key0 = k0 + warp * S::KEYS;
+#pragma unroll
+  for (int st = 0; st < S::STAGES - 1; ++st) issue(st, key0 + st * STEP);
+
+  // ---- q and the new key rotated, as in attn_decode_fused_kernel; q stays bf16, the scale goes onto the scores ----
+  if (early) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  static_assert(D <= S::THREADS, "one element of v per thread");
+  const float v_new = threadIdx.x < D ? bf16_bits_to_float(ld_after_wait_u16(v + b * v_ld + (long long)kvh * D + threadIdx.x)) : 0.f;
+  // element pairs (D / 2 per head, the key last), four per thread on their way at once
+  constexpr int PAIRS = 4;
+  for (int i0 = threadIdx.x; i0 < (heads + 1) * (D / 2); i0 += PAIRS * S::THREADS) {
+    float x[PAIRS], y[PAIRS], cs[PAIRS], sn[PAIRS];
+    int ea[PAIRS], eb[PAIRS];
+#pragma unroll
+    for (int u = 0; u < PAIRS; ++u) {
+      const int i = i0 + u * S::THREADS;
+      const int hsel = i / (D / 2), pr = i % (D / 2);
+      if (hsel > heads) break;
+      const bf16* src = hsel == heads ? k + b * k_ld + (long long)kvh * D : q + b * q_ld + (long long)(kvh * g_total + g_offset + hsel) * D;
+      if (pr < half) {
+        ea[u] = interleaved ? 2 * pr : pr;
+        eb[u] = interleaved ? 2 * pr + 1 : pr + half;
+        if (rope_table) {
+          const float2 t = __ldg(rope_table + (long long)pos * half + pr);
+          cs[u] = t.x;
+          sn[u] = t.y;
+        } else {
+          const float inv_freq = exp2f(-log2_theta * (2.f * float(pr) / float(rotary_dim)));
+          sincosf(float(pos) * inv_freq, &sn[u], &cs[u]);
+        }
+      } else {
+        ea[u] = rotary_dim + 2 * (pr - half);
+        eb[u] = ea[u] + 1;
+      }
+      x[u] = bf16_bits_to_float(ld_after_wait_u16(src + ea[u]));
+      y[u] = bf16_bits_to_float(ld_after_wait_u16(src + eb[u]));
+    }
+#pragma unroll
+    for (int u = 0; u < PAIRS; ++u) {
+      const int hsel = (i0 + u * S::THREADS) / (D / 2);
+      if (hsel > heads) break;
+      float ra = x[u], rb = y[u];
+      if ((i0 + u * S::THREADS) % (D / 2) < half) {
+        ra = x[u] * cs[u] - y[u] * sn[u];
+        rb = y[u] * cs[u] + x[u] * sn[u];
+      }
+      if (hsel == heads) {
+        knew_s[ea[u]] = __float2bfloat16(ra);
+        knew_s[eb[u]] = __float2bfloat16(rb);
+      } else {
+        tile_ptr<D>(q_s, hsel, ea[u] >> 3)[ea[u] & 7] = __float2bfloat16(ra);
+        tile_ptr<D>(q_s, hsel, eb[u] >> 3)[eb[u] & 7] = __float2bfloat16(rb);
+      }
+    }
+  }
+  for (int i = heads * (D / 8) + threadIdx.x; i < 16 * (D / 8); i += S::THREADS)
+    *reinterpret_cast<uint4*>(tile_ptr<D>(q_s, i / (D / 8), i % (D / 8))) = make_uint4(0, 0, 0, 0);
+  if (threadIdx.x < D) vnew_s[threadIdx.x] = __float2bfloat16(v_new);
+  __syncthreads();
+  if (owns_new && blockIdx.z == 0) {  // persist the new key / value for later steps
+    for (int i = threadIdx.x; i < D; i += S::THREADS) {
+      kcache[((long long)bh * max_seq + pos) * D + i] = knew_s[i];
+      vcache[((long long)bh * max_seq + pos) * D + i] = vnew_s[i];
+    }
+  }
+
+  // fragments: rows g and g + 8 of the 16 heads, columns 2 t and 2 t + 1 of a tile of eight
+  const int g = lane >> 2, t4 = lane & 3, id = lane >> 3, r8 = lane & 7;
+  uint32_t qf[D / 16][4];
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) ldmatrix_x4(qf[ks], tile_ptr<D>(q_s, (id & 1) * 8 + r8, ks * 2 + (id >> 1)));
+  float o[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[n][j] = 0.f;
+
+  auto step = [&](bf16* kt, bf16* vt, int valid) {  // `valid` (1 to 16) keys of the tile count
+    float sc[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sc[n][j] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+      uint32_t kb[4];
+      ldmatrix_x4(kb, tile_ptr<D>(kt, (id >> 1) * 8 + r8, ks * 2 + (id & 1)));
+      mma_bf16_16816(sc[0], qf[ks], kb[0], kb[1]);
+      mma_bf16_16816(sc[1], qf[ks], kb[2], kb[3]);
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sc[n][j] = n * 8 + 2 * t4 + (j & 1) < valid ? sc[n][j] * scale_log2e : -INFINITY;
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      float mx = fmaxf(fmaxf(sc[0][2 * hh], sc[0][2 * hh + 1]), fmaxf(sc[1][2 * hh], sc[1][2 * hh + 1]));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float m_new = fmaxf(m[hh], mx);
+      const float corr = exp2f(m[hh] - m_new);
+      m[hh] = m_new;
+      l[hh] *= corr;
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          sc[n][2 * hh + j] = exp2f(sc[n][2 * hh + j] - m_new);
+          l[hh] += sc[n][2 * hh + j];
+        }
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) {
+        o[n][2 * hh] *= corr;
+        o[n][2 * hh + 1] *= corr;
+      }
+    }
+    uint32_t part[3][4];  // p = part[0] + part[1] + part[2]: what the first two leave has 8 bits at most
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // {keys 0-7, rows g}, {0-7, g + 8}, {8-15, g}, {8-15, g + 8}
+      float p0 = sc[i >> 1][(i & 1) * 2], p1 = sc[i >> 1][(i & 1) * 2 + 1];
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        part[u][i] = pack_bf16x2(p0, p1);
+        p0 -= __uint_as_float(part[u][i] << 16);
+        p1 -= __uint_as_float(part[u][i] & 0xFFFF0000u);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < D / 16; ++n) {
+      uint32_t vb[4];
+      ldmatrix_x4_trans(vb, tile_ptr<D>(vt, (id & 1) * 8 + r8, n * 2 + (id >> 1)));
+      // the tile's sum first, then an fp32 addition that rounds to nearest: the MMA's own additions cut off what does not fit, which over
+      // 2000 keys in one accumulator came to 4.5e-7 of the result (the kernel above: 2.4e-7)
+      float t[2][4] = {};
+#pragma unroll
+      for (int u = 2; u >= 0; --u) {  // (the small parts first)
+        mma_bf16_16816(t[0], part[u], vb[0], vb[1]);
+        mma_bf16_16816(t[1], part[u], vb[2], vb[3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        o[2 * n][j] += t[0][j];
+        o[2 * n + 1][j] += t[1][j];
+      }
+    }
+  };
+  for (int it = 0; key0 < k1; key0 += STEP, ++it) {
+    issue((it + S::STAGES - 1) % S::STAGES, key0 + (S::STAGES - 1) * STEP);
+    cp_async_wait_group<S::STAGES - 1>();
+    __syncwarp();  // (the lanes read what others have copied)
+    bf16* kt = ring + (it % S::STAGES) * 2 * S::TILE;
+    if (owns_new && pos - key0 < S::KEYS) {  // (the last tile of the last split: its last key is the new one)
+      for (int c = lane; c < D / 8; c += 32) {
+        *reinterpret_cast<uint4*>(tile_ptr<D>(kt, pos - key0, c)) = reinterpret_cast<const uint4*>(knew_s)[c];
+        *reinterpret_cast<uint4*>(tile_ptr<D>(kt + S::TILE, pos - key0, c)) = reinterpret_cast<const uint4*>(vnew_s)[c];
+      }
+      __syncwarp();
+    }
+    step(kt, kt + S::TILE, min(S::KEYS, k1 - key0));
+    __syncwarp();  // nobody copies over this stage before all have read it
+  }
+  cp_async_wait_group<0>();
+
+  // ---- merge the warps ----
+  float finite = 0.f;
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) finite += o[n][j] * 0.f;
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    finite += l[hh] * 0.f;
+    l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 1);
+    l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 2);
+    if (t4 == 0) {
+      red_m[warp][g + 8 * hh] = m[hh];
+      red_l[warp][g + 8 * hh] = l[hh];
+    }
+  }
+  const bool again = __syncthreads_or(finite != 0.f);  // (NaN != 0; every ring has been read)
+  float* red_o = reinterpret_cast<float*>(dec_ring);  // [warp][16 heads][D]
+  int warps = min(S::WARPS, (k1 - k0 + S::KEYS - 1) / S::KEYS);  // (those that had keys; below 1: an empty split)
+  if (!again) {
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      if (g + 8 * hh >= heads) continue;
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n)
+        *reinterpret_cast<float2*>(red_o + (warp * 16 + g + 8 * hh) * S::OUT_LD + n * 8 + 2 * t4) = make_float2(o[n][2 * hh], o[n][2 * hh + 1]);
+    }
+  } else {  // a key at a time per warp, head by head
+    warps = S::WARPS;
+    for (int h = 0; h < heads; ++h) {
+      float qv[D / 32], acc[D / 32], mh = -INFINITY, lh = 0.f;
+#pragma unroll
+      for (int e = 0; e < D / 32; ++e) {
+        const int at = e * 32 + lane;
+        qv[e] = __bfloat162float(tile_ptr<D>(q_s, h, at >> 3)[at & 7]) * scale_log2e;
+        acc[e] = 0.f;
+      }
+      for (int key = k0 + warp; key < k1; key += S::WARPS) {
+        const bool fresh = owns_new && key == pos;
+        const bf16* kr = fresh ? knew_s : kbase + (long long)key * D;
+        const bf16* vr = fresh ? vnew_s : vbase + (long long)key * D;
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < D / 32; ++e) s += __bfloat162float(kr[e * 32 + lane]) * qv[e];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        const float m_new = fmaxf(mh, s), base = m_new == -INFINITY ? 0.f : m_new;  // (keys masked by scores of -inf so far)
+        const float corr = exp2f(mh - base), pexp = exp2f(s - base);
+        lh = lh * corr + pexp;
+#pragma unroll
+        for (int e = 0; e < D / 32; ++e) acc[e] = acc[e] * corr + pexp * __bfloat162float(vr[e * 32 + lane]);
+        mh = m_new;
+      }
+#pragma unroll
+      for (int e = 0; e < D / 32; ++e) red_o[(warp * 16 + h) * S::OUT_LD + e * 32 + lane] = acc[e];
+      if (lane == 0) {
+        red_m[warp][h] = mh;
+        red_l[warp][h] = lh;
+      }
+    }
+  }
+  __syncthreads();
+  // four elements per thread: a group of four heads of 128 is one round of the CTA
+  auto store = [&](int qh, int d, float4 x, float ll) {
+    bf16* dst = out + (long long)b * out_ld + (long long)qh * D + d;
+    dst[0] = __float2bfloat16(ll > 0.f ? x.x / ll : 0.f);
+    dst[1] = __float2bfloat16(ll > 0.f ? x.y / ll : 0.f);
+    dst[2] = __float2bfloat16(ll > 0.f ? x.z / ll : 0.f);
+    dst[3] = __float2bfloat16(ll > 0.f ? x.w / ll : 0.f);
+  };
+  auto add = [](float4& acc, const float4& x, float c) {
+    acc.x += x.x * c;
+    acc.y += x.y * c;
+    acc.z += x.z * c;
+    acc.w += x.w * c;
+  };
+  for (int i = threadIdx.x; i < heads * (D / 4); i += S::THREADS) {
+    const int h = i / (D / 4), d = i % (D / 4) * 4;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < S::WARPS; ++w)
+      if (w < warps) mm = fmaxf(mm, red_m[w][h]);
+    float ll = 0.f;
+    float4 oo = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < S::WARPS; ++w) {
+      if (w >= warps) continue;
+      const float c = red_m[w][h] == -INFINITY ? 0.f : exp2f(red_m[w][h] - mm);
+      ll += red_l[w][h] * c;
+      add(oo, *reinterpret_cast<const float4*>(red_o + (w * 16 + h) * S::OUT_LD + d), c);
+    }
+    const int qh = kvh * g_total + g_offset + h;
+    const long long row = (long long)b * q_heads + qh;
+    if (splits == 1) {
+      store(qh, d, oo, ll);
+    } else {
+      *reinterpret_cast<float4*>(part_o + (row * splits + split) * D + d) = oo;
+      if (d == 0) { part_ml[(row * splits + split) * 2] = mm; part_ml[(row * splits + split) * 2 + 1] = ll; }
+    }
+  }
+  if (splits == 1) return;
+  // last split to arrive merges the partial results of all splits
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint32_t old = atomicAdd(counters + bh, 1u);
+    const bool last = old == uint32_t(splits - 1);
+    if (last) counters[bh] = 0;
+    is_last = last ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < heads * (D / 4); i += S::THREADS) {
+    const int h = i / (D / 4), d = i % (D / 4) * 4;
+    const int qh = kvh * g_total + g_offset + h;
+    const long long row = (long long)b * q_heads + qh;
+    // (all loads of a batch of eight splits before the first use, as in attn_decode_fused_kernel)
+    float mm = -INFINITY, ll = 0.f;
+    float4 oo = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      float2 ml[8];
+      float4 os[8];
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8) {
+        const bool live = s0 + q8 < splits;
+        const long long pr = row * splits + s0 + q8;
+        ml[q8] = live ? make_float2(__ldcg(part_ml + pr * 2), __ldcg(part_ml + pr * 2 + 1)) : make_float2(-INFINITY, 0.f);
+        os[q8] = live ? __ldcg(reinterpret_cast<const float4*>(part_o + pr * D + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      float m_new = mm;
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8) m_new = fmaxf(m_new, ml[q8].x);
+      const float c_old = mm == -INFINITY ? 0.f : exp2f(mm - m_new);
+      ll *= c_old;
+      oo = make_float4(oo.x * c_old, oo.y * c_old, oo.z * c_old, oo.w * c_old);
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8) {
+        const float c = ml[q8].x == -INFINITY ? 0.f : exp2f(ml[q8].x - m_new);
+        ll += ml[q8].y * c;
+        add(oo, os[q8], c);
+      }
+      mm = m_new;
+    }
+    store(qh, d, oo, ll);
+  }
+}
+
 // table[pos * (rotary_dim / 2) + p] = (cos, sin)(pos * theta^(-2p / rotary_dim)), the angles of the rotary embedding
 __global__ void rope_table_kernel(float2* __restrict__ table, int positions, int half, int rotary_dim, float log2_theta) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1027,27 +1408,41 @@ extern "C" int tpb_attn_decode_fused(const void* q, const void* k, const void* v
   const float sl2 = scale * 1.4426950408889634f;
   const float l2t = log2f(theta);
   int done = 0, launches = 0;
+  // four heads and more fill a quarter and more of the rows of an MMA; below that the rows that would be empty cost more than they bring
+  const bool tensor = g_total >= 4 && !(reinterpret_cast<uintptr_t>(part_o) & 15);
   while (done < g_total) {
     const int left = g_total - done;
-    const int gmax = head_dim == 128 ? 4 : 8;
-    int gnow = 1;
-    while (gnow * 2 <= left && gnow * 2 <= gmax) gnow *= 2;
+    const int gnow = tensor ? 16 : (left >= 2 ? 2 : 1);  // (larger groups come here only with partials off a 16-byte boundary)
     // equal groups share one launch (grid z) when the caller's counter array has a counter for each of them
-    int reps = left / gnow;
+    int reps = tensor ? (left + 15) / 16 : left / gnow;
     if (splits > 1 && (long long)batch * kv_heads * reps > counter_elems) reps = 1;
     dim3 grid(batch * kv_heads, splits, reps);
-#define DECF(D, G)                                                                                                           \
-  if (!dec_smem_ready<attn_decode_fused_kernel<D, G>>(dec_ring_bytes<D>() + DEC_EARLY_PAD)) return TPB_ERR_CUDA;                               \
-  launch_dependent(attn_decode_fused_kernel<D, G>, grid, dim3(DEC_THREADS), dec_ring_bytes<D>() + (early && first ? DEC_EARLY_PAD : 0), s, first && (early || pdl_enabled()), (const bf16*)q, (const bf16*)k, (const bf16*)v, \
-                (bf16*)kcache, (bf16*)vcache, (bf16*)out, part_o, part_ml, (uint32_t*)counters, pos_ptr, q_heads, kv_heads, g_total, \
-                done, max_seq, splits, sl2, rotary_dim, l2t, interleaved, q_ld, k_ld, v_ld, (const float2*)rope_table, out_ld, (early && first) ? 1 : 0)
     const bool first = launches == 0;  // (a second group of heads follows the first group's launch, which writes the new cache row)
-    if (head_dim == 128) {
-      if (gnow == 1) { DECF(128, 1); } else if (gnow == 2) { DECF(128, 2); } else { DECF(128, 4); }
+    const bool ahead = early && first;
+    auto launch = [&](auto kernel, int threads, size_t smem) {
+      launch_dependent(kernel, grid, dim3(threads), smem, s, first && (early || pdl_enabled()), (const bf16*)q, (const bf16*)k, (const bf16*)v,
+                       (bf16*)kcache, (bf16*)vcache, (bf16*)out, part_o, part_ml, (uint32_t*)counters, pos_ptr, q_heads, kv_heads, g_total, done,
+                       max_seq, splits, sl2, rotary_dim, l2t, interleaved, q_ld, k_ld, v_ld, (const float2*)rope_table, out_ld, ahead ? 1 : 0);
+    };
+#define DECF(D, G)                                                                                                  \
+  do {                                                                                                              \
+    if (!dec_smem_ready<attn_decode_fused_kernel<D, G>>(dec_ring_bytes<D>() + DEC_EARLY_PAD)) return TPB_ERR_CUDA;  \
+    launch(attn_decode_fused_kernel<D, G>, DEC_THREADS, dec_ring_bytes<D>() + (ahead ? DEC_EARLY_PAD : 0));         \
+  } while (0)
+#define DECG(D)                                                                                   \
+  do {                                                                                            \
+    if (!dec_smem_ready<attn_decode_gqa_kernel<D>>(GqaShape<D>::RING)) return TPB_ERR_CUDA;       \
+    launch(attn_decode_gqa_kernel<D>, GqaShape<D>::THREADS, GqaShape<D>::RING);                   \
+  } while (0)
+    if (tensor) {
+      if (head_dim == 128) DECG(128); else DECG(64);
+    } else if (head_dim == 128) {
+      if (gnow == 1) DECF(128, 1); else DECF(128, 2);
     } else {
-      if (gnow == 1) { DECF(64, 1); } else if (gnow == 2) { DECF(64, 2); } else if (gnow == 4) { DECF(64, 4); } else { DECF(64, 8); }
+      if (gnow == 1) DECF(64, 1); else DECF(64, 2);
     }
 #undef DECF
+#undef DECG
     done += gnow * reps;
     ++launches;
   }

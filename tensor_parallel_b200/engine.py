@@ -196,8 +196,8 @@ class DecoderEngine:
         self.next_ids = torch.zeros(B, dtype=torch.int64, device=dev)
         self.rope_angles = native.rope_table(max_seq, spec.rotary_dim, self.theta, dev) if spec.rotary_dim else None
         # split the key range only when (batch x kv heads) alone cannot occupy the SMs
-        # (a KV head's query heads run in groups of up to 4 (head_dim 128) or 8 (64) per CTA, all groups in one launch)
-        ctas = B * self.nkv * math.ceil(self.nq / self.nkv / (4 if D == 128 else 8))
+        # (a KV head's query heads share a CTA, from 17 on in groups of 16, all groups in one launch)
+        ctas = B * self.nkv * math.ceil(self.nq / self.nkv / 16)
         self.splits = 1 if ctas >= 128 else max(1, min(8, math.ceil(256 / ctas)))
         self.attn_ws = (torch.empty(B * self.nq * self.splits * D, dtype=torch.float32, device=dev),
                         torch.empty(B * self.nq * self.splits * 2, dtype=torch.float32, device=dev),
