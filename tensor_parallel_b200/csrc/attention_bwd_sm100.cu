@@ -1013,21 +1013,6 @@ static int step_rows(int head_dim, int bias_mode, int streamed, int heads, int b
   return streamed <= 2 * BWW_T && rows >= 256 ? BW_T : BWW_T;
 }
 
-// Tensor map over a bf16 score bias [batch or 1][heads or 1][sq][sk] (keys contiguous); box = [rows queries][keys].
-static int bw_bias_tmap(CUtensorMap* map, const void* bias, int batch, int heads, int sq, int sk, long long sb, long long sh, long long sqs, int rows,
-                        int keys, bool swizzled) {
-  EncodeTiledFn fn = fa_encode_fn();
-  if (!fn) return TPB_ERR_DRIVER;
-  cuuint64_t dims[4] = {cuuint64_t(sk), cuuint64_t(sq), cuuint64_t(sh ? heads : 1), cuuint64_t(sb ? batch : 1)};
-  cuuint64_t strides[3] = {cuuint64_t(sqs) * 2, cuuint64_t(sh ? sh : sqs) * 2, cuuint64_t(sb ? sb : sqs) * 2};
-  cuuint32_t box[4] = {cuuint32_t(keys), cuuint32_t(rows), 1, 1}, estr[4] = {1, 1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(bias), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
-             ? TPB_OK
-             : TPB_ERR_TMAP;
-}
-
 }  // namespace tpb
 
 using namespace tpb;
@@ -1096,8 +1081,8 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   const int kv_rows = step_rows(head_dim, bias_mode, sq, kv_heads, batch), q_rows = step_rows(head_dim, bias_mode, sk, q_heads, batch);
   CUtensorMap b_kv = q64, b_q = q64;
   if (bias_mode == 2) {  // (a wide dQ step takes two boxes)
-    rc = bw_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, kv_rows, BW_R, false);
-    if (rc == TPB_OK) rc = bw_bias_tmap(&b_q, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_R, BW_T, true);
+    rc = fa_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, kv_rows, BW_R, false);
+    if (rc == TPB_OK) rc = fa_bias_tmap(&b_q, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, BW_R, BW_T, true);
     if (rc != TPB_OK) return rc;
   }
   auto launch = [&](auto dkv, const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap* t1, const CUtensorMap* t2, const CUtensorMap& tb, dim3 grid) {

@@ -371,27 +371,49 @@ constexpr int FA2_M = 256;
 constexpr int FA2_THREADS = 384;
 constexpr float FA2_RESCALE_LOG2 = 8.f;
 
+__device__ __forceinline__ void tmem_load(uint32_t at, uint32_t (&r)[16]) { tmem_ld_x16(at, r); }
+__device__ __forceinline__ void tmem_load(uint32_t at, uint32_t (&r)[32]) { tmem_ld_x32(at, r); }
+__device__ __forceinline__ void tmem_store(uint32_t at, const uint32_t (&r)[16]) { tmem_st_x16(at, r); }
+__device__ __forceinline__ void tmem_store(uint32_t at, const uint32_t (&r)[32]) { tmem_st_x32(at, r); }
+
+// Keys per tile.  128: one CTA fills an SM.  64, at head_dim 64: half of the tensor-memory columns and registers, two CTAs per SM.  What bounds
+// the softmax is not its instructions (a third of the issue slots) but the chain of a step, from scores to probabilities and through the tensor
+// core to the next scores, which two query tiles do not fill; four do better, although a step of half the keys has most of its chain.
+template <int D, int N>
+struct Fa2 {
+  static constexpr int CTAS = N == 64 ? 2 : 1;
+  static constexpr int W = N == 64 ? 16 : 32;  // columns per TMEM access beside a row of scores in registers
+  static constexpr int REGS_OTHER = N == 64 ? 32 : 56, REGS_SOFTMAX = N == 64 ? 104 : 224;
+  static_assert(4 * 32 * REGS_OTHER + 8 * 32 * REGS_SOFTMAX <= (N == 64 ? 80 : 168) * FA2_THREADS, "registers of a CTA at its launch");
+};
+
 // POLY of every 4 pairs of exponentials run on the FMA pipe.  BIAS: the score-bias code exists only where it is needed - 0 none, 1 any bias,
-// loaded in vectors or one by one, 2 bf16 rows in vectors (bias_vector_rows), those of a whole tile ahead.  2 holds 64 registers of raw
-// biases; in one instantiation with 1 they spill there too (2 x 1001, 16 heads of 128, causal, a dense bf16 bias: 296 us, apart 239 us;
-// 4 x 500, 16 heads of 64: 77 and 70 us; fp32 bias of 16 x 512, 32 heads of 64: 282 and 217 us).
-template <int D, int POLY, int BIAS>
-__global__ void __launch_bounds__(FA2_THREADS, 1)
+// loaded in vectors or one by one, 2 bf16 tiles by TMA, 3 bf16 rows in vectors (bias_vector_rows), those of a whole tile ahead.  3 holds 64 registers
+// of raw biases; in one instantiation with 1 they spill there too (2 x 1001, 16 heads of 128, causal, a dense bf16 bias: 296 us, apart 239 us;
+// fp32 bias of 16 x 512, 32 heads of 64: 282 and 217 us).
+template <int D, int N, int POLY, int BIAS>
+__global__ void __launch_bounds__(FA2_THREADS, Fa2<D, N>::CTAS)
 attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                         const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
+                         const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_b, const FaParams p) {
   constexpr int DB = D / 64;
-  constexpr uint32_t T_BYTES = DB * FA_BLOCK_BYTES;  // one 128-row tile of Q, K or V
-  constexpr uint32_t TMEM_COLS = 512;
-  constexpr uint32_t O_COL0 = 256;
-  constexpr uint32_t IDESC_QK = make_idesc_bf16(FA_M, FA_N, false, false);
+  constexpr uint32_t Q_BYTES = DB * FA_BLOCK_BYTES;  // one tile of 128 queries
+  constexpr uint32_t T_BYTES = DB * N * 128;         // one tile of N keys or values
+  constexpr uint32_t TMEM_COLS = 512 / Fa2<D, N>::CTAS;
+  constexpr uint32_t O_COL0 = 2 * N;
+  constexpr bool BIAS_TMA = BIAS == 2, BIAS_ROWS = BIAS == 3;
+  constexpr uint32_t B_BYTES = FA_M * N * 2;         // biases of a tile
+  constexpr int W = Fa2<D, N>::W;
+  static_assert(O_COL0 + 2 * D <= TMEM_COLS, "tensor memory columns");
+  constexpr uint32_t IDESC_QK = make_idesc_bf16(FA_M, N, false, false);
   constexpr uint32_t IDESC_PV = make_idesc_bf16(FA_M, D, false, true);
 
   extern __shared__ uint8_t fa_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_s = smem;                 // [2 tiles]
-  uint8_t* k_s = q_s + 2 * T_BYTES;    // [2 stages]
+  uint8_t* k_s = q_s + 2 * Q_BYTES;    // [2 stages]
   uint8_t* v_s = k_s + 2 * T_BYTES;    // [2 stages]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + 2 * T_BYTES);
+  uint8_t* b_s = v_s + 2 * T_BYTES;    // [2 tiles], BIAS_TMA only: swizzled blocks of [128 queries][64 keys]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(b_s + (BIAS_TMA ? 2 * B_BYTES : 0));
   uint64_t* q_full = bars;
   uint64_t* k_full = bars + 1;    // [2]
   uint64_t* k_empty = bars + 3;   // [2]
@@ -400,7 +422,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   uint64_t* s_full = bars + 9;    // [2 tiles]
   uint64_t* p_full = bars + 11;   // [2 tiles]
   uint64_t* o_full = bars + 13;   // [2 tiles]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* b_full = bars + 15;   // [2 tiles], BIAS_TMA
+  uint64_t* b_empty = bars + 17;  // [2 tiles]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be uniform)
@@ -414,7 +438,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   for (int t = 0; t < 2; ++t) {
     int kv_end = p.sk;
     if (p.causal) kv_end = min(p.sk, q0 + t * FA_M + FA_M + shift);
-    n_tiles[t] = (q0 + t * FA_M < p.sq && kv_end > 0) ? (kv_end + FA_N - 1) / FA_N : 0;
+    n_tiles[t] = (q0 + t * FA_M < p.sq && kv_end > 0) ? (kv_end + N - 1) / N : 0;
   }
   const int n_max = max(n_tiles[0], n_tiles[1]);
 
@@ -431,6 +455,10 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       mbar_init(&s_full[s], 1);
       mbar_init(&p_full[s], 4);  // one arrival per softmax warp of the tile
       mbar_init(&o_full[s], 1);
+      if (BIAS_TMA) {
+        mbar_init(&b_full[s], 1);
+        mbar_init(&b_empty[s], 4);
+      }
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -450,26 +478,44 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   };
 
   if (warp < 4) {
-    setmaxnreg_dec<56>();
+    setmaxnreg_dec<Fa2<D, N>::REGS_OTHER>();
     if (warp == 0) {
       // ---------------- TMA producer ----------------
       if (elect_one() && n_max > 0) {
-        mbar_expect_tx(q_full, 2 * T_BYTES);
+        mbar_expect_tx(q_full, 2 * Q_BYTES);
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-          for (int d = 0; d < DB; ++d) tma_load_4d(q_s + t * T_BYTES + d * FA_BLOCK_BYTES, &tmap_q, q_full, d * 64, q0 + t * FA_M, h, b);
+          for (int d = 0; d < DB; ++d) tma_load_4d(q_s + t * Q_BYTES + d * FA_BLOCK_BYTES, &tmap_q, q_full, d * 64, q0 + t * FA_M, h, b);
         for (int j = 0; j < n_max && !*abort_flag; ++j) {
           const int s = j & 1;
           const uint32_t par = ((j >> 1) & 1) ^ 1;
           if (!mbar_wait(&k_empty[s], par)) { give_up(STATUS_TIMEOUT_MBAR); break; }
           mbar_expect_tx(&k_full[s], T_BYTES);
 #pragma unroll
-          for (int d = 0; d < DB; ++d) tma_load_4d(k_s + s * T_BYTES + d * FA_BLOCK_BYTES, &tmap_k, &k_full[s], d * 64, j * FA_N, kvh, b);
+          for (int d = 0; d < DB; ++d) tma_load_4d(k_s + s * T_BYTES + d * (N * 128), &tmap_k, &k_full[s], d * 64, j * N, kvh, b);
           if (!mbar_wait(&v_empty[s], par)) { give_up(STATUS_TIMEOUT_MBAR); break; }
           mbar_expect_tx(&v_full[s], T_BYTES);
 #pragma unroll
-          for (int d = 0; d < DB; ++d) tma_load_4d(v_s + s * T_BYTES + d * FA_BLOCK_BYTES, &tmap_v, &v_full[s], d * 64, j * FA_N, kvh, b);
+          for (int d = 0; d < DB; ++d) tma_load_4d(v_s + s * T_BYTES + d * (N * 128), &tmap_v, &v_full[s], d * 64, j * N, kvh, b);
+        }
+      }
+    } else if (BIAS_TMA && warp == 2) {
+      // ---------------- biases, one tile per query tile: the next is on its way as soon as the last has been read ----------------
+      if (elect_one()) {
+        for (int j = 0; j < n_max && !*abort_flag; ++j) {
+          bool ok = true;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (!ok || j >= n_tiles[t]) continue;
+            ok = mbar_wait(&b_empty[t], (j & 1) ^ 1);
+            if (!ok) continue;
+            mbar_expect_tx(&b_full[t], B_BYTES);
+#pragma unroll
+            for (int c = 0; c < N / 64; ++c)
+              tma_load_4d(b_s + t * B_BYTES + c * FA_BLOCK_BYTES, &tmap_b, &b_full[t], j * N + c * 64, q0 + t * FA_M, p.bias_sh ? h : 0, p.bias_sb ? b : 0);
+          }
+          if (!ok) { give_up(STATUS_TIMEOUT_MBAR); break; }
         }
       }
     } else if (warp == 1) {
@@ -483,16 +529,16 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
           for (int d = 0; d < DB; ++d) {
 #pragma unroll
             for (int kk = 0; kk < 64 / 16; ++kk)
-              umma_bf16_lead(leader, tmem_base + t * FA_N, q_lo + (t * T_BYTES + d * FA_BLOCK_BYTES) / 16 + kk * 2, k_lo + d * (FA_BLOCK_BYTES / 16) + kk * 2,
+              umma_bf16_lead(leader, tmem_base + t * N, q_lo + (t * Q_BYTES + d * FA_BLOCK_BYTES) / 16 + kk * 2, k_lo + d * (N * 128 / 16) + kk * 2,
                              IDESC_QK, (d | kk) ? 1u : 0u);
           }
           umma_commit_lead(leader, &s_full[t]);
         };
         auto issue_pv = [&](int t, int j) {  // O_t (+)= P_t(j) V(j): P from tensor memory, V tile [128 keys][D] MN-major
-          const uint32_t v_lo = desc_mnmajor_lo(smem_u32(v_s + (j & 1) * T_BYTES), FA_BLOCK_BYTES);
+          const uint32_t v_lo = desc_mnmajor_lo(smem_u32(v_s + (j & 1) * T_BYTES), N * 128);
 #pragma unroll
-          for (int kk = 0; kk < FA_N / 16; ++kk)
-            umma_bf16_tmem_a_lead(leader, tmem_base + O_COL0 + t * FA_N, tmem_base + t * FA_N + kk * 8, v_lo + kk * (16 * 128 / 16), IDESC_PV,
+          for (int kk = 0; kk < N / 16; ++kk)
+            umma_bf16_tmem_a_lead(leader, tmem_base + O_COL0 + t * D, tmem_base + t * N + kk * 8, v_lo + kk * (16 * 128 / 16), IDESC_PV,
                                   (j | kk) ? 1u : 0u);
         };
         auto wait_all = [&](uint64_t* bar, uint32_t parity) {
@@ -534,31 +580,31 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     }
   } else {
     // ---------------- softmax warps ----------------
-    setmaxnreg_inc<224>();
+    setmaxnreg_inc<Fa2<D, N>::REGS_SOFTMAX>();
     const int t = (warp - 4) >> 2;
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;
     const int qi = q0 + t * FA_M + row;
     const int my_tiles = n_tiles[t];
-    const uint32_t s_addr = tmem_base + (uint32_t(quarter * 32) << 16) + t * FA_N;  // scores, and in their first 64 columns P
-    const uint32_t o_addr = tmem_base + (uint32_t(quarter * 32) << 16) + O_COL0 + t * FA_N;
+    const uint32_t s_addr = tmem_base + (uint32_t(quarter * 32) << 16) + t * N;  // scores, and in their first half P
+    const uint32_t o_addr = tmem_base + (uint32_t(quarter * 32) << 16) + O_COL0 + t * D;
     float m_run = -INFINITY, l_run = 0.f;
     const long long bias_row = BIAS ? (b * p.bias_sb + h * p.bias_sh + (long long)min(qi, p.sq - 1) * p.bias_sq) : 0;
     bool alive = true;
 
     for (int j = 0; j < my_tiles; ++j) {
-      const int key0 = j * FA_N;
+      const int key0 = j * N;
       const int visible = min(p.sk, p.causal ? qi + shift + 1 : p.sk) - key0;  // keys [0, visible) of this tile count, the others become -inf
       // only tiles that touch the diagonal or the end of the keys need per-element work
-      const bool plain = key0 + FA_N <= p.sk && (!p.causal || key0 + FA_N - 1 <= q0 + t * FA_M + shift);
+      const bool plain = key0 + N <= p.sk && (!p.causal || key0 + N - 1 <= q0 + t * FA_M + shift);
       // the row's biases of a whole tile, fetched BEFORE the wait for its scores: loaded where they are used, they would add
       // sixteen global round trips to the chain of every tile
-      uint4 bias_raw[BIAS == 2 ? FA_N / 8 : 1];
-      const bool ahead = BIAS == 2 && plain;
+      uint4 bias_raw[BIAS_ROWS ? N / 8 : 1];
+      const bool ahead = BIAS_ROWS && plain;
       if (ahead) {
         const uint4* src = reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.bias) + bias_row + key0);
 #pragma unroll
-        for (int c = 0; c < FA_N / 8; ++c) bias_raw[BIAS == 2 ? c : 0] = __ldg(src + c);
+        for (int c = 0; c < N / 8; ++c) bias_raw[BIAS_ROWS ? c : 0] = __ldg(src + c);
       }
       if (*abort_flag || !mbar_wait(&s_full[t], j & 1)) {
         if (!*abort_flag) give_up(STATUS_TIMEOUT_MBAR);
@@ -566,49 +612,63 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         break;
       }
       tc_fence_after();
-      uint32_t r[FA_N];
+      uint32_t r[N];
       float m_tile = -INFINITY;
       if (!BIAS) {
 #pragma unroll
-        for (int c = 0; c < FA_N; c += 32) tmem_ld_x32(s_addr + c, *reinterpret_cast<uint32_t(*)[32]>(r + c));
+        for (int c = 0; c < N; c += 32) tmem_ld_x32(s_addr + c, *reinterpret_cast<uint32_t(*)[32]>(r + c));
         tmem_ld_wait();
         if (!plain) {
 #pragma unroll
-          for (int i = 0; i < FA_N; ++i)
+          for (int i = 0; i < N; ++i)
             if (i >= visible) r[i] = 0xff800000u;
         }
         float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < FA_N; i += 4) {
+        for (int i = 0; i < N; i += 4) {
           m0 = fmax3(m0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
           m1 = fmax3(m1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
         }
         m_tile = fmaxf(m0, m1) * p.scale_log2e;  // (the scale is positive: the maximum commutes with it)
-      } else if (ahead) {
+      } else if (ahead || BIAS_TMA) {
+        if (BIAS_TMA && !mbar_wait(&b_full[t], j & 1)) {
+          give_up(STATUS_TIMEOUT_MBAR);
+          alive = false;
+          break;
+        }
         // whole tile visible: two scores per instruction, no masks (this path is bound by instruction issue: 16 x 512 tokens, 32
         // heads of 64, 218 us with a mask and a multiply per score, 151 us like this, 79 us without a bias)
 #pragma unroll
-        for (int c0 = 0; c0 < FA_N; c0 += 32) {  // a quarter at a time: the scores take the registers that the biases leave
+        for (int c0 = 0; c0 < N; c0 += 32) {  // a quarter at a time: the scores take the registers that the biases leave
           tmem_ld_x32(s_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(r + c0));
           tmem_ld_wait();
 #pragma unroll
           for (int c = c0; c < c0 + 32; c += 8) {
-            const uint4 u = bias_raw[BIAS == 2 ? c / 8 : 0];
+            const uint4 u = BIAS_TMA ? *reinterpret_cast<const uint4*>(b_s + t * B_BYTES + (c >> 6) * FA_BLOCK_BYTES + row * 128 + (((c >> 3 & 7) ^ (row & 7)) << 4))
+                                     : bias_raw[BIAS_ROWS ? c / 8 : 0];
             const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float b0, b1, s0, s1;
               ffma2(b0, b1, __uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u), 1.4426950408889634f, 1.4426950408889634f, 0.f, 0.f);
               ffma2(s0, s1, __uint_as_float(r[c + 2 * i]), __uint_as_float(r[c + 2 * i + 1]), p.scale_log2e, p.scale_log2e, b0, b1);
+              if (BIAS_TMA && !plain) {
+                if (c + 2 * i >= visible) s0 = -INFINITY;
+                if (c + 2 * i + 1 >= visible) s1 = -INFINITY;
+              }
               r[c + 2 * i] = __float_as_uint(s0);
               r[c + 2 * i + 1] = __float_as_uint(s1);
               m_tile = fmax3(m_tile, s0, s1);
             }
           }
         }
+        if (BIAS_TMA) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&b_empty[t]);
+        }
       } else {
 #pragma unroll
-        for (int c0 = 0; c0 < FA_N; c0 += 32) {
+        for (int c0 = 0; c0 < N; c0 += 32) {
           float bv[4][8];  // (all of a quarter's biases are on their way before the wait for its scores)
 #pragma unroll
           for (int c = 0; c < 32; c += 8)
@@ -639,13 +699,13 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       }
       if (j > 0 && __any_sync(0xffffffffu, rescale)) {
 #pragma unroll
-        for (int c = 0; c < D; c += 32) {
-          uint32_t o[32];
-          tmem_ld_x32(o_addr + c, o);
+        for (int c = 0; c < D; c += W) {
+          uint32_t o[W];
+          tmem_load(o_addr + c, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-          tmem_st_x32(o_addr + c, o);
+          for (int i = 0; i < W; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+          tmem_store(o_addr + c, o);
         }
       }
       l_run *= factor;
@@ -654,10 +714,10 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       const float nbase = m_run == -INFINITY ? 0.f : -m_run;
       float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
-      for (int c = 0; c < FA_N / 2; c += 32) {
-        uint32_t packed[32];
+      for (int c = 0; c < N / 2; c += W) {
+        uint32_t packed[W];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < W; ++i) {
           float t0, t1;
           ffma2(t0, t1, __uint_as_float(r[2 * (c + i)]), __uint_as_float(r[2 * (c + i) + 1]), mul, mul, nbase, nbase);
           float p0, p1;
@@ -672,7 +732,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
           fadd2(sum0, sum1, sum0, sum1, p0, p1);
           packed[i] = pack_bf16x2(p0, p1);
         }
-        tmem_st_x32(s_addr + c, packed);
+        tmem_store(s_addr + c, packed);
       }
       l_run += sum0 + sum1;
       tmem_st_wait();
@@ -754,17 +814,29 @@ static int fa_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
-template <int D, int POLY, int BIAS>
-static int fa2_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, dim3 grid, cudaStream_t stream) {
-  constexpr size_t smem = size_t(D / 64) * FA_BLOCK_BYTES * 6 + 1024 + 256;
+// Keys per tile (see Fa2) of a launch at head_dim 64, bias as BIAS above: 64 where there are CTAs for a second one per SM (us in tiles of 128 / 64,
+// heads in brackets: 16 x 512 (32) 77 / 59, causal 69 / 54, a bias by TMA 114 / 89, fp32 215 / 194; 32 x 129 (16) 28 / 18; but 8 x 512 (8), 128 CTAs, 11.9 / 13.3, by
+// TMA 17.5 / 19.0, and 2 x 1000 (12), 96 CTAs, 18.3 / 21.3).  Long causal rows without a bias fill their tiles of 128 (4 x 2048 (12) 65.0 / 65.9, 2 x 4096 (16)
+// 140 / 144; 4 x 1001 (32) 50.1 / 47.9), and rows in registers pay for fewer of those where tiles are whole (mask of 16 x 512 (32) 107 / 123, causal
+// 242 / 184, of 16 x 200 (16) 28 / 22).
+static int fa2_tile_keys(int bias, long long ctas, int sk, bool causal) {
+  if (ctas <= 148) return 128;
+  if (bias == 0) return causal && sk > 1024 ? 128 : 64;
+  return bias == 3 && !causal && sk > 256 ? 128 : 64;
+}
+
+template <int D, int N, int BIAS>
+static int fa2_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tb, const FaParams& p, dim3 grid, cudaStream_t stream) {
+  constexpr size_t smem = size_t(D / 64) * (2 * FA_BLOCK_BYTES + 4 * N * 128) + (BIAS == 2 ? 2 * FA_M * N * 2 : 0) + 1024 + 256;
+  static_assert(Fa2<D, N>::CTAS * (smem + 1024) <= 228 * 1024, "shared memory of an SM");
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(attn_fwd_pingpong_kernel<D, POLY, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return TPB_ERR_CUDA;
+    if (cudaFuncSetAttribute(attn_fwd_pingpong_kernel<D, N, 1, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return TPB_ERR_CUDA;
     configured[dev].store(true, std::memory_order_release);
   }
-  attn_fwd_pingpong_kernel<D, POLY, BIAS><<<grid, FA2_THREADS, smem, stream>>>(tq, tk, tv, p);
+  attn_fwd_pingpong_kernel<D, N, 1, BIAS><<<grid, FA2_THREADS, smem, stream>>>(tq, tk, tv, tb, p);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
@@ -812,10 +884,21 @@ extern "C" int tpb_attn_prefill_sm100(const void* q, const void* k, const void* 
     dim3 grid((sq + FA2_M - 1) / FA2_M, q_heads, batch);
     // one pair of exponentials in four runs as a cubic on the FMA pipe (measured best of 0 / 1 / 2 / 3 in four:
     // 206 / 199 / 205 / 236 us at batch 4, 2048 tokens, 32 heads of 128, causal, before the warp-uniform issue loop: 161 us with it)
-    if (bias && p.bias_kind == 2 && p.bias_vec)
-      return head_dim == 128 ? fa2_launch<128, 1, 2>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, 2>(tq, tk, tv, p, grid, s);
-    if (bias) return head_dim == 128 ? fa2_launch<128, 1, 1>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, 1>(tq, tk, tv, p, grid, s);
-    return head_dim == 128 ? fa2_launch<128, 1, 0>(tq, tk, tv, p, grid, s) : fa2_launch<64, 1, 0>(tq, tk, tv, p, grid, s);
+    // bf16 rows in vectors come by TMA where it can address them, as in the backward; at head_dim 128, where shared memory has no room, and where
+    // one row serves all queries (padding masks), by loads
+    const bool vectors = p.bias_kind == 2 && p.bias_vec, by_tma = vectors && head_dim == 64 && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0;
+    const int mode = !bias ? 0 : by_tma ? 2 : vectors ? 3 : 1;
+    CUtensorMap tb = tq;
+    if (by_tma) rc = fa_bias_tmap(&tb, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, FA_M, 64, true);
+    if (head_dim == 128)
+      return mode == 0 ? fa2_launch<128, 128, 0>(tq, tk, tv, tb, p, grid, s) : mode == 3 ? fa2_launch<128, 128, 3>(tq, tk, tv, tb, p, grid, s) : fa2_launch<128, 128, 1>(tq, tk, tv, tb, p, grid, s);
+    const bool narrow = fa2_tile_keys(mode, (long long)grid.x * grid.y * grid.z, sk, causal) == 64;
+    if (narrow && rc == TPB_OK) rc = fa_tmap(&tk, k, head_dim, 64, sk, kv_heads, batch, k_ss, k_sh, k_sb);
+    if (narrow && rc == TPB_OK) rc = fa_tmap(&tv, v, head_dim, 64, sk, kv_heads, batch, v_ss, v_sh, v_sb);
+    if (rc != TPB_OK) return rc;
+#define FA2_64(BIAS) (narrow ? fa2_launch<64, 64, BIAS>(tq, tk, tv, tb, p, grid, s) : fa2_launch<64, 128, BIAS>(tq, tk, tv, tb, p, grid, s))
+    return mode == 0 ? FA2_64(0) : mode == 1 ? FA2_64(1) : mode == 2 ? FA2_64(2) : FA2_64(3);
+#undef FA2_64
   }
   dim3 grid((sq + FA_M - 1) / FA_M, q_heads, batch);
   return head_dim == 128 ? fa_launch<128>(tq, tk, tv, p, grid, s) : fa_launch<64>(tq, tk, tv, p, grid, s);

@@ -128,6 +128,21 @@ static int fa_tmap(CUtensorMap* map, const void* ptr, int head_dim, int box_rows
   return r == CUDA_SUCCESS ? TPB_OK : TPB_ERR_TMAP;
 }
 
+// Tensor map over a bf16 score bias [batch or 1][heads or 1][sq][sk] (keys contiguous); box = [rows queries][keys].
+static int fa_bias_tmap(CUtensorMap* map, const void* bias, int batch, int heads, int sq, int sk, long long sb, long long sh, long long sqs, int rows,
+                        int keys, bool swizzled) {
+  EncodeTiledFn fn = fa_encode_fn();
+  if (!fn) return TPB_ERR_DRIVER;
+  cuuint64_t dims[4] = {cuuint64_t(sk), cuuint64_t(sq), cuuint64_t(sh ? heads : 1), cuuint64_t(sb ? batch : 1)};
+  cuuint64_t strides[3] = {cuuint64_t(sqs) * 2, cuuint64_t(sh ? sh : sqs) * 2, cuuint64_t(sb ? sb : sqs) * 2};
+  cuuint32_t box[4] = {cuuint32_t(keys), cuuint32_t(rows), 1, 1}, estr[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(bias), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? TPB_OK
+             : TPB_ERR_TMAP;
+}
+
 // The tensor-map encoder needs a context bound to the calling thread (autograd worker threads have none at first).
 static int fa_bind_thread() {
   static thread_local int bound_device = -1;
