@@ -9,8 +9,8 @@
 //
 // Two launches, dK / dV and dQ, both free of atomics and therefore deterministic (the optional bias gradient is the exception: fp32
 // atomic adds).  A CTA keeps 128 "resident" rows (the TMEM lanes) and streams the other sequence through.  There are two kernels, each a
-// template of both launches: attn_bwd_tcgen05_kernel streams 64 rows per step (described here), attn_bwd_wide_kernel 128 (described
-// there); step_rows below says which launch takes which.
+// template of both launches: attn_bwd_tcgen05_kernel streams 64 rows per step (described here), attn_bwd_wide_kernel 128, or 64
+// with two CTAs per SM (described there); two_per_sm and step_rows below say which launch takes which.
 //
 //   dK / dV (DKV = true) : resident = 128 keys of one KV head (K and V tiles), streamed = queries (Q and dO, over all
 //                          query heads of the group):  S^T = K Q^T and dP^T = V dO^T land in TMEM with a key per lane,
@@ -532,28 +532,35 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 // for 47 % (dQ 50 %) of the causal launch below.  (Next would be shared memory: 192 KB read and 64 KB filled per 2048 clocks of dK / dV products.)
 // Whole backward, 32 heads of 128: 4 x 2048 causal 558 -> 507 us, 2 x 2080 344 -> 323, without a mask 560 -> 518; 1 x 1000 65.7 -> 61.3.
 // Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.  Short and ragged sequences: step_rows.
-constexpr int BWW_WARPS = 16;                            // elementwise warps
-constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
-constexpr int BWW_T = 128;                               // streamed rows per step
-constexpr int BWW_S1 = 3, BWW_S2 = 2;                    // ring depths: Q (dK / dV) or K (dQ); dO or V
-constexpr int BWW_BARS = 1 + 2 * (BWW_S1 + BWW_S2) + 7;
-constexpr uint32_t BWW_BIAS = BWW_T * BW_R * 2;          // bias elements of one step
-constexpr size_t bww_smem_bytes(int d, int bias) {
-  return size_t(2 + BWW_S1 + BWW_S2) * (d / 64) * FA_BLOCK_BYTES + (bias == 2 ? BWW_S1 * BWW_BIAS : 0) + 2 * BWW_T * sizeof(float2) + BWW_BARS * 8 + 16;
-}
+//
+// T = 64 is the same with 64 streamed rows, at head_dim 64: half of the tensor-memory columns, registers and shared memory, and two CTAs per SM, which fill
+// each other's chains, prologues and epilogues.
+template <int D, int T, int BIAS>
+struct Bww {
+  static constexpr int CTAS = T == 64 ? 2 : 1;
+  static constexpr int WARPS = 16 / CTAS;                  // elementwise warps
+  static constexpr int THREADS = 64 + 32 * WARPS;
+  static constexpr int S1 = T == 64 && BIAS == 2 ? 2 : 3, S2 = 2;  // ring depths: Q (dK / dV) or K (dQ), with the bias; dO or V
+  static constexpr int BARS = 1 + 2 * (S1 + S2) + 7;
+  static constexpr uint32_t TILE = D / 64 * T * 128;       // one streamed tile
+  static constexpr uint32_t BIAS_BYTES = T * BW_R * 2;     // bias elements of one step
+  static constexpr size_t SMEM = size_t(2 * (D / 64)) * FA_BLOCK_BYTES + (S1 + S2) * TILE + (BIAS == 2 ? S1 * BIAS_BYTES : 0) + 2 * T * sizeof(float2) + BARS * 8 + 16;
+  static_assert(CTAS * (SMEM + 1024) <= 228 * 1024, "shared memory of an SM");
+};
 
-template <int D, bool DKV, int BIAS>
-__global__ void __launch_bounds__(BWW_THREADS, 1)
+template <int D, bool DKV, int BIAS, int T>
+__global__ void __launch_bounds__(Bww<D, T, BIAS>::THREADS, Bww<D, T, BIAS>::CTAS)
 attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_constant__ CUtensorMap tmap_r2,
                      const __grid_constant__ CUtensorMap tmap_t1, const __grid_constant__ CUtensorMap tmap_t2,
                      const __grid_constant__ CUtensorMap tmap_b, const BwParams p) {
-  constexpr int DB = D / 64;
-  constexpr uint32_t TILE = DB * FA_BLOCK_BYTES;  // 128 rows
-  constexpr uint32_t TMEM_COLS = 512, S_COL = 0, DP_COL = BWW_T, ACC0_COL = 2 * BWW_T, ACC1_COL = ACC0_COL + D;
-  constexpr bool RES_TMEM = !DKV || D == 64;  // the resident tiles as tensor-memory operands, where 512 columns leave room
+  using B = Bww<D, T, BIAS>;
+  constexpr int DB = D / 64, BWW_S1 = B::S1, BWW_S2 = B::S2, BWW_WARPS = B::WARPS;
+  constexpr uint32_t R_TILE = DB * FA_BLOCK_BYTES, TILE = B::TILE, T_BLOCK = T * 128, BWW_BIAS = B::BIAS_BYTES;
+  constexpr uint32_t TMEM_COLS = 512 / B::CTAS, S_COL = 0, DP_COL = T, ACC0_COL = 2 * T, ACC1_COL = ACC0_COL + D;
+  constexpr bool RES_TMEM = !DKV || (D == 64 && T == 128);  // the resident tiles as tensor-memory operands, where the columns leave room
   constexpr uint32_t RES_COL = ACC0_COL + (DKV ? 2 : 1) * D;
-  static_assert(!RES_TMEM || RES_COL + D <= TMEM_COLS, "tensor memory columns");
-  constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BWW_T, false, false);
+  static_assert(ACC0_COL + (DKV ? 2 : 1) * D <= TMEM_COLS && (!RES_TMEM || RES_COL + D <= TMEM_COLS), "tensor memory columns");
+  constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, T, false, false);
   constexpr uint32_t IDESC_ACC = make_idesc_bf16(BW_R, D, false, true);
 
   extern __shared__ __align__(1024) uint8_t bww_smem[];
@@ -563,12 +570,12 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
     return;
   }
   uint8_t* r1_s = smem;
-  uint8_t* r2_s = r1_s + TILE;
-  uint8_t* t1_s = r2_s + TILE;            // [BWW_S1]
+  uint8_t* r2_s = r1_s + R_TILE;
+  uint8_t* t1_s = r2_s + R_TILE;            // [BWW_S1]
   uint8_t* t2_s = t1_s + BWW_S1 * TILE;   // [BWW_S2]
   uint8_t* bias_s = t2_s + BWW_S2 * TILE;     // [BWW_S1], BIAS == 2 only
   float* stat_s = reinterpret_cast<float*>(bias_s + (BIAS == 2 ? BWW_S1 * BWW_BIAS : 0));  // dK / dV, [2 steps]: -lse * log2(e) of 128 streamed queries (-inf = no such query), -delta * scale
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + 4 * BWW_T);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + 4 * T);
   uint64_t* r_full = bars;
   uint64_t* t1_full = bars + 1;
   uint64_t* t1_empty = t1_full + BWW_S1;
@@ -592,8 +599,8 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
     r0 = blockIdx.x * BW_R;
     kvh = blockIdx.y;
     head = kvh * group;
-    const int q_steps = (p.sq + BWW_T - 1) / BWW_T;
-    step0 = p.causal ? max(0, r0 - shift) / BWW_T : 0;
+    const int q_steps = (p.sq + T - 1) / T;
+    step0 = p.causal ? max(0, r0 - shift) / T : 0;
     per_head = max(0, q_steps - step0);
     n_steps = per_head * group;
   } else {
@@ -603,7 +610,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
     int kv_end = p.sk;
     if (p.causal) kv_end = min(p.sk, r0 + BW_R + shift);
     step0 = 0;
-    per_head = kv_end > 0 ? (kv_end + BWW_T - 1) / BWW_T : 0;
+    per_head = kv_end > 0 ? (kv_end + T - 1) / T : 0;
     n_steps = per_head;
   }
 
@@ -646,33 +653,33 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
 
   if (warp == 0) {
     // ---------------- TMA producer (the whole warp stays together: all lanes write statistics) ----------------
-    auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row, int h) {
+    auto load = [&](uint8_t* dst, uint32_t block, const CUtensorMap* map, uint64_t* bar, int row, int h) {
 #pragma unroll
-      for (int d = 0; d < DB; ++d) tma_load_4d(dst + d * FA_BLOCK_BYTES, map, bar, d * 64, row, h, b);
+      for (int d = 0; d < DB; ++d) tma_load_4d(dst + d * block, map, bar, d * 64, row, h, b);
     };
     if (n_steps > 0) {
       if (lane == 0) {
-        mbar_expect_tx(r_full, 2 * TILE);
-        load(r1_s, &tmap_r1, r_full, r0, DKV ? kvh : head);
-        load(r2_s, &tmap_r2, r_full, r0, DKV ? kvh : head);
+        mbar_expect_tx(r_full, 2 * R_TILE);
+        load(r1_s, FA_BLOCK_BYTES, &tmap_r1, r_full, r0, DKV ? kvh : head);
+        load(r2_s, FA_BLOCK_BYTES, &tmap_r2, r_full, r0, DKV ? kvh : head);
       }
       int g = 0, local = 0;  // query head of the group (dK / dV), step within it
       for (int n = 0; n < n_steps; ++n) {
         const int s1 = n % BWW_S1, s2 = n % BWW_S2;
         bool ok = !*abort_flag && mbar_wait(&t1_empty[s1], ((n / BWW_S1) & 1) ^ 1);
-        const int row0 = (step0 + local) * BWW_T;
+        const int row0 = (step0 + local) * T;
         const int t_head = DKV ? head + g : kvh;
         if (++local == per_head) { local = 0; ++g; }
         if (ok && lane == 0) {
           mbar_expect_tx(&t1_full[s1], TILE + (BIAS == 2 ? BWW_BIAS : 0));
-          load(t1_s + s1 * TILE, &tmap_t1, &t1_full[s1], row0, t_head);
+          load(t1_s + s1 * TILE, T_BLOCK, &tmap_t1, &t1_full[s1], row0, t_head);
           if (BIAS == 2) {
             const int bh = p.b_sh ? (DKV ? t_head : head) : 0, bb = p.b_sb ? b : 0;
-            if (DKV) {  // [128 queries][128 keys]
+            if (DKV) {  // [T queries][128 keys]
               tma_load_4d(bias_s + s1 * BWW_BIAS, &tmap_b, &t1_full[s1], r0, row0, bh, bb);
-            } else {  // two swizzled blocks of [128 queries][64 keys]
+            } else {  // swizzled blocks of [128 queries][64 keys]
               tma_load_4d(bias_s + s1 * BWW_BIAS, &tmap_b, &t1_full[s1], row0, r0, bh, bb);
-              tma_load_4d(bias_s + s1 * BWW_BIAS + FA_BLOCK_BYTES, &tmap_b, &t1_full[s1], row0 + 64, r0, bh, bb);
+              if (T == 128) tma_load_4d(bias_s + s1 * BWW_BIAS + FA_BLOCK_BYTES, &tmap_b, &t1_full[s1], row0 + 64, r0, bh, bb);
             }
           }
         }
@@ -683,12 +690,12 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         }
         if (lane == 0) {
           mbar_expect_tx(&t2_full[s2], TILE);
-          load(t2_s + s2 * TILE, &tmap_t2, &t2_full[s2], row0, t_head);
+          load(t2_s + s2 * TILE, T_BLOCK, &tmap_t2, &t2_full[s2], row0, t_head);
         }
         if (DKV) {
-          float2 st[BWW_T / 32];
+          float2 st[T / 32];
 #pragma unroll
-          for (int i = 0; i < BWW_T / 32; ++i) {
+          for (int i = 0; i < T / 32; ++i) {
             const int qi = row0 + i * 32 + lane;
             st[i] = make_float2(-INFINITY, 0.f);
             if (qi < p.sq) {
@@ -705,9 +712,9 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
             break;
           }
 #pragma unroll
-          for (int i = 0; i < BWW_T / 32; ++i) {
-            stat_s[s2 * 2 * BWW_T + i * 32 + lane] = st[i].x;
-            stat_s[(s2 * 2 + 1) * BWW_T + i * 32 + lane] = st[i].y;
+          for (int i = 0; i < T / 32; ++i) {
+            stat_s[s2 * 2 * T + i * 32 + lane] = st[i].x;
+            stat_s[(s2 * 2 + 1) * T + i * 32 + lane] = st[i].y;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&t2_full[s2]);
@@ -725,17 +732,17 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         for (int d = 0; d < DB; ++d) {
 #pragma unroll
           for (int kk = 0; kk < 64 / 16; ++kk) {
-            const uint32_t off = d * (FA_BLOCK_BYTES >> 4) + kk * 2;
-            if (!RES_TMEM) umma_bf16_lead(leader, col, (which ? r2_lo : r1_lo) + off, t_lo + off, IDESC_S, (d | kk) ? 1u : 0u);
+            const uint32_t off = d * (T_BLOCK >> 4) + kk * 2;
+            if (!RES_TMEM) umma_bf16_lead(leader, col, (which ? r2_lo : r1_lo) + d * (FA_BLOCK_BYTES >> 4) + kk * 2, t_lo + off, IDESC_S, (d | kk) ? 1u : 0u);
             else umma_bf16_tmem_a_lead(leader, col, tmem_base + RES_COL + which * (D / 2) + (d * 4 + kk) * 8, t_lo + off, IDESC_S, (d | kk) ? 1u : 0u);
           }
         }
         umma_commit_lead(leader, which ? dp_full : s_full);
       };
       auto accumulate = [&](uint32_t acc_col, uint32_t a_col, uint32_t tile, bool first) {
-        const uint32_t t_lo = desc_mnmajor_lo(tile, FA_BLOCK_BYTES);
+        const uint32_t t_lo = desc_mnmajor_lo(tile, T_BLOCK);
 #pragma unroll
-        for (int kk = 0; kk < BWW_T / 16; ++kk)  // (the bf16 operand of 32 streamed rows lies in the first half of their own columns)
+        for (int kk = 0; kk < T / 16; ++kk)  // (the bf16 operand of 32 streamed rows lies in the first half of their own columns)
           umma_bf16_tmem_a_lead(leader, tmem_base + acc_col, tmem_base + a_col + (kk >> 1) * 32 + (kk & 1) * 8, t_lo + kk * (16 * 128 >> 4), IDESC_ACC,
                                 (!first || kk) ? 1u : 0u);
       };
@@ -780,8 +787,9 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
       umma_commit_lead(leader, acc_full);
     }
   } else {
-    // ---------------- elementwise warps: four threads per TMEM lane, 32 of the step's columns each ----------------
-    constexpr int HC = BWW_T / 4, HD = D / 4;
+    // ---------------- elementwise warps: two or four threads per TMEM lane, 32 of the step's columns each ----------------
+    constexpr int HC = T / (BWW_WARPS / 4), HD = D / (BWW_WARPS / 4);
+    static_assert(HC == 32, "columns per thread");
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
     const int part = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
@@ -829,13 +837,13 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
     };
 
     for (int n = 0; alive && n < n_steps; ++n) {
-      const float* neg_lse = stat_s + (n % BWW_S2) * 2 * BWW_T + part * HC;
-      const float* neg_delta = neg_lse + BWW_T;
+      const float* neg_lse = stat_s + (n % BWW_S2) * 2 * T + part * HC;
+      const float* neg_delta = neg_lse + T;
       if (DKV && !wait_all(&t2_full[n % BWW_S2], (n / BWW_S2) & 1)) break;
       if (BIAS == 2 && !wait_all(&t1_full[n % BWW_S1], (n / BWW_S1) & 1)) break;
       if (!wait_all(s_full, n & 1)) break;
       tc_fence_after();
-      const int col0 = (step0 + local) * BWW_T + part * HC;  // first query (DKV) or key of my columns
+      const int col0 = (step0 + local) * T + part * HC;  // first query (DKV) or key of my columns
       const int b_head = DKV ? head + g : head;
       if (++local == per_head) { local = 0; ++g; }
       // score bias: element (query, key) = (col0 + c, ri) for dK / dV - there the lanes of a warp own consecutive keys - and
@@ -958,20 +966,19 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-template <int D, bool DKV, int BIAS>
+template <int D, bool DKV, int BIAS, int T>
 static int bw_launch_wide(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& tb,
                           const BwParams& p, dim3 grid, cudaStream_t stream) {
-  constexpr size_t smem = bww_smem_bytes(D, BIAS);
-  static_assert(smem <= 227 * 1024, "shared memory of a CTA");
+  constexpr size_t smem = Bww<D, T, BIAS>::SMEM;
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(attn_bwd_wide_kernel<D, DKV, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_bwd_wide_kernel<D, DKV, BIAS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
       return TPB_ERR_CUDA;
     configured[dev].store(true, std::memory_order_release);
   }
-  attn_bwd_wide_kernel<D, DKV, BIAS><<<grid, BWW_THREADS, smem, stream>>>(r1, r2, t1, t2, tb, p);
+  attn_bwd_wide_kernel<D, DKV, BIAS, T><<<grid, Bww<D, T, BIAS>::THREADS, smem, stream>>>(r1, r2, t1, t2, tb, p);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
@@ -992,7 +999,7 @@ static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtenso
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
-// Streamed rows per step of a launch, 64 or 128: which kernel it takes.  bias_mode as BIAS above; heads: of the launch's grid (KV heads for
+// Streamed rows per step of a launch with one CTA per SM, 64 or 128: which kernel it takes.  bias_mode as BIAS above; heads: of the launch's grid (KV heads for
 // dK / dV).  What decides is how many rows of the last step are empty, in every product and elementwise pass, against what a step costs.
 // Times are of whole backwards, both launches in steps of 64 / of 128 rows, in us, causal where no bias is named.
 //   head_dim 128 with a bias: 64, the wide rings leave no room for it.
@@ -1005,12 +1012,20 @@ static int bw_launch(const CUtensorMap& r1, const CUtensorMap& r2, const CUtenso
 //   head_dim 64 with a bias: 64 only for up to 64 rows (32 heads: 4 x 64 10 %, with a padding mask 7 % longer in wide steps); beyond, the wide
 //   kernel's warps, twice as many per bias element, decide (4 x 300 0.79 of the time, 2 x 900 0.71, with a mask 0.76 and 0.64).
 static int step_rows(int head_dim, int bias_mode, int streamed, int heads, int batch) {
-  const bool half = streamed % BWW_T > 0 && streamed % BWW_T <= BW_T;
-  if (head_dim == 128) return bias_mode || (half && streamed < 3 * BWW_T) ? BW_T : BWW_T;
-  if (bias_mode) return streamed <= BW_T ? BW_T : BWW_T;
+  const bool half = streamed % 128 > 0 && streamed % 128 <= BW_T;
+  if (head_dim == 128) return bias_mode || (half && streamed < 3 * 128) ? BW_T : 128;
+  if (bias_mode) return streamed <= BW_T ? BW_T : 128;
   const long long rows = (long long)heads * batch;
-  if (half) return streamed < 3 * BWW_T || (streamed < 5 * BWW_T && rows >= 64) ? BW_T : BWW_T;
-  return streamed <= 2 * BWW_T && rows >= 256 ? BW_T : BWW_T;
+  if (half) return streamed < 3 * 128 || (streamed < 5 * 128 && rows >= 64) ? BW_T : 128;
+  return streamed <= 2 * 128 && rows >= 256 ? BW_T : 128;
+}
+
+// Whether a launch over `resident` rows takes the wide kernel with two CTAs per SM and steps of 64 rows (head_dim 64): where there are CTAs for it; causal
+// CTAs differ in length, so that it takes a second round of them.  Whole backwards in us, as step_rows has it / with two CTAs per SM: 16 x 512, 32 heads
+// 256 / 187, causal 209 / 156, with a bias 278 / 219; 4 x 2048, 12 heads 263 / 225, causal 168 / 157; 32 x 129, 16 heads 72 / 55; 4 x 300, 16 heads (192 CTAs)
+// 30.3 / 24.8, causal with a mask 46.5 / 49.1; 2 x 1000, 12 heads (192) 54.6 / 48.5, causal 42.6 / 45.9; 1 x 512, 8 heads (32) 20.6 / 23.0.
+static bool two_per_sm(int head_dim, int resident, int heads, int batch, bool causal) {
+  return head_dim == 64 && (long long)((resident + BW_R - 1) / BW_R) * heads * batch > (causal ? 296 : 148);
 }
 
 }  // namespace tpb
@@ -1078,7 +1093,8 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   // a dense bf16 bias travels by TMA (strides and base are multiples of 16 bytes); fp32 ones, unaligned rows and masks that
   // broadcast over the queries are loaded element by element
   const int bias_mode = !bias ? 0 : (p.bias_kind == 2 && p.bias_vec && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0 ? 2 : 1);
-  const int kv_rows = step_rows(head_dim, bias_mode, sq, kv_heads, batch), q_rows = step_rows(head_dim, bias_mode, sk, q_heads, batch);
+  const bool kv_two = two_per_sm(head_dim, sk, kv_heads, batch, causal), q_two = two_per_sm(head_dim, sq, q_heads, batch, causal);
+  const int kv_rows = kv_two ? BW_T : step_rows(head_dim, bias_mode, sq, kv_heads, batch), q_rows = q_two ? BW_T : step_rows(head_dim, bias_mode, sk, q_heads, batch);
   CUtensorMap b_kv = q64, b_q = q64;
   if (bias_mode == 2) {  // (a wide dQ step takes two boxes)
     rc = fa_bias_tmap(&b_kv, bias, batch, q_heads, sq, sk, bias_sb, bias_sh, bias_sq, kv_rows, BW_R, false);
@@ -1087,10 +1103,15 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   }
   auto launch = [&](auto dkv, const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap* t1, const CUtensorMap* t2, const CUtensorMap& tb, dim3 grid) {
     constexpr bool DKV = decltype(dkv)::value;
-    const bool wide = (DKV ? kv_rows : q_rows) == BWW_T;
+    const bool wide = (DKV ? kv_rows : q_rows) == 128;
 #define BW_ONE(D, BIAS)                                                                  \
-  (wide ? bw_launch_wide<D, DKV, BIAS>(r1, r2, t1[1], t2[1], tb, p, grid, s)             \
+  (wide ? bw_launch_wide<D, DKV, BIAS, 128>(r1, r2, t1[1], t2[1], tb, p, grid, s)        \
         : bw_launch<D, DKV, BIAS>(r1, r2, t1[0], t2[0], tb, p, grid, s))
+    if (head_dim == 64 && (DKV ? kv_two : q_two)) {
+#define BW_TWO(BIAS) bw_launch_wide<64, DKV, BIAS, 64>(r1, r2, t1[0], t2[0], tb, p, grid, s)
+      return bias_mode == 0 ? BW_TWO(0) : bias_mode == 1 ? BW_TWO(1) : BW_TWO(2);
+#undef BW_TWO
+    }
     if (head_dim == 64) return bias_mode == 0 ? BW_ONE(64, 0) : bias_mode == 1 ? BW_ONE(64, 1) : BW_ONE(64, 2);
     return bias_mode == 0   ? BW_ONE(128, 0)
            : bias_mode == 1 ? bw_launch<128, DKV, 1>(r1, r2, t1[0], t2[0], tb, p, grid, s)

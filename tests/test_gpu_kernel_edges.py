@@ -826,6 +826,46 @@ def test_norm_of_as_many_rows_as_an_int_counts():
     torch.cuda.empty_cache()
 
 
+def _attention_double(q, k, v, causal, bias):
+    """Output, and what backward needs, of 64-bit attention over leaves of q, k, v and the bias."""
+    scores = torch.einsum("bqhd,bkhd->bhqk", q, k.repeat_interleave(q.shape[2] // k.shape[2], 2)) / math.sqrt(q.shape[-1])
+    if bias is not None:
+        scores = scores + bias
+    if causal:
+        sq, sk = scores.shape[-2:]
+        scores = scores.masked_fill(torch.ones(sq, sk, dtype=torch.bool, device=q.device).triu(sk - sq + 1), -math.inf)
+    return torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1).nan_to_num(0.0), v.repeat_interleave(q.shape[2] // v.shape[2], 2))
+
+
+# more CTAs than SMs (causal: than two rounds of them) at head_dim 64: two CTAs per SM.  Lengths off the tiles of 64 and 128, one tile, several, more
+# keys than queries; grouped heads.
+@pytest.mark.parametrize("b,sq,sk,hq,hkv,causal", [(5, 129, 129, 32, 32, False), (10, 130, 193, 32, 16, True), (5, 200, 72, 32, 32, False), (3, 257, 320, 64, 64, True),
+                                                   (2, 1, 64, 160, 160, True), (4, 264, 264, 40, 40, False)])
+@pytest.mark.parametrize("bias", ["none", "dense", "rows off 16 bytes", "fp32", "padding"])
+def test_attention_with_two_ctas_per_sm(b, sq, sk, hq, hkv, causal, bias):
+    nat = _native()
+    torch.manual_seed(sq + sk)
+    q, k, v = (torch.randn(b, s, h, 64, device="cuda", dtype=torch.bfloat16).requires_grad_() for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
+    g = torch.randn(b, sq, hq, 64, device="cuda", dtype=torch.bfloat16)
+    added = None
+    if bias == "padding":
+        added = torch.zeros(b, 1, 1, sk, device="cuda", dtype=torch.bfloat16)
+        added[0, :, :, sk - sk // 3:] = -math.inf
+    elif bias != "none":
+        pitch = (sk + 7) // 8 * 8 + (1 if bias == "rows off 16 bytes" else 0)
+        added = torch.randn(1, hq, sq, pitch, device="cuda", dtype=torch.float32 if bias == "fp32" else torch.bfloat16)[..., :sk].detach().requires_grad_()
+    out = nat.attention(q, k, v, causal, added)
+    out.backward(g)
+    nat.device_state(q.device).check_status()
+    leaves = [t.detach().double().requires_grad_() for t in (q, k, v) + ((added,) if added is not None and added.requires_grad else ())]
+    want = _attention_double(*leaves[:3], causal, leaves[3] if len(leaves) > 3 else None if added is None else added.double())
+    want.backward(g.double())
+    # probabilities, dS and results are rounded to bf16 (2^-9 each, independent from element to element), as in test_attention_backward_by_step
+    assert (out.double() - want).norm() <= 0.01 * want.norm()
+    for t, ref in zip((q, k, v) + ((added,) if len(leaves) > 3 else ()), leaves):
+        assert (t.grad.double() - ref.grad).norm() <= 0.01 * ref.grad.norm() + 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("cols", [8, 264, 776, 1024, 1536, 1544, 1800, 2048, 2568, 3072, 3080, 3584, 4096, 4104, 5120, 6152, 8192])
 @pytest.mark.parametrize("mode", [0, 1])
