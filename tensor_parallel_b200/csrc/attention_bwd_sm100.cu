@@ -74,6 +74,14 @@ struct BwParams {
 
 // ---- what the elementwise warps of both kernels do with 32 columns (streamed rows) of one TMEM lane (resident row) ----
 
+// Bits lo to hi - 1 of 32.
+__device__ __forceinline__ uint32_t bw_bits(int lo, int hi) {
+  uint32_t bits = 0xffffffffu;
+  if (lo > 0) bits = lo < 32 ? bits << lo : 0u;
+  if (hi < 32) bits = hi > 0 ? bits & (0xffffffffu >> (32 - hi)) : 0u;
+  return bits;
+}
+
 // Bits of the columns from col0 on that are visible pairs with resident row ri; only steps that touch the diagonal or an end have any cleared.
 template <bool DKV>
 __device__ __forceinline__ uint32_t bw_visible(const BwParams& p, int ri, int shift, int col0) {
@@ -84,10 +92,7 @@ __device__ __forceinline__ uint32_t bw_visible(const BwParams& p, int ri, int sh
   } else {
     hi = min(32, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0);  // key <= query + shift
   }
-  uint32_t visible = 0xffffffffu;
-  if (lo > 0) visible = lo < 32 ? visible << lo : 0u;
-  if (hi < 32) visible = hi > 0 ? visible & (0xffffffffu >> (32 - hi)) : 0u;
-  return visible;
+  return bw_bits(lo, hi);
 }
 
 // Eight score biases of resident row `row` from column `col` of a step on, out of the step's tile in shared memory.
@@ -966,6 +971,267 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
+// ---- gradient of a bias that several (batch, head) pairs share ----
+//
+// d(bias)[i, j] = sum over the pairs of P (dP - delta).  Inside the dQ launch every pair adds its own 4 bytes per score into one fp32 buffer: 134 M
+// reductions for 16 x 512 tokens and 32 heads, 126 us of its 235.  Here a CTA owns a tile of 128 queries x 128 keys of the bias and walks the pairs:
+// S = Q K^T and dP = dO V^T once more (seven tile products become nine), the sum of P (dP - delta) in registers, one store at the end and no
+// buffer to clear.  Sums run in a fixed order.
+//
+//   warp 0     : TMA producer, the four tiles of a pair (Q, dO, K, V) per stage of a ring
+//   warp 1     : MMA issuer, S and dP of pair n + 1 while the other warps are at pair n (two buffers of each: 512 TMEM columns)
+//   warps 2-17 : a thread per query and 32 keys, their sums in registers, their biases (the same for every pair) in slots of its own in shared memory
+//
+// Tile and pair take 2000 clocks: an exponential per score, 1024 on the special-function unit, and the latencies of barrier and TMEM around
+// them, which two halves of the keys with barriers of their own hide in part (114 -> 110 us).  16 x 512 tokens, 32 heads: 110 us; whole
+// backward with it 333 us, with reductions in the dQ launch, the buffer to clear and the cast to bf16 361.  Where it pays: ops/native.py.
+constexpr int BG_STAGES = 3, BG_WARPS = 16, BG_THREADS = 64 + 32 * BG_WARPS;
+constexpr int BG_HALVES = 2, BG_COLS = BW_R / BG_HALVES;  // products, hand-over and warps by halves of the keys: while one half waits, the other computes
+template <int D>
+constexpr size_t bg_smem_bytes() { return size_t(BG_STAGES) * 4 * (D / 64) * FA_BLOCK_BYTES + BW_R * BW_R * 2 + 20 * 8 + 1024; }
+
+struct BgParams {
+  int batch, sq, sk, q_heads, kv_heads, causal;
+  float scale_log2e;
+  const float *lse, *delta;  // [batch][q_heads][sq]
+  const bf16* bias;          // element strides over (head, query), keys contiguous; b_sh = 0: shared by the heads too
+  void* dbias;               // in the bias' own strides
+  int dbias_fp32;
+  long long b_sh, b_sq;
+  uint32_t* status;
+};
+
+template <int D>
+__global__ void __launch_bounds__(BG_THREADS, 1)
+attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do, const __grid_constant__ CUtensorMap tmap_k,
+                      const __grid_constant__ CUtensorMap tmap_v, const BgParams p) {
+  constexpr int DB = D / 64;
+  constexpr uint32_t TILE = DB * FA_BLOCK_BYTES, STAGE = 4 * TILE;
+  constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BG_COLS, false, false);
+  extern __shared__ uint8_t bg_smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(bg_smem_raw) + 1023) & ~uintptr_t(1023));
+  uint4* bias_s = reinterpret_cast<uint4*>(smem + BG_STAGES * STAGE);  // [4 chunks of 8 keys][threads], private
+  uint64_t* t_full = reinterpret_cast<uint64_t*>(bias_s + 4 * 32 * BG_WARPS);
+  uint64_t* t_empty = t_full + BG_STAGES;
+  uint64_t* s_full = t_empty + BG_STAGES;      // [2 buffers][2 halves of the keys]: S and dP of a pair are there
+  uint64_t* s_done = s_full + 2 * BG_HALVES;   // and have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_done + 2 * BG_HALVES);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int k0 = blockIdx.x * BW_R, q0 = blockIdx.y * BW_R, plane = blockIdx.z;
+  const int shift = p.sk - p.sq, group = p.q_heads / p.kv_heads;
+  const int heads = p.b_sh ? 1 : p.q_heads;  // heads that share the plane
+  const bool any = !p.causal || k0 <= min(p.sq, q0 + BW_R) - 1 + shift;  // (otherwise no query of the tile sees a key of it)
+  const int pairs = any ? p.batch * heads : 0;
+
+  if (threadIdx.x == 0) {
+    prefetch_tmap(&tmap_q);
+    prefetch_tmap(&tmap_do);
+    prefetch_tmap(&tmap_k);
+    prefetch_tmap(&tmap_v);
+    for (int s = 0; s < BG_STAGES; ++s) {
+      mbar_init(&t_full[s], 1);
+      mbar_init(&t_empty[s], 1);
+    }
+    for (int s = 0; s < 2 * BG_HALVES; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&s_done[s], BG_WARPS / BG_HALVES);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  auto give_up = [&]() {
+    atomicMax(p.status, STATUS_TIMEOUT_MBAR);
+    *abort_flag = 1;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int n = 0, b = 0, h = plane; n < pairs; ++n) {
+        const int s = n % BG_STAGES;
+        if (*abort_flag || !mbar_wait(&t_empty[s], ((n / BG_STAGES) & 1) ^ 1)) {
+          if (!*abort_flag) give_up();
+          break;
+        }
+        uint8_t* dst = smem + s * STAGE;
+        mbar_expect_tx(&t_full[s], STAGE);
+#pragma unroll
+        for (int d = 0; d < DB; ++d) {
+          tma_load_4d(dst + d * FA_BLOCK_BYTES, &tmap_q, &t_full[s], d * 64, q0, h, b);
+          tma_load_4d(dst + 2 * TILE + d * FA_BLOCK_BYTES, &tmap_k, &t_full[s], d * 64, k0, h / group, b);
+          tma_load_4d(dst + TILE + d * FA_BLOCK_BYTES, &tmap_do, &t_full[s], d * 64, q0, h, b);
+          tma_load_4d(dst + 3 * TILE + d * FA_BLOCK_BYTES, &tmap_v, &t_full[s], d * 64, k0, h / group, b);
+        }
+        if (heads > 1 && ++h < heads) continue;
+        if (heads > 1) h = 0;
+        ++b;
+      }
+    }
+  } else if (warp == 1) {
+    const uint32_t leader = elect_one();
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+      const bool there = __all_sync(0xffffffffu, !*abort_flag && mbar_wait(bar, parity));
+      if (!there && leader && !*abort_flag) give_up();
+      tc_fence_after();
+      return there;
+    };
+    for (int n = 0; n < pairs; ++n) {
+      const int s = n % BG_STAGES, buf = n & 1;
+      if (!wait_all(&t_full[s], (n / BG_STAGES) & 1)) break;
+      const uint32_t at = smem_u32(smem + s * STAGE);
+      bool ok = true;
+#pragma unroll
+      for (int half = 0; half < BG_HALVES; ++half) {
+        if (n >= 2) ok = ok && wait_all(&s_done[buf * BG_HALVES + half], ((n >> 1) & 1) ^ 1);
+        if (!ok) break;
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+          const uint32_t a_lo = desc_kmajor_lo(at + which * TILE), b_lo = desc_kmajor_lo(at + (2 + which) * TILE + half * BG_COLS * 128);
+#pragma unroll
+          for (int i = 0; i < DB * 4; ++i) {
+            const uint32_t off = (i >> 2) * (FA_BLOCK_BYTES >> 4) + (i & 3) * 2;
+            umma_bf16_lead(leader, tmem_base + buf * 256 + which * 128 + half * BG_COLS, a_lo + off, b_lo + off, IDESC_S, i ? 1u : 0u);
+          }
+        }
+        umma_commit_lead(leader, &s_full[buf * BG_HALVES + half]);
+      }
+      if (!ok) break;
+      umma_commit_lead(leader, &t_empty[s]);
+    }
+  } else {
+    constexpr int HC = BW_R / 4;
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
+    const int ri = q0 + quarter * 32 + lane, col0 = k0 + part * HC;
+    const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16) + part * HC;
+    const bool row_ok = ri < p.sq;
+    const long long row_at = plane * p.b_sh + (long long)ri * p.b_sq + col0;
+    const uint32_t visible = row_ok ? bw_bits(0, min(p.sk, p.causal ? ri + shift + 1 : p.sk) - col0) : 0u;
+    const bool masked = __any_sync(0xffffffffu, visible != 0xffffffffu);  // (per warp)
+    uint4* my_bias = bias_s + threadIdx.x - 64;
+#pragma unroll
+    for (int c = 0; c < HC; c += 8) {
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if (row_ok && col0 + c + 8 <= p.sk) {
+        u = __ldg(reinterpret_cast<const uint4*>(p.bias + row_at + c));
+      } else if (row_ok) {
+        uint32_t* w = &u.x;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (col0 + c + i < p.sk) w[i >> 1] |= uint32_t(__bfloat16_as_ushort(p.bias[row_at + c + i])) << (16 * (i & 1));
+      }
+      my_bias[c / 8 * (32 * BG_WARPS)] = u;
+    }
+    float acc[HC];
+#pragma unroll
+    for (int c = 0; c < HC; ++c) acc[c] = 0.f;
+    // my row of the pairs' statistics: the pairs are batches (one head's plane) or all heads of all batches, one [sq] row apart or q_heads of them
+    const long long stat_step = heads > 1 ? p.sq : (long long)p.q_heads * p.sq;
+    const float *lse_at = p.lse + (long long)plane * p.sq + ri, *delta_at = p.delta + (long long)plane * p.sq + ri;
+    float l2 = -INFINITY, del = 0.f;  // -lse * log2(e) (-inf: no such query, or none of its keys visible) and -delta
+    auto stats = [&]() {
+      const float l = __ldg(lse_at);
+      l2 = l != -INFINITY ? -l * 1.4426950408889634f : -INFINITY;
+      del = -__ldg(delta_at);
+      lse_at += stat_step;
+      delta_at += stat_step;
+    };
+    if (row_ok && pairs > 0) stats();
+    bool alive = true;
+    for (int n = 0; n < pairs; ++n) {
+      const int buf = n & 1;
+      const float l2_now = l2, del_now = del;
+      if (row_ok && n + 1 < pairs) stats();
+      if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&s_full[buf * BG_HALVES + part * BG_HALVES / 4], (n >> 1) & 1))) {
+        if (lane == 0 && !*abort_flag) give_up();
+        alive = false;
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int c0 = 0; c0 < HC; c0 += 16) {
+        uint32_t sv[16], dv[16];
+        tmem_ld_x16(t_lane + buf * 256 + c0, sv);
+        tmem_ld_x16(t_lane + buf * 256 + 128 + c0, dv);
+        const uint4 u0 = my_bias[(c0 / 8) * (32 * BG_WARPS)], u1 = my_bias[(c0 / 8 + 1) * (32 * BG_WARPS)];
+        const uint32_t bw[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};  // bf16 pairs
+        tmem_ld_wait();
+        if (c0 + 16 == HC) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_done[buf * BG_HALVES + part * BG_HALVES / 4]);
+        }
+        float odd0 = 0.f, odd1 = 0.f;  // not 0 if a dP is not finite
+#pragma unroll
+        for (int c = 0; c < 16; c += 2) {
+          constexpr float LOG2E = 1.4426950408889634f;
+          const uint32_t w = bw[c / 2];
+          float x0, x1, g0, g1;
+          ffma2(x0, x1, __uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u), LOG2E, LOG2E, l2_now, l2_now);
+          ffma2(x0, x1, __uint_as_float(sv[c]), __uint_as_float(sv[c + 1]), p.scale_log2e, p.scale_log2e, x0, x1);
+          sv[c] = __float_as_uint(ex2_approx(x0));
+          sv[c + 1] = __float_as_uint(ex2_approx(x1));
+          fadd2(g0, g1, __uint_as_float(dv[c]), __uint_as_float(dv[c + 1]), del_now, del_now);
+          dv[c] = __float_as_uint(g0);
+          dv[c + 1] = __float_as_uint(g1);
+          ffma2(odd0, odd1, g0, g1, 0.f, 0.f, odd0, odd1);
+        }
+        // pairs of a query and a key that are out of range or masked contribute nothing, whatever their dP is
+        if (masked) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            if (!(visible >> (c0 + c) & 1)) sv[c] = 0u;
+        }
+        if (odd0 + odd1 != 0.f) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            if (sv[c] == 0u) dv[c] = 0u;
+        }
+#pragma unroll
+        for (int c = 0; c < 16; c += 2)
+          ffma2(acc[c0 + c], acc[c0 + c + 1], __uint_as_float(sv[c]), __uint_as_float(sv[c + 1]), __uint_as_float(dv[c]), __uint_as_float(dv[c + 1]), acc[c0 + c],
+                acc[c0 + c + 1]);
+      }
+    }
+    if (alive && row_ok) {
+#pragma unroll
+      for (int c = 0; c < HC; c += 8) {
+        if (col0 + c + 8 <= p.sk) {
+          if (p.dbias_fp32) {
+            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.dbias) + row_at + c);
+            dst[0] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+            dst[1] = make_float4(acc[c + 4], acc[c + 5], acc[c + 6], acc[c + 7]);
+          } else {
+            *reinterpret_cast<uint4*>(static_cast<bf16*>(p.dbias) + row_at + c) =
+                make_uint4(pack_bf16x2(acc[c], acc[c + 1]), pack_bf16x2(acc[c + 2], acc[c + 3]), pack_bf16x2(acc[c + 4], acc[c + 5]), pack_bf16x2(acc[c + 6], acc[c + 7]));
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (col0 + c + i >= p.sk) continue;
+            if (p.dbias_fp32) static_cast<float*>(p.dbias)[row_at + c + i] = acc[c + i];
+            else static_cast<bf16*>(p.dbias)[row_at + c + i] = __float2bfloat16(acc[c + i]);
+          }
+        }
+      }
+    }
+  }
+
+  // ---------------- teardown ----------------
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+
 template <int D, bool DKV, int BIAS, int T>
 static int bw_launch_wide(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& tb,
                           const BwParams& p, dim3 grid, cudaStream_t stream) {
@@ -1125,4 +1391,52 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   p.out1 = nullptr;
   p.dbias = dbias;
   return launch(std::false_type{}, q128, do128, ks, vs, b_q, dim3((sq + BW_R - 1) / BW_R, q_heads, batch));
+}
+
+// Gradient of a bf16 score bias that the batches share (bias_sb = 0; bias_sh = 0: the heads as well), for head_dim 64: dbias has the bias' strides and
+// is written, not added to.  lse, delta: [batch][q_heads][sq], delta as tpb_attn_backward_sm100 left it.  Other arguments as there.
+extern "C" int tpb_attn_bias_grad_sm100(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* delta, int batch, int sq,
+                                        int sk, int q_heads, int kv_heads, int head_dim, long long q_sb, long long q_ss, long long q_sh, long long k_sb,
+                                        long long k_ss, long long k_sh, long long v_sb, long long v_ss, long long v_sh, long long do_sb, long long do_ss,
+                                        long long do_sh, int causal, float scale, const void* bias, long long bias_sh, long long bias_sq, void* dbias,
+                                        int dbias_fp32, void* status, void* stream_) {
+  if (!q || !k || !v || !dout || !lse || !delta || !bias || !dbias || !status || batch <= 0 || sq <= 0 || sk <= 0 || q_heads <= 0 || kv_heads <= 0 ||
+      q_heads % kv_heads || bias_sq <= 0 || bias_sh < 0 || !(scale > 0.f))
+    return TPB_ERR_ARG;
+  const int q_tiles = (sq + BW_R - 1) / BW_R, k_tiles = (sk + BW_R - 1) / BW_R, planes = bias_sh ? q_heads : 1;
+  if (head_dim != 64 || q_tiles > 65535 || planes > 65535) return TPB_ERR_SIZE;
+  const long long strides[] = {q_ss, k_ss, v_ss, do_ss, q_heads > 1 ? q_sh : 0, q_heads > 1 ? do_sh : 0, kv_heads > 1 ? k_sh : 0,
+                               kv_heads > 1 ? v_sh : 0, batch > 1 ? q_sb : 0, batch > 1 ? k_sb : 0, batch > 1 ? v_sb : 0, batch > 1 ? do_sb : 0, bias_sh, bias_sq};
+  for (long long s : strides)
+    if (s & 7) return TPB_ERR_ALIGN;
+  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dout | (uintptr_t)bias | (uintptr_t)dbias) & 15) return TPB_ERR_ALIGN;
+  if (fa_bind_thread() != TPB_OK) return TPB_ERR_CUDA;
+  CUtensorMap tq, tdo, tk, tv;
+  int rc = fa_tmap(&tq, q, head_dim, BW_R, sq, q_heads, batch, q_ss, q_sh, q_sb);
+  if (rc == TPB_OK) rc = fa_tmap(&tdo, dout, head_dim, BW_R, sq, q_heads, batch, do_ss, do_sh, do_sb);
+  if (rc == TPB_OK) rc = fa_tmap(&tk, k, head_dim, BW_R, sk, kv_heads, batch, k_ss, k_sh, k_sb);
+  if (rc == TPB_OK) rc = fa_tmap(&tv, v, head_dim, BW_R, sk, kv_heads, batch, v_ss, v_sh, v_sb);
+  if (rc != TPB_OK) return rc;
+  BgParams p;
+  memset(&p, 0, sizeof(p));
+  p.batch = batch; p.sq = sq; p.sk = sk; p.q_heads = q_heads; p.kv_heads = kv_heads; p.causal = causal;
+  p.scale_log2e = scale * 1.4426950408889634f;
+  p.lse = lse;
+  p.delta = delta;
+  p.bias = static_cast<const bf16*>(bias);
+  p.dbias = dbias;
+  p.dbias_fp32 = dbias_fp32;
+  p.b_sh = bias_sh; p.b_sq = bias_sq;
+  p.status = static_cast<uint32_t*>(status);
+  constexpr size_t smem = bg_smem_bytes<64>();
+  static_assert(smem <= 227 * 1024, "shared memory of a CTA");
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(attn_bias_grad_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return TPB_ERR_CUDA;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  attn_bias_grad_kernel<64><<<dim3(k_tiles, q_tiles, planes), BG_THREADS, smem, static_cast<cudaStream_t>(stream_)>>>(tq, tdo, tk, tv, p);
+  return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }

@@ -657,6 +657,23 @@ def attention_forward(q, k, v, causal, scale, want_lse=False, bias=None, out=Non
 LIB.tpb_attn_backward.argtypes = [c_void_p] * 10 + [c_int] * 6 + [c_ll] * 21 + [c_int, c_float, c_void_p]
 LIB.tpb_attn_backward_bias.argtypes = [c_void_p] * 10 + [c_int] * 6 + [c_ll] * 21 + [c_int, c_float, c_void_p, c_int] + [c_ll] * 4 + [c_void_p, c_void_p]
 LIB.tpb_attn_backward_sm100.argtypes = [c_void_p] * 10 + [c_int] * 6 + [c_ll] * 21 + [c_int, c_float, c_void_p, c_int] + [c_ll] * 4 + [c_void_p, c_void_p, c_void_p]
+LIB.tpb_attn_bias_grad_sm100.argtypes = [c_void_p] * 6 + [c_int] * 6 + [c_ll] * 12 + [c_int, c_float, c_void_p, c_ll, c_ll, c_void_p, c_int, c_void_p, c_void_p]
+
+
+def _bias_grad_tiles(b, sq, sk, hq, d, bias4, strides) -> bool:
+    """Whether the gradient of a bf16 score bias that the batches share is summed up tile by tile (``tpb_attn_bias_grad_sm100``, a CTA per tile of
+    128 x 128 pairs), not added up by the dQ launch.  It recomputes the scores of every batch, and pays where its CTAs fill the SMs with whole
+    tiles.  Whole backwards at head_dim 64, added up / summed by tile, in us: 16 x 512, 32 heads 361 / 333, 8 heads (128 CTAs) 104 / 91; 16 x 256, 32
+    heads (128) 116 / 111, 16 heads (64) 62 / 70; 16 x 200, 32 heads 102 / 102; 4 x 1024, 32 heads 559 / 349.  With one or two batches, nothing or
+    little to sum: 1 x 512, 32 heads (512) 44 / 48, 8 heads 34 / 29; 1 x 1024, 32 heads 187 / 147."""
+    sb, sh, sr, sc = strides
+    if d != 64 or bias4.dtype != torch.bfloat16 or sb != 0 or sc != 1 or sr <= 0 or sr % 8 or sh % 8 or bias4.data_ptr() % 16:
+        return False
+    tiles, planes = -(-sq // 128) * -(-sk // 128), hq if sh else 1
+    ctas = tiles * planes
+    if ctas < 120 or sq * sk < 0.75 * tiles * 128 * 128:
+        return False
+    return ctas <= 148 or ctas >= 1024 or b * (1 if sh else hq) >= 4
 
 
 def _bias_view(bias):
@@ -665,9 +682,9 @@ def _bias_view(bias):
     return bias4, [0 if bias4.shape[i] == 1 else bias4.stride(i) for i in range(4)]
 
 
-def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_dbias=False):
+def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_dbias=False, dbias_dtype=torch.float32):
     """Gradients of :func:`attention_forward` (scores are recomputed tile by tile).  With ``bias`` the scores are
-    re-biased; ``want_dbias`` also returns the gradient of the bias (fp32, in the bias' own shape)."""
+    re-biased; ``want_dbias`` also returns the gradient of the bias (summed in fp32, returned as ``dbias_dtype``, in the bias' own shape)."""
     global _launches
     q, k, v, dout = (t if _strided_ok(t) else t.contiguous() for t in (q, k, v, dout))
     b, sq, hq, d = q.shape
@@ -677,15 +694,16 @@ def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_d
     dv = torch.empty(b, sk, hkv, d, dtype=q.dtype, device=q.device)
     delta = torch.empty(b, hq, sq, dtype=torch.float32, device=q.device)
     scale = 1.0 / math.sqrt(d) if scale is None else scale
-    bias4, bstr, dbias = None, [0, 0, 0, 0], None
+    bias4, bstr, dbias, tiles = None, [0, 0, 0, 0], None, False
     if bias is not None:
         bias4, bstr = _bias_view(bias)
         if want_dbias:  # dense fp32 buffer in the bias' shape: the kernel addresses it with the bias' broadcast pattern
-            dbias = torch.zeros(bias4.shape, dtype=torch.float32, device=q.device)
-            dstr = [0 if dbias.shape[i] == 1 else dbias.stride(i) for i in range(4)]
+            dstr = [0 if n == 1 else math.prod(bias4.shape[i + 1:]) for i, n in enumerate(bias4.shape)]
             if dstr != bstr:  # a non-contiguous bias view: keep one addressing for both
                 bias4 = bias4.contiguous()
                 bstr = dstr
+            tiles = not _LEGACY_ATTENTION and dbias_dtype in (torch.float32, torch.bfloat16) and _bias_grad_tiles(b, sq, sk, hq, d, bias4, bstr)
+            dbias = torch.empty(bias4.shape, dtype=dbias_dtype, device=q.device) if tiles else torch.zeros(bias4.shape, dtype=torch.float32, device=q.device)
     bias_is_fp32 = 1 if (bias4 is not None and bias4.dtype == torch.float32) else 0
     if not _LEGACY_ATTENTION:  # tcgen05 kernels (two launches of one template) + the delta kernel
         status = device_state(q.device).status
@@ -695,11 +713,18 @@ def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_d
                                           v.stride(0), v.stride(1), v.stride(2), out.stride(0), out.stride(1), out.stride(2),
                                           dout.stride(0), dout.stride(1), dout.stride(2), dq.stride(0), dq.stride(1), dq.stride(2),
                                           dk.stride(0), dk.stride(1), dk.stride(2), int(causal), scale, _ptr(bias4), bias_is_fp32,
-                                          bstr[0], bstr[1], bstr[2], bstr[3], _ptr(dbias), _ptr(status), _stream()),
+                                          bstr[0], bstr[1], bstr[2], bstr[3], None if tiles else _ptr(dbias), _ptr(status), _stream()),
               "tpb_attn_backward_sm100")
         _launches += 3
+        if tiles:
+            check(LIB.tpb_attn_bias_grad_sm100(_ptr(q), _ptr(k), _ptr(v), _ptr(dout), _ptr(lse), _ptr(delta), b, sq, sk, hq, hkv, d,
+                                               q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
+                                               v.stride(0), v.stride(1), v.stride(2), dout.stride(0), dout.stride(1), dout.stride(2),
+                                               int(causal), scale, _ptr(bias4), bstr[1], bstr[2], _ptr(dbias), int(dbias_dtype == torch.float32),
+                                               _ptr(status), _stream()), "tpb_attn_bias_grad_sm100")
+            _launches += 1
         if want_dbias:
-            return dq, dk, dv, dbias.reshape(bias.shape)
+            return dq, dk, dv, dbias.reshape(bias.shape).to(dbias_dtype)
         return dq, dk, dv
     check(LIB.tpb_attn_backward_bias(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(dout), _ptr(lse), _ptr(delta), _ptr(dq), _ptr(dk), _ptr(dv),
                                      b, sq, sk, hq, hkv, d,
@@ -711,7 +736,7 @@ def attention_backward(q, k, v, out, dout, lse, causal, scale, bias=None, want_d
                                      _ptr(dbias), _stream()), "tpb_attn_backward")
     _launches += 3
     if want_dbias:
-        return dq, dk, dv, dbias.reshape(bias.shape)
+        return dq, dk, dv, dbias.reshape(bias.shape).to(dbias_dtype)
     return dq, dk, dv
 
 
@@ -728,9 +753,9 @@ class _AttentionFn(torch.autograd.Function):
         q, k, v, out, lse = ctx.saved_tensors[:5]
         bias = ctx.saved_tensors[5] if ctx.has_bias else None
         want_dbias = ctx.has_bias and ctx.needs_input_grad[5]
-        grads = attention_backward(q, k, v, out, grad.to(q.dtype), lse, ctx.causal, ctx.scale, bias=bias, want_dbias=want_dbias)
-        dbias = grads[3].to(bias.dtype) if want_dbias else None
-        return grads[0], grads[1], grads[2], None, None, dbias
+        grads = attention_backward(q, k, v, out, grad.to(q.dtype), lse, ctx.causal, ctx.scale, bias=bias, want_dbias=want_dbias,
+                                   dbias_dtype=bias.dtype if want_dbias else torch.float32)
+        return grads[0], grads[1], grads[2], None, None, grads[3] if want_dbias else None
 
 
 def _keys_contiguous(bias):

@@ -866,6 +866,34 @@ def test_attention_with_two_ctas_per_sm(b, sq, sk, hq, hkv, causal, bias):
         assert (t.grad.double() - ref.grad).norm() <= 0.01 * ref.grad.norm() + 1e-6
 
 
+# a tile per CTA for the gradient of a shared bias: whole tiles, ragged ones, rows of a multiple of eight, more keys than queries, a plane for all heads
+@pytest.mark.parametrize("b,sq,sk,hq,hkv,shared", [(3, 256, 256, 32, 32, False), (1, 240, 248, 30, 15, False), (2, 384, 1000, 6, 6, False), (5, 1152, 1792, 2, 1, True)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_attention_bias_gradient_by_tiles(b, sq, sk, hq, hkv, shared, causal, dtype):
+    """Against 64 bits; the same bits every time; masked pairs contribute nothing, whatever their values."""
+    nat = _native()
+    torch.manual_seed(sq)
+    q, k, v = (torch.randn(b, s, h, 64, device="cuda", dtype=torch.bfloat16) for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
+    g = torch.randn(b, sq, hq, 64, device="cuda", dtype=torch.bfloat16)
+    bias = torch.randn(1, 1 if shared else hq, sq, sk, device="cuda", dtype=torch.bfloat16)
+    bias[..., 3] = -math.inf
+    strides = [0 if n == 1 else st for n, st in zip(bias.shape, bias.stride())]
+    assert nat._bias_grad_tiles(b, sq, sk, hq, 64, bias, strides)
+    out, lse = nat.attention_forward(q, k, v, causal, None, want_lse=True, bias=bias)
+    got = nat.attention_backward(q, k, v, out, g, lse, causal, None, bias=bias, want_dbias=True, dbias_dtype=dtype)[3]
+    assert got.dtype == dtype and got.shape == bias.shape and not bool(got[..., 3].any())
+    assert torch.equal(got, nat.attention_backward(q, k, v, out, g, lse, causal, None, bias=bias, want_dbias=True, dbias_dtype=dtype)[3])
+    leaf = bias.double().requires_grad_()
+    _attention_double(q.double(), k.double(), v.double(), causal, leaf).backward(g.double())
+    # delta is taken from the rounded output (2^-9, independent over 64 elements); bf16 results are rounded once more
+    assert (got.double() - leaf.grad).norm() <= 0.006 * leaf.grad.norm()
+    v2 = v.clone()
+    v2[:, 3] = math.inf  # dP is not finite where the probability is 0
+    inf = nat.attention_backward(q, k, v2, out, g, lse, causal, None, bias=bias, want_dbias=True, dbias_dtype=dtype)[3]
+    assert torch.equal(inf, got)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("cols", [8, 264, 776, 1024, 1536, 1544, 1800, 2048, 2568, 3072, 3080, 3584, 4096, 4104, 5120, 6152, 8192])
 @pytest.mark.parametrize("mode", [0, 1])
