@@ -73,8 +73,11 @@ class T5Attention(nn.Module):
 
     def compute_bias(self, query_length: int, key_length: int, device):
         # query i sits at position i + key_length - query_length: the distances run from -(key_length - 1) to query_length - 1
-        distance = torch.arange(1 - key_length, max(query_length, 1 - key_length), device=device)  # (none without queries and keys)
-        buckets = relative_position_bucket(distance, not self.is_decoder, self.relative_attention_num_buckets, self.relative_attention_max_distance)
+        first, last = 1 - key_length, max(query_length, 1 - key_length)  # (none without queries and keys)
+        rule = (not self.is_decoder, self.relative_attention_num_buckets, self.relative_attention_max_distance)
+        buckets = OF.relative_buckets(first, last - first, device, *rule)
+        if buckets is None:
+            buckets = relative_position_bucket(torch.arange(first, last, device=device), *rule)
         return OF.relative_bias(self.relative_attention_bias, buckets, query_length, key_length)  # [1, heads, q, k]
 
     def forward(self, hidden_states, mask=None, key_value_states=None, position_bias=None, past_key_value=None, use_cache=False):

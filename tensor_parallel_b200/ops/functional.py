@@ -186,6 +186,18 @@ def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
     return relative_bias_ref(embedding, buckets, queries, keys)
 
 
+def relative_buckets(first: int, count: int, device, bidirectional: bool, buckets: int, max_distance: int):
+    """Relative-position buckets of the distances ``first``, ``first + 1``, ... by one kernel, or None where the caller has to take the steps over
+    tensors (other devices, tracing, dispatch modes, ranges that the kernel does not cover)."""
+    exact = buckets // (4 if bidirectional else 2)
+    if (torch.device(device).type != "cuda" or _FORCE_TORCH or not 0 < count <= 2 ** 31 or exact < 1 or max_distance <= exact
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()):
+        return None
+    from tensor_parallel_b200.ops import native
+
+    return native.relative_buckets(first, count, device, bidirectional, buckets, max_distance)
+
+
 def gelu(x, approximate: str = "none"):
     nat = _native(x)
     if nat is not None and nat.elementwise_supported(x):

@@ -861,6 +861,19 @@ def relative_bias_supported(table: torch.Tensor, queries: int, keys: int) -> boo
             and keys > 0)
 
 
+LIB.tpb_relative_buckets.argtypes = [c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_void_p]
+
+
+def relative_buckets(first: int, count: int, device, bidirectional: bool, buckets: int, max_distance: int) -> torch.Tensor:
+    """int64 ``[count]``: the relative-position buckets of the distances from ``first`` up (T5: exact below half of a direction's buckets,
+    logarithmic up to ``max_distance``)."""
+    global _launches
+    out = torch.empty(count, dtype=torch.int64, device=device)
+    check(LIB.tpb_relative_buckets(_ptr(out), first, count, int(bidirectional), buckets, max_distance, _stream()), "tpb_relative_buckets")
+    _launches += 1
+    return out
+
+
 class _RelativeBiasFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, table, buckets, queries, keys):

@@ -826,6 +826,20 @@ def test_norm_of_as_many_rows_as_an_int_counts():
     torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("bidirectional", [False, True])
+@pytest.mark.parametrize("buckets,max_distance", [(32, 128), (32, 20), (4, 100), (7, 90), (12, 1000), (64, 100000), (30, 333), (256, 4096)])
+def test_relative_buckets_are_those_of_the_tensor_steps(bidirectional, buckets, max_distance):
+    from tensor_parallel_b200.models.t5 import relative_position_bucket
+
+    device = torch.device("cuda", 0)
+    for first, count in ((-200000, 400001), (-511, 1023), (0, 1), (1, 70), (-(2 ** 40), 300), (2 ** 40, 300)):
+        got = OF.relative_buckets(first, count, device, bidirectional, buckets, max_distance)
+        assert got is not None
+        assert torch.equal(got, relative_position_bucket(torch.arange(first, first + count, device=device), bidirectional, buckets, max_distance))
+    for args in ((0, 0, device, bidirectional, buckets, max_distance), (0, 5, "cpu", bidirectional, buckets, max_distance), (0, 5, device, True, 3, 100), (0, 5, device, False, 32, 16)):
+        assert OF.relative_buckets(*args) is None
+
+
 def _attention_double(q, k, v, causal, bias):
     """Output, and what backward needs, of 64-bit attention over leaves of q, k, v and the bias."""
     scores = torch.einsum("bqhd,bkhd->bhqk", q, k.repeat_interleave(q.shape[2] // k.shape[2], 2)) / math.sqrt(q.shape[-1])
