@@ -55,6 +55,25 @@ class Linear(nn.Linear):
         return OF.linear(x, self.weight, self.bias)
 
 
+def _only_multiplies(module: nn.Module) -> bool:
+    """False for a module whose call does more than one product with its weight: another class (wrappers of parallel shards, adapters,
+    parametrisations), a bias, a ``forward`` put on the instance, hooks of its own or of all modules, a weight that is a tensor subclass."""
+    every = torch.nn.modules.module
+    hooks = (module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks, every._global_forward_hooks,
+             every._global_forward_pre_hooks, every._global_backward_hooks, every._global_backward_pre_hooks)
+    return (type(module) is Linear and module.bias is None and "forward" not in vars(module) and type(module.weight) in (nn.Parameter, torch.Tensor)
+            and not any(hooks))
+
+
+def linears(x, *modules: nn.Module):
+    """``tuple(module(x) for module in modules)``, as one autograd node where the modules are plain projections."""
+    if all(type(m) is Linear and _only_multiplies(m) for m in modules):
+        outs = OF.linears(x, [m.weight for m in modules])
+        if outs is not None:
+            return tuple(outs)
+    return tuple(m(x) for m in modules)
+
+
 class Conv1D(nn.Module):
     """GPT-2 style linear layer storing ``weight[in, out]`` and its width as ``nf``."""
 

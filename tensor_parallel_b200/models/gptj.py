@@ -8,7 +8,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from tensor_parallel_b200.models.common import CausalLMBase, LayerNorm, Linear, ModelOutput, ShapedConfig, init_weights_, past_length, update_kv
+from tensor_parallel_b200.models.common import CausalLMBase, LayerNorm, Linear, ModelOutput, ShapedConfig, init_weights_, linears, past_length, update_kv
 from tensor_parallel_b200.ops import functional as OF
 
 
@@ -40,7 +40,7 @@ class GPTJAttention(nn.Module):
 
     def _qkv(self, hidden_states):
         b, s, _ = hidden_states.shape
-        return tuple(p(hidden_states).view(b, s, -1, self.head_dim) for p in (self.q_proj, self.k_proj, self.v_proj))
+        return tuple(t.view(b, s, -1, self.head_dim) for t in linears(hidden_states, self.q_proj, self.k_proj, self.v_proj))
 
     def forward(self, hidden_states, layer_past=None, attention_mask=None, position_ids=None, use_cache=False):
         b, s, _ = hidden_states.shape

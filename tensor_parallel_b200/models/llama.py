@@ -11,7 +11,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from tensor_parallel_b200.models.common import CausalLMBase, Linear, ModelOutput, RMSNorm, ShapedConfig, init_weights_, past_length, update_kv
+from tensor_parallel_b200.models.common import CausalLMBase, Linear, ModelOutput, RMSNorm, ShapedConfig, init_weights_, linears, past_length, update_kv
 from tensor_parallel_b200.ops import functional as OF
 
 
@@ -47,9 +47,7 @@ class LlamaAttention(nn.Module):
     def forward(self, hidden_states, attention_mask=None, position_ids=None, past_key_value=None,
                 output_attentions=False, use_cache=False):
         b, s, _ = hidden_states.shape
-        q = self.q_proj(hidden_states).view(b, s, -1, self.head_dim)
-        k = self.k_proj(hidden_states).view(b, s, -1, self.head_dim)
-        v = self.v_proj(hidden_states).view(b, s, -1, self.head_dim)
+        q, k, v = (t.view(b, s, -1, self.head_dim) for t in linears(hidden_states, self.q_proj, self.k_proj, self.v_proj))
         q = OF.apply_rope(q, position_ids, self.rope_theta)
         k = OF.apply_rope(k, position_ids, self.rope_theta)
         k_all, v_all, present = update_kv(past_key_value, k, v)
@@ -66,7 +64,7 @@ class LlamaMLP(nn.Module):
         self.down_proj = Linear(config.intermediate_size, config.hidden_size, bias=False)
 
     def forward(self, x):
-        return self.down_proj(OF.swiglu(self.gate_proj(x), self.up_proj(x)))
+        return self.down_proj(OF.swiglu(*linears(x, self.gate_proj, self.up_proj)))
 
 
 class LlamaDecoderLayer(nn.Module):

@@ -12,7 +12,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from tensor_parallel_b200.models.common import Linear, ModelOutput, RMSNorm, ShapedConfig, init_weights_
+from tensor_parallel_b200.models.common import Linear, ModelOutput, RMSNorm, ShapedConfig, init_weights_, linears
 from tensor_parallel_b200.ops import functional as OF
 
 
@@ -83,17 +83,22 @@ class T5Attention(nn.Module):
     def forward(self, hidden_states, mask=None, key_value_states=None, position_bias=None, past_key_value=None, use_cache=False):
         b, s, _ = hidden_states.shape
         d = self.key_value_proj_dim
-        q = self.q(hidden_states).view(b, s, -1, d)
         is_cross = key_value_states is not None
         if is_cross and past_key_value is not None:
+            q = self.q(hidden_states)
             k_cache, v_cache = past_key_value[0], past_key_value[1]
         else:
             source = key_value_states if is_cross else hidden_states
-            k_cache = self.k(source).view(b, source.shape[1], -1, d).transpose(1, 2)
-            v_cache = self.v(source).view(b, source.shape[1], -1, d).transpose(1, 2)
+            if is_cross:
+                q, (k, v) = self.q(hidden_states), linears(source, self.k, self.v)
+            else:
+                q, k, v = linears(source, self.q, self.k, self.v)
+            k_cache = k.view(b, source.shape[1], -1, d).transpose(1, 2)
+            v_cache = v.view(b, source.shape[1], -1, d).transpose(1, 2)
             if not is_cross and past_key_value is not None:
                 k_cache = torch.cat((past_key_value[0], k_cache), dim=2)
                 v_cache = torch.cat((past_key_value[1], v_cache), dim=2)
+        q = q.view(b, s, -1, d)
         key_length = k_cache.shape[2]
         if position_bias is None:
             if self.has_relative_attention_bias:
@@ -151,7 +156,7 @@ class T5DenseGatedActDense(nn.Module):
         self.wo = Linear(config.d_ff, config.d_model, bias=False)
 
     def forward(self, x):
-        return self.wo(OF.geglu(self.wi_0(x), self.wi_1(x), approximate="tanh"))
+        return self.wo(OF.geglu(*linears(x, self.wi_0, self.wi_1), approximate="tanh"))
 
 
 class T5LayerFF(nn.Module):

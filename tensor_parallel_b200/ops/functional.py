@@ -125,6 +125,12 @@ def linear(x, weight, bias=None):
     return F.linear(x, weight, bias)
 
 
+def linears(x, weights):
+    """Several projections of ``x`` by one autograd node, or None where each has to be its own."""
+    nat = _native(x)
+    return nat.linears(x, weights) if nat is not None and nat.linears_supported(x, weights) else None
+
+
 def rms_norm(x, weight, eps: float = 1e-6):
     nat = _native(x)
     if nat is not None and nat.norm_supported(x):

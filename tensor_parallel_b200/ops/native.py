@@ -402,6 +402,17 @@ def linear(x, weight, bias=None):
     return AUTOGRAD.linear(x, weight, bias)
 
 
+def linears_supported(x, weights) -> bool:
+    """Whether several projections of ``x`` gain from one node (:func:`linears`): an input that takes a gradient, and the C++ nodes."""
+    return (AUTOGRAD is not None and torch.is_grad_enabled() and x.requires_grad and not torch._C._is_tracing()
+            and all(gemm_supported(x, w) for w in weights))
+
+
+def linears(x, weights):
+    """``[x @ w.T for w in weights]`` in one autograd node, which adds the input's gradients up inside its GEMMs."""
+    return AUTOGRAD.linears(x, list(weights))
+
+
 # ------------------------------------------------------------------------------------------------
 # norms
 # ------------------------------------------------------------------------------------------------

@@ -40,6 +40,8 @@ def _gemm(x, w, out, bias, residual, tokens, features, k, ldx, ldw, ld_out, act,
     y = a.float() @ b.float().t()
     if bias:
         y = y + _memory(bias, features, torch.bfloat16).float()
+    if residual:
+        y = y + _matrix(residual, tokens, features, ld_out).float()
     _matrix(out, tokens, features, ld_out).copy_(y)
     return _gemm.code
 
@@ -142,6 +144,67 @@ def test_linear_node(nodes, with_bias, frozen, form):
         assert (got is None) == (want is None)
         if want is not None:
             _close(got, want)
+
+
+@pytest.mark.parametrize("frozen", [(), (0,), (1, 3), (2,)])
+@pytest.mark.parametrize("unused", [(), (0,), (2,), (0, 1)])
+@pytest.mark.parametrize("form", ["plain", "three dimensions", "strided", "fp32 gradient"])
+def test_node_of_several_projections(nodes, frozen, unused, form):
+    """Against projections with nodes of their own: what an unused one leaves without a gradient, frozen leaves, shapes and strides."""
+    torch.manual_seed(0)
+    x = torch.randn(2, 5, 24, dtype=torch.bfloat16) if form == "three dimensions" else torch.randn(24, 10, dtype=torch.bfloat16).t()
+    if form == "plain":
+        x = x.contiguous()
+    values = [x] + [torch.randn(n, 24, dtype=torch.bfloat16) * 0.1 for n in (16, 8, 16)]
+    results = []
+    for call in (lambda x, ws: nodes.AUTOGRAD.linears(x, ws), lambda x, ws: [F.linear(x, w) for w in ws]):
+        leaves = [v.detach().requires_grad_(i not in frozen) for i, v in enumerate(values)]
+        outs = call(leaves[0], leaves[1:])
+        used = [o.float() if form == "fp32 gradient" else o for i, o in enumerate(outs) if i not in unused]
+        if any(o.requires_grad for o in used):
+            torch.autograd.backward(used, [torch.ones_like(o) + torch.arange(o.shape[-1]) // 4 / 4 for o in used])
+        results.append([o.detach() for o in outs] + [t.grad for t in leaves])
+    for got, want in zip(*results):
+        assert (got is None) == (want is None)
+        if want is not None:
+            _close(got, want)
+
+
+def test_modules_that_do_more_than_multiply_are_called_as_they_are(nodes, monkeypatch):
+    from tensor_parallel_b200.models import common
+
+    joint = []
+    monkeypatch.setattr(common.OF, "linears", lambda x, ws: joint.append(len(ws)) or [F.linear(x, w) for w in ws])
+
+    class Wrapped(common.Linear):
+        pass
+
+    def plain():
+        return common.Linear(8, 4, bias=False)
+
+    def hooked():
+        m = plain()
+        m.register_forward_hook(lambda module, args, out: out + 1)
+        return m
+
+    def replaced():
+        m = plain()
+        m.forward = lambda x: F.linear(x, m.weight) * 2
+        return m
+
+    x = torch.randn(3, 8)
+    for make in (lambda: Wrapped(8, 4, bias=False), lambda: common.Linear(8, 4), lambda: torch.nn.Linear(8, 4, bias=False), hooked, replaced,
+                 lambda: torch.nn.utils.parametrizations.weight_norm(plain()), lambda: torch.nn.Sequential(plain())):
+        modules = [plain(), make()]
+        assert all(torch.equal(a, m(x)) for a, m in zip(common.linears(x, *modules), modules)) and not joint
+    handle = torch.nn.modules.module.register_module_forward_pre_hook(lambda module, args: None)
+    common.linears(x, plain(), plain())
+    handle.remove()
+    assert not joint
+    modules = [plain(), plain()]
+    assert all(torch.equal(a, m(x)) for a, m in zip(common.linears(x, *modules), modules)) and joint == [2]
+    monkeypatch.undo()
+    assert len(common.linears(x.requires_grad_(), *modules)) == 2  # (on the CPU every module is called)
 
 
 @pytest.mark.parametrize("mode,dtype,wdtype,with_bias,with_weight", [(0, torch.bfloat16, torch.bfloat16, False, True), (0, torch.float32, torch.float32, False, True),
