@@ -28,6 +28,8 @@ struct Library {
   decltype(&tpb_norm_fwd) norm_fwd = nullptr;
   decltype(&tpb_norm_bwd) norm_bwd = nullptr;
   decltype(&tpb_norm_bwd_parts) norm_bwd_parts = nullptr;
+  decltype(&tpb_col_sum_parts) col_sum_parts = nullptr;
+  decltype(&tpb_col_sum) col_sum = nullptr;
 };
 Library lib;
 PyObject* error_text = nullptr;     // (code, what) -> message
@@ -116,6 +118,17 @@ std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
   return shape;
 }
 
+// The gradient of a bias: column sums of g in fp32, as `dtype`.
+Tensor column_sums(const Tensor& g, at::ScalarType dtype) {
+  if (!lib.col_sum || g.size(0) == 0 || g.size(1) % 8 || (dtype != at::kBFloat16 && dtype != at::kFloat) || reinterpret_cast<uintptr_t>(g.const_data_ptr()) % 16)
+    return g.sum(at::IntArrayRef{0}, false, at::kFloat).to(dtype);  // (summed in fp32 without an fp32 copy of the gradient)
+  const int rows = int(g.size(0)), cols = int(g.size(1)), parts = lib.col_sum_parts(rows, cols);
+  Tensor out = at::empty({cols}, g.options().dtype(dtype)), partials = parts > 1 ? at::empty({parts, cols}, g.options().dtype(at::kFloat)) : Tensor();
+  check(lib.col_sum(g.const_data_ptr(), out.mutable_data_ptr(), parts > 1 ? partials.data_ptr<float>() : nullptr, rows, cols, dtype == at::kFloat, stream_of(g)),
+        "tpb_col_sum");  // (not among the launches: those of a linear layer are its GEMMs)
+  return out;
+}
+
 struct LinearFn : torch::autograd::Function<LinearFn> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_) {
     const Tensor bias = or_undefined(bias_);
@@ -134,7 +147,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     if (ctx->needs_input_grad(0)) gx = gemm(g, weight, Tensor(), false, true).view(ctx->saved_data["shape"].toIntVector());
     if (ctx->needs_input_grad(1)) gw = gemm(g, x2d, Tensor(), true, true);
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2))
-      gb = g.sum(at::IntArrayRef{0}, false, at::kFloat).to(grad.scalar_type());  // (summed in fp32 without an fp32 copy of the gradient)
+      gb = column_sums(g, grad.scalar_type());
     return {gx, gw, gb};
   }
 };
@@ -250,6 +263,12 @@ void bind(const py::dict& addresses, py::function text, py::function reserve) {
   entry(lib.norm_fwd, addresses, "tpb_norm_fwd");
   entry(lib.norm_bwd, addresses, "tpb_norm_bwd");
   entry(lib.norm_bwd_parts, addresses, "tpb_norm_bwd_parts");
+  if (addresses.contains("tpb_col_sum")) {
+    entry(lib.col_sum_parts, addresses, "tpb_col_sum_parts");
+    entry(lib.col_sum, addresses, "tpb_col_sum");
+  } else {
+    lib.col_sum = nullptr;
+  }
   Py_XDECREF(error_text);
   Py_XDECREF(reserve_slots);
   error_text = text.release().ptr();  // (kept for the life of the process, beyond the interpreter's teardown of module globals)

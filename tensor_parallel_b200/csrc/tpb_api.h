@@ -124,6 +124,11 @@ int tpb_norm_bwd_parts(int rows, int cols);
 int tpb_norm_bwd(const void* dy, const void* x, const void* weight, const float* rstd, const float* mean, void* dx, float* part_w,
                  float* part_b, void* dweight, void* dbias, int rows, int cols, int mode, int dtype, int grad_dtype, void* stream);
 
+// Column sums in fp32 of g[rows, cols] (bf16, contiguous, 16-byte aligned, cols a multiple of 8), stored as bf16 (out_dtype 0) or fp32 (1); partials:
+// fp32 [tpb_col_sum_parts(rows, cols)][cols], not needed for one part.
+int tpb_col_sum_parts(int rows, int cols);
+int tpb_col_sum(const void* g, void* out, float* partials, int rows, int cols, int out_dtype, void* stream);
+
 // Sizes of the structures above as this library was built, one byte-count per 16 bits (plan, reduction context, options), for callers that
 // are built apart from it.
 #define TPB_API_LAYOUT ((unsigned long long)sizeof(tpb_gemm_plan_t) | (unsigned long long)sizeof(tpb_reduce_ctx_t) << 16 | (unsigned long long)sizeof(tpb_gemm_opts_t) << 32)

@@ -213,8 +213,8 @@ def _reserve_slots(index: int, elems: int) -> int:
 
 
 def _bind_autograd():
-    names = ("tpb_gemm_plan_ex", "tpb_gemm_bf16_ex", "tpb_norm_fwd", "tpb_norm_bwd", "tpb_norm_bwd_parts")
-    AUTOGRAD.bind({n: ctypes.cast(getattr(LIB, n), c_void_p).value for n in names}, _error_text, _reserve_slots)
+    names = ("tpb_gemm_plan_ex", "tpb_gemm_bf16_ex", "tpb_norm_fwd", "tpb_norm_bwd", "tpb_norm_bwd_parts", "tpb_col_sum_parts", "tpb_col_sum")
+    AUTOGRAD.bind({n: ctypes.cast(getattr(LIB, n), c_void_p).value for n in names if hasattr(LIB, n)}, _error_text, _reserve_slots)
 
 
 if AUTOGRAD is not None:

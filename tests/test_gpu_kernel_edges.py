@@ -826,6 +826,25 @@ def test_norm_of_as_many_rows_as_an_int_counts():
     torch.cuda.empty_cache()
 
 
+# one share of the rows and several, remainders of 32 rows and of 64 columns, one row, columns that take the sum over tensors
+@pytest.mark.parametrize("rows,cols", [(1, 8), (33, 72), (256, 3072), (257, 640), (1000, 520), (4097, 64), (70, 36)])
+def test_bias_gradient(rows, cols):
+    """Column sums against 64 bits, the same bits every time; a gradient that is not contiguous."""
+    nat = _native()
+    torch.manual_seed(rows)
+    x, w = torch.randn(rows, 64, device="cuda", dtype=torch.bfloat16), torch.randn(cols, 64, device="cuda", dtype=torch.bfloat16)
+    for g in (torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16), torch.randn(cols, rows, device="cuda", dtype=torch.bfloat16).t()):
+        got = []
+        for _ in range(2):
+            b = torch.zeros(cols, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+            nat.linear(x, w, b).backward(g)
+            got.append(b.grad)
+        want = g.double().sum(0)
+        assert torch.equal(*got) and got[0].dtype == torch.bfloat16
+        # one bf16 rounding behind fp32 sums of numbers of magnitude 1
+        assert bool(((got[0].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * rows).all())
+
+
 @pytest.mark.parametrize("bidirectional", [False, True])
 @pytest.mark.parametrize("buckets,max_distance", [(32, 128), (32, 20), (4, 100), (7, 90), (12, 1000), (64, 100000), (30, 333), (256, 4096)])
 def test_relative_buckets_are_those_of_the_tensor_steps(bidirectional, buckets, max_distance):
