@@ -112,10 +112,23 @@ Tensor gemm(const Tensor& x_in, const Tensor& w_in, const Tensor& bias, bool x_t
   return out;
 }
 
-std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
+// What a call costs beside its launches is tensor operations that change nothing, 0.5 to 1 us each: a view or a conversion is taken only where
+// shape or type ask for it.
+Tensor rows_of(const Tensor& x) { return x.dim() == 2 ? x : x.reshape({-1, x.size(-1)}); }
+Tensor as_type(const Tensor& t, at::ScalarType dtype) { return t.scalar_type() == dtype ? t : t.to(dtype); }
+
+// Rows as the leading dimensions of x have it.
+Tensor shaped_as(const Tensor& rows, const Tensor& x) {
+  if (x.dim() == 2) return rows;
   std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
-  shape.back() = last;
-  return shape;
+  shape.back() = rows.size(1);
+  return rows.view(shape);
+}
+// The shape of an input, kept for its gradient where that is not its rows' (empty otherwise).
+std::vector<int64_t> shape_of(const Tensor& x) { return x.dim() == 2 ? std::vector<int64_t>() : x.sizes().vec(); }
+Tensor in_shape(const Tensor& rows, const c10::IValue& shape) {
+  const auto sizes = shape.toIntVector();
+  return sizes.empty() ? rows : rows.view(sizes);
 }
 
 // The gradient of a bias: column sums of g in fp32, as `dtype`.
@@ -132,19 +145,19 @@ Tensor column_sums(const Tensor& g, at::ScalarType dtype) {
 struct LinearFn : torch::autograd::Function<LinearFn> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_) {
     const Tensor bias = or_undefined(bias_);
-    const Tensor x2d = x.reshape({-1, x.size(-1)});
+    const Tensor x2d = rows_of(x);
     const Tensor out = gemm(x2d, weight, bias, false, false);
     ctx->save_for_backward({x2d, weight});
-    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["shape"] = shape_of(x);
     ctx->saved_data["bias"] = bias.defined();
-    return out.view(with_last(x, weight.size(0)));
+    return shaped_as(out, x);
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &x2d = saved[0], &weight = saved[1], &grad = grads[0];
-    const Tensor g = grad.reshape({-1, grad.size(-1)}).to(at::kBFloat16).contiguous();
+    const Tensor g = as_type(rows_of(grad), at::kBFloat16).contiguous();
     Tensor gx, gw, gb;
-    if (ctx->needs_input_grad(0)) gx = gemm(g, weight, Tensor(), false, true).view(ctx->saved_data["shape"].toIntVector());
+    if (ctx->needs_input_grad(0)) gx = in_shape(gemm(g, weight, Tensor(), false, true), ctx->saved_data["shape"]);
     if (ctx->needs_input_grad(1)) gw = gemm(g, x2d, Tensor(), true, true);
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2))
       gb = column_sums(g, grad.scalar_type());
@@ -156,14 +169,14 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
 // reads and writes each of them once more (three of 8192 x 4096: 59 us); here the second and third GEMM add to what the one before stored.
 struct LinearsFn : torch::autograd::Function<LinearsFn> {
   static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& x, at::TensorList weights) {
-    const Tensor x2d = x.reshape({-1, x.size(-1)});
+    const Tensor x2d = rows_of(x);
     torch::autograd::variable_list outs, saved{x2d};
     for (const Tensor& w : weights) {
-      outs.push_back(gemm(x2d, w, Tensor(), false, false).view(with_last(x, w.size(0))));
+      outs.push_back(shaped_as(gemm(x2d, w, Tensor(), false, false), x));
       saved.push_back(w);
     }
     ctx->save_for_backward(saved);
-    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["shape"] = shape_of(x);
     ctx->set_materialize_grads(false);
     return outs;
   }
@@ -173,11 +186,11 @@ struct LinearsFn : torch::autograd::Function<LinearsFn> {
     Tensor gx;
     for (size_t i = 0; i < grads.size(); ++i) {
       if (!grads[i].defined()) continue;  // (nobody used that projection)
-      const Tensor g = grads[i].reshape({-1, grads[i].size(-1)}).to(at::kBFloat16).contiguous();
+      const Tensor g = as_type(rows_of(grads[i]), at::kBFloat16).contiguous();
       if (ctx->needs_input_grad(0)) gx = gemm(g, saved[1 + i], Tensor(), false, true, gx);
       if (ctx->needs_input_grad(1 + i)) out[1 + i] = gemm(g, saved[0], Tensor(), true, true);
     }
-    if (gx.defined()) out[0] = gx.view(ctx->saved_data["shape"].toIntVector());
+    if (gx.defined()) out[0] = in_shape(gx, ctx->saved_data["shape"]);
     return out;
   }
 };
@@ -188,7 +201,7 @@ Tensor linear(const Tensor& x, const Tensor& weight, const std::optional<Tensor>
   const Tensor bias = or_undefined(bias_);
   if (at::GradMode::is_enabled() && (x.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad())))
     return LinearFn::apply(x, weight, bias_);
-  return gemm(x.reshape({-1, x.size(-1)}), weight, bias, false, false).view(with_last(x, weight.size(0)));
+  return shaped_as(gemm(rows_of(x), weight, bias, false, false), x);
 }
 
 int dtype_code(const Tensor& t) {
@@ -203,29 +216,29 @@ struct NormFn : torch::autograd::Function<NormFn> {
                         double eps, int64_t mode) {
     const Tensor weight = or_undefined(weight_), bias = or_undefined(bias_);
     const int dtype = dtype_code(x);
-    const Tensor x2d = x.reshape({-1, x.size(-1)}).contiguous();
-    const Tensor w = weight.defined() ? weight.to(x.scalar_type()).contiguous() : Tensor();
-    const Tensor b = bias.defined() ? bias.to(x.scalar_type()).contiguous() : Tensor();
+    const Tensor x2d = rows_of(x).contiguous();
+    const Tensor w = weight.defined() ? as_type(weight, x.scalar_type()).contiguous() : Tensor();
+    const Tensor b = bias.defined() ? as_type(bias, x.scalar_type()).contiguous() : Tensor();
     const int64_t rows = x2d.size(0), cols = x2d.size(1);
     Tensor out = at::empty_like(x2d);
-    Tensor rstd = at::empty({rows}, x2d.options().dtype(at::kFloat));
-    Tensor mean = mode == 1 ? at::empty_like(rstd) : Tensor();
-    check(lib.norm_fwd(x2d.const_data_ptr(), nullptr, data(w), data(b), out.mutable_data_ptr(), nullptr, rstd.data_ptr<float>(),
-                       mean.defined() ? mean.data_ptr<float>() : nullptr, int(rows), int(cols), float(eps), int(mode), dtype, stream_of(x2d)),
+    Tensor stats = at::empty({mode == 1 ? 2 : 1, rows}, x2d.options().dtype(at::kFloat));  // 1 / deviation, and for LayerNorm the mean, of every row
+    float* rstd = stats.data_ptr<float>();
+    check(lib.norm_fwd(x2d.const_data_ptr(), nullptr, data(w), data(b), out.mutable_data_ptr(), nullptr, rstd, mode == 1 ? rstd + rows : nullptr, int(rows),
+                       int(cols), float(eps), int(mode), dtype, stream_of(x2d)),
           "tpb_norm_fwd");
     launched.fetch_add(1, std::memory_order_relaxed);
-    ctx->save_for_backward({x2d, w, rstd, mean});
-    ctx->saved_data["shape"] = x.sizes().vec();
-    ctx->saved_data["mode"] = mode;
-    ctx->saved_data["wdtype"] = weight.defined() ? int64_t(weight.scalar_type()) : int64_t(-1);
-    ctx->saved_data["bdtype"] = bias.defined() ? int64_t(bias.scalar_type()) : int64_t(-1);
-    return out.view(x.sizes());
+    ctx->save_for_backward({x2d, w, stats});
+    ctx->saved_data["shape"] = shape_of(x);
+    ctx->saved_data["meta"] = std::vector<int64_t>{mode, weight.defined() ? int64_t(weight.scalar_type()) : int64_t(-1),
+                                                   bias.defined() ? int64_t(bias.scalar_type()) : int64_t(-1)};
+    return shaped_as(out, x);
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x2d = saved[0], &w = saved[1], &rstd = saved[2], &mean = saved[3];
-    const int64_t mode = ctx->saved_data["mode"].toInt(), wdtype = ctx->saved_data["wdtype"].toInt(), bdtype = ctx->saved_data["bdtype"].toInt();
-    const Tensor g = grads[0].reshape(x2d.sizes()).to(x2d.scalar_type()).contiguous();
+    const Tensor &x2d = saved[0], &w = saved[1], &stats = saved[2];
+    const auto meta = ctx->saved_data["meta"].toIntVector();
+    const int64_t mode = meta[0], wdtype = meta[1], bdtype = meta[2];
+    const Tensor g = as_type(rows_of(grads[0]), x2d.scalar_type()).contiguous();
     const int64_t rows = x2d.size(0), cols = x2d.size(1);
     Tensor dx = at::empty_like(x2d);
     // column sums: one fp32 partial row per CTA, added up by a second kernel that writes the gradients in their own dtype
@@ -234,17 +247,19 @@ struct NormFn : torch::autograd::Function<NormFn> {
     const int parts = lib.norm_bwd_parts(int(rows), int(cols));
     const auto fp32 = x2d.options().dtype(at::kFloat);
     const auto as_grad = narrow ? x2d.options().dtype(at::kBFloat16) : fp32;
-    Tensor part_w = has_w ? at::empty({parts, cols}, fp32) : Tensor(), part_b = has_b ? at::empty({parts, cols}, fp32) : Tensor();
+    Tensor partials = has_w || has_b ? at::empty({int(has_w) + int(has_b), parts, cols}, fp32) : Tensor();
+    float* part_w = has_w ? partials.data_ptr<float>() : nullptr;
+    float* part_b = has_b ? partials.data_ptr<float>() + (has_w ? int64_t(parts) * cols : 0) : nullptr;
+    const float* rstd = stats.const_data_ptr<float>();
     Tensor dw = has_w ? at::empty({cols}, as_grad) : Tensor(), db = has_b ? at::empty({cols}, as_grad) : Tensor();
     auto out = [](Tensor& t) { return t.defined() ? t.mutable_data_ptr() : nullptr; };
-    check(lib.norm_bwd(g.const_data_ptr(), x2d.const_data_ptr(), data(w), rstd.const_data_ptr<float>(), mode == 1 ? mean.const_data_ptr<float>() : nullptr,
-                       dx.mutable_data_ptr(), static_cast<float*>(out(part_w)), static_cast<float*>(out(part_b)), out(dw), out(db), int(rows), int(cols),
-                       int(mode), dtype_code(x2d), narrow ? 0 : 1, stream_of(x2d)),
+    check(lib.norm_bwd(g.const_data_ptr(), x2d.const_data_ptr(), data(w), rstd, mode == 1 ? rstd + rows : nullptr, dx.mutable_data_ptr(), part_w, part_b, out(dw),
+                       out(db), int(rows), int(cols), int(mode), dtype_code(x2d), narrow ? 0 : 1, stream_of(x2d)),
           "tpb_norm_bwd");
     launched.fetch_add(has_w || has_b ? 2 : 1, std::memory_order_relaxed);
-    if (has_w) dw = dw.to(at::ScalarType(wdtype));
-    if (has_b) db = db.to(at::ScalarType(bdtype));
-    return {dx.view(ctx->saved_data["shape"].toIntVector()), dw, db, Tensor(), Tensor()};
+    if (has_w) dw = as_type(dw, at::ScalarType(wdtype));
+    if (has_b) db = as_type(db, at::ScalarType(bdtype));
+    return {in_shape(dx, ctx->saved_data["shape"]), dw, db, Tensor(), Tensor()};
   }
 };
 

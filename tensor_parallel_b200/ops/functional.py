@@ -16,15 +16,19 @@ import torch
 import torch.nn.functional as F
 
 _FORCE_TORCH = bool(os.environ.get("TENSOR_PARALLEL_USE_NATIVE"))
+_native_module = None
 
 
 def _native(x: torch.Tensor):
     """The native module if ``x`` should run on hand-written kernels, else ``None``."""
+    global _native_module
     if not x.is_cuda or _FORCE_TORCH:
         return None
-    from tensor_parallel_b200.ops import native  # raises if the library is missing on a GPU box
+    if _native_module is None:  # (an import statement per call costs as much as all other checks)
+        from tensor_parallel_b200.ops import native  # raises if the library is missing on a GPU box
 
-    return native
+        _native_module = native
+    return _native_module
 
 
 # -- reference definitions ---------------------------------------------------------------------
