@@ -538,31 +538,32 @@ attn_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __gri
 // Whole backward, 32 heads of 128: 4 x 2048 causal 558 -> 507 us, 2 x 2080 344 -> 323, without a mask 560 -> 518; 1 x 1000 65.7 -> 61.3.
 // Attention layer with relative positions (16 x 512, 32 heads of 64, with the projections) 1473 -> 1434.  Short and ragged sequences: step_rows.
 //
-// T = 64 is the same with 64 streamed rows, at head_dim 64: half of the tensor-memory columns, registers and shared memory, and two CTAs per SM, which fill
-// each other's chains, prologues and epilogues.
-template <int D, int T, int BIAS>
+// T = 64 is the same with 64 streamed rows, at head_dim 64 and for dQ at 128: half of the tensor-memory columns, registers and shared memory, and two CTAs per
+// SM, which fill each other's chains, prologues and epilogues.
+template <int D, bool DKV, int T, int BIAS>
 struct Bww {
   static constexpr int CTAS = T == 64 ? 2 : 1;
   static constexpr int WARPS = 16 / CTAS;                  // elementwise warps
   static constexpr int THREADS = 64 + 32 * WARPS;
-  static constexpr int S1 = T == 64 && BIAS == 2 ? 2 : 3, S2 = 2;  // ring depths: Q (dK / dV) or K (dQ), with the bias; dO or V
+  static constexpr int S1 = T == 64 && (BIAS == 2 || D == 128) ? 2 : 3, S2 = T == 64 && D == 128 ? 1 : 2;  // ring depths: Q (dK / dV) or K (dQ), with the bias; dO or V
   static constexpr int BARS = 1 + 2 * (S1 + S2) + 7;
   static constexpr uint32_t TILE = D / 64 * T * 128;       // one streamed tile
   static constexpr uint32_t BIAS_BYTES = T * BW_R * 2;     // bias elements of one step
-  static constexpr size_t SMEM = size_t(2 * (D / 64)) * FA_BLOCK_BYTES + (S1 + S2) * TILE + (BIAS == 2 ? S1 * BIAS_BYTES : 0) + 2 * T * sizeof(float2) + BARS * 8 + 16;
+  static constexpr size_t STATS = DKV ? 2 * T * sizeof(float2) : 0;
+  static constexpr size_t SMEM = size_t(2 * (D / 64)) * FA_BLOCK_BYTES + (S1 + S2) * TILE + (BIAS == 2 ? S1 * BIAS_BYTES : 0) + STATS + BARS * 8 + 16;
   static_assert(CTAS * (SMEM + 1024) <= 228 * 1024, "shared memory of an SM");
 };
 
 template <int D, bool DKV, int BIAS, int T>
-__global__ void __launch_bounds__(Bww<D, T, BIAS>::THREADS, Bww<D, T, BIAS>::CTAS)
+__global__ void __launch_bounds__(Bww<D, DKV, T, BIAS>::THREADS, Bww<D, DKV, T, BIAS>::CTAS)
 attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_constant__ CUtensorMap tmap_r2,
                      const __grid_constant__ CUtensorMap tmap_t1, const __grid_constant__ CUtensorMap tmap_t2,
                      const __grid_constant__ CUtensorMap tmap_b, const BwParams p) {
-  using B = Bww<D, T, BIAS>;
+  using B = Bww<D, DKV, T, BIAS>;
   constexpr int DB = D / 64, BWW_S1 = B::S1, BWW_S2 = B::S2, BWW_WARPS = B::WARPS;
   constexpr uint32_t R_TILE = DB * FA_BLOCK_BYTES, TILE = B::TILE, T_BLOCK = T * 128, BWW_BIAS = B::BIAS_BYTES;
   constexpr uint32_t TMEM_COLS = 512 / B::CTAS, S_COL = 0, DP_COL = T, ACC0_COL = 2 * T, ACC1_COL = ACC0_COL + D;
-  constexpr bool RES_TMEM = !DKV || (D == 64 && T == 128);  // the resident tiles as tensor-memory operands, where the columns leave room
+  constexpr bool RES_TMEM = T == 128 ? !DKV || D == 64 : !DKV && D == 64;  // the resident tiles as tensor-memory operands, where the columns leave room
   constexpr uint32_t RES_COL = ACC0_COL + (DKV ? 2 : 1) * D;
   static_assert(ACC0_COL + (DKV ? 2 : 1) * D <= TMEM_COLS && (!RES_TMEM || RES_COL + D <= TMEM_COLS), "tensor memory columns");
   constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, T, false, false);
@@ -580,7 +581,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
   uint8_t* t2_s = t1_s + BWW_S1 * TILE;   // [BWW_S2]
   uint8_t* bias_s = t2_s + BWW_S2 * TILE;     // [BWW_S1], BIAS == 2 only
   float* stat_s = reinterpret_cast<float*>(bias_s + (BIAS == 2 ? BWW_S1 * BWW_BIAS : 0));  // dK / dV, [2 steps]: -lse * log2(e) of 128 streamed queries (-inf = no such query), -delta * scale
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + 4 * T);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + B::STATS / sizeof(float));
   uint64_t* r_full = bars;
   uint64_t* t1_full = bars + 1;
   uint64_t* t1_empty = t1_full + BWW_S1;
@@ -744,6 +745,11 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         }
         umma_commit_lead(leader, which ? dp_full : s_full);
       };
+      // (dQ reads its V tile in dP only; dO is read again, in dV)
+      auto dp_scores = [&](int n) {
+        scores(1, smem_u32(t2_s + (n % BWW_S2) * TILE));
+        if (!DKV) umma_commit_lead(leader, &t2_empty[n % BWW_S2]);
+      };
       auto accumulate = [&](uint32_t acc_col, uint32_t a_col, uint32_t tile, bool first) {
         const uint32_t t_lo = desc_mnmajor_lo(tile, T_BLOCK);
 #pragma unroll
@@ -764,7 +770,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
       bool ok = wait_all(RES_TMEM ? res_full : r_full, 0) && t1_there(0);
       if (ok) scores(0, t1_at(0));
       ok = ok && t2_there(0);
-      if (ok) scores(1, t2_at(0));
+      if (ok) dp_scores(0);
       for (int n = 0; ok && n < n_steps; ++n) {
         const bool more = n + 1 < n_steps;
         ok = wait_all(s_done, n & 1);
@@ -782,11 +788,10 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         if (!ok) break;
         accumulate(ACC0_COL, DP_COL, t1_at(n), n == 0);
         umma_commit_lead(leader, &t1_empty[n % BWW_S1]);
-        if (!DKV) umma_commit_lead(leader, &t2_empty[n % BWW_S2]);
         if (more) {
           ok = t2_there(n + 1);
           if (!ok) break;
-          scores(1, t2_at(n + 1));
+          dp_scores(n + 1);
         }
       }
       umma_commit_lead(leader, acc_full);
@@ -948,18 +953,22 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         bf16* base = a == 0 ? p.out0 : p.out1;
         const long long sb = a == 0 ? p.o0_sb : p.o1_sb, ss = a == 0 ? p.o0_ss : p.o1_ss, sh = a == 0 ? p.o0_sh : p.o1_sh;
         bf16* orow = base + b * sb + (long long)min(ri, limit - 1) * ss + (long long)o_head * sh + part * HD;
-        uint32_t o[HD];
-        if (n_steps > 0) {
-          __syncwarp();
-          const uint32_t at = t_lane + (a == 0 ? ACC0_COL : ACC1_COL) + part * HD;
-          if constexpr (HD == 32) tmem_ld_x32(at, o);
-          else tmem_ld_x16(at, o);
-          tmem_ld_wait();
-        } else {
+        constexpr int W = HD < 32 ? HD : 32;
 #pragma unroll
-          for (int i = 0; i < HD; ++i) o[i] = 0u;
+        for (int c = 0; c < HD; c += W) {
+          uint32_t o[W];
+          if (n_steps > 0) {
+            __syncwarp();
+            const uint32_t at = t_lane + (a == 0 ? ACC0_COL : ACC1_COL) + part * HD + c;
+            if constexpr (W == 32) tmem_ld_x32(at, o);
+            else tmem_ld_x16(at, o);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i) o[i] = 0u;
+          }
+          if (ri < limit) bw_store_row(orow + c, o);
         }
-        if (ri < limit) bw_store_row(orow, o);
       }
     }
   }
@@ -1235,7 +1244,7 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 template <int D, bool DKV, int BIAS, int T>
 static int bw_launch_wide(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& tb,
                           const BwParams& p, dim3 grid, cudaStream_t stream) {
-  constexpr size_t smem = Bww<D, T, BIAS>::SMEM;
+  constexpr size_t smem = Bww<D, DKV, T, BIAS>::SMEM;
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
@@ -1244,7 +1253,7 @@ static int bw_launch_wide(const CUtensorMap& r1, const CUtensorMap& r2, const CU
       return TPB_ERR_CUDA;
     configured[dev].store(true, std::memory_order_release);
   }
-  attn_bwd_wide_kernel<D, DKV, BIAS, T><<<grid, Bww<D, T, BIAS>::THREADS, smem, stream>>>(r1, r2, t1, t2, tb, p);
+  attn_bwd_wide_kernel<D, DKV, BIAS, T><<<grid, Bww<D, DKV, T, BIAS>::THREADS, smem, stream>>>(r1, r2, t1, t2, tb, p);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
@@ -1292,6 +1301,13 @@ static int step_rows(int head_dim, int bias_mode, int streamed, int heads, int b
 // 30.3 / 24.8, causal with a mask 46.5 / 49.1; 2 x 1000, 12 heads (192) 54.6 / 48.5, causal 42.6 / 45.9; 1 x 512, 8 heads (32) 20.6 / 23.0.
 static bool two_per_sm(int head_dim, int resident, int heads, int batch, bool causal) {
   return head_dim == 64 && (long long)((resident + BW_R - 1) / BW_R) * heads * batch > (causal ? 296 : 148);
+}
+
+// The dQ launch at head_dim 128, whose resident tiles and rings of steps of 64 keys just fit half of an SM (with them in shared memory and not in tensor memory, an
+// MMA reads twice as much): for sequences of a few steps, whose fill and drain count.  Whole backwards in us, 32 heads, wide / so: 16 x 512 336 / 321, causal 292 / 269;
+// 16 x 100 57.2 / 49.3; 3 x 200 33.8 / 30.9; 16 heads 4 x 300 37.3 / 34.6, 2 x 700 55.9 / 52.6, causal 45.3 / 45.5; but 1 x 2048 219 / 222, causal 153 / 163, 4 x 2048 causal 505 / 510.
+static bool dq_two_per_sm_128(int head_dim, int sq, int sk, int heads, int batch) {
+  return head_dim == 128 && sk <= 640 && (long long)((sq + BW_R - 1) / BW_R) * heads * batch > 148;
 }
 
 }  // namespace tpb
@@ -1359,7 +1375,7 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
   // a dense bf16 bias travels by TMA (strides and base are multiples of 16 bytes); fp32 ones, unaligned rows and masks that
   // broadcast over the queries are loaded element by element
   const int bias_mode = !bias ? 0 : (p.bias_kind == 2 && p.bias_vec && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0 ? 2 : 1);
-  const bool kv_two = two_per_sm(head_dim, sk, kv_heads, batch, causal), q_two = two_per_sm(head_dim, sq, q_heads, batch, causal);
+  const bool kv_two = two_per_sm(head_dim, sk, kv_heads, batch, causal), q_two = two_per_sm(head_dim, sq, q_heads, batch, causal) || (bias_mode == 0 && dq_two_per_sm_128(head_dim, sq, sk, q_heads, batch));
   const int kv_rows = kv_two ? BW_T : step_rows(head_dim, bias_mode, sq, kv_heads, batch), q_rows = q_two ? BW_T : step_rows(head_dim, bias_mode, sk, q_heads, batch);
   CUtensorMap b_kv = q64, b_q = q64;
   if (bias_mode == 2) {  // (a wide dQ step takes two boxes)
@@ -1379,6 +1395,9 @@ extern "C" int tpb_attn_backward_sm100(const void* q, const void* k, const void*
 #undef BW_TWO
     }
     if (head_dim == 64) return bias_mode == 0 ? BW_ONE(64, 0) : bias_mode == 1 ? BW_ONE(64, 1) : BW_ONE(64, 2);
+    if constexpr (!DKV) {
+      if (bias_mode == 0 && q_two) return bw_launch_wide<128, DKV, 0, 64>(r1, r2, t1[0], t2[0], tb, p, grid, s);
+    }
     return bias_mode == 0   ? BW_ONE(128, 0)
            : bias_mode == 1 ? bw_launch<128, DKV, 1>(r1, r2, t1[0], t2[0], tb, p, grid, s)
                             : bw_launch<128, DKV, 2>(r1, r2, t1[0], t2[0], tb, p, grid, s);

@@ -870,16 +870,16 @@ def _attention_double(q, k, v, causal, bias):
     return torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1).nan_to_num(0.0), v.repeat_interleave(q.shape[2] // v.shape[2], 2))
 
 
-# more CTAs than SMs (causal: than two rounds of them) at head_dim 64: two CTAs per SM.  Lengths off the tiles of 64 and 128, one tile, several, more
+# more CTAs than SMs (causal: than two rounds of them) at head_dim 64, and in dQ at head_dim 128: two CTAs per SM.  Lengths off the tiles of 64 and 128, one tile, several, more
 # keys than queries; grouped heads.
 @pytest.mark.parametrize("b,sq,sk,hq,hkv,causal", [(5, 129, 129, 32, 32, False), (10, 130, 193, 32, 16, True), (5, 200, 72, 32, 32, False), (3, 257, 320, 64, 64, True),
                                                    (2, 1, 64, 160, 160, True), (4, 264, 264, 40, 40, False)])
-@pytest.mark.parametrize("bias", ["none", "dense", "rows off 16 bytes", "fp32", "padding"])
-def test_attention_with_two_ctas_per_sm(b, sq, sk, hq, hkv, causal, bias):
+@pytest.mark.parametrize("d,bias", [(64, "none"), (64, "dense"), (64, "rows off 16 bytes"), (64, "fp32"), (64, "padding"), (128, "none")])
+def test_attention_with_two_ctas_per_sm(b, sq, sk, hq, hkv, causal, d, bias):
     nat = _native()
     torch.manual_seed(sq + sk)
-    q, k, v = (torch.randn(b, s, h, 64, device="cuda", dtype=torch.bfloat16).requires_grad_() for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
-    g = torch.randn(b, sq, hq, 64, device="cuda", dtype=torch.bfloat16)
+    q, k, v = (torch.randn(b, s, h, d, device="cuda", dtype=torch.bfloat16).requires_grad_() for s, h in ((sq, hq), (sk, hkv), (sk, hkv)))
+    g = torch.randn(b, sq, hq, d, device="cuda", dtype=torch.bfloat16)
     added = None
     if bias == "padding":
         added = torch.zeros(b, 1, 1, sk, device="cuda", dtype=torch.bfloat16)
