@@ -983,21 +983,21 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
 // ---- gradient of a bias that several (batch, head) pairs share ----
 //
 // d(bias)[i, j] = sum over the pairs of P (dP - delta).  Inside the dQ launch every pair adds its own 4 bytes per score into one fp32 buffer: 134 M
-// reductions for 16 x 512 tokens and 32 heads, 126 us of its 235.  Here a CTA owns a tile of 128 queries x 128 keys of the bias and walks the pairs:
+// reductions for 16 x 512 tokens and 32 heads, 126 us of its 235.  Here a CTA owns a tile of 128 queries x 64 keys of the bias and walks the pairs:
 // S = Q K^T and dP = dO V^T once more (seven tile products become nine), the sum of P (dP - delta) in registers, one store at the end and no
 // buffer to clear.  Sums run in a fixed order.
 //
-//   warp 0     : TMA producer, the four tiles of a pair (Q, dO, K, V) per stage of a ring
-//   warp 1     : MMA issuer, S and dP of pair n + 1 while the other warps are at pair n (two buffers of each: 512 TMEM columns)
-//   warps 2-17 : a thread per query and 32 keys, their sums in registers, their biases (the same for every pair) in slots of its own in shared memory
+//   warp 0    : TMA producer, the four tiles of a pair (Q, dO, K, V) per stage of a ring
+//   warp 1    : MMA issuer, S and dP of pair n + 1 while the other warps are at pair n (two buffers of each: 256 TMEM columns)
+//   warps 2-9 : two threads per query, 32 keys each, their sums in registers, their biases (the same for every pair) in slots of their own in
+//               shared memory
 //
-// Tile and pair take 2000 clocks: an exponential per score, 1024 on the special-function unit, and the latencies of barrier and TMEM around
-// them, which two halves of the keys with barriers of their own hide in part (114 -> 110 us).  16 x 512 tokens, 32 heads: 110 us; whole
-// backward with it 333 us, with reductions in the dQ launch, the buffer to clear and the cast to bf16 361.  Where it pays: ops/native.py.
-constexpr int BG_STAGES = 3, BG_WARPS = 16, BG_THREADS = 64 + 32 * BG_WARPS;
-constexpr int BG_HALVES = 2, BG_COLS = BW_R / BG_HALVES;  // products, hand-over and warps by halves of the keys: while one half waits, the other computes
+// Two CTAs per SM.  One with tiles of 128 keys, sixteen such warps and a third less to load took 110 us for that shape (2000 clocks per tile and pair, half of them an
+// exponential per score on the special-function unit, the rest latencies of barrier and TMEM that warps in step do not hide from each other); this one
+// takes 88 us.  Whole backward with it 307 us, with reductions in the dQ launch, the buffer to clear and the cast to bf16 353.  Where it pays: ops/native.py.
+constexpr int BG_STAGES = 2, BG_KEYS = 64, BG_WARPS = 8, BG_THREADS = 64 + 32 * BG_WARPS;
 template <int D>
-constexpr size_t bg_smem_bytes() { return size_t(BG_STAGES) * 4 * (D / 64) * FA_BLOCK_BYTES + BW_R * BW_R * 2 + 20 * 8 + 1024; }
+constexpr size_t bg_smem_bytes() { return size_t(BG_STAGES) * 2 * (D / 64) * (FA_BLOCK_BYTES + BG_KEYS * 128) + BW_R * BG_KEYS * 2 + 16 * 8; }
 
 struct BgParams {
   int batch, sq, sk, q_heads, kv_heads, causal;
@@ -1011,24 +1011,29 @@ struct BgParams {
 };
 
 template <int D>
-__global__ void __launch_bounds__(BG_THREADS, 1)
+__global__ void __launch_bounds__(BG_THREADS, 2)
 attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const BgParams p) {
   constexpr int DB = D / 64;
-  constexpr uint32_t TILE = DB * FA_BLOCK_BYTES, STAGE = 4 * TILE;
-  constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BG_COLS, false, false);
-  extern __shared__ uint8_t bg_smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(bg_smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr uint32_t TILE = DB * FA_BLOCK_BYTES, K_BLOCK = BG_KEYS * 128, K_TILE = DB * K_BLOCK, STAGE = 2 * (TILE + K_TILE);  // Q, dO, K, V
+  constexpr uint32_t TMEM_COLS = 256;
+  constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BG_KEYS, false, false);
+  extern __shared__ __align__(1024) uint8_t bg_smem[];
+  uint8_t* smem = bg_smem;
+  if (smem_u32(smem) & 1023) {  // (the swizzle patterns need it, and there is no room to round up)
+    if (threadIdx.x == 0) atomicMax(p.status, STATUS_BAD_ARG);
+    return;
+  }
   uint4* bias_s = reinterpret_cast<uint4*>(smem + BG_STAGES * STAGE);  // [4 chunks of 8 keys][threads], private
   uint64_t* t_full = reinterpret_cast<uint64_t*>(bias_s + 4 * 32 * BG_WARPS);
   uint64_t* t_empty = t_full + BG_STAGES;
-  uint64_t* s_full = t_empty + BG_STAGES;      // [2 buffers][2 halves of the keys]: S and dP of a pair are there
-  uint64_t* s_done = s_full + 2 * BG_HALVES;   // and have been read
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_done + 2 * BG_HALVES);
+  uint64_t* s_full = t_empty + BG_STAGES;  // [2 buffers]: S and dP of a pair are there
+  uint64_t* s_done = s_full + 2;           // and have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_done + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int k0 = blockIdx.x * BW_R, q0 = blockIdx.y * BW_R, plane = blockIdx.z;
+  const int k0 = blockIdx.x * BG_KEYS, q0 = blockIdx.y * BW_R, plane = blockIdx.z;
   const int shift = p.sk - p.sq, group = p.q_heads / p.kv_heads;
   const int heads = p.b_sh ? 1 : p.q_heads;  // heads that share the plane
   const bool any = !p.causal || k0 <= min(p.sq, q0 + BW_R) - 1 + shift;  // (otherwise no query of the tile sees a key of it)
@@ -1043,15 +1048,15 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       mbar_init(&t_full[s], 1);
       mbar_init(&t_empty[s], 1);
     }
-    for (int s = 0; s < 2 * BG_HALVES; ++s) {
+    for (int s = 0; s < 2; ++s) {
       mbar_init(&s_full[s], 1);
-      mbar_init(&s_done[s], BG_WARPS / BG_HALVES);
+      mbar_init(&s_done[s], BG_WARPS);
     }
     *abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -1076,9 +1081,9 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
         for (int d = 0; d < DB; ++d) {
           tma_load_4d(dst + d * FA_BLOCK_BYTES, &tmap_q, &t_full[s], d * 64, q0, h, b);
-          tma_load_4d(dst + 2 * TILE + d * FA_BLOCK_BYTES, &tmap_k, &t_full[s], d * 64, k0, h / group, b);
+          tma_load_4d(dst + 2 * TILE + d * K_BLOCK, &tmap_k, &t_full[s], d * 64, k0, h / group, b);
           tma_load_4d(dst + TILE + d * FA_BLOCK_BYTES, &tmap_do, &t_full[s], d * 64, q0, h, b);
-          tma_load_4d(dst + 3 * TILE + d * FA_BLOCK_BYTES, &tmap_v, &t_full[s], d * 64, k0, h / group, b);
+          tma_load_4d(dst + 2 * TILE + K_TILE + d * K_BLOCK, &tmap_v, &t_full[s], d * 64, k0, h / group, b);
         }
         if (heads > 1 && ++h < heads) continue;
         if (heads > 1) h = 0;
@@ -1096,28 +1101,22 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     for (int n = 0; n < pairs; ++n) {
       const int s = n % BG_STAGES, buf = n & 1;
       if (!wait_all(&t_full[s], (n / BG_STAGES) & 1)) break;
+      if (n >= 2 && !wait_all(&s_done[buf], ((n >> 1) & 1) ^ 1)) break;
       const uint32_t at = smem_u32(smem + s * STAGE);
-      bool ok = true;
 #pragma unroll
-      for (int half = 0; half < BG_HALVES; ++half) {
-        if (n >= 2) ok = ok && wait_all(&s_done[buf * BG_HALVES + half], ((n >> 1) & 1) ^ 1);
-        if (!ok) break;
+      for (int which = 0; which < 2; ++which) {
+        const uint32_t a_lo = desc_kmajor_lo(at + which * TILE), b_lo = desc_kmajor_lo(at + 2 * TILE + which * K_TILE);
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const uint32_t a_lo = desc_kmajor_lo(at + which * TILE), b_lo = desc_kmajor_lo(at + (2 + which) * TILE + half * BG_COLS * 128);
-#pragma unroll
-          for (int i = 0; i < DB * 4; ++i) {
-            const uint32_t off = (i >> 2) * (FA_BLOCK_BYTES >> 4) + (i & 3) * 2;
-            umma_bf16_lead(leader, tmem_base + buf * 256 + which * 128 + half * BG_COLS, a_lo + off, b_lo + off, IDESC_S, i ? 1u : 0u);
-          }
-        }
-        umma_commit_lead(leader, &s_full[buf * BG_HALVES + half]);
+        for (int i = 0; i < DB * 4; ++i)
+          umma_bf16_lead(leader, tmem_base + (buf * 2 + which) * BG_KEYS, a_lo + (i >> 2) * (FA_BLOCK_BYTES >> 4) + (i & 3) * 2, b_lo + (i >> 2) * (K_BLOCK >> 4) + (i & 3) * 2,
+                         IDESC_S, i ? 1u : 0u);
       }
-      if (!ok) break;
+      umma_commit_lead(leader, &s_full[buf]);
       umma_commit_lead(leader, &t_empty[s]);
     }
   } else {
-    constexpr int HC = BW_R / 4;
+    constexpr int HC = BG_KEYS / (BG_WARPS / 4);
+    static_assert(HC == 32, "keys per thread");
     const int quarter = warp & 3, part = (warp - 2) >> 2;
     const int ri = q0 + quarter * 32 + lane, col0 = k0 + part * HC;
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16) + part * HC;
@@ -1159,7 +1158,7 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       const int buf = n & 1;
       const float l2_now = l2, del_now = del;
       if (row_ok && n + 1 < pairs) stats();
-      if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&s_full[buf * BG_HALVES + part * BG_HALVES / 4], (n >> 1) & 1))) {
+      if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&s_full[buf], (n >> 1) & 1))) {
         if (lane == 0 && !*abort_flag) give_up();
         alive = false;
         break;
@@ -1168,15 +1167,15 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
       for (int c0 = 0; c0 < HC; c0 += 16) {
         uint32_t sv[16], dv[16];
-        tmem_ld_x16(t_lane + buf * 256 + c0, sv);
-        tmem_ld_x16(t_lane + buf * 256 + 128 + c0, dv);
+        tmem_ld_x16(t_lane + buf * 2 * BG_KEYS + c0, sv);
+        tmem_ld_x16(t_lane + (buf * 2 + 1) * BG_KEYS + c0, dv);
         const uint4 u0 = my_bias[(c0 / 8) * (32 * BG_WARPS)], u1 = my_bias[(c0 / 8 + 1) * (32 * BG_WARPS)];
         const uint32_t bw[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};  // bf16 pairs
         tmem_ld_wait();
         if (c0 + 16 == HC) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&s_done[buf * BG_HALVES + part * BG_HALVES / 4]);
+          if (lane == 0) mbar_arrive(&s_done[buf]);
         }
         float odd0 = 0.f, odd1 = 0.f;  // not 0 if a dP is not finite
 #pragma unroll
@@ -1238,7 +1237,7 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 template <int D, bool DKV, int BIAS, int T>
@@ -1422,7 +1421,7 @@ extern "C" int tpb_attn_bias_grad_sm100(const void* q, const void* k, const void
   if (!q || !k || !v || !dout || !lse || !delta || !bias || !dbias || !status || batch <= 0 || sq <= 0 || sk <= 0 || q_heads <= 0 || kv_heads <= 0 ||
       q_heads % kv_heads || bias_sq <= 0 || bias_sh < 0 || !(scale > 0.f))
     return TPB_ERR_ARG;
-  const int q_tiles = (sq + BW_R - 1) / BW_R, k_tiles = (sk + BW_R - 1) / BW_R, planes = bias_sh ? q_heads : 1;
+  const int q_tiles = (sq + BW_R - 1) / BW_R, k_tiles = (sk + BG_KEYS - 1) / BG_KEYS, planes = bias_sh ? q_heads : 1;
   if (head_dim != 64 || q_tiles > 65535 || planes > 65535) return TPB_ERR_SIZE;
   const long long strides[] = {q_ss, k_ss, v_ss, do_ss, q_heads > 1 ? q_sh : 0, q_heads > 1 ? do_sh : 0, kv_heads > 1 ? k_sh : 0,
                                kv_heads > 1 ? v_sh : 0, batch > 1 ? q_sb : 0, batch > 1 ? k_sb : 0, batch > 1 ? v_sb : 0, batch > 1 ? do_sb : 0, bias_sh, bias_sq};
@@ -1433,8 +1432,8 @@ extern "C" int tpb_attn_bias_grad_sm100(const void* q, const void* k, const void
   CUtensorMap tq, tdo, tk, tv;
   int rc = fa_tmap(&tq, q, head_dim, BW_R, sq, q_heads, batch, q_ss, q_sh, q_sb);
   if (rc == TPB_OK) rc = fa_tmap(&tdo, dout, head_dim, BW_R, sq, q_heads, batch, do_ss, do_sh, do_sb);
-  if (rc == TPB_OK) rc = fa_tmap(&tk, k, head_dim, BW_R, sk, kv_heads, batch, k_ss, k_sh, k_sb);
-  if (rc == TPB_OK) rc = fa_tmap(&tv, v, head_dim, BW_R, sk, kv_heads, batch, v_ss, v_sh, v_sb);
+  if (rc == TPB_OK) rc = fa_tmap(&tk, k, head_dim, BG_KEYS, sk, kv_heads, batch, k_ss, k_sh, k_sb);
+  if (rc == TPB_OK) rc = fa_tmap(&tv, v, head_dim, BG_KEYS, sk, kv_heads, batch, v_ss, v_sh, v_sb);
   if (rc != TPB_OK) return rc;
   BgParams p;
   memset(&p, 0, sizeof(p));
@@ -1448,7 +1447,7 @@ extern "C" int tpb_attn_bias_grad_sm100(const void* q, const void* k, const void
   p.b_sh = bias_sh; p.b_sq = bias_sq;
   p.status = static_cast<uint32_t*>(status);
   constexpr size_t smem = bg_smem_bytes<64>();
-  static_assert(smem <= 227 * 1024, "shared memory of a CTA");
+  static_assert(2 * (smem + 1024) <= 228 * 1024, "shared memory of an SM");
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;

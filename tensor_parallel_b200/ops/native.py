@@ -673,18 +673,15 @@ LIB.tpb_attn_bias_grad_sm100.argtypes = [c_void_p] * 6 + [c_int] * 6 + [c_ll] * 
 
 def _bias_grad_tiles(b, sq, sk, hq, d, bias4, strides) -> bool:
     """Whether the gradient of a bf16 score bias that the batches share is summed up tile by tile (``tpb_attn_bias_grad_sm100``, a CTA per tile of
-    128 x 128 pairs), not added up by the dQ launch.  It recomputes the scores of every batch, and pays where its CTAs fill the SMs with whole
-    tiles.  Whole backwards at head_dim 64, added up / summed by tile, in us: 16 x 512, 32 heads 361 / 333, 8 heads (128 CTAs) 104 / 91; 16 x 256, 32
-    heads (128) 116 / 111, 16 heads (64) 62 / 70; 16 x 200, 32 heads 102 / 102; 4 x 1024, 32 heads 559 / 349.  With one or two batches, nothing or
-    little to sum: 1 x 512, 32 heads (512) 44 / 48, 8 heads 34 / 29; 1 x 1024, 32 heads 187 / 147."""
+    128 queries x 64 keys), not added up by the dQ launch.  It recomputes the scores of every batch, and pays where its CTAs find an SM each and
+    their tiles are mostly full.  Whole backwards at head_dim 64, added up / summed by tile, in us: 16 x 512, 32 heads 353 / 307, 8 heads (256 CTAs) 104 / 89;
+    16 x 256, 32 heads 117 / 107, 16 heads (128) 62.6 / 61.9, 8 heads (64) 37 / 42; 16 x 200, 16 heads (128, three fifths full) 56.7 / 61.1; 16 x 128, 32 heads
+    (64) 44 / 51; 1 x 512, 8 heads (256) 34 / 28; 4 x 1024, 32 heads 556 / 321."""
     sb, sh, sr, sc = strides
     if d != 64 or bias4.dtype != torch.bfloat16 or sb != 0 or sc != 1 or sr <= 0 or sr % 8 or sh % 8 or bias4.data_ptr() % 16:
         return False
-    tiles, planes = -(-sq // 128) * -(-sk // 128), hq if sh else 1
-    ctas = tiles * planes
-    if ctas < 120 or sq * sk < 0.75 * tiles * 128 * 128:
-        return False
-    return ctas <= 148 or ctas >= 1024 or b * (1 if sh else hq) >= 4
+    tiles = -(-sq // 128) * -(-sk // 64)
+    return tiles * (hq if sh else 1) >= 120 and sq * sk >= 0.75 * tiles * 128 * 64
 
 
 def _bias_view(bias):
