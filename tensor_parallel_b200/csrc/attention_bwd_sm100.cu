@@ -745,10 +745,11 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         }
         umma_commit_lead(leader, which ? dp_full : s_full);
       };
-      // (dQ reads its V tile in dP only; dO is read again, in dV)
+      // dQ reads its V tile in dP only (dO is read again, in dV).  Two CTAs per SM, with their short rings, free it at once (head_dim 64, 2 x 4096, 16 heads:
+      // whole backward 500 -> 496 us); with one CTA the extra commit in the middle of a step's chain costs more (head_dim 128, causal: 441 -> 444 us).
       auto dp_scores = [&](int n) {
         scores(1, smem_u32(t2_s + (n % BWW_S2) * TILE));
-        if (!DKV) umma_commit_lead(leader, &t2_empty[n % BWW_S2]);
+        if (!DKV && T == 64) umma_commit_lead(leader, &t2_empty[n % BWW_S2]);
       };
       auto accumulate = [&](uint32_t acc_col, uint32_t a_col, uint32_t tile, bool first) {
         const uint32_t t_lo = desc_mnmajor_lo(tile, T_BLOCK);
@@ -788,6 +789,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
         if (!ok) break;
         accumulate(ACC0_COL, DP_COL, t1_at(n), n == 0);
         umma_commit_lead(leader, &t1_empty[n % BWW_S1]);
+        if (!DKV && T == 128) umma_commit_lead(leader, &t2_empty[n % BWW_S2]);
         if (more) {
           ok = t2_there(n + 1);
           if (!ok) break;
