@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "launch.cuh"
 #include "ptx_sm100.cuh"
@@ -63,19 +64,46 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// block-wide sum of up to two values; blockDim.x <= 1024
+// block-wide sums of two values, or (not BOTH) of the second only, whose shuffles no compiler takes out; blockDim.x <= 1024
+template <bool BOTH>
 __device__ __forceinline__ void block_sum2(float& a, float& b) {
   __shared__ float sa[32], sb[32];
-  a = warp_sum(a);
+  if (BOTH) a = warp_sum(a);
   b = warp_sum(b);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
   __syncthreads();
-  if (lane == 0) { sa[warp] = a; sb[warp] = b; }
+  if (lane == 0) {
+    if (BOTH) sa[warp] = a;
+    sb[warp] = b;
+  }
   __syncthreads();
-  a = lane < nw ? sa[lane] : 0.f;
-  b = lane < nw ? sb[lane] : 0.f;
-  a = warp_sum(a);
-  b = warp_sum(b);
+  if (BOTH) a = warp_sum(lane < nw ? sa[lane] : 0.f);
+  b = warp_sum(lane < nw ? sb[lane] : 0.f);
+}
+
+template <typename T> struct Raw8 { uint4 u[sizeof(T) / 2]; };  // 8 elements as they lie in memory
+template <typename T> __device__ __forceinline__ Raw8<T> load_raw(const T* p) {
+  Raw8<T> r;
+#pragma unroll
+  for (int i = 0; i < int(sizeof(T) / 2); ++i) r.u[i] = reinterpret_cast<const uint4*>(p)[i];
+  return r;
+}
+__device__ __forceinline__ void unpack(const Raw8<bf16>& r, float (&v)[8]) {
+  const uint32_t w[4] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+__device__ __forceinline__ void pack(const float (&v)[8], Raw8<float>& r) {
+  r.u[0] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+  r.u[1] = make_uint4(__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7]));
+}
+__device__ __forceinline__ void unpack(const Raw8<float>& r, float (&v)[8]) {
+  const uint32_t w[8] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w, r.u[1].x, r.u[1].y, r.u[1].z, r.u[1].w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -86,40 +114,70 @@ __device__ __forceinline__ void block_sum2(float& a, float& b) {
 constexpr int NORM_THREADS = 256;
 constexpr int NORM_MAXV = 8;  // cols <= 16384
 
-// MAXV = vectors of 8 elements a thread may hold (cols <= 256 * 8 * MAXV); small MAXV keeps the register count
-// low so that more rows are in flight per SM.
-template <typename T, int MODE, int MAXV>
-__global__ void __launch_bounds__(NORM_THREADS)
+// CTAs of a row each that an SM is to hold, at least: the most that registers allow without spills.  A row is bound by the chain load - sums - store, so
+// that rows in flight are what counts: RMSNorm bf16 8192 x 5120 with six / five CTAs 29.8 / 31.2 us, 8192 x 8192 with five / four 43.6 / 46.7; LayerNorm
+// 4096 wide spills with six (600 rows 3.86 -> 4.33), 5120 wide loses with four (8192 rows 41.9 -> 44.6), 8192 wide with three (56 -> 63).
+template <typename T, int MODE, int MAXV, bool RES>
+constexpr int norm_row_ctas_per_sm() {
+  if (RES || sizeof(T) == 4) return 1;
+  if (MODE == 0) return MAXV <= 2 ? 8 : MAXV == 3 ? 6 : MAXV == 4 ? 5 : 4;
+  return MAXV == 1 ? 8 : MAXV <= 3 ? 5 : 4;
+}
+
+// MAXV = vectors of 8 elements a thread may hold (cols <= 256 * 8 * MAXV).  RES = there is a residual; without one the row waits for its sums as it lies
+// in memory: 32 registers a thread for up to 4096 bf16 columns, so that eight rows are in flight per SM, and the weights are fetched before the sums are
+// known.  RMSNorm bf16 8192 x 4096 29.6 -> 21.9 us (6.1 TB/s), 1000 x 4096 in L2 / in memory 5.1 -> 3.7 / 6.8 -> 5.0, 20 x 4096 2.5 -> 2.0.
+template <typename T, int MODE, int MAXV, bool RES>
+__global__ void __launch_bounds__(NORM_THREADS, norm_row_ctas_per_sm<T, MODE, MAXV, RES>())
 norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
                 const T* __restrict__ bias, T* __restrict__ out, T* __restrict__ sum_out, float* __restrict__ rstd_out,
                 float* __restrict__ mean_out, int cols, float eps) {
+  constexpr bool EARLY = !RES && MODE == 0 && sizeof(T) * MAXV <= 4;  // weights before the sums, where registers allow it
   pdl_wait();
   const size_t row = blockIdx.x;
   const T* xr = x + row * cols;
   const int nvec = cols >> 3;
-  float v[MAXV][8];
-  float s1 = 0.f, s2 = 0.f;
+  Raw8<typename std::conditional<RES, float, T>::type> held[MAXV];
+  Raw8<T> wr[EARLY ? MAXV : 1];
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
     const int vi = threadIdx.x + i * NORM_THREADS;
     if (vi < nvec) {
-      Vec8<T>::load(xr + vi * 8, v[i]);
-      if (residual) {
-        float r[8];
+      if constexpr (RES) {
+        float v[8], r[8];
+        Vec8<T>::load(xr + vi * 8, v);
         Vec8<T>::load(residual + row * cols + vi * 8, r);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[i][j] += r[j];
+        for (int j = 0; j < 8; ++j) v[j] += r[j];
         if (sum_out) {
           // round to the storage type first so that the statistics match what later kernels will read
-          Vec8<T>::store(sum_out + row * cols + vi * 8, v[i]);
-          Vec8<T>::load(sum_out + row * cols + vi * 8, v[i]);
+          Vec8<T>::store(sum_out + row * cols + vi * 8, v);
+          Vec8<T>::load(sum_out + row * cols + vi * 8, v);
         }
+        pack(v, held[i]);
+      } else {
+        held[i] = load_raw(xr + vi * 8);
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { s1 += v[i][j]; s2 += v[i][j] * v[i][j]; }
     }
   }
-  block_sum2(s1, s2);
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) {
+      const int vi = threadIdx.x + i * NORM_THREADS;
+      if (vi < nvec && weight) wr[i] = load_raw(weight + vi * 8);
+    }
+  }
+  float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    if (int(threadIdx.x) + i * NORM_THREADS < nvec) {
+      float v[8];
+      unpack(held[i], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { s1 += v[j]; s2 += v[j] * v[j]; }
+    }
+  }
+  block_sum2<MODE == 1>(s1, s2);
   const float inv_n = 1.f / float(cols);
   const float mean = MODE == 1 ? s1 * inv_n : 0.f;
   const float var = MODE == 1 ? fmaxf(s2 * inv_n - mean * mean, 0.f) : s2 * inv_n;
@@ -132,12 +190,14 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T
   for (int i = 0; i < MAXV; ++i) {
     const int vi = threadIdx.x + i * NORM_THREADS;
     if (vi < nvec) {
-      float w[8], b[8], o[8];
-      if (weight) Vec8<T>::load(weight + vi * 8, w);
+      float v[8], w[8], b[8], o[8];
+      unpack(held[i], v);
+      if constexpr (EARLY) { if (weight) unpack(wr[i], w); }
+      else if (weight) Vec8<T>::load(weight + vi * 8, w);
       if (MODE == 1 && bias) Vec8<T>::load(bias + vi * 8, b);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        float y = (v[i][j] - mean) * rstd;
+        float y = (v[j] - mean) * rstd;
         if (weight) y *= w[j];
         if (MODE == 1 && bias) y += b[j];
         o[j] = y;
@@ -155,27 +215,6 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T
 // in registers kept 32 KB per SM in flight, too little for the latency of a loaded memory system.  RMSNorm 8192 x 4096 bf16 63 -> 48 us
 // (4.2 TB/s), 8192 x 8192 122 -> 86; LayerNorm 1999 x 5120 fp32 44 -> 40 us, 8192 x 8192 fp32 201 -> 162; 20 x 4096 5.0 and 5.0.
 constexpr int NORM_BWD_MAXC = 8192;  // 1024 threads
-
-template <typename T> struct Raw8 { uint4 u[sizeof(T) / 2]; };  // 8 elements as they lie in memory
-template <typename T> __device__ __forceinline__ Raw8<T> load_raw(const T* p) {
-  Raw8<T> r;
-#pragma unroll
-  for (int i = 0; i < int(sizeof(T) / 2); ++i) r.u[i] = reinterpret_cast<const uint4*>(p)[i];
-  return r;
-}
-__device__ __forceinline__ void unpack(const Raw8<bf16>& r, float (&v)[8]) {
-  const uint32_t w[4] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[2 * i] = __uint_as_float(w[i] << 16);
-    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-}
-__device__ __forceinline__ void unpack(const Raw8<float>& r, float (&v)[8]) {
-  const uint32_t w[8] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w, r.u[1].x, r.u[1].y, r.u[1].z, r.u[1].w};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
-}
 
 // The 8 columns of a thread in 16-byte chunks: bf16 one chunk, fp32 two, which lie blockDim.x chunks apart so that a warp's accesses are
 // contiguous (cp.async goes past L1: chunks side by side would fetch every 32-byte sector twice).
@@ -228,16 +267,17 @@ struct RowRing {
   static __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory"); }
 };
 
-// Block-wide sums of two values per row, one barrier per row: `turn` alternates between two sets of warp sums.
+// Block-wide sums of two values per row, or (not BOTH) of the second only; one barrier per row: `turn` alternates between two sets of warp sums.
+template <bool BOTH>
 __device__ __forceinline__ void row_sum2(float2 (*warp_sums)[32], int turn, float& a, float& b) {
-  a = warp_sum(a);
+  if (BOTH) a = warp_sum(a);
   b = warp_sum(b);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   if (nw == 1) return;
   if (lane == 0) warp_sums[turn][warp] = make_float2(a, b);
   __syncthreads();
   const float2 w = lane < nw ? warp_sums[turn][lane] : make_float2(0.f, 0.f);
-  a = warp_sum(w.x);
+  if (BOTH) a = warp_sum(w.x);
   b = warp_sum(w.y);
 }
 
@@ -297,7 +337,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
         s2 += g * xh;
       }
     }
-    row_sum2(warp_sums, it & 1, s1, s2);
+    row_sum2<MODE == 1>(warp_sums, it & 1, s1, s2);
     const float c1 = MODE == 1 ? s1 * inv_n : 0.f;
     const float c2 = s2 * inv_n;
     {
@@ -354,7 +394,7 @@ norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, cons
       s1 += v[j];
       s2 += v[j] * v[j];
     }
-    row_sum2(warp_sums, it & 1, s1, s2);
+    row_sum2<MODE == 1>(warp_sums, it & 1, s1, s2);
     const float mean = MODE == 1 ? s1 * inv_n : 0.f;
     const float var = MODE == 1 ? fmaxf(s2 * inv_n - mean * mean, 0.f) : s2 * inv_n;
     const float rstd = rsqrtf(var + eps);
@@ -378,11 +418,12 @@ norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, cons
 
 // A CTA per row, with the row added up in the order of norm_fwd_rows_kernel, so that its result does not depend on which of the two a call takes:
 // thread t stands for threads t, t + 256, ... of a ring CTA (`ring_threads`, a multiple of 32), which own the same columns and end up in the
-// same place among the warps' sums.  Several rows per SM in flight, each in registers, no row waits for another's barrier; where the lines lie:
-// norm_takes_row_cta.  RMSNorm bf16 4000 x 5120, input in L2 / in memory: 13.7 / 17.6 us (rings 18.4 / 19.4; rows in one CTA that loads the next row
-// only when it is done 17.4 / 25.0); LayerNorm bf16 4000 x 4096 14.0 / 18.1 (17.6 / 18.9); 8192 x 8192 56 us, 4.8 TB/s (70).
+// same place among the warps' sums.  Several rows per SM in flight, each in registers as it lies in memory, no row waits for another's barrier; where
+// the lines lie: norm_takes_row_cta.  RMSNorm bf16 4000 x 5120, input in L2 / in memory: 12.8 / 16.6 us (rings 17.0 / 17.8; converted to fp32 while it
+// waits 13.5 / 17.5), 8192 x 8192 43.6 us, 6.2 TB/s (rings 51.0; converted 49.7); LayerNorm bf16 4000 x 4096 13.8 / 18.0, 8192 x 8192 56 us, 4.8 TB/s
+// (rings 69).
 template <typename T, int MODE, int MAXV>
-__global__ void __launch_bounds__(NORM_THREADS)
+__global__ void __launch_bounds__(NORM_THREADS, norm_row_ctas_per_sm<T, MODE, MAXV, false>())
 norm_fwd_row_kernel(const T* __restrict__ x, const T* __restrict__ weight, const T* __restrict__ bias, T* __restrict__ out, float* __restrict__ rstd_out,
                     float* __restrict__ mean_out, int cols, int ring_threads, float eps) {
   constexpr int CHUNKS = RowCols<T>::CHUNKS, WIDTH = RowCols<T>::WIDTH;
@@ -392,30 +433,39 @@ norm_fwd_row_kernel(const T* __restrict__ x, const T* __restrict__ weight, const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto column = [&](int i, int chunk) { return (int(threadIdx.x) + i * NORM_THREADS + chunk * ring_threads) * WIDTH; };
   auto mine = [&](int i, int chunk) { return int(threadIdx.x) + i * NORM_THREADS < ring_threads && column(i, chunk) < cols; };
-  auto load = [&](const T* row, int i, float (&f)[8]) {
+  auto load = [&](const T* row, int i) {
     Raw8<T> r;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) r.u[c] = mine(i, c) ? *reinterpret_cast<const uint4*>(row + column(i, c)) : make_uint4(0, 0, 0, 0);
-    unpack(r, f);
+    return r;
   };
-  float v[MAXV][8];
+  constexpr bool EARLY = sizeof(T) * MAXV == 2;
+  Raw8<T> held[MAXV], wr[EARLY ? MAXV : 1], br[EARLY && MODE == 1 ? MAXV : 1];
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) load(x + at, i, v[i]);
+  for (int i = 0; i < MAXV; ++i) held[i] = load(x + at, i);
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) {
+      if (weight) wr[i] = load(weight, i);
+      if constexpr (MODE == 1) { if (bias) br[i] = load(bias, i); }
+    }
+  }
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
-    float s1 = 0.f, s2 = 0.f;
+    float s1 = 0.f, s2 = 0.f, v[8];
+    unpack(held[i], v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      s1 += v[i][j];
-      s2 += v[i][j] * v[i][j];
+      s1 += v[j];
+      s2 += v[j] * v[j];
     }
-    s1 = warp_sum(s1);
+    if (MODE == 1) s1 = warp_sum(s1);
     s2 = warp_sum(s2);
     if (lane == 0) warp_sums[warp + i * (NORM_THREADS / 32)] = make_float2(s1, s2);
   }
   __syncthreads();
   const float2 sums = lane < ring_threads >> 5 ? warp_sums[lane] : make_float2(0.f, 0.f);
-  const float s1 = warp_sum(sums.x), s2 = warp_sum(sums.y);
+  const float s1 = MODE == 1 ? warp_sum(sums.x) : 0.f, s2 = warp_sum(sums.y);
   const float inv_n = 1.f / float(cols);
   const float mean = MODE == 1 ? s1 * inv_n : 0.f;
   const float var = MODE == 1 ? fmaxf(s2 * inv_n - mean * mean, 0.f) : s2 * inv_n;
@@ -426,12 +476,13 @@ norm_fwd_row_kernel(const T* __restrict__ x, const T* __restrict__ weight, const
   }
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
-    float w[8], b[8], o[8];
-    if (weight) load(weight, i, w);
-    if (MODE == 1 && bias) load(bias, i, b);
+    float v[8], w[8], b[8], o[8];
+    unpack(held[i], v);
+    if (weight) unpack(EARLY ? wr[EARLY ? i : 0] : load(weight, i), w);
+    if (MODE == 1 && bias) unpack(EARLY ? br[EARLY && MODE == 1 ? i : 0] : load(bias, i), b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      float y = (v[i][j] - mean) * rstd;
+      float y = (v[j] - mean) * rstd;
       if (weight) y *= w[j];
       if (MODE == 1 && bias) y += b[j];
       o[j] = y;
@@ -834,17 +885,17 @@ static inline bool norm_filled(int cols) { return (cols > NORM_THREADS * 6 && co
 // norm_fwd_row_kernel (true) or norm_fwd_rows_kernel for a forward without a residual, which give the same bits.  Times in us as row / ring, "hot"
 // with the input in L2, as the kernel before leaves it, "cold" with it in memory.
 static inline bool norm_takes_row_cta(int rows, int cols, int mode, int dtype) {
-  // fp32: RMSNorm of many rows that fill the threads (8192 x 4096 43.1 / 47.7, 16384 x 2048 41.6 / 48.2, 32768 x 4096 159 / 192; 4000 x 4096 25.5 / 22.6)
+  // fp32: RMSNorm of many rows that fill the threads (8192 x 4096 42.1 / 47.3, 16384 x 2048 41.4 / 47.8; cold 4000 x 2048 12.6 / 12.3, 2000 x 4096 12.7 / 12.5)
   if (dtype == 1) return mode == 0 && norm_filled(cols) && rows >= 8192;
-  // one row per SM: the ring kernel's CTA has more threads for it (LayerNorm 100 x 8192 4.1 / 3.2, 20 x 4096 2.8 / 2.4)
+  // one row per SM: the ring kernel's CTA has more threads for it (LayerNorm 100 x 8192 4.2 / 3.3, 20 x 5120 3.5 / 2.6; RMSNorm 100 x 8192 3.4 / 3.0)
   if (cols > 1536 && rows <= 148) return false;
-  // wide rows: RMSNorm 2000 x 5120 hot 7.4 / 10.2, cold 10.6 / 11.0; 2000 x 3072 6.3 / 7.5, 8.3 / 7.9; LayerNorm 2000 x 4096 8.1 / 10.2, 10.7 / 11.4; 1000 x
-  // 8192 9.0 / 11.0, 11.4 / 12.8.  But 4000 x 2560 10.2 / 10.4, 13.0 / 10.8, LayerNorm 4000 x 3072 13.4 / 13.5, 16.5 / 15.9: rings
+  // wide rows: RMSNorm 2000 x 5120 hot 7.2 / 9.5, cold 10.1 / 10.7; 2000 x 3072 5.7 / 7.3, 7.5 / 7.7; LayerNorm 2000 x 5120 10.6 / 11.9, 13.3 / 13.8; 1000 x
+  // 8192 9.0 / 11.2, 11.3 / 12.8.  But 4000 x 2560 9.3 / 10.0, 11.8 / 10.7, LayerNorm 4000 x 3072 13.2 / 13.5, 16.6 / 16.1: rings
   if (cols > 3072 || (mode == 0 && cols > 2560)) return true;
-  // middle widths: hot faster, cold slower (RMSNorm 4000 x 1536 6.8 / 7.5, 8.6 / 7.7; LayerNorm 4000 x 2048 9.2 / 10.1, 11.6 / 11.0), so by whether
+  // middle widths: hot faster, cold slower (RMSNorm 4000 x 1536 6.5 / 7.0, 8.6 / 7.6; LayerNorm 4000 x 2048 8.9 / 10.1, 10.8 / 11.0), so by whether
   // input and output can be hot
   if (mode == 0 ? cols > 1024 && cols <= 1536 : cols > 1536 && cols <= 2048) return (long long)rows * cols <= 1 << 24;
-  // narrow RMSNorm rows that are all resident at once (300 x 768 2.15 / 2.31, 1000 x 512 2.55 / 2.64; 2000 x 768 4.1 / 3.2, 300 x 256 2.2 / 2.2)
+  // narrow RMSNorm rows that are all resident at once (300 x 768 2.2 / 2.3, 1000 x 1024 2.8 / 2.8; 2000 x 768 3.9 / 3.2, 300 x 256 2.1 / 2.0)
   return mode == 0 && cols > 256 && cols <= 1024 && rows <= 8 * 148;
 }
 
@@ -868,8 +919,8 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
   if (!x || !out || rows <= 0 || cols <= 0) return TPB_ERR_ARG;
   if ((cols & 7) || cols > NORM_THREADS * 8 * NORM_MAXV) return TPB_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  // bf16 RMSNorm rows that fill 256 threads: a CTA per row in an order of its own whatever their number (600 x 4096 3.3 us, ring 4.4; 1000 x 2048 3.2
-  // and 3.7; 32768 x 4096 106 and 107; 20 x 4096 2.7 and 2.4; 2048 x 4096 10.2 and 9.3)
+  // bf16 RMSNorm rows that fill 256 threads: a CTA per row in an order of its own whatever their number (600 x 4096 3.0 us, ring 4.4; 1000 x 2048 3.0
+  // and 3.7; 20 x 4096 2.1 and 2.4; 2000 x 4096 in memory 7.9 and 9.3)
   const bool one_cta = mode == 0 && norm_filled(cols) && dtype == 0;
   if (!residual && !one_cta && cols <= NORM_BWD_MAXC && norm_takes_row_cta(rows, cols, mode, dtype)) {
 #define LAUNCH(T, M, V)                                                                                                                        \
@@ -903,7 +954,7 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
     TPB_CHECK_LAUNCH();
   }
 #define LAUNCH3(T, M, V)                                                                                              \
-  launch_kernel(norm_fwd_kernel<T, M, V>, dim3(rows), dim3(NORM_THREADS), 0, s, (const T*)x, (const T*)residual, (const T*)weight, \
+  launch_kernel(residual ? norm_fwd_kernel<T, M, V, true> : norm_fwd_kernel<T, M, V, false>, dim3(rows), dim3(NORM_THREADS), 0, s, (const T*)x, (const T*)residual, (const T*)weight, \
                 (const T*)bias, (T*)out, (T*)sum_out, rstd_out, mean_out, cols, eps)
 #define LAUNCH(T, M)                                                                     \
   do {                                                                                   \

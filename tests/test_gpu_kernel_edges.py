@@ -946,6 +946,28 @@ def test_norm_of_a_row_does_not_depend_on_the_others(dtype, cols, mode, with_wei
     assert (out[:64].double() - _norm_double(x[:64], w, mode) - (0 if b is None else b.double())).norm() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * out[:64].double().norm()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("cols", [1544, 2048, 3080, 4096, 8200, 12296, 16384])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("with_weight", [False, True])
+def test_norm_with_a_residual_of_zeros(dtype, cols, mode, with_weight):
+    """Rows held as they lie in memory and as sums in fp32: the same numbers, and the same bits where both are added up in the same order."""
+    nat = _native()
+    torch.manual_seed(cols)
+    x = (torch.randn(150, cols, device="cuda") * 2 + 0.1).to(dtype)
+    w = torch.randn(cols, device="cuda").to(dtype) if with_weight else None
+    b = torch.randn(cols, device="cuda").to(dtype) if with_weight and mode else None
+    out, rstd, _ = nat.norm_forward(x, w, b, 1e-6, mode, want_stats=True)
+    summed = torch.empty_like(x)
+    for kwargs in (dict(), dict(sum_out=summed)):
+        other, r, _ = nat.norm_forward(x, w, b, 1e-6, mode, residual=torch.zeros_like(x), want_stats=True, **kwargs)
+        if cols > 8192 or (mode == 0 and dtype == torch.bfloat16):
+            assert torch.equal(other, out) and torch.equal(r, rstd)
+        want = _norm_double(x, w, mode) + (0 if b is None else b.double())
+        assert (other.double() - want).norm() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * want.norm()
+    assert torch.equal(summed, x)
+
+
 def _norm_double(x, w, mode):
     y = x.double()
     if mode:
