@@ -126,7 +126,7 @@ constexpr int norm_row_ctas_per_sm() {
 
 // MAXV = vectors of 8 elements a thread may hold (cols <= 256 * 8 * MAXV).  RES = there is a residual; without one the row waits for its sums as it lies
 // in memory: 32 registers a thread for up to 4096 bf16 columns, so that eight rows are in flight per SM, and the weights are fetched before the sums are
-// known.  RMSNorm bf16 8192 x 4096 29.6 -> 21.9 us (6.1 TB/s), 1000 x 4096 in L2 / in memory 5.1 -> 3.7 / 6.8 -> 5.0, 20 x 4096 2.5 -> 2.0.
+// known.  RMSNorm bf16 8192 x 4096 29.6 -> 22.7 us (5.9 TB/s), 1000 x 4096 in L2 / in memory 5.1 -> 3.5 / 6.8 -> 5.1, 20 x 4096 2.5 -> 2.1; 8192 x 12288 148 -> 63.
 template <typename T, int MODE, int MAXV, bool RES>
 __global__ void __launch_bounds__(NORM_THREADS, norm_row_ctas_per_sm<T, MODE, MAXV, RES>())
 norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
