@@ -17,6 +17,7 @@
 // GQA / MQA, causal masking with a cached prefix (sk >= sq) and arbitrary q / k / v strides are supported.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -42,26 +43,27 @@ __device__ __forceinline__ float bias_at(const BiasArgs& ba, long long idx) {
 
 // 16-byte accesses: D / 8 lanes per row, four rows per lane group in flight, rows in memory order (head fastest), so that a warp
 // reads whole contiguous stretches of `out` and `dout`.  Memory-bound: 4 x 2048 x 32 heads of 128, 134 MB, 68 -> 33 us against a
-// warp per row with 2-byte loads.
-template <int D>
+// warp per row with 2-byte loads; I = unsigned where row numbers fit, whose divisions are a fraction of
+// 64-bit ones: 30.6 -> 25.8 us; 16 x 512 x 32 heads of 64 16.1 -> 14.7, 1 x 100 x 12 3.2 -> 2.7.
+template <int D, typename I>
 __global__ void __launch_bounds__(256)
 attn_bwd_delta_vec_kernel(const bf16* __restrict__ out, const bf16* __restrict__ dout, float* __restrict__ delta, int sq, int heads,
-                          long long o_sb, long long o_ss, long long o_sh, long long do_sb, long long do_ss, long long do_sh, long long rows) {
+                          long long o_sb, long long o_ss, long long o_sh, long long do_sb, long long do_ss, long long do_sh, I rows) {
   constexpr int LANES = D / 8, GROUPS = 256 / LANES, U = 4;
   const int part = threadIdx.x % LANES;
-  const long long r0 = blockIdx.x * (long long)(GROUPS * U) + threadIdx.x / LANES;
+  const I r0 = blockIdx.x * I(GROUPS * U) + threadIdx.x / LANES;
   uint4 o[U], g[U];
   long long dst[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const long long r = r0 + u * GROUPS;  // (b, i, h)
+    const I r = r0 + u * GROUPS;  // (b, i, h)
     o[u] = g[u] = make_uint4(0, 0, 0, 0);
     dst[u] = -1;
     if (r < rows) {
-      const long long t = r / heads;
-      const int h = int(r - t * heads);
-      const long long b = t / sq;
-      const int i = int(t - b * sq);
+      const I t = r / I(heads);
+      const int h = int(r - t * I(heads));
+      const long long b = t / I(sq);
+      const int i = int(t - I(b) * I(sq));
       o[u] = *reinterpret_cast<const uint4*>(out + b * o_sb + (long long)i * o_ss + (long long)h * o_sh + part * 8);
       g[u] = *reinterpret_cast<const uint4*>(dout + b * do_sb + (long long)i * do_ss + (long long)h * do_sh + part * 8);
       dst[u] = (b * heads + h) * sq + i;
@@ -397,12 +399,13 @@ extern "C" int tpb_attn_bwd_delta(const void* out, const void* dout, float* delt
   const long long rows = (long long)batch * heads * sq;
   const bool vec = !((o_sb | o_ss | o_sh | do_sb | do_ss | do_sh) & 7) && !((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout)) & 15);
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  if (vec && head_dim == 128)
-    attn_bwd_delta_vec_kernel<128><<<int((rows + 63) / 64), 256, 0, s>>>((const bf16*)out, (const bf16*)dout, delta, sq, heads, o_sb, o_ss, o_sh, do_sb,
-                                                                         do_ss, do_sh, rows);
-  else if (vec && head_dim == 64)
-    attn_bwd_delta_vec_kernel<64><<<int((rows + 127) / 128), 256, 0, s>>>((const bf16*)out, (const bf16*)dout, delta, sq, heads, o_sb, o_ss, o_sh, do_sb,
-                                                                          do_ss, do_sh, rows);
+#define DELTA(D, I)                                                                                                                              \
+  attn_bwd_delta_vec_kernel<D, I><<<int((rows + 8192 / D - 1) / (8192 / D)), 256, 0, s>>>((const bf16*)out, (const bf16*)dout, delta, sq, heads, o_sb, o_ss, \
+                                                                                         o_sh, do_sb, do_ss, do_sh, static_cast<I>(rows))
+  const bool small = rows <= INT_MAX;  // (row numbers of the last CTA go beyond `rows`, by less than 128)
+  if (vec && head_dim == 128) { if (small) DELTA(128, unsigned); else DELTA(128, long long); }
+  else if (vec && head_dim == 64) { if (small) DELTA(64, unsigned); else DELTA(64, long long); }
+#undef DELTA
   else attn_bwd_delta_kernel<<<int((rows + 7) / 8), 256, 0, s>>>(
       (const bf16*)out, (const bf16*)dout, delta, sq, heads, head_dim, o_sb, o_ss, o_sh, do_sb, do_ss, do_sh, rows);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;

@@ -3,6 +3,7 @@ range, each against an fp32 / fp64 PyTorch statement of the same operation.
 
 Tolerances: a bf16 result is half a unit in the last place (2^-9 relative) off its exact value by rounding alone; 2^-8 of the value
 leaves room for the fp32 accumulation in front of it, plus an absolute term of a few fp32 roundings of the largest term."""
+import ctypes
 import math
 
 import pytest
@@ -966,6 +967,25 @@ def test_norm_with_a_residual_of_zeros(dtype, cols, mode, with_weight):
         want = _norm_double(x, w, mode) + (0 if b is None else b.double())
         assert (other.double() - want).norm() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * want.norm()
     assert torch.equal(summed, x)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("batch", [1, 3, 2 ** 20 - 1, 2 ** 20 + 1])
+def test_row_sums_of_the_attention_backward(d, batch):
+    """Row numbers below and above 2^31 (2048 rows per sequence, sequences that share their memory)."""
+    nat = _native()
+    torch.manual_seed(d)
+    sq, heads = 64, 32
+    out, dout = (torch.randn(sq, heads, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    delta = torch.full((batch, heads, sq), math.nan, device="cuda")
+    entry = nat.LIB.tpb_attn_bwd_delta  # (only the backward calls it; undeclared pointers would be cut to 32 bits)
+    entry.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 4 + [ctypes.c_longlong] * 6 + [ctypes.c_void_p]
+    nat.check(entry(out.data_ptr(), dout.data_ptr(), delta.data_ptr(), batch, sq, heads, d, 0, heads * d, d, 0, heads * d, d, nat._stream()),
+              "tpb_attn_bwd_delta")
+    want = (out.double() * dout.double()).sum(-1).t()
+    size = (out.double() * dout.double()).abs().sum(-1).t()
+    assert bool(((delta[0].double() - want).abs() <= 2.0 ** -24 * d * size).all())  # (products are exact in fp32, at most d roundings of partial sums)
+    assert all(torch.equal(part, delta[:1].expand_as(part)) for part in delta.split(2 ** 16))
 
 
 def _norm_double(x, w, mode):
