@@ -658,13 +658,17 @@ attn_decode_fused_kernel(const bf16* q, const bf16* k, const bf16* v,
 // (for the scores) and head elements (for the output) its columns.  Head by head on the CUDA cores, every key costs about 45 instructions
 // per query head and four keys, and the kernel above is bound by them (16 sequences x 1024 keys, 128 / 8 heads of 64: 57 us for 34 MB).
 // A warp takes 16 keys per iteration from a ring of its own (cp.async; keys past the end arrive as zeros, the new key is put into its row of
-// the last tile), keeps its own running maximum and sum, and the warps' results are merged at the end.  Nothing is held in fewer bits
-// than on the CUDA cores: q, K and V are bf16 numbers as they are, and a probability enters as the exact sum of three bf16 numbers (8 bits
-// each, fp32 has 24), in three MMAs.  Only where a result is not finite - 0 * inf in one of the three parts is NaN - the CTA does its keys
-// again on the CUDA cores.  Partial results against 64 bits, 16 heads of 64, 30 / 1000 / 4000 keys: 1.2 / 2.2 / 2.8e-7 of the result on the CUDA
-// cores, 1.0 / 1.8 / 2.1e-7 here (two bf16 numbers per probability: 2e-6).  Replayed from a CUDA graph, caches in memory: 16 x 1024 keys, 128 / 8 heads of
-// 64 57 -> 13 us; 8 x 2048, 32 / 8 heads of 128 54 -> 22 us; 16 x 2048, 40 / 10 heads of 128 165 -> 48 us; 20 keys, 128 / 8 heads of 64 9.7 -> 7.4 us, four
-// heads of 64 6.0 -> 5.3 us, 8 x 60 keys of them 6.4 -> 6.7 us (the worst of 100 shapes).
+// the last tile), keeps its own running maximum and sum, and the warps' results are merged at the end.  q, K and V are bf16 numbers as they are,
+// and a probability enters as the sum of three bf16 numbers (8 bits each, fp32 has 24; exact above 2^-100; far below, the third is too small for a bf16
+// number), in three MMAs.  An MMA's additions cut off what does not fit beside their largest term, so no sum runs on in an accumulator: a step's 16
+// products are added up in one, and the steps in fp32, scores over the head as well as outputs over the keys.  Only where a result is not finite -
+// 0 * inf in one of the three parts is NaN - the CTA does its keys again on the CUDA cores.
+// Results before their rounding, against 64 bits, on the CUDA cores / here: 128 / 8 heads of 64, 30 / 1000 / 2400 keys 1.1 / 1.7 / 2.0e-7 and 1.0 / 1.5 / 1.6e-7,
+// 16 / 4 heads of 128 1.3 / 1.9 / 2.1e-7 and 1.0 / 1.6 / 1.8e-7 (a score in one accumulator: 1.4 / 2.1 / 2.3e-7); with eight channels of magnitude 30 whose
+// products cancel 8.3 / 2.4 / 2.8e-6 and 4.1 / 1.1 / 1.3e-6 (5.4 / 3.8 / 5.5e-6).  (What is cut off shifts all scores alike, which their softmax does not see.)
+// Replayed from a CUDA graph, caches in memory: 16 x 1024 keys, 128 / 8 heads of 64 57 -> 13 us; 8 x 2048, 32 / 8 heads of 128 54 -> 22 us; 16 x 2048,
+// 40 / 10 heads of 128 165 -> 48 us; 20 keys, 128 / 8 heads of 64 9.7 -> 7.3 us, four heads of 64 5.9 -> 5.8; but 60 and 150 keys of groups of four heads
+// of 64 6.1 to 6.5 -> 6.3 to 6.6, 5 % more at worst (the host does not know the number of keys).
 template <int D>
 struct GqaShape {
   static constexpr int WARPS = D == 64 ? 8 : 4, THREADS = WARPS * 32, STAGES = 3, KEYS = 16;
@@ -811,8 +815,13 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
     for (int ks = 0; ks < D / 16; ++ks) {
       uint32_t kb[4];
       ldmatrix_x4(kb, tile_ptr<D>(kt, (id >> 1) * 8 + r8, ks * 2 + (id & 1)));
-      mma_bf16_16816(sc[0], qf[ks], kb[0], kb[1]);
-      mma_bf16_16816(sc[1], qf[ks], kb[2], kb[3]);
+      float t[2][4] = {};
+      mma_bf16_16816(t[0], qf[ks], kb[0], kb[1]);
+      mma_bf16_16816(t[1], qf[ks], kb[2], kb[3]);
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sc[n][j] += t[n][j];
     }
 #pragma unroll
     for (int n = 0; n < 2; ++n)
@@ -855,8 +864,7 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
     for (int n = 0; n < D / 16; ++n) {
       uint32_t vb[4];
       ldmatrix_x4_trans(vb, tile_ptr<D>(vt, (id & 1) * 8 + r8, n * 2 + (id >> 1)));
-      // the tile's sum first, then an fp32 addition that rounds to nearest: the MMA's own additions cut off what does not fit, which over
-      // 2000 keys in one accumulator came to 4.5e-7 of the result (the kernel above: 2.4e-7)
+      // (over 2000 keys in one accumulator, what was cut off came to 4.5e-7 of the result)
       float t[2][4] = {};
 #pragma unroll
       for (int u = 2; u >= 0; --u) {  // (the small parts first)

@@ -672,6 +672,38 @@ def test_decode_attention_keeps_its_partial_results_in_32_bits(hq, hkv, d, split
             assert (got.double() - want).norm() <= 1e-6 * want.norm()
 
 
+@pytest.mark.parametrize("group,d", [(4, 128), (16, 128), (16, 64)])
+@pytest.mark.parametrize("outlier", [0, 8, 30, 100])
+@pytest.mark.parametrize("ctx", [30, 1000, 2400])
+def test_decode_attention_of_grouped_heads_is_as_exact_as_of_single_ones(group, d, outlier, ctx):
+    """Outputs before their rounding against 64 bits, from heads that share a KV head and from the same heads two by two, which take a kernel with fp32
+    multiplications and additions on the CUDA cores; also where scores are small sums of large products (a few channels of magnitude `outlier`)."""
+    nat = _native()
+    torch.manual_seed(group + d + outlier)
+    b, splits = 4, 2
+    kc, vc = (torch.randn(b, 1, ctx + 8, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    qkv = torch.randn(b, (group + 2) * d, device="cuda", dtype=torch.bfloat16)
+    for c in (2, 17, 40, 59) if outlier else ():  # two channels whose products with q are each other's negative
+        c2 = (c + 21) % d
+        qkv.view(b, -1, d)[:, :group, c2] = qkv.view(b, -1, d)[:, :group, c] = outlier * (1 + 0.3 * torch.rand(b, group, device="cuda"))
+        kc[..., c] = outlier * (1 + 0.3 * torch.rand(b, 1, ctx + 8, device="cuda"))
+        kc[..., c2] = -kc[..., c]
+    q, k, v = qkv.split([group * d, d, d], dim=1)
+    at = torch.tensor([ctx], device="cuda", dtype=torch.int32)
+
+    def merged(q, heads):
+        part_o, part_ml = torch.empty(b, heads, splits, d, device="cuda"), torch.empty(b, heads, splits, 2, device="cuda")
+        nat.attn_decode_fused(q, k, v, kc, vc, at, 0, 10000.0, splits=splits, workspace=(part_o, part_ml, torch.zeros(b * heads, dtype=torch.int32, device="cuda")))
+        w = (part_ml[..., 0].double() - part_ml[..., 0].double().amax(-1, keepdim=True)).exp2()
+        return (part_o.double() * w[..., None]).sum(2) / (part_ml[..., 1].double() * w).sum(2)[..., None]
+
+    got = merged(q, group)
+    single = torch.cat([merged(q[:, i * d : (i + 2) * d], 2) for i in range(0, group, 2)], dim=1)
+    kd, vd = (t[:, :, : ctx + 1].double().expand(-1, group, -1, -1) for t in (kc, vc))
+    want = torch.einsum("bhn,bhnd->bhd", (torch.einsum("bhd,bhnd->bhn", q.reshape(b, group, d).double(), kd) / math.sqrt(d)).softmax(-1), vd)
+    assert (got - want).norm() <= (single - want).norm()
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (16, 1, 64), (2, 2, 64)])
 @pytest.mark.parametrize("splits", [1, 3])
 def test_decode_attention_of_infinite_values(hq, hkv, d, splits):
