@@ -958,6 +958,7 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
   }
   __syncthreads();
   // four elements per thread: a group of four heads of 128 is one round of the CTA
+  const bool vec = !(reinterpret_cast<uintptr_t>(part_o) & 15);  // (partials of a caller's workspace, which may begin anywhere)
   auto store = [&](int qh, int d, float4 x, float ll) {
     bf16* dst = out + (long long)b * out_ld + (long long)qh * D + d;
     dst[0] = __float2bfloat16(ll > 0.f ? x.x / ll : 0.f);
@@ -991,7 +992,9 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
     if (splits == 1) {
       store(qh, d, oo, ll);
     } else {
-      *reinterpret_cast<float4*>(part_o + (row * splits + split) * D + d) = oo;
+      float* dst = part_o + (row * splits + split) * D + d;
+      if (vec) *reinterpret_cast<float4*>(dst) = oo;
+      else dst[0] = oo.x, dst[1] = oo.y, dst[2] = oo.z, dst[3] = oo.w;
       if (d == 0) { part_ml[(row * splits + split) * 2] = mm; part_ml[(row * splits + split) * 2 + 1] = ll; }
     }
   }
@@ -1023,7 +1026,10 @@ attn_decode_gqa_kernel(const bf16* q, const bf16* k, const bf16* v, bf16* __rest
         const bool live = s0 + q8 < splits;
         const long long pr = row * splits + s0 + q8;
         ml[q8] = live ? make_float2(__ldcg(part_ml + pr * 2), __ldcg(part_ml + pr * 2 + 1)) : make_float2(-INFINITY, 0.f);
-        os[q8] = live ? __ldcg(reinterpret_cast<const float4*>(part_o + pr * D + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* src = part_o + pr * D + d;
+        os[q8] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live && vec) os[q8] = __ldcg(reinterpret_cast<const float4*>(src));
+        else if (live) os[q8] = make_float4(__ldcg(src), __ldcg(src + 1), __ldcg(src + 2), __ldcg(src + 3));
       }
       float m_new = mm;
 #pragma unroll
@@ -1417,10 +1423,10 @@ extern "C" int tpb_attn_decode_fused(const void* q, const void* k, const void* v
   const float l2t = log2f(theta);
   int done = 0, launches = 0;
   // four heads and more fill a quarter and more of the rows of an MMA; below that the rows that would be empty cost more than they bring
-  const bool tensor = g_total >= 4 && !(reinterpret_cast<uintptr_t>(part_o) & 15);
+  const bool tensor = g_total >= 4;
   while (done < g_total) {
     const int left = g_total - done;
-    const int gnow = tensor ? 16 : (left >= 2 ? 2 : 1);  // (larger groups come here only with partials off a 16-byte boundary)
+    const int gnow = tensor ? 16 : (left >= 2 ? 2 : 1);
     // equal groups share one launch (grid z) when the caller's counter array has a counter for each of them
     int reps = tensor ? (left + 15) / 16 : left / gnow;
     if (splits > 1 && (long long)batch * kv_heads * reps > counter_elems) reps = 1;

@@ -753,6 +753,24 @@ def test_decode_attention_of_grouped_heads_beside_other_keys(hq, hkv, d, splits,
         assert bool(((out.double() - want).abs()[fin] <= (2.0 ** -8 * want.abs() + 1e-5)[fin]).all())  # one bf16 rounding
 
 
+@pytest.mark.parametrize("hq,hkv,d", [(4, 1, 64), (23, 1, 64), (8, 2, 128)])
+@pytest.mark.parametrize("off", [1, 2])
+def test_decode_attention_with_partials_anywhere(hq, hkv, d, off):
+    """Partial results off a 16-byte boundary: the same kernel, one launch, the same bits."""
+    nat = _native()
+    torch.manual_seed(hq)
+    b, splits, ctx, smax = 2, 3, 90, 128
+    kc, vc = (torch.randn(b, hkv, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    q, k, v = torch.randn(b, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16).split([hq * d, hkv * d, hkv * d], dim=1)
+    at = torch.tensor([ctx], device="cuda", dtype=torch.int32)
+    outs = []
+    for o in (0, off):
+        ws = (torch.empty(b * hq * splits * d + o, device="cuda")[o:], torch.empty(b * hq * splits * 2, device="cuda"), torch.zeros(b * hq, dtype=torch.int32, device="cuda"))
+        outs.append(nat.attn_decode_fused(q, k, v, kc.clone(), vc.clone(), at, 0, 10000.0, splits=splits, workspace=ws))
+        assert nat.LIB.tpb_last_launches() == 1
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(2, 2, 128), (2, 1, 64), (4, 1, 128), (8, 1, 64), (6, 2, 128)])
 @pytest.mark.parametrize("rotary_dim", [0, 32, None])
 @pytest.mark.parametrize("interleaved", [False, True])
