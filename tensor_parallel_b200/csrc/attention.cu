@@ -8,6 +8,7 @@
 //                         arbitrary q / k / v strides), fp32 online softmax, optional log-sum-exp output
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -318,7 +319,7 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kcache, 
   float m[G], l[G], acc[G][EPL];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY;
+    m[g] = -FLT_MAX;  // (not -inf: a score of -inf, of a masked key, would make NaN of -inf - -inf)
     l[g] = 0.f;
 #pragma unroll
     for (int e = 0; e < EPL; ++e) acc[g][e] = 0.f;
@@ -521,7 +522,7 @@ attn_decode_fused_kernel(const bf16* q, const bf16* k, const bf16* v,
   float m[G], l[G], acc[G][EPL];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY;
+    m[g] = -FLT_MAX;  // (not -inf: a score of -inf, of a masked key, would make NaN of -inf - -inf)
     l[g] = 0.f;
 #pragma unroll
     for (int e = 0; e < EPL; ++e) acc[g][e] = 0.f;

@@ -723,12 +723,11 @@ def test_decode_attention_of_infinite_values(hq, hkv, d, splits):
     assert bool((out[..., 3] == float("inf")).all() and (out[..., 5] == float("-inf")).all()) and not out.isnan().any()
 
 
-@pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (16, 1, 64), (23, 1, 64)])
+@pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (16, 1, 64), (23, 1, 64), (1, 1, 128), (2, 1, 64), (3, 1, 128)])
 @pytest.mark.parametrize("splits,off", [(1, 0), (3, 0), (3, 1)])
-@pytest.mark.parametrize("bad", [False, True])
-def test_decode_attention_of_grouped_heads_beside_other_keys(hq, hkv, d, splits, off, bad):
-    """A masked-out key (-inf scores) and an infinite value change their own sequence only, and leave the others' bits alone; the new key at every
-    place of a tile of 16; partial results off a 16-byte boundary."""
+def test_decode_attention_of_grouped_heads_beside_other_keys(hq, hkv, d, splits, off):
+    """Masked-out keys (-inf scores), the first of every lane's range among them, and an infinite value change their own sequence only, and leave the others'
+    bits alone; the new key at every place of a tile of 16; partial results off a 16-byte boundary."""
     nat = _native()
     torch.manual_seed(hq)
     b, smax = 3, 64
@@ -737,20 +736,38 @@ def test_decode_attention_of_grouped_heads_beside_other_keys(hq, hkv, d, splits,
         qkv = torch.randn(b, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16).abs()
         q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
         at = torch.tensor([ctx], device="cuda", dtype=torch.int32)
-        ws = (torch.empty(b * hq * splits * d + off, device="cuda")[off:], torch.empty(b * hq * splits * 2, device="cuda"), torch.zeros(b * hq, dtype=torch.int32, device="cuda"))
-        k2, v2 = kc.clone(), vc.clone()
-        if bad:
-            if not off:  # (the kernel for one and two heads, which also takes such workspaces, makes NaN of a range that begins with -inf)
-                k2[1, :, 11] = float("-inf")  # (q is positive: the score is -inf, the probability 0)
-            v2[1, :, 7, 3] = float("inf")
-        out = nat.attn_decode_fused(q, k, v, k2, v2, at, 0, 10000.0, splits=splits, workspace=ws).view(b, hq, d)
-        assert torch.equal(k2[:, :, ctx], k.view(b, hkv, d)) and torch.equal(v2[:, :, ctx], v.view(b, hkv, d))
-        kd, vd = (t[:, :, : ctx + 1].double().repeat_interleave(hq // hkv, 1) for t in (k2, v2))
-        p = (torch.einsum("bhd,bhnd->bhn", q.reshape(b, hq, d).double(), kd) / math.sqrt(d)).softmax(-1)
-        want = torch.einsum("bhn,bhnd->bhd", p, vd)
-        assert torch.equal(out.isinf(), want.isinf()) and not out.isnan().any()
-        fin = want.isfinite()
-        assert bool(((out.double() - want).abs()[fin] <= (2.0 ** -8 * want.abs() + 1e-5)[fin]).all())  # one bf16 rounding
+        outs = []
+        for bad in (False, True):
+            ws = (torch.empty(b * hq * splits * d + off, device="cuda")[off:], torch.empty(b * hq * splits * 2, device="cuda"), torch.zeros(b * hq, dtype=torch.int32, device="cuda"))
+            k2, v2 = kc.clone(), vc.clone()
+            if bad:
+                k2[1, :, [0, 1, 2, 3, 11, 14, 15, 16, 17, 29]] = float("-inf")  # (q is positive: the score is -inf, the probability 0)
+                v2[1, :, 7, 3] = float("inf")
+            out = nat.attn_decode_fused(q, k, v, k2, v2, at, 0, 10000.0, splits=splits, workspace=ws).view(b, hq, d)
+            assert torch.equal(k2[:, :, ctx], k.view(b, hkv, d)) and torch.equal(v2[:, :, ctx], v.view(b, hkv, d))
+            kd, vd = (t[:, :, : ctx + 1].double().repeat_interleave(hq // hkv, 1) for t in (k2, v2))
+            p = (torch.einsum("bhd,bhnd->bhn", q.reshape(b, hq, d).double(), kd) / math.sqrt(d)).softmax(-1)
+            want = torch.einsum("bhn,bhnd->bhd", p, vd)
+            outs.append(out)
+            assert torch.equal(out.isinf(), want.isinf()) and not out.isnan().any()
+            fin = want.isfinite()
+            assert bool(((out.double() - want).abs()[fin] <= (2.0 ** -8 * want.abs() + 1e-5)[fin]).all())  # one bf16 rounding
+        assert torch.equal(outs[0][[0, 2]], outs[1][[0, 2]])
+
+
+@pytest.mark.parametrize("group,d", [(1, 64), (2, 128), (8, 64)])
+def test_decode_attention_of_a_cache_that_begins_with_masked_keys(group, d):
+    nat = _native()
+    torch.manual_seed(d)
+    b, n, smax = 2, 100, 128
+    kc, vc = (torch.randn(b, 1, smax, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    q = torch.randn(b, group, d, device="cuda", dtype=torch.bfloat16).abs()
+    kc[:, :, :40] = float("-inf")
+    for splits in (1, 4):
+        out = nat.attn_decode(q, kc, vc, torch.tensor([n], device="cuda", dtype=torch.int32), 0, splits=splits).view(b, group, d)
+        kd, vd = kc[:, :, 40:n].double().expand(-1, group, -1, -1), vc[:, :, 40:n].double().expand(-1, group, -1, -1)
+        want = torch.einsum("bhn,bhnd->bhd", (torch.einsum("bhd,bhnd->bhn", q.double(), kd) / math.sqrt(d)).softmax(-1), vd)
+        assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all())  # one bf16 rounding
 
 
 @pytest.mark.parametrize("hq,hkv,d", [(4, 1, 64), (23, 1, 64), (8, 2, 128)])
