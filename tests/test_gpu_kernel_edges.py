@@ -967,6 +967,34 @@ def test_attention_with_two_ctas_per_sm(b, sq, sk, hq, hkv, causal, d, bias):
         assert (t.grad.double() - ref.grad).norm() <= 0.01 * ref.grad.norm() + 1e-6
 
 
+@pytest.mark.parametrize("bias", ["none", "dense", "fp32", "mask"])
+@pytest.mark.parametrize("at", [3, 70, 127])
+def test_attention_does_not_round_the_largest_probability_of_the_first_128_keys(bias, at):
+    """One key with nearly all of the weight, so that the output is its value, rounded once; tiles of 64 keys at head_dim 64."""
+    nat = _native()
+    torch.manual_seed(at)
+    b, s, h = 10, 140, 16
+    scores = torch.full((h, s), -12.0, device="cuda")
+    scores[:, 0] = 0.0
+    scores[:, at] = 4 + torch.rand(h, device="cuda")  # less than 2^8 above the first key
+    scores = scores.bfloat16()
+    q, k = (torch.zeros(b, s, h, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    v = torch.randn(b, s, h, 64, device="cuda", dtype=torch.bfloat16)
+    added = None
+    if bias == "none":
+        q[..., 0], k[..., 0] = 8, scores.t()
+    elif bias == "mask":
+        scores = scores[:1].expand(h, s)
+        added = scores[0].view(1, 1, 1, s).repeat(b, 1, 1, 1)
+    else:
+        added = torch.zeros(1, h, s, 144, device="cuda", dtype=torch.float32 if bias == "fp32" else torch.bfloat16)[..., :s]
+        added.copy_(scores[None, :, None])
+    out, _ = nat.attention_forward(q, k, v, False, None, want_lse=True, bias=added)
+    want = torch.einsum("hk,bkhd->bhd", scores.double().softmax(-1), v.double())[:, None]
+    # one bf16 rounding (2^-8 at most); the other keys have 2 % of the weight, each rounded once more, and V is below 5
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -8 * 0.02 * 5).all())
+
+
 # a tile per CTA for the gradient of a shared bias: whole tiles, ragged ones, rows of a multiple of eight, more keys than queries, a plane for all heads
 @pytest.mark.parametrize("b,sq,sk,hq,hkv,shared", [(3, 256, 256, 32, 32, False), (1, 240, 248, 30, 15, False), (2, 384, 1000, 6, 6, False), (5, 1152, 1792, 2, 1, True)])
 @pytest.mark.parametrize("causal", [False, True])
