@@ -131,9 +131,16 @@ Tensor in_shape(const Tensor& rows, const c10::IValue& shape) {
   return sizes.empty() ? rows : rows.view(sizes);
 }
 
+// Whether something goes on around a gradient that a kernel would drop out of: a graph of its own (create_graph), a batch of gradients
+// (is_grads_batched) or another transform, a tensor subclass.
+bool more_than_numbers(const Tensor& g) {
+  return (at::GradMode::is_enabled() && g.requires_grad()) || !g.has_storage() || g.unsafeGetTensorImpl()->is_python_dispatch();
+}
+
 // The gradient of a bias: column sums of g in fp32, as `dtype`.
 Tensor column_sums(const Tensor& g, at::ScalarType dtype) {
-  if (!lib.col_sum || g.size(0) == 0 || g.size(1) % 8 || (dtype != at::kBFloat16 && dtype != at::kFloat) || reinterpret_cast<uintptr_t>(g.const_data_ptr()) % 16)
+  if (!lib.col_sum || more_than_numbers(g) || g.size(0) == 0 || g.size(1) % 8 || (dtype != at::kBFloat16 && dtype != at::kFloat) ||
+      reinterpret_cast<uintptr_t>(g.const_data_ptr()) % 16)
     return g.sum(at::IntArrayRef{0}, false, at::kFloat).to(dtype);  // (summed in fp32 without an fp32 copy of the gradient)
   const int rows = int(g.size(0)), cols = int(g.size(1)), parts = lib.col_sum_parts(rows, cols);
   Tensor out = at::empty({cols}, g.options().dtype(dtype)), partials = parts > 1 ? at::empty({parts, cols}, g.options().dtype(at::kFloat)) : Tensor();

@@ -85,13 +85,27 @@ def _norm_bwd(dy, x, weight, rstd, mean, dx, part_w, part_b, dw, db, rows, cols,
     return 0
 
 
+def _col_sum_parts(rows, cols):
+    return 2
+
+
+def _col_sum(g, out, partials, rows, cols, fp32, stream):
+    _memory(out, cols, torch.float32 if fp32 else torch.bfloat16).copy_(_matrix(g, rows, cols, cols).float().sum(0))
+    _col_sum.calls += 1
+    return 0
+
+
+_col_sum.calls = 0
+
+
 @pytest.fixture
 def nodes():
     from tensor_parallel_b200.ops import native
 
     signatures = dict(tpb_gemm_plan_ex=(_plan, [_i] * 7 + [_p]), tpb_gemm_bf16_ex=(_gemm, [_p] * 5 + [_i] * 7 + [_f] + [_p] * 4),
                       tpb_norm_fwd=(_norm_fwd, [_p] * 8 + [_i, _i, _f, _i, _i, _p]), tpb_norm_bwd=(_norm_bwd, [_p] * 10 + [_i] * 5 + [_p]),
-                      tpb_norm_bwd_parts=(_norm_bwd_parts, [_i, _i]))
+                      tpb_norm_bwd_parts=(_norm_bwd_parts, [_i, _i]), tpb_col_sum_parts=(_col_sum_parts, [_i, _i]),
+                      tpb_col_sum=(_col_sum, [_p] * 3 + [_i] * 3 + [_p]))
     stubs = {name: ctypes.CFUNCTYPE(_i, *args)(fn) for name, (fn, args) in signatures.items()}
     context = native.ReduceCtx()
     native.AUTOGRAD.bind({n: ctypes.cast(s, _p).value for n, s in stubs.items()}, native._error_text, lambda index, elems: ctypes.addressof(context))
@@ -144,6 +158,25 @@ def test_linear_node(nodes, with_bias, frozen, form):
         assert (got is None) == (want is None)
         if want is not None:
             _close(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gradient_of_a_bias_of_its_own_takes_part_in_what_goes_on_around_it(nodes, dtype):
+    """The layer's bias alone is trained: its gradient of a batch of gradients, and a graph through it; one gradient takes the kernel."""
+    torch.manual_seed(3)
+    x, w = torch.randn(10, 24, dtype=torch.bfloat16), torch.randn(16, 24, dtype=torch.bfloat16)
+    b = torch.zeros(16, dtype=torch.bfloat16, requires_grad=True)
+    out = nodes.linear(x, w, b).to(dtype)
+    g = torch.randn(3, 10, 16).to(dtype)
+    before = _col_sum.calls
+    (batched,) = torch.autograd.grad(out, b, g, is_grads_batched=True, retain_graph=True)
+    single = torch.stack([torch.autograd.grad(out, b, t, retain_graph=True)[0] for t in g])
+    _close(batched, single)
+    assert _col_sum.calls == before + 3
+    leaf = g[0].clone().requires_grad_()
+    (once,) = torch.autograd.grad(out, b, leaf, create_graph=True)
+    (twice,) = torch.autograd.grad(once.float().square().sum(), leaf)
+    _close(twice, (2 * once.detach().float()).expand(10, 16).to(dtype))
 
 
 @pytest.mark.parametrize("frozen", [(), (0,), (1, 3), (2,)])
