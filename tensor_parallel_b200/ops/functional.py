@@ -198,10 +198,12 @@ def relative_bias(embedding: torch.nn.Module, buckets, queries: int, keys: int):
 
 def relative_buckets(first: int, count: int, device, bidirectional: bool, buckets: int, max_distance: int):
     """Relative-position buckets of the distances ``first``, ``first + 1``, ... by one kernel, or None where the caller has to take the steps over
-    tensors (other devices, tracing, dispatch modes, ranges that the kernel does not cover)."""
-    exact = buckets // (4 if bidirectional else 2)
-    if (torch.device(device).type != "cuda" or _FORCE_TORCH or not 0 < count <= 2 ** 31 or exact < 1 or max_distance <= exact
-            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()):
+    tensors (other devices than the current one, functorch transforms, tracing, dispatch modes, ranges that the kernel does not cover)."""
+    exact, device = buckets // (4 if bidirectional else 2), torch.device(device)
+    if (device.type != "cuda" or _FORCE_TORCH or not 0 < count <= 2 ** 31 or type(buckets) is not int or type(max_distance) is not int
+            or not 0 < exact < max_distance < 2 ** 31 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()
+            or device.index not in (None, torch.cuda.current_device())):
         return None
     from tensor_parallel_b200.ops import native
 

@@ -2,6 +2,7 @@
 out its rows, and the relative-position bias by distance against the lookup of every pair."""
 import ctypes
 import re
+import sys
 import types
 
 import pytest
@@ -312,3 +313,24 @@ def test_a_step_says_what_its_kernels_reported(code, words):
         with pytest.raises(TPCollectiveError, match=words):
             DecoderEngine._raise_on_status(engine)
     assert int(status.sum()) == 0
+
+
+@pytest.mark.parametrize("buckets,max_distance,inside", [(32, 128, "vmap"), (32, 128, "grad"), (32, 128, "jvp"), (32, 128, "another device"), (32, 128.0, ""),
+                                                         (32, 2 ** 31, ""), (32, 128, "plain")])
+def test_relative_buckets_of_a_program_that_transforms_its_functions(monkeypatch, buckets, max_distance, inside):
+    """The kernel is asked for only where its result is a plain tensor on the current device, and for numbers that its entry takes."""
+    asked = []
+    monkeypatch.setitem(sys.modules, "tensor_parallel_b200.ops.native", types.SimpleNamespace(relative_buckets=lambda *a: asked.append(a)))
+    import tensor_parallel_b200.ops as ops
+
+    monkeypatch.setattr(ops, "native", sys.modules["tensor_parallel_b200.ops.native"], raising=False)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    device = "cuda:1" if inside == "another device" else "cuda:0"
+
+    def call(t):
+        assert OF.relative_buckets(-3, 7, device, True, buckets, max_distance) is None
+        return t.sum()
+
+    transform = dict(vmap=torch.vmap, grad=torch.func.grad, jvp=lambda f: lambda t: torch.func.jvp(f, (t,), (t,))).get(inside, lambda f: f)
+    transform(call)(torch.ones(2, 3) if inside == "vmap" else torch.ones(3))
+    assert len(asked) == (inside == "plain")
