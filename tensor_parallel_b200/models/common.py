@@ -65,9 +65,10 @@ def _only_multiplies(module: nn.Module) -> bool:
             and not any(hooks))
 
 
-def linears(x, *modules: nn.Module):
-    """``tuple(module(x) for module in modules)``, as one autograd node where the modules are plain projections."""
-    if all(type(m) is Linear and _only_multiplies(m) for m in modules):
+def linears(x, *modules: nn.Module, joint: bool = True):
+    """``tuple(module(x) for module in modules)``, as one autograd node where the modules are plain projections.  ``joint=False`` where a result leaves the
+    caller with its graph, as cached keys and values do: a backward through one of them would free what the others have saved."""
+    if joint and all(type(m) is Linear and _only_multiplies(m) for m in modules):
         outs = OF.linears(x, [m.weight for m in modules])
         if outs is not None:
             return tuple(outs)

@@ -38,13 +38,13 @@ class GPTJAttention(nn.Module):
         self.v_proj = Linear(self.embed_dim, self.embed_dim, bias=False)
         self.out_proj = Linear(self.embed_dim, self.embed_dim, bias=False)
 
-    def _qkv(self, hidden_states):
+    def _qkv(self, hidden_states, cached):
         b, s, _ = hidden_states.shape
-        return tuple(t.view(b, s, -1, self.head_dim) for t in linears(hidden_states, self.q_proj, self.k_proj, self.v_proj))
+        return tuple(t.view(b, s, -1, self.head_dim) for t in linears(hidden_states, self.q_proj, self.k_proj, self.v_proj, joint=not cached))
 
     def forward(self, hidden_states, layer_past=None, attention_mask=None, position_ids=None, use_cache=False):
         b, s, _ = hidden_states.shape
-        q, k, v = self._qkv(hidden_states)
+        q, k, v = self._qkv(hidden_states, use_cache or layer_past is not None)
         q = OF.apply_rope(q, position_ids, self.rope_theta, self.rotary_dim, interleaved=True)
         k = OF.apply_rope(k, position_ids, self.rope_theta, self.rotary_dim, interleaved=True)
         k_all, v_all, present = update_kv(layer_past, k, v)
@@ -64,7 +64,7 @@ class CodeGenAttention(GPTJAttention):
         self.qkv_proj = Linear(self.embed_dim, 3 * self.embed_dim, bias=False)
         self.out_proj = Linear(self.embed_dim, self.embed_dim, bias=False)
 
-    def _qkv(self, hidden_states):
+    def _qkv(self, hidden_states, cached):
         b, s, _ = hidden_states.shape
         fused = self.qkv_proj(hidden_states).view(b, s, self.MP, 3, -1, self.head_dim)
         q, v, k = fused[:, :, :, 0], fused[:, :, :, 1], fused[:, :, :, 2]

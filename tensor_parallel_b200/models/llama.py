@@ -47,7 +47,8 @@ class LlamaAttention(nn.Module):
     def forward(self, hidden_states, attention_mask=None, position_ids=None, past_key_value=None,
                 output_attentions=False, use_cache=False):
         b, s, _ = hidden_states.shape
-        q, k, v = (t.view(b, s, -1, self.head_dim) for t in linears(hidden_states, self.q_proj, self.k_proj, self.v_proj))
+        cached = use_cache or past_key_value is not None
+        q, k, v = (t.view(b, s, -1, self.head_dim) for t in linears(hidden_states, self.q_proj, self.k_proj, self.v_proj, joint=not cached))
         q = OF.apply_rope(q, position_ids, self.rope_theta)
         k = OF.apply_rope(k, position_ids, self.rope_theta)
         k_all, v_all, present = update_kv(past_key_value, k, v)

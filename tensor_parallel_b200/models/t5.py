@@ -89,10 +89,11 @@ class T5Attention(nn.Module):
             k_cache, v_cache = past_key_value[0], past_key_value[1]
         else:
             source = key_value_states if is_cross else hidden_states
+            joint = past_key_value is None and not (self.is_decoder and use_cache)
             if is_cross:
-                q, (k, v) = self.q(hidden_states), linears(source, self.k, self.v)
+                q, (k, v) = self.q(hidden_states), linears(source, self.k, self.v, joint=joint)
             else:
-                q, k, v = linears(source, self.q, self.k, self.v)
+                q, k, v = linears(source, self.q, self.k, self.v, joint=joint)
             k_cache = k.view(b, source.shape[1], -1, d).transpose(1, 2)
             v_cache = v.view(b, source.shape[1], -1, d).transpose(1, 2)
             if not is_cross and past_key_value is not None:

@@ -240,6 +240,50 @@ def test_modules_that_do_more_than_multiply_are_called_as_they_are(nodes, monkey
     assert len(common.linears(x.requires_grad_(), *modules)) == 2  # (on the CPU every module is called)
 
 
+@pytest.mark.parametrize("use_cache,past", [(False, False), (True, False), (False, True)])
+@pytest.mark.parametrize("model", ["llama", "gptj", "t5 encoder", "t5 decoder", "t5 cross-attention"])
+def test_cached_keys_and_values_have_graphs_of_their_own(monkeypatch, model, use_cache, past):
+    """A backward through cached keys and then one through the values, which left the layer with their graph."""
+    from tensor_parallel_b200.models import common, gptj, llama, t5
+
+    joint = []
+
+    class Joint(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x, *ws):
+            joint.append(len(ws))
+            ctx.save_for_backward(x, *ws)
+            return tuple(F.linear(x, w) for w in ws)
+
+        @staticmethod
+        def backward(ctx, *gs):
+            x, *ws = ctx.saved_tensors
+            return (sum(g @ w for g, w in zip(gs, ws)), *(g.flatten(0, 1).t() @ x.flatten(0, 1) for g in gs))
+
+    monkeypatch.setattr(common.OF, "linears", lambda x, ws: Joint.apply(x, *ws))
+    torch.manual_seed(0)
+    x = torch.randn(2, 5, 32, requires_grad=True)
+    before = tuple(torch.randn(2, 2, 3, 16, requires_grad=True) for _ in range(2)) if past and model != "t5 encoder" else None
+    positions = torch.arange(5)[None].expand(2, 5)
+    if model == "llama":
+        layer = llama.LlamaAttention(llama.LlamaConfig(hidden_size=32, num_attention_heads=2, num_key_value_heads=2))
+        out, _, present = layer(x, position_ids=positions, past_key_value=before, use_cache=use_cache)
+    elif model == "gptj":
+        layer = gptj.GPTJAttention(gptj.GPTJConfig(n_embd=32, n_head=2, rotary_dim=8))
+        out, present = layer(x, position_ids=positions, layer_past=before, use_cache=use_cache)
+    else:
+        layer = t5.T5Attention(t5.T5Config(d_model=32, num_heads=2, d_kv=16), True, model != "t5 encoder")
+        out, present, _ = layer(x, key_value_states=torch.randn(2, 4, 32, requires_grad=True) if "cross" in model else None, past_key_value=before, use_cache=use_cache)
+    escapes = (use_cache or past) and model != "t5 encoder"
+    assert joint == ([] if escapes else [2 if "cross" in model else 3])
+    if present is not None:
+        for t in present:
+            if t.requires_grad:
+                t.sum().backward()
+    else:
+        out.sum().backward()
+
+
 @pytest.mark.parametrize("mode,dtype,wdtype,with_bias,with_weight", [(0, torch.bfloat16, torch.bfloat16, False, True), (0, torch.float32, torch.float32, False, True),
                                                                    (1, torch.bfloat16, torch.bfloat16, True, True), (1, torch.float32, torch.bfloat16, True, True),
                                                                    (1, torch.bfloat16, torch.float32, False, True), (0, torch.bfloat16, None, False, False)])
