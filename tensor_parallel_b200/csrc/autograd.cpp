@@ -191,8 +191,8 @@ struct LinearsFn : torch::autograd::Function<LinearsFn> {
     const auto saved = ctx->get_saved_variables();
     torch::autograd::variable_list out(1 + grads.size());
     Tensor gx;
-    for (size_t i = 0; i < grads.size(); ++i) {
-      if (!grads[i].defined()) continue;  // (nobody used that projection)
+    for (size_t i = grads.size(); i-- > 0;) {  // (the engine's order, so that there are only roundings fewer; q, the largest where k and v have fewer heads, last)
+      if (!grads[i].defined()) continue;       // (nobody used that projection)
       const Tensor g = as_type(rows_of(grads[i]), at::kBFloat16).contiguous();
       if (ctx->needs_input_grad(0)) gx = gemm(g, saved[1 + i], Tensor(), false, true, gx);
       if (ctx->needs_input_grad(1 + i)) out[1 + i] = gemm(g, saved[0], Tensor(), true, true);

@@ -101,7 +101,8 @@ int tpb_set_wait_limit(double seconds);
 
 // out[tokens, features] = act(x[tokens, k] @ w[features, k]^T + bias_scale * bias) + residual
 // (bf16 operands, fp32 accumulation).  With rc->world > 1 the product is additionally summed over all ranks
-// inside the same kernel (every rank must launch it with the same shapes).
+// inside the same kernel (every rank must launch it with the same shapes).  `residual` may be `out`: every element is read by the thread that
+// then stores it, once its sum is complete.
 int tpb_gemm_bf16(const void* x, const void* w, void* out, const void* bias, const void* residual, int tokens,
                   int features, int k, int ldx, int ldw, int ld_out, int act, float bias_scale,
                   const tpb_gemm_plan_t* plan, const tpb_reduce_ctx_t* rc, void* stream);

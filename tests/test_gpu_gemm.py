@@ -194,6 +194,63 @@ def test_gemm_operands_transposed_in_memory(tokens, features, k, x_t, w_t):
     _check(out, _ref(x, w, bias), k)
 
 
+# few rows, split-K (plans with several shares), one CTA per tile, pair tiles of 128 and 256 columns; ragged rows, widths off a multiple of 8 and 16
+ADD_TO = [(8, 4096, 4096), (20, 768, 3072), (33, 1028, 12288), (1, 520, 16384), (64, 4096, 16384), (130, 256, 8192), (200, 4096, 11008), (100, 772, 768),
+          (1000, 2052, 768), (1000, 2048, 2048), (2000, 4096, 1024), (2049, 4100, 512), (4100, 5120, 9000)]
+
+
+@pytest.mark.parametrize("tokens,features,k", ADD_TO)
+def test_gemm_adds_to_what_it_stores(tokens, features, k):
+    """The residual in the result's own buffer: the bits of a residual beside it, every time."""
+    nat = _native()
+    torch.manual_seed(7)
+    g = torch.randn(tokens, k, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(k, features, device="cuda", dtype=torch.bfloat16) / k ** 0.5
+    r = torch.randn(tokens, features, device="cuda", dtype=torch.bfloat16)
+    want = nat.gemm_nt(g, w, w_t=True, residual=r)
+    for _ in range(3):
+        buf = r.clone()
+        assert nat.gemm_nt(g, w, w_t=True, residual=buf, out=buf) is buf and torch.equal(buf, want)
+    nat.device_state(g.device).check_status()
+    _check(want, _ref(g, w.t(), residual=r), k)
+
+
+def test_the_sizes_above_take_every_route():
+    nat = _native()
+    plans = [nat.gemm_plan(*size, 1, 0, 0, no_swap=True) for size in ADD_TO]
+    assert {p.pair for p in plans} == {0, 128, 256} and {1, 2, 3} <= {p.k_splits for p in plans}
+
+
+@pytest.mark.parametrize("tokens,inputs,outputs", [(20, 768, (768, 192, 192)), (130, 256, (8192, 8192)), (33, 1028, (12288, 64)), (100, 772, (768, 768, 768)),
+                                                   (2049, 1024, (1024, 512, 512)), (1000, 2052, (768, 768))])
+@pytest.mark.parametrize("frozen", [(), (1,), (0,)])
+def test_joint_projections_against_64_bits(tokens, inputs, outputs, frozen):
+    """Projections of one input in one node: no gradient further off than with nodes of their own, whose sum is rounded more often."""
+    nat = _native()
+    torch.manual_seed(tokens)
+    values = [torch.randn(tokens, inputs, device="cuda", dtype=torch.bfloat16)]
+    values += [(torch.randn(n, inputs, device="cuda") / inputs ** 0.5).bfloat16() for n in outputs]
+    grads = [torch.randn(tokens, n, device="cuda", dtype=torch.bfloat16) for n in outputs]
+
+    def run(call, dtype):
+        leaves = [t.to(dtype, copy=True).requires_grad_(i not in frozen) for i, t in enumerate(values)]
+        outs = call(leaves[0], leaves[1:])
+        torch.autograd.backward([o for o in outs if o.requires_grad], [g.to(dtype) for o, g in zip(outs, grads) if o.requires_grad])
+        return [o.detach() for o in outs] + [t.grad for t in leaves]
+
+    assert nat.linears_supported(values[0].clone().requires_grad_(), values[1:])
+    joint = run(nat.linears, torch.bfloat16)
+    alone = run(lambda x, ws: [nat.linear(x, w) for w in ws], torch.bfloat16)
+    want = run(lambda x, ws: [x @ w.t() for w in ws], torch.float64)
+    for i, (a, b, ref) in enumerate(zip(joint, alone, want)):
+        if ref is None:
+            assert a is None and b is None
+        elif i == len(outputs):  # the input's gradient
+            assert (a.double() - ref).norm() <= (b.double() - ref).norm() and (a.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+        else:
+            assert torch.equal(a, b)
+
+
 def test_linear_backward_reads_operands_in_place():
     """dX and dW of the autograd linear against fp32 autograd; no transpose kernel is launched."""
     nat = _native()
