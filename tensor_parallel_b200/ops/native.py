@@ -62,7 +62,8 @@ _launches = 0
 class _Module(types.ModuleType):
     @property
     def launch_count(self):
-        """Kernels launched through this binding since import, or since it was last set (bench.py reports the delta)."""
+        """Kernels launched through this binding since import, or since it was last set (bench.py reports the delta), but for the column sums
+        that are the gradient of a linear layer's bias."""
         return self._launches + (0 if self.AUTOGRAD is None else self.AUTOGRAD.launches())
 
     @launch_count.setter

@@ -344,10 +344,11 @@ def test_changed_inputs_are_noticed(nodes):
         out.sum().backward()
 
 
-@pytest.mark.parametrize("layer", ["linear", "norm"])
+@pytest.mark.parametrize("layer", ["linear", "linears", "norm"])
 def test_transforms_are_refused(nodes, layer):
     x, w = _linear_case()
-    call = (lambda t: nodes.linear(t, w)) if layer == "linear" else (lambda t: nodes.rms_norm(t, torch.ones(16, dtype=t.dtype), 1e-6))
+    call = dict(linear=lambda t: nodes.linear(t, w), linears=lambda t: sum(nodes.linears(t, [w, w])),
+                norm=lambda t: nodes.rms_norm(t, torch.ones(16, dtype=t.dtype), 1e-6))[layer]
     with pytest.raises(RuntimeError):
         torch.func.vmap(call)(x.detach()[None])
     with pytest.raises(RuntimeError):
