@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(NORM_THREADS, norm_row_ctas_per_sm<T, MODE, MA
 norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
                 const T* __restrict__ bias, T* __restrict__ out, T* __restrict__ sum_out, float* __restrict__ rstd_out,
                 float* __restrict__ mean_out, int cols, float eps) {
-  constexpr bool EARLY = !RES && MODE == 0 && sizeof(T) * MAXV <= 4;  // weights before the sums, where registers allow it
+  constexpr bool EARLY = !RES && MAXV <= 2;  // weights before the sums, where registers allow it
   pdl_wait();
   const size_t row = blockIdx.x;
   const T* xr = x + row * cols;
@@ -953,9 +953,14 @@ extern "C" int tpb_norm_fwd(const void* x, const void* residual, const void* wei
 #undef LAUNCH
     TPB_CHECK_LAUNCH();
   }
-#define LAUNCH3(T, M, V)                                                                                              \
-  launch_kernel(residual ? norm_fwd_kernel<T, M, V, true> : norm_fwd_kernel<T, M, V, false>, dim3(rows), dim3(NORM_THREADS), 0, s, (const T*)x, (const T*)residual, (const T*)weight, \
-                (const T*)bias, (T*)out, (T*)sum_out, rstd_out, mean_out, cols, eps)
+  // (without a residual only rows wider than the rings' and the bf16 RMSNorm rows above come here)
+#define LAUNCH3(T, M, V)                                                                                                                     \
+  do {                                                                                                                                       \
+    auto kernel = norm_fwd_kernel<T, M, V, true>;                                                                                            \
+    if constexpr (V == 8 || (M == 0 && sizeof(T) == 2 && V <= 2)) { if (!residual) kernel = norm_fwd_kernel<T, M, V, false>; }               \
+    launch_kernel(kernel, dim3(rows), dim3(NORM_THREADS), 0, s, (const T*)x, (const T*)residual, (const T*)weight, (const T*)bias, (T*)out,  \
+                  (T*)sum_out, rstd_out, mean_out, cols, eps);                                                                               \
+  } while (0)
 #define LAUNCH(T, M)                                                                     \
   do {                                                                                   \
     if (cols <= NORM_THREADS * 8) LAUNCH3(T, M, 1);                                      \
