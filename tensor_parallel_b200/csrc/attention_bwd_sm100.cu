@@ -998,8 +998,8 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmap_r1, const __grid_c
 // exponential per score on the special-function unit, the rest latencies of barrier and TMEM that warps in step do not hide from each other); this one
 // takes 88 us.  Whole backward with it 307 us, with reductions in the dQ launch, the buffer to clear and the cast to bf16 353.  Where it pays: ops/native.py.
 constexpr int BG_STAGES = 2, BG_KEYS = 64, BG_WARPS = 8, BG_THREADS = 64 + 32 * BG_WARPS;
-template <int D>
-constexpr size_t bg_smem_bytes() { return size_t(BG_STAGES) * 2 * (D / 64) * (FA_BLOCK_BYTES + BG_KEYS * 128) + BW_R * BG_KEYS * 2 + 16 * 8; }
+constexpr size_t BG_SMEM = size_t(BG_STAGES) * 2 * (FA_BLOCK_BYTES + BG_KEYS * 128) + BW_R * BG_KEYS * 2 + 16 * 8;
+static_assert(2 * (BG_SMEM + 1024) <= 228 * 1024, "shared memory of an SM");
 
 struct BgParams {
   int batch, sq, sk, q_heads, kv_heads, causal;
@@ -1012,12 +1012,10 @@ struct BgParams {
   uint32_t* status;
 };
 
-template <int D>
 __global__ void __launch_bounds__(BG_THREADS, 2)
 attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const BgParams p) {
-  constexpr int DB = D / 64;
-  constexpr uint32_t TILE = DB * FA_BLOCK_BYTES, K_BLOCK = BG_KEYS * 128, K_TILE = DB * K_BLOCK, STAGE = 2 * (TILE + K_TILE);  // Q, dO, K, V
+  constexpr uint32_t TILE = FA_BLOCK_BYTES, K_TILE = BG_KEYS * 128, STAGE = 2 * (TILE + K_TILE);  // Q, dO, K, V of one pair, head_dim 64
   constexpr uint32_t TMEM_COLS = 256;
   constexpr uint32_t IDESC_S = make_idesc_bf16(BW_R, BG_KEYS, false, false);
   extern __shared__ __align__(1024) uint8_t bg_smem[];
@@ -1080,13 +1078,10 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
         uint8_t* dst = smem + s * STAGE;
         mbar_expect_tx(&t_full[s], STAGE);
-#pragma unroll
-        for (int d = 0; d < DB; ++d) {
-          tma_load_4d(dst + d * FA_BLOCK_BYTES, &tmap_q, &t_full[s], d * 64, q0, h, b);
-          tma_load_4d(dst + 2 * TILE + d * K_BLOCK, &tmap_k, &t_full[s], d * 64, k0, h / group, b);
-          tma_load_4d(dst + TILE + d * FA_BLOCK_BYTES, &tmap_do, &t_full[s], d * 64, q0, h, b);
-          tma_load_4d(dst + 2 * TILE + K_TILE + d * K_BLOCK, &tmap_v, &t_full[s], d * 64, k0, h / group, b);
-        }
+        tma_load_4d(dst, &tmap_q, &t_full[s], 0, q0, h, b);
+        tma_load_4d(dst + 2 * TILE, &tmap_k, &t_full[s], 0, k0, h / group, b);
+        tma_load_4d(dst + TILE, &tmap_do, &t_full[s], 0, q0, h, b);
+        tma_load_4d(dst + 2 * TILE + K_TILE, &tmap_v, &t_full[s], 0, k0, h / group, b);
         if (heads > 1 && ++h < heads) continue;
         if (heads > 1) h = 0;
         ++b;
@@ -1109,9 +1104,7 @@ attn_bias_grad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       for (int which = 0; which < 2; ++which) {
         const uint32_t a_lo = desc_kmajor_lo(at + which * TILE), b_lo = desc_kmajor_lo(at + 2 * TILE + which * K_TILE);
 #pragma unroll
-        for (int i = 0; i < DB * 4; ++i)
-          umma_bf16_lead(leader, tmem_base + (buf * 2 + which) * BG_KEYS, a_lo + (i >> 2) * (FA_BLOCK_BYTES >> 4) + (i & 3) * 2, b_lo + (i >> 2) * (K_BLOCK >> 4) + (i & 3) * 2,
-                         IDESC_S, i ? 1u : 0u);
+        for (int i = 0; i < 4; ++i) umma_bf16_lead(leader, tmem_base + (buf * 2 + which) * BG_KEYS, a_lo + i * 2, b_lo + i * 2, IDESC_S, i ? 1u : 0u);
       }
       umma_commit_lead(leader, &s_full[buf]);
       umma_commit_lead(leader, &t_empty[s]);
@@ -1448,15 +1441,13 @@ extern "C" int tpb_attn_bias_grad_sm100(const void* q, const void* k, const void
   p.dbias_fp32 = dbias_fp32;
   p.b_sh = bias_sh; p.b_sq = bias_sq;
   p.status = static_cast<uint32_t*>(status);
-  constexpr size_t smem = bg_smem_bytes<64>();
-  static_assert(2 * (smem + 1024) <= 228 * 1024, "shared memory of an SM");
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(attn_bias_grad_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return TPB_ERR_CUDA;
+    if (cudaFuncSetAttribute(attn_bias_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BG_SMEM)) != cudaSuccess) return TPB_ERR_CUDA;
     configured[dev].store(true, std::memory_order_release);
   }
-  attn_bias_grad_kernel<64><<<dim3(k_tiles, q_tiles, planes), BG_THREADS, smem, static_cast<cudaStream_t>(stream_)>>>(tq, tdo, tk, tv, p);
+  attn_bias_grad_kernel<<<dim3(k_tiles, q_tiles, planes), BG_THREADS, BG_SMEM, static_cast<cudaStream_t>(stream_)>>>(tq, tdo, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }

@@ -391,11 +391,11 @@ struct Fa2 {
   static_assert(4 * 32 * REGS_OTHER + 8 * 32 * REGS_SOFTMAX <= (N == 64 ? 80 : 168) * FA2_THREADS, "registers of a CTA at its launch");
 };
 
-// POLY of every 4 pairs of exponentials run on the FMA pipe.  BIAS: the score-bias code exists only where it is needed - 0 none, 1 any bias,
+// BIAS: the score-bias code exists only where it is needed - 0 none, 1 any bias,
 // loaded in vectors or one by one, 2 bf16 tiles by TMA, 3 bf16 rows in vectors (bias_vector_rows), those of a whole tile ahead.  3 holds 64 registers
 // of raw biases; in one instantiation with 1 they spill there too (2 x 1001, 16 heads of 128, causal, a dense bf16 bias: 296 us, apart 239 us;
 // fp32 bias of 16 x 512, 32 heads of 64: 282 and 217 us).
-template <int D, int N, int POLY, int BIAS>
+template <int D, int N, int BIAS>
 __global__ void __launch_bounds__(FA2_THREADS, Fa2<D, N>::CTAS)
 attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_b, const FaParams p) {
@@ -725,7 +725,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
           float t0, t1;
           ffma2(t0, t1, __uint_as_float(r[2 * (c + i)]), __uint_as_float(r[2 * (c + i) + 1]), mul, mul, nbase, nbase);
           float p0, p1;
-          if ((i & 3) < POLY) {
+          // one pair of exponentials in four as a cubic on the FMA pipe (measured best of 0 / 1 / 2 / 3 in four: 206 / 199 / 205 / 236 us at
+          // batch 4, 2048 tokens, 32 heads of 128, causal, before the warp-uniform issue loop: 161 us with it)
+          if ((i & 3) == 0) {
             ex2_poly2(t0, t1);
             p0 = t0;
             p1 = t1;
@@ -837,10 +839,10 @@ static int fa2_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TPB_ERR_CUDA;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(attn_fwd_pingpong_kernel<D, N, 1, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return TPB_ERR_CUDA;
+    if (cudaFuncSetAttribute(attn_fwd_pingpong_kernel<D, N, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return TPB_ERR_CUDA;
     configured[dev].store(true, std::memory_order_release);
   }
-  attn_fwd_pingpong_kernel<D, N, 1, BIAS><<<grid, FA2_THREADS, smem, stream>>>(tq, tk, tv, tb, p);
+  attn_fwd_pingpong_kernel<D, N, BIAS><<<grid, FA2_THREADS, smem, stream>>>(tq, tk, tv, tb, p);
   return cudaGetLastError() == cudaSuccess ? TPB_OK : TPB_ERR_CUDA;
 }
 
@@ -886,8 +888,6 @@ extern "C" int tpb_attn_prefill_sm100(const void* q, const void* k, const void* 
   static const bool one_tile = getenv("TPB_ATTN_ONE_TILE") != nullptr;  // (A/B switch: the kernel with one query tile per CTA)
   if (!one_tile && sq > FA_M) {
     dim3 grid((sq + FA2_M - 1) / FA2_M, q_heads, batch);
-    // one pair of exponentials in four runs as a cubic on the FMA pipe (measured best of 0 / 1 / 2 / 3 in four:
-    // 206 / 199 / 205 / 236 us at batch 4, 2048 tokens, 32 heads of 128, causal, before the warp-uniform issue loop: 161 us with it)
     // bf16 rows in vectors come by TMA where it can address them, as in the backward; at head_dim 128, where shared memory has no room, and where
     // one row serves all queries (padding masks), by loads
     const bool vectors = p.bias_kind == 2 && p.bias_vec, by_tma = vectors && head_dim == 64 && bias_sq > 0 && bias_sb >= 0 && bias_sh >= 0;
