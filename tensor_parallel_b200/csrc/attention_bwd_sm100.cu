@@ -1,14 +1,14 @@
 // Attention backward for sm_100a on tcgen05 tensor cores, with an optional additive score bias (scores = S * scale + bias;
-// d(bias) = P * (dP - delta), summed over whatever dimensions the bias broadcasts over, is added into an fp32 buffer by the
-// dQ launch, which visits every (query, key) pair exactly once).
+// d(bias) = P * (dP - delta), summed over whatever dimensions the bias broadcasts over, comes from attn_bias_grad_kernel for a dense bf16
+// bias that the batches share, and is otherwise added into an fp32 buffer by the dQ launch, which visits every (query, key) pair exactly once).
 //
 //   P  = exp(S * scale - lse)          S  = Q K^T
 //   dV = P^T dO                        dP = dO V^T
 //   dS = P * (dP - delta) * scale      delta[i] = sum_d out[i, d] * dout[i, d]
 //   dQ = dS K                          dK = dS^T Q
 //
-// Two launches, dK / dV and dQ, both free of atomics and therefore deterministic (the optional bias gradient is the exception: fp32
-// atomic adds).  A CTA keeps 128 "resident" rows (the TMEM lanes) and streams the other sequence through.  There are two kernels, each a
+// Two launches, dK / dV and dQ, and where it is taken that of the bias gradient, free of atomics and therefore deterministic (a bias gradient
+// that the dQ launch adds up is the exception: fp32 atomic adds).  A CTA keeps 128 "resident" rows (the TMEM lanes) and streams the other sequence through.  There are two kernels, each a
 // template of both launches: attn_bwd_tcgen05_kernel streams 64 rows per step (described here), attn_bwd_wide_kernel 128, or 64
 // with two CTAs per SM (described there); two_per_sm and step_rows below say which launch takes which.
 //
@@ -1300,6 +1300,8 @@ static bool two_per_sm(int head_dim, int resident, int heads, int batch, bool ca
 // The dQ launch at head_dim 128, whose resident tiles and rings of steps of 64 keys just fit half of an SM (with them in shared memory and not in tensor memory, an
 // MMA reads twice as much): for sequences of a few steps, whose fill and drain count.  Whole backwards in us, 32 heads, wide / so: 16 x 512 336 / 321, causal 292 / 269;
 // 16 x 100 57.2 / 49.3; 3 x 200 33.8 / 30.9; 16 heads 4 x 300 37.3 / 34.6, 2 x 700 55.9 / 52.6, causal 45.3 / 45.5; but 1 x 2048 219 / 222, causal 153 / 163, 4 x 2048 causal 505 / 510.
+// From 641 to 1152 keys either is ahead by up to 5 % (2 x 768, 16 heads 55.5 / 53.7, causal 44.9 / 46.6; 4 x 1024, 32 heads 242 / 250, causal 194 / 184), from
+// 1280 on wide steps in most (4 x 1536, 32 heads 499 / 563, 2 x 2048 422 / 462, causal 266 / 300), so the line stays where the gain ends.
 static bool dq_two_per_sm_128(int head_dim, int sq, int sk, int heads, int batch) {
   return head_dim == 128 && sk <= 640 && (long long)((sq + BW_R - 1) / BW_R) * heads * batch > 148;
 }

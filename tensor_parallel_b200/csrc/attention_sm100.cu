@@ -640,8 +640,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
           alive = false;
           break;
         }
-        // whole tile visible: two scores per instruction, no masks (this path is bound by instruction issue: 16 x 512 tokens, 32
-        // heads of 64, 218 us with a mask and a multiply per score, 151 us like this, 79 us without a bias)
+        // two scores per instruction; rows in registers come here for whole tiles only, tiles by TMA always, with a select per score
+        // where some are not visible (16 x 512 tokens, 32 heads of 64: 218 us with a mask and a multiply per score, 148 us with rows in registers, 90 us
+        // by TMA with two CTAs per SM; 59 us without a bias)
 #pragma unroll
         for (int c0 = 0; c0 < N; c0 += 32) {  // a quarter at a time: the scores take the registers that the biases leave
           tmem_ld_x32(s_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(r + c0));
@@ -713,7 +714,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         }
       }
       l_run *= factor;
-      // ---- probabilities (bf16 pairs, key 2c and 2c + 1 in column c of this row) over the scores' first 64 columns ----
+      // ---- probabilities (bf16 pairs, key 2c and 2c + 1 in column c of this row) over the first half of the scores' columns ----
       const float mul = BIAS ? 1.f : p.scale_log2e;
       const float nbase = m_run == -INFINITY ? 0.f : -m_run;
       float sum0 = 0.f, sum1 = 0.f;
@@ -821,7 +822,7 @@ static int fa_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
 }
 
 // Keys per tile (see Fa2) of a launch at head_dim 64, bias as BIAS above: 64 where there are CTAs for a second one per SM (us in tiles of 128 / 64,
-// heads in brackets: 16 x 512 (32) 77 / 59, causal 69 / 54, a bias by TMA 114 / 89, fp32 215 / 194; 32 x 129 (16) 28 / 18; but 8 x 512 (8), 128 CTAs, 11.9 / 13.3, by
+// heads in brackets: 16 x 512 (32) 77 / 59, causal 69 / 55, a bias by TMA 114 / 90, fp32 215 / 197; 32 x 129 (16) 28 / 18; but 8 x 512 (8), 128 CTAs, 11.9 / 13.3, by
 // TMA 17.5 / 19.0, and 2 x 1000 (12), 96 CTAs, 18.3 / 21.3).  Long causal rows without a bias fill their tiles of 128 (4 x 2048 (12) 65.0 / 65.9, 2 x 4096 (16)
 // 140 / 144; 4 x 1001 (32) 50.1 / 47.9), and rows in registers pay for fewer of those where tiles are whole (mask of 16 x 512 (32) 107 / 123, causal
 // 242 / 184, of 16 x 200 (16) 28 / 22).

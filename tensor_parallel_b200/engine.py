@@ -196,7 +196,9 @@ class DecoderEngine:
         self.next_ids = torch.zeros(B, dtype=torch.int64, device=dev)
         self.rope_angles = native.rope_table(max_seq, spec.rotary_dim, self.theta, dev) if spec.rotary_dim else None
         # split the key range only when (batch x kv heads) alone cannot occupy the SMs
-        # (a KV head's query heads share a CTA, from 17 on in groups of 16, all groups in one launch)
+        # (a KV head's query heads share a CTA from four on, in groups of 16, all groups in one launch; one to three run two by two.  More than
+        # eight splits cost more in their merge than they bring: one sequence, 128 / 8 heads of 64, 64 CTAs, 1000 keys 8.3 us, with 16 splits 8.9;
+        # four sequences of 32 / 8 heads of 128, 2500 keys 16.6 and 23.7)
         ctas = B * self.nkv * math.ceil(self.nq / self.nkv / 16)
         self.splits = 1 if ctas >= 128 else max(1, min(8, math.ceil(256 / ctas)))
         self.attn_ws = (torch.empty(B * self.nq * self.splits * D, dtype=torch.float32, device=dev),
